@@ -18,7 +18,7 @@ LIB_PATH = os.path.join(_HERE, "_lib", "libdynamix_g2.so")
 G2_OK = 0
 STATUS = {0: "ok", 1: "invalid argument", 2: "CUDA runtime error", 3: "unsupported device or feature",
           4: "size exceeds a kernel limit"}
-DEVERR_TIMEOUT, DEVERR_BOUNDS, DEVERR_RANGE, DEVERR_RANGE_CHECK = 1, 2, 4, 8
+DEVERR_TIMEOUT, DEVERR_BOUNDS, DEVERR_RANGE, DEVERR_RANGE_CHECK, DEVERR_RESIDUAL = 1, 2, 4, 8, 16
 
 BK = 64          # source segment width (pixels)
 PAD = 128        # packed bins and packed_cols are multiples of this
@@ -27,7 +27,10 @@ TC_BM, TC_BN = 128, 256
 PLAIN_BM, PLAIN_BN = 128, 128
 MAX_JOBS = 32
 ITEM_EMPTY = -1
-KIND_FP16, KIND_E4M3 = 0, 1
+KIND_FP16, KIND_E4M3, KIND_E2M1 = 0, 1, 2
+KIND_BLOCKED = 256
+E2M1_CHUNK = 4080
+RES_SECTOR = 64  # packed columns per residual list
 
 # numpy mirror of g2_gram_item (48 bytes, 8-byte aligned)
 ITEM_DTYPE = np.dtype([("job", "<i4"), ("i0", "<i4"), ("j0", "<i4"), ("a_k0", "<i4"), ("b_k0", "<i4"),
@@ -60,6 +63,13 @@ SIGNATURES = {
     "g2_gram_tc": (C.c_int, [_p, _i32, _p, _i64, _p, _i64, _p, _i64, _p, _i32, _p]),
     "g2_gram_tc_pair": (C.c_int, [_p, _i32, _p, _i64, _p, _i64, _p, _i64, _p, _i32, _p]),
     "g2_gram_tc_wide": (C.c_int, [_p, _i32, _p, _i64, _p, _i64, _p, _i64, _p, _i32, _p]),
+    "g2_gram_tc_e2m1": (C.c_int, [_p, _i32, _p, _i64, _p, _i64, _p, _i64, _p, _i32, _p]),
+    "g2_pack_u8_residual": (C.c_int, [_p, _i64, _i64, _i64, _i32, _p, _p, _p, _i64, _p, _i64, _i64, _p, _p, _i32, _p,
+                                      _p]),
+    "g2_count_tail": (C.c_int, [_p, _i64, _i64, _p, _i64, _i64, _p, _p]),
+    "g2_residual_sums": (C.c_int, [_p, _i64, _i64, _i64, _i32, _p, _p, _i32, _p, _i32, _p, _p, _p, _p, _p]),
+    "g2_e2m1_offset": (C.c_int, [_p, _p, _i32, _i64, _p, _p, _p]),
+    "g2_operand_expand": (C.c_int, [_p, _i64, _i64, _i64, _i32, _i32, _p, _p, _i32, _p, _p, _p]),
     "g2_gram_workers": (C.c_int, [_i32, _p]),
     "g2_plain_direct": (C.c_int, [_p, _i32, _p, _i64, _p, _i64, _p, _p]),
     "g2_plain_dp4a": (C.c_int, [_p, _i32, _p, _i64, _p, _i64, _p, _i64, _p, _p]),
@@ -153,4 +163,6 @@ def device_error_message(code):
         msgs.append("a count does not fit the packing")
     if code & DEVERR_RANGE_CHECK:
         msgs.append("a count may not fit the packing (unchecked)")
+    if code & DEVERR_RESIDUAL:
+        msgs.append("more large counts than the narrow operand's residual lists hold")
     return "; ".join(msgs) or "device error %d" % code

@@ -52,28 +52,46 @@ constexpr int EPI_THREADS = 128;
 constexpr int EPI_WARPS = EPI_THREADS / 32;
 constexpr int SMEM_BAR_OFF = STAGES * STAGE_BYTES;
 constexpr int SMEM_BYTES = 1024 /*alignment slack*/ + SMEM_BAR_OFF + 256 + 2 * NDIAG_PAD * 4;
+constexpr int F4_SMEM_BYTES = SMEM_BYTES - STAGES * (B_BYTES - 112 * ROW_BYTES);  // e2m1 items: 112 B rows per CTA
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 
 struct MapsParam {
   CUtensorMap map[G2_MAX_JOBS];  // box: one stage row (128 B) x 128 rows, 128-byte swizzle
   int32_t kind[G2_MAX_JOBS];
   int32_t ones[G2_MAX_JOBS];
+  uint32_t blocked;              // bit per job: K-blocked operand, 3-D map (128 B, rows, blocks)
 };
 
 __device__ __forceinline__ int stage_elems(int kind) { return kind == G2_KIND_E4M3 ? 128 : 64; }
 
+// e2m1 operands (G2_KIND_E2M1, kind::mxf4, twice the e4m3 MMA rate): 256
+// elements per 128-byte stage row.  The MMA reads block scales from TMEM, so
+// the two accumulators give up 32 columns to a block of ones: 256 x 224 items
+// (224 = the largest multiple of 32 with 2 n <= 480).
+constexpr int F4_BN = 224;
+constexpr int F4_STAGE = 256;
+constexpr int F4_B_BYTES = (F4_BN / 2) * ROW_BYTES;
+constexpr uint32_t F4_SCALE_COL = 480;
+constexpr uint32_t F4_SCALE_ONES = 0x7F7F7F7Fu;  // e8m0 2^0, four per column and lane
+struct MapsParamF4 : MapsParam {
+  CUtensorMap map_b[G2_MAX_JOBS];  // box: 128 B x 112 rows of one block
+};
+
 // Columns of the item's MMA: the frames (and the row of ones) left from j0,
 // rounded up to a multiple of 32, at most 256.
+template <bool F4 = false>
 __device__ __forceinline__ int item_n(const g2_gram_item& w, const MapsParam& maps) {
   const int live = w.nframes + (w.s_off >= 0 && maps.ones[w.job] ? 1 : 0) - w.j0;
   const int n = (live + 31) & ~31;
-  return n < 32 ? 32 : (n > BN ? BN : n);
+  constexpr int most = F4 ? F4_BN : BN;
+  return n < 32 ? 32 : (n > most ? most : n);
 }
 
+template <bool F4 = false>
 __device__ __forceinline__ bool item_ok(const g2_gram_item& w, const MapsParam& maps, int n_jobs,
                                         int64_t numer_len, int64_t sums_len) {
   if (w.job < 0 || w.job >= n_jobs) return false;
-  const int bk = stage_elems(maps.kind[w.job]);
+  const int bk = F4 ? F4_STAGE : stage_elems(maps.kind[w.job]);
   return w.k_len > 0 && (w.k_len % bk) == 0 && (w.a_k0 % bk) == 0 && (w.b_k0 % bk) == 0 && w.nframes > 0 &&
          w.i0 >= 0 && w.j0 >= 0 && w.j0 < w.nframes + 1 && w.out_off >= 0 && w.out_off + w.nframes <= numer_len &&
          w.shift >= 0 && w.shift <= 32 &&
@@ -93,22 +111,43 @@ __device__ __forceinline__ bool named_bar_any(uint32_t id, uint32_t n, bool v) {
   return r != 0;
 }
 
+template <bool F4>
+struct PairMaps {
+  using type = MapsParam;
+};
+template <>
+struct PairMaps<true> {
+  using type = MapsParamF4;
+};
+
+// An epilogue sum as int64: e2m1 sums are signed (two's complement throughout).
+template <bool F4>
+__device__ __forceinline__ unsigned long long widen(uint32_t v) {
+  return F4 ? static_cast<unsigned long long>(static_cast<long long>(static_cast<int32_t>(v)))
+            : static_cast<unsigned long long>(v);
+}
+
+// F4: e2m1 operands on kind::mxf4 (every job); else e4m3 / fp16 operands.
+template <bool F4>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
-    gram_pair_kernel(const __grid_constant__ MapsParam maps, int n_jobs, const g2_gram_item* __restrict__ items,
+    gram_pair_kernel(const __grid_constant__ typename PairMaps<F4>::type maps, int n_jobs, const g2_gram_item* __restrict__ items,
                      int64_t n_items, unsigned long long* __restrict__ numer, int64_t numer_len,
                      unsigned long long* __restrict__ sums, int64_t sums_len, int32_t* __restrict__ err) {
+  constexpr int SB = F4 ? F4_B_BYTES : B_BYTES;  // B bytes per stage and CTA
+  constexpr int ACC_STEP = F4 ? F4_BN : BN;      // TMEM columns from one accumulator to the next
+  constexpr int BAR_OFF = STAGES * (A_BYTES + SB);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * A_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + SMEM_BAR_OFF);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + BAR_OFF);
   uint64_t* empty = full + STAGES;
   uint64_t* accf = empty + STAGES;
   uint64_t* acce = accf + 2;
   uint64_t* drain = acce + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint32_t* diag = reinterpret_cast<uint32_t*>(smem + SMEM_BAR_OFF + 256);
+  uint32_t* diag = reinterpret_cast<uint32_t*>(smem + BAR_OFF + 256);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -138,6 +177,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (F4) {
+    // the scale columns of both CTAs hold ones before the leader's first MMA
+    if (warp >= 2)
+      tmem_fill_x32(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + F4_SCALE_COL, F4_SCALE_ONES);
+    tc_fence_before();
+    cluster_sync_all();
+    tc_fence_after();
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
@@ -146,14 +193,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       uint32_t phase = 0;
       int64_t issued = 0;
       bool ok = true;
+      g2_gram_item next = {};
+      if (cluster < n_items) next = items[cluster];
       for (int64_t it = cluster; it < n_items && ok; it += n_clusters) {
-        const g2_gram_item w = items[it];
+        // the next item is read an item ahead, so the ring does not run dry
+        // for the latency of its record
+        const g2_gram_item w = next;
+        if (it + n_clusters < n_items) next = items[it + n_clusters];
         if (w.job == G2_ITEM_EMPTY) continue;
-        if (!item_ok(w, maps, n_jobs, numer_len, sums_len)) continue;
+        if (!item_ok<F4>(w, maps, n_jobs, numer_len, sums_len)) continue;
         const CUtensorMap* m = &maps.map[w.job];
-        const int bk = stage_elems(maps.kind[w.job]);
+        const CUtensorMap* mb = m;
+        if constexpr (F4) mb = &maps.map_b[w.job];
+        const bool blocked = F4 || ((maps.blocked >> w.job) & 1u);
+        const int bk = F4 ? F4_STAGE : stage_elems(maps.kind[w.job]);
         const int nk = w.k_len / bk;
-        const int n = item_n(w, maps);
+        const int n = item_n<F4>(w, maps);
         const int32_t arow = w.i0 + static_cast<int32_t>(rank) * HALF;
         const int32_t brow = w.j0 + static_cast<int32_t>(rank) * (n / 2);
         for (int kb = 0; kb < nk; ++kb) {
@@ -161,10 +216,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
             ok = false;
             break;
           }
-          if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2 * STAGE_BYTES);
+          if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2 * (A_BYTES + SB));
           const uint32_t fb = mapa_shared(smem_addr(&full[stage]), 0);
-          tma_load_2d_pair(sA + stage * A_BYTES, m, fb, w.a_k0 + kb * bk, arow);
-          tma_load_2d_pair(sB + stage * B_BYTES, m, fb, w.b_k0 + kb * bk, brow);
+          if (blocked) {
+            tma_load_3d_pair(sA + stage * A_BYTES, m, fb, arow, w.a_k0 / bk + kb);
+            tma_load_3d_pair(sB + stage * SB, mb, fb, brow, w.b_k0 / bk + kb);
+          } else {
+            tma_load_2d_pair(sA + stage * A_BYTES, m, fb, w.a_k0 + kb * bk, arow);
+            tma_load_2d_pair(sB + stage * SB, mb, fb, w.b_k0 + kb * bk, brow);
+          }
           ++issued;
           if (++stage == STAGES) {
             stage = 0;
@@ -191,19 +251,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       uint32_t phase = 0;
       int64_t local = 0;
       bool ok = true;
+      g2_gram_item next = {};
+      if (cluster < n_items) next = items[cluster];
       for (int64_t it = cluster; it < n_items && ok; it += n_clusters) {
-        const g2_gram_item w = items[it];
+        // the next item is read an item ahead, so the ring does not run dry
+        // for the latency of its record
+        const g2_gram_item w = next;
+        if (it + n_clusters < n_items) next = items[it + n_clusters];
         if (w.job == G2_ITEM_EMPTY) continue;
-        if (!item_ok(w, maps, n_jobs, numer_len, sums_len)) continue;
+        if (!item_ok<F4>(w, maps, n_jobs, numer_len, sums_len)) continue;
         const bool fp8 = maps.kind[w.job] == G2_KIND_E4M3;
-        const int n = item_n(w, maps);
-        const uint32_t idesc = idesc_f32acc(BM, static_cast<uint32_t>(n));
+        const int n = item_n<F4>(w, maps);
+        const uint32_t idesc = F4 ? idesc_mxf4(BM, static_cast<uint32_t>(n)) : idesc_f32acc(BM, static_cast<uint32_t>(n));
         const int buf = static_cast<int>(local & 1);
         const uint32_t ap = static_cast<uint32_t>((local >> 1) & 1);
         if (!mbar_wait_cluster(&acce[buf], ap ^ 1, abort_flag, err)) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BN);
-        const int nk = w.k_len / stage_elems(maps.kind[w.job]);
+        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * ACC_STEP);
+        const int bk = F4 ? F4_STAGE : stage_elems(maps.kind[w.job]);
+        const int nk = w.k_len / bk;
         for (int kb = 0; kb < nk; ++kb) {
           if (!mbar_wait_cluster(&full[stage], phase, abort_flag, err)) {
             ok = false;
@@ -211,8 +277,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
           }
           tc_fence_after();
           const uint32_t a0 = smem_addr(sA + stage * A_BYTES);
-          const uint32_t b0 = smem_addr(sB + stage * B_BYTES);
-          if (fp8) {
+          const uint32_t b0 = smem_addr(sB + stage * SB);
+          if constexpr (F4) {
+            const uint32_t sc = tmem_base + F4_SCALE_COL;
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              tc_mma_pair_mxf4(d_tmem, smem_desc_sw128(a0 + kk * 32), smem_desc_sw128(b0 + kk * 32), idesc, sc, sc,
+                               (kb | kk) != 0 ? 1u : 0u);
+          } else if (fp8) {
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
               tc_mma_pair_f8f6f4(d_tmem, smem_desc_sw128(a0 + kk * 32), smem_desc_sw128(b0 + kk * 32), idesc,
@@ -249,7 +321,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         --local;
         continue;
       }
-      if (!item_ok(w, maps, n_jobs, numer_len, sums_len)) {
+      if (!item_ok<F4>(w, maps, n_jobs, numer_len, sums_len)) {
         if (etid == 0 && rank == 0) atomicOr(err, G2_DEVERR_BOUNDS);
         --local;
         continue;
@@ -260,11 +332,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       const bool ok = mbar_wait_cluster(&accf[buf], ap, abort_flag, err);
       if (named_bar_any(1, EPI_THREADS, !ok)) break;
       tc_fence_after();
-      const float unscale = maps.kind[w.job] == G2_KIND_E4M3 ? 262144.0f : 281474976710656.0f;
-      const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
+      // e2m1 codes hold u / 2
+      const float unscale = F4 ? 4.0f : (maps.kind[w.job] == G2_KIND_E4M3 ? 262144.0f : 281474976710656.0f);
+      const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * ACC_STEP);
       const int i0 = w.i0 + static_cast<int>(rank) * HALF;  // first frame of this CTA's rows
       const bool row_live = i0 + row < w.nframes;
-      const int n = item_n(w, maps);
+      const int n = item_n<F4>(w, maps);
       const int lag0 = w.j0 - i0 - (HALF - 1);
       const int ones_col = w.s_off >= 0 ? w.nframes - w.j0 : -1;  // -1 or >= n: not in this block
       // rows past the frames (the row of ones among them) contribute nothing;
@@ -280,13 +353,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         tmem_ld_32x32b_x32(tbase + static_cast<uint32_t>(cc * 32), v);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __float2uint_rn(__uint_as_float(v[j]) * us);
+        for (int j = 0; j < 32; ++j) {
+          const float x = __uint_as_float(v[j]) * us;
+          v[j] = F4 ? static_cast<uint32_t>(__float2int_rn(x)) : __float2uint_rn(x);
+        }
         const int jx = ones_col - cc * 32;
         if (jx >= 0 && jx < 32) {  // warp-uniform
 #pragma unroll
           for (int j = 0; j < 32; ++j)
             if (j == jx) {
-              if (v[j]) atomicAdd(&sums[w.s_off + i0 + row], static_cast<unsigned long long>(v[j]));
+              if (v[j]) atomicAdd(&sums[w.s_off + i0 + row], widen<F4>(v[j]));
               v[j] = 0;
             }
         }
@@ -309,7 +385,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         if (s) {
           const int tau = lag0 + d;
           if (tau >= 0 && tau < w.nframes)
-            atomicAdd(&numer[w.out_off + tau], static_cast<unsigned long long>(s) << w.shift);
+            atomicAdd(&numer[w.out_off + tau], widen<F4>(s) << w.shift);
           dacc[d] = 0;
         }
       }
@@ -430,9 +506,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
           const uint32_t fb = mapa_shared(smem_addr(&full[stage]), 0);
           uint8_t* st = smem + stage * W_STAGE_BYTES;
           const int32_t kc = w.a_k0 + kb * bk;
-          tma_load_2d_pair(st, m, fb, kc, arow);
-          if (n0) tma_load_2d_pair(st + A_BYTES, m, fb, w.b_k0 + kb * bk, brow0);
-          if (n1) tma_load_2d_pair(st + A_BYTES + B_BYTES, m, fb, w.b_k0 + kb * bk, brow1);
+          if ((maps.blocked >> w.job) & 1u) {
+            tma_load_3d_pair(st, m, fb, arow, kc / bk);
+            if (n0) tma_load_3d_pair(st + A_BYTES, m, fb, brow0, w.b_k0 / bk + kb);
+            if (n1) tma_load_3d_pair(st + A_BYTES + B_BYTES, m, fb, brow1, w.b_k0 / bk + kb);
+          } else {
+            tma_load_2d_pair(st, m, fb, kc, arow);
+            if (n0) tma_load_2d_pair(st + A_BYTES, m, fb, w.b_k0 + kb * bk, brow0);
+            if (n1) tma_load_2d_pair(st + A_BYTES + B_BYTES, m, fb, w.b_k0 + kb * bk, brow1);
+          }
           ++issued;
           if (++stage == W_STAGES) {
             stage = 0;
@@ -622,7 +704,11 @@ int max_clusters(const void* kernel, int smem, int* out) {
 }
 
 int pair_max_clusters(int* out) {
-  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel), g2::pair::SMEM_BYTES, out);
+  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<false>), g2::pair::SMEM_BYTES, out);
+}
+
+int f4_max_clusters(int* out) {
+  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<true>), g2::pair::F4_SMEM_BYTES, out);
 }
 
 int wide_max_clusters(int* out) {
@@ -636,17 +722,23 @@ int pair_maps(const g2_job* jobs, int32_t n_jobs, g2::pair::MapsParam* maps) {
     const g2_job& jb = jobs[j];
     if (!jb.packed_dev || !aligned(jb.packed_dev, 16) || jb.nframes <= 0 || jb.nframes >= (1ll << 31) ||
         jb.packed_cols <= 0 || jb.packed_cols % G2_PAD != 0 || jb.packed_cols >= (1ll << 31) ||
-        (jb.elem_kind != G2_KIND_FP16 && jb.elem_kind != G2_KIND_E4M3) || (jb.ones_row != 0 && jb.ones_row != 1))
+        ((jb.elem_kind & ~G2_KIND_BLOCKED) != G2_KIND_FP16 && (jb.elem_kind & ~G2_KIND_BLOCKED) != G2_KIND_E4M3) ||
+        (jb.ones_row != 0 && jb.ones_row != 1))
       return G2_ERR_ARG;
   }
   std::memset(maps, 0, sizeof(*maps));
   for (int j = 0; j < n_jobs; ++j) {
-    const int eb = jobs[j].elem_kind == G2_KIND_E4M3 ? 1 : 2;
+    const int32_t kind = jobs[j].elem_kind & ~G2_KIND_BLOCKED;
+    const bool blocked = (jobs[j].elem_kind & G2_KIND_BLOCKED) != 0;
+    const int eb = kind == G2_KIND_E4M3 ? 1 : 2;
     const uint64_t rows = static_cast<uint64_t>(jobs[j].nframes) + (jobs[j].ones_row ? 1 : 0);
-    const int st = encode_tmap_2d(&maps->map[j], jobs[j].packed_dev, eb, jobs[j].packed_cols, rows,
-                                  pair::ROW_BYTES / eb, pair::HALF);
+    const int st = blocked ? encode_tmap_blocked(&maps->map[j], jobs[j].packed_dev, jobs[j].packed_cols * eb, rows,
+                                                 pair::HALF)
+                           : encode_tmap_2d(&maps->map[j], jobs[j].packed_dev, eb, jobs[j].packed_cols, rows,
+                                            pair::ROW_BYTES / eb, pair::HALF);
     if (st != G2_OK) return st;
-    maps->kind[j] = jobs[j].elem_kind;
+    if (blocked) maps->blocked |= 1u << j;
+    maps->kind[j] = kind;
     maps->ones[j] = jobs[j].ones_row;
   }
   return G2_OK;
@@ -655,10 +747,10 @@ int pair_maps(const g2_job* jobs, int32_t n_jobs, g2::pair::MapsParam* maps) {
 
 extern "C" int g2_gram_workers(int32_t pair, int32_t* workers) {
   using namespace g2;
-  if (!workers || pair < 0 || pair > 2) return G2_ERR_ARG;
+  if (!workers || pair < 0 || pair > 3) return G2_ERR_ARG;
   if (pair) {
     int n = 0;
-    const int st = pair == 2 ? wide_max_clusters(&n) : pair_max_clusters(&n);
+    const int st = pair == 3 ? f4_max_clusters(&n) : (pair == 2 ? wide_max_clusters(&n) : pair_max_clusters(&n));
     if (st != G2_OK) return st;
     *workers = n;
     return G2_OK;
@@ -697,7 +789,7 @@ int launch_pair(bool wide, const g2_job* jobs, int32_t n_jobs, const g2_gram_ite
     pair::gram_wide_kernel<<<g, pair::NUM_THREADS, pair::W_SMEM_BYTES, as_stream(stream)>>>(
         maps, n_jobs, items_dev, n_items, nm, numer_len, sm, sums_len, err_dev);
   else
-    pair::gram_pair_kernel<<<g, pair::NUM_THREADS, pair::SMEM_BYTES, as_stream(stream)>>>(
+    pair::gram_pair_kernel<false><<<g, pair::NUM_THREADS, pair::SMEM_BYTES, as_stream(stream)>>>(
         maps, n_jobs, items_dev, n_items, nm, numer_len, sm, sums_len, err_dev);
   return launch_status();
 }
@@ -715,4 +807,43 @@ extern "C" int g2_gram_tc_wide(const g2_job* jobs, int32_t n_jobs, const g2_gram
                                int32_t* err_dev, int32_t grid, void* stream) {
   return launch_pair(true, jobs, n_jobs, items_dev, n_items, numer_dev, numer_len, sums_dev, sums_len, err_dev, grid,
                      stream);
+}
+
+extern "C" int g2_gram_tc_e2m1(const g2_job* jobs, int32_t n_jobs, const g2_gram_item* items_dev, int64_t n_items,
+                               uint64_t* numer_dev, int64_t numer_len, uint64_t* sums_dev, int64_t sums_len,
+                               int32_t* err_dev, int32_t grid, void* stream) {
+  using namespace g2;
+  if (!jobs || n_jobs < 1 || n_jobs > G2_MAX_JOBS || n_items < 0 || !numer_dev || numer_len <= 0 || !err_dev ||
+      sums_len < 0 || (sums_len > 0 && !sums_dev) || (n_items > 0 && !items_dev))
+    return G2_ERR_ARG;
+  for (int j = 0; j < n_jobs; ++j) {
+    const g2_job& jb = jobs[j];
+    if (!jb.packed_dev || !aligned(jb.packed_dev, 16) || jb.nframes <= 0 || jb.nframes >= (1ll << 31) ||
+        jb.packed_cols <= 0 || jb.packed_cols % pair::F4_STAGE != 0 || jb.packed_cols >= (1ll << 31) ||
+        jb.elem_kind != G2_KIND_E2M1 || (jb.ones_row != 0 && jb.ones_row != 1))
+      return G2_ERR_ARG;
+  }
+  if (n_items == 0) return G2_OK;
+  pair::MapsParamF4 maps;
+  std::memset(&maps, 0, sizeof(maps));
+  for (int j = 0; j < n_jobs; ++j) {
+    const uint64_t rows = static_cast<uint64_t>(jobs[j].nframes) + (jobs[j].ones_row ? 1 : 0);
+    const uint64_t bytes = static_cast<uint64_t>(jobs[j].packed_cols) / 2;
+    int st = encode_tmap_blocked(&maps.map[j], jobs[j].packed_dev, bytes, rows, pair::HALF);
+    if (st == G2_OK) st = encode_tmap_blocked(&maps.map_b[j], jobs[j].packed_dev, bytes, rows, pair::F4_BN / 2);
+    if (st != G2_OK) return st;
+    maps.kind[j] = jobs[j].elem_kind;
+    maps.ones[j] = jobs[j].ones_row;
+  }
+  int max_cl = 0;
+  const int st = f4_max_clusters(&max_cl);
+  if (st != G2_OK) return st;
+  int64_t clusters = grid > 0 ? (grid + 1) / 2 : max_cl;
+  if (clusters > max_cl) clusters = max_cl;
+  if (clusters > n_items) clusters = n_items;
+  pair::gram_pair_kernel<true><<<static_cast<unsigned>(2 * clusters), pair::NUM_THREADS, pair::F4_SMEM_BYTES,
+                                 as_stream(stream)>>>(
+      maps, n_jobs, items_dev, n_items, reinterpret_cast<unsigned long long*>(numer_dev), numer_len,
+      reinterpret_cast<unsigned long long*>(sums_dev), sums_len, err_dev);
+  return launch_status();
 }

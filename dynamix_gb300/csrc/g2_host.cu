@@ -28,26 +28,44 @@ int sm_count_current() {
   return n;
 }
 
+namespace {
+int encoder() {
+  std::lock_guard<std::mutex> lk(g_mu);
+  if (g_encode) return G2_OK;
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess || fn == nullptr)
+    return G2_ERR_UNSUPPORTED;
+  g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  return G2_OK;
+}
+}  // namespace
+
 int encode_tmap_2d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t cols, uint64_t rows,
                    uint32_t box_cols, uint32_t box_rows) {
-  {
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (!g_encode) {
-      void* fn = nullptr;
-      cudaDriverEntryPointQueryResult q;
-      if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
-              cudaSuccess ||
-          q != cudaDriverEntryPointSuccess || fn == nullptr)
-        return G2_ERR_UNSUPPORTED;
-      g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    }
-  }
+  const int st = encoder();
+  if (st != G2_OK) return st;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols * static_cast<uint64_t>(elem_bytes)};
   const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUtensorMapDataType dt = elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUresult r = g_encode(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? G2_OK : G2_ERR_ARG;
+}
+
+int encode_tmap_blocked(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint32_t box_rows) {
+  const int st = encoder();
+  if (st != G2_OK) return st;
+  if (row_bytes == 0 || row_bytes % 128 != 0) return G2_ERR_ARG;
+  const cuuint64_t dims[3] = {128, rows, row_bytes / 128};
+  const cuuint64_t strides[2] = {128, 128 * rows};
+  const cuuint32_t box[3] = {128, box_rows, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? G2_OK : G2_ERR_ARG;

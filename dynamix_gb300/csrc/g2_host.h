@@ -26,4 +26,9 @@ int sm_count_current();
 int encode_tmap_2d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t cols, uint64_t rows,
                    uint32_t box_cols, uint32_t box_rows);
 
+// Encode a 3-D tiled tensor map (128 bytes, rows, blocks) over a K-blocked
+// matrix (G2_KIND_BLOCKED) of `rows` rows of `row_bytes` bytes, with a
+// (128 bytes x box_rows x 1) box, 128-byte swizzle, zero fill outside.
+int encode_tmap_blocked(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint32_t box_rows);
+
 }  // namespace g2

@@ -90,6 +90,16 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// 3-D tiled load of the box at (0, c1 = row, c2 = block) of a K-blocked matrix.
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int32_t c1,
+                                            int32_t c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+          smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_addr(bar)), "r"(0), "r"(c1), "r"(c2)
+      : "memory");
+}
+
 // 1-D bulk copy of `bytes` (a multiple of 16; both addresses 16-byte
 // aligned) from global into this CTA's shared memory, completing on the
 // mbarrier with its byte count.
@@ -239,6 +249,15 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
       "l"(reinterpret_cast<uint64_t>(map)), "r"(mbar_cluster_addr), "r"(c0), "r"(c1)
       : "memory");
 }
+// The same of the box at (0, c1 = row, c2 = block) of a K-blocked matrix.
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint32_t mbar_cluster_addr,
+                                                 int32_t c1, int32_t c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+      "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(mbar_cluster_addr), "r"(0), "r"(c1), "r"(c2)
+      : "memory");
+}
 // One warp in EACH CTA of the pair performs these, collectively.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(dst_smem)),
@@ -269,6 +288,35 @@ __device__ __forceinline__ void tc_mma_pair_f8f6f4(uint32_t d_tmem, uint64_t a_d
       "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// The block-scaled kinds read one e8m0 scale per 32 elements of A and of B from
+// TMEM columns (sa, sb); with every byte of those columns 127 the scales are 1.
+// kind::mxf4: A and B are e2m1 (two per byte, K = 64 per MMA), fp32 D.
+__device__ __forceinline__ void tc_mma_pair_mxf4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                 uint32_t sa_tmem, uint32_t sb_tmem, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%5], p;\n\t}" ::"r"(
+          d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sa_tmem), "r"(sb_tmem), "r"(accumulate)
+      : "memory");
+}
+// Instruction descriptor of kind::mxf4: A and B format 1 (e2m1) at bits 7-9 /
+// 10-11, both K-major, N>>3 at bits 17-22, scale type 1 (e8m0) at bit 23,
+// M>>7 at bits 27-28, K = 64 (bit 31 clear), scale ids 0; D is fp32.
+__host__ __device__ constexpr uint32_t idesc_mxf4(uint32_t M, uint32_t N) {
+  return (1u << 7) | (1u << 10) | ((N >> 3) << 17) | (1u << 23) | ((M >> 7) << 27);
+}
+// One value into 32 columns of this warp's 32 TMEM lanes (whole warp).
+__device__ __forceinline__ void tmem_fill_x32(uint32_t taddr, uint32_t v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(
+          taddr),
+      "r"(v)
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 // Arrive once on the mbarrier at this offset in every CTA of `cta_mask` when
 // all pair MMAs issued so far by this thread complete.

@@ -1,0 +1,875 @@
+// Narrow operands for u8 stacks whose large counts are rare.
+//
+// The Gram's rate doubles from 16-bit to 8-bit operands and again to 4-bit
+// ones, but a narrow element holds only small counts exactly: e4m3 bytes 0-16,
+// e2m1 codes (in halves) -4..4, so that u = lo - 3 covers the counts 0-7.
+// Photon counts have a thin tail (at 0.1 photons per pixel one count in 2e8
+// exceeds 7), so each count v is split as v = lo + r, lo = min(v, 7 or 16): lo
+// goes into the packed operand, and the few r > 0 into lists, one per 64 packed
+// columns.  With
+//   v v' = lo lo' + (r lo' + lo r') + r r',   lo lo' = u u' + 3 (lo + lo') - 9
+// the tensor-core Gram of the operand gives the sums of u u' (e4m3: lo lo'),
+// offset_kernel adds the terms in 3 from the bin sums, and residual_kernel the
+// others, in int64, exactly.  A list that overflows sets G2_DEVERR_RESIDUAL: the
+// caller packs the stack into a wider element.
+//
+// pack_walk_kernel moves the bytes by work units, 32 units of one class per
+// block of a source chunk, a warp per block:
+//  * e2m1: the packed order inside a bin is free (every Gram entry sums over
+//    the bin), so the layout is built from the pack's own units: 16 bytes from
+//    two 16-pixel runs, 4 bytes from two 4-pixel runs, 4 bytes from 8 gathered
+//    pixels.  Eight counts become eight codes in five instructions (code8).
+//    No byte is shared between chunks and no unit is a single byte.
+//  * e4m3: the units of the e4m3 layout (g2_pack_e4m3_units).
+// Counts that may need a residual (a byte of 8 or more, or of 16 or
+// more) are found by one OR over the unit's words and take a slow path.
+#include "g2_ptx.cuh"
+#include "g2_host.h"
+
+namespace g2 {
+namespace tail {
+
+// Pixels per source chunk, frames per step and bytes of one staged frame row
+// (the chunk from its 16-byte aligned start, and spare words for reads past it).
+template <bool E2M1>
+struct Cfg {
+  static constexpr int CH = E2M1 ? G2_E2M1_CHUNK : G2_PACK_CHUNK;
+  static constexpr int F = E2M1 ? 4 : 8;
+  static constexpr int ROW = CH + 48;
+  static_assert(ROW % 16 == 0 && CH % 16 == 0 && CH <= 0xFFF, "bulk copy rows, 12-bit sources");
+};
+constexpr int THREADS = 256;
+constexpr int MOVERS = THREADS / 32 - 1;
+constexpr int STAGES = 2;
+constexpr int CTAS_PER_SM = 5;
+constexpr uint32_t UNIT_VEC = 1, UNIT_WORD = 2, UNIT_GATHER = 3, UNIT_BYTE = 4;
+constexpr uint32_t NO_SRC = 0xFFF;
+constexpr int SECTOR = 64;                            // packed columns per residual list
+
+struct Residuals {
+  uint32_t* count;  // per sector
+  uint2* list;      // [sector][cap]: {frame, column in the sector | r << 8}
+  uint32_t cap;
+  uint32_t n_sectors;
+};
+
+// Offset of byte x of row t in a K-blocked operand whose blocks hold `pitch` =
+// 128 * rows bytes (blocks of 128 bytes of every row, so that the 128 rows a
+// Gram stage reads lie side by side).
+__device__ __forceinline__ int64_t blk_off(uint32_t x, int64_t t, int64_t pitch) {
+  return static_cast<int64_t>(x >> 7) * pitch + t * 128 + (x & 127u);
+}
+
+// e2m1 codes of u = count - 3, counts 0-7, as the byte table of a prmt (the
+// code of -3 is 0xB, of 4 is 4), and the counts of the 16 codes.
+constexpr uint32_t CODES_LO = 0x00090A0Bu, CODES_HI = 0x04030201u;
+__device__ __forceinline__ uint32_t e2m1_count(uint32_t code) {
+  return static_cast<uint32_t>(0x0000012300076543ull >> (4 * code)) & 15u;
+}
+// Eight counts below 8 (bytes of a, bytes of b) as eight codes: packed into
+// nibbles they are the selectors of two prmt table reads.  The columns of the
+// result are a0 a2 b0 b2 a1 a3 b1 b3.
+__device__ __forceinline__ uint32_t code8(uint32_t a, uint32_t b) {
+  const uint32_t w = a + (b << 4);
+  return __byte_perm(CODES_LO, CODES_HI, w) + (__byte_perm(CODES_LO, CODES_HI, w >> 16) << 4);
+}
+
+// The low parts of four counts w, appending residuals.  E2M1: `col` is the
+// first column of the counts' word of 8, plus 2 for its b half; e4m3: the
+// column of the first count.
+template <bool E2M1>
+__device__ __noinline__ uint32_t encode_word(uint32_t w, uint32_t col, uint32_t t, const Residuals& res,
+                                             int32_t* err) {
+  constexpr uint32_t top = E2M1 ? 7 : 16;
+  uint32_t out = 0;
+#pragma unroll 1
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t v = (w >> (8 * j)) & 255u;
+    uint32_t e = v;
+    if (v > top) {
+      e = top;
+      const uint32_t c = col + (E2M1 ? ((j & 1) << 2 | j >> 1) : j), s = c / SECTOR;
+      const uint32_t slot = s < res.n_sectors ? atomicAdd(&res.count[s], 1u) : res.cap;
+      if (slot < res.cap)
+        res.list[static_cast<size_t>(s) * res.cap + slot] = make_uint2(t, (c % SECTOR) | ((v - top) << 8));
+      else
+        atomicOr(err, G2_DEVERR_RESIDUAL);
+    }
+    out |= e << (8 * j);
+  }
+  return out;
+}
+
+// bits of a byte that mark a count the fast path cannot move as it is
+template <bool E2M1>
+__device__ __forceinline__ constexpr uint32_t high_bits() { return E2M1 ? 0xF8F8F8F8u : 0xF0F0F0F0u; }
+
+// Sixteen counts, the first of each word in column col + i * step.
+template <bool E2M1>
+__device__ __forceinline__ void encode16(uint4& v, uint32_t col, uint32_t step, uint32_t t, const Residuals& res,
+                                         int32_t* err) {
+  constexpr uint32_t hb = high_bits<E2M1>();
+  if (v.x & hb) v.x = encode_word<E2M1>(v.x, col, t, res, err);
+  if (v.y & hb) v.y = encode_word<E2M1>(v.y, col + step, t, res, err);
+  if (v.z & hb) v.z = encode_word<E2M1>(v.z, col + 2 * step, t, res, err);
+  if (v.w & hb) v.w = encode_word<E2M1>(v.w, col + 3 * step, t, res, err);
+}
+
+// 16 consecutive bytes at byte offset o of the staged row (any alignment):
+// the two aligned 16-byte words around them, realigned by selects and shifts
+__device__ __forceinline__ uint4 load16(const uint8_t* base, uint32_t o) {
+  const uint4 q0 = *reinterpret_cast<const uint4*>(base + (o & ~15u));
+  const uint4 q1 = *reinterpret_cast<const uint4*>(base + (o & ~15u) + 16);
+  const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+  const uint32_t k = (o >> 2) & 3u, sh = 8 * (o & 3u);
+  uint32_t x[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const uint32_t lo = (k & 1u) ? w[i + 1] : w[i];
+    const uint32_t hi = (k & 1u) ? w[i + 3] : w[i + 2];
+    x[i] = (k & 2u) ? hi : lo;
+  }
+  return make_uint4(__funnelshift_r(x[0], x[1], sh), __funnelshift_r(x[1], x[2], sh),
+                    __funnelshift_r(x[2], x[3], sh), __funnelshift_r(x[3], x[4], sh));
+}
+__device__ __forceinline__ uint32_t load4(const uint8_t* base, uint32_t o) {
+  const uint32_t* p = reinterpret_cast<const uint32_t*>(base + (o & ~3u));
+  return __funnelshift_r(p[0], p[1], 8 * (o & 3u));
+}
+
+// One e2m1 unit over the step's nf frames (the first is frame t of the whole
+// stack; its chunk starts at staged byte `phase`, each later frame's `step`
+// bytes further on, mod 16): {class << 30 | destination, sources...}.
+__device__ __forceinline__ void move_e2m1(const uint4& u, const uint8_t* base, uint32_t phase, uint32_t step,
+                                          uint8_t* out, int64_t pitch, uint32_t row_bytes, int nf, uint32_t t,
+                                          const Residuals& res, int32_t* err, bool& bad) {
+  using C = Cfg<true>;
+  constexpr uint32_t hb = high_bits<true>();
+  const uint32_t cls = u.x >> 30, dst = u.x & 0x3FFFFFFFu;
+  const uint32_t sa = u.y & 0xFFFFu, sb = u.y >> 16;
+  if (cls == UNIT_VEC) {
+    if (dst >= row_bytes / 16 || sa > C::CH - 16 || sb > C::CH - 16) {
+      bad = true;
+      return;
+    }
+    uint8_t* o = out + blk_off(16 * dst, 0, pitch);
+#pragma unroll
+    for (int f = 0; f < C::F; ++f) {
+      if (f >= nf) break;
+      const uint32_t d = ((phase + f * step) & 15u) + f * C::ROW;
+      uint4 a = load16(base, d + sa);
+      uint4 b = load16(base, d + sb);
+      if ((a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) & hb) {
+        encode16<true>(a, 32 * dst, 8, t + f, res, err);
+        encode16<true>(b, 32 * dst + 2, 8, t + f, res, err);
+      }
+      *reinterpret_cast<uint4*>(o + f * 128) =
+          make_uint4(code8(a.x, b.x), code8(a.y, b.y), code8(a.z, b.z), code8(a.w, b.w));
+    }
+  } else if (cls == UNIT_WORD) {
+    if (dst >= row_bytes / 4 || sa > C::CH - 4 || sb > C::CH - 4) {
+      bad = true;
+      return;
+    }
+    uint8_t* o = out + blk_off(4 * dst, 0, pitch);
+#pragma unroll
+    for (int f = 0; f < C::F; ++f) {
+      if (f >= nf) break;
+      const uint32_t d = ((phase + f * step) & 15u) + f * C::ROW;
+      uint32_t a = load4(base, d + sa), b = load4(base, d + sb);
+      if ((a | b) & hb) {
+        if (a & hb) a = encode_word<true>(a, 8 * dst, t + f, res, err);
+        if (b & hb) b = encode_word<true>(b, 8 * dst + 2, t + f, res, err);
+      }
+      *reinterpret_cast<uint32_t*>(o + f * 128) = code8(a, b);
+    }
+  } else if (cls == UNIT_GATHER) {
+    if (dst >= row_bytes / 4) {
+      bad = true;
+      return;
+    }
+    const uint32_t s[8] = {u.y & 0xFFFu,  (u.y >> 12) & 0xFFFu, (u.y >> 24) | ((u.z & 0xFu) << 8), (u.z >> 4) & 0xFFFu,
+                           (u.z >> 16) & 0xFFFu, (u.z >> 28) | ((u.w & 0xFFu) << 4), (u.w >> 8) & 0xFFFu, u.w >> 20};
+    uint8_t* o = out + blk_off(4 * dst, 0, pitch);
+#pragma unroll
+    for (int f = 0; f < C::F; ++f) {
+      if (f >= nf) break;
+      const uint8_t* q = base + ((phase + f * step) & 15u) + f * C::ROW;
+      uint32_t a = 0, b = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {  // 12-bit sources below CH, or NO_SRC: a column of padding (count 3, u = 0)
+        a |= (s[j] < C::CH ? static_cast<uint32_t>(q[s[j]]) : 3u) << (8 * j);
+        b |= (s[4 + j] < C::CH ? static_cast<uint32_t>(q[s[4 + j]]) : 3u) << (8 * j);
+      }
+      if ((a | b) & hb) {
+        if (a & hb) a = encode_word<true>(a, 8 * dst, t + f, res, err);
+        if (b & hb) b = encode_word<true>(b, 8 * dst + 2, t + f, res, err);
+      }
+      *reinterpret_cast<uint32_t*>(o + f * 128) = code8(a, b);
+    }
+  }
+}
+
+// One e4m3 unit: {destination, sources, sources, class}.
+__device__ __forceinline__ void move_e4m3(const uint4& u, const uint8_t* base, uint32_t phase, uint32_t step,
+                                          uint8_t* out, int64_t pitch, uint32_t row_bytes, int nf, uint32_t t,
+                                          const Residuals& res, int32_t* err, bool& bad) {
+  using C = Cfg<false>;
+  constexpr uint32_t hb = high_bits<false>();
+  if (u.w == UNIT_VEC) {
+    if (u.x >= row_bytes / 16 || u.y > C::CH - 16) {
+      bad = true;
+      return;
+    }
+    uint8_t* o = out + blk_off(16 * u.x, 0, pitch);
+#pragma unroll
+    for (int f = 0; f < C::F; ++f) {
+      if (f >= nf) break;
+      uint4 v = load16(base, ((phase + f * step) & 15u) + f * C::ROW + u.y);
+      if ((v.x | v.y | v.z | v.w) & hb) encode16<false>(v, 16 * u.x, 4, t + f, res, err);
+      *reinterpret_cast<uint4*>(o + f * 128) = v;
+    }
+  } else if (u.w == UNIT_WORD || u.w == UNIT_GATHER) {
+    const uint32_t s0 = u.y & 0xFFFFu, s1 = u.y >> 16, s2 = u.z & 0xFFFFu, s3 = u.z >> 16;
+    const bool word = u.w == UNIT_WORD;
+    if (u.x >= row_bytes / 4 || (word && u.y > C::CH - 4) ||
+        (!word && (s0 >= C::CH || s1 >= C::CH || s2 >= C::CH || s3 >= C::CH))) {
+      bad = true;
+      return;
+    }
+    uint8_t* o = out + blk_off(4 * u.x, 0, pitch);
+#pragma unroll
+    for (int f = 0; f < C::F; ++f) {
+      if (f >= nf) break;
+      const uint32_t d = ((phase + f * step) & 15u) + f * C::ROW;
+      const uint8_t* q = base + d;
+      uint32_t v = word ? load4(base, d + u.y)
+                        : static_cast<uint32_t>(q[s0]) | (static_cast<uint32_t>(q[s1]) << 8) |
+                              (static_cast<uint32_t>(q[s2]) << 16) | (static_cast<uint32_t>(q[s3]) << 24);
+      if (v & hb) v = encode_word<false>(v, 4 * u.x, t + f, res, err);
+      *reinterpret_cast<uint32_t*>(o + f * 128) = v;
+    }
+  } else if (u.w == UNIT_BYTE) {
+    if (u.x >= row_bytes || u.y >= C::CH) {
+      bad = true;
+      return;
+    }
+    uint8_t* o = out + blk_off(u.x, 0, pitch);
+#pragma unroll
+    for (int f = 0; f < C::F; ++f) {
+      if (f >= nf) break;
+      uint32_t v = base[((phase + f * step) & 15u) + f * C::ROW + u.y];
+      if (v & hb) v = encode_word<false>(v, u.x, t + f, res, err);
+      o[f * 128] = static_cast<uint8_t>(v);
+    }
+  }
+}
+
+// Persistent CTAs; a work item is a step of F frames over one band of chunks.
+// The CTA walks the band chunk by chunk through a ring of STAGES staged chunks:
+// warp 0 lane 0 bulk-copies the F frames' binned span of the chunk, the mover
+// warps take its blocks in turn (block j of the layout goes to warp j mod
+// MOVERS, its units read one block ahead).  The 128-byte lines of a packed
+// row hold units of neighbouring chunks, so walking them in one CTA completes
+// a line within microseconds; with a CTA per chunk (walking frames) a third
+// of the written bytes left L2 as partly filled lines (T = 10,000 frames of
+// 514 x 1030, DRAM read 7.05 GB of 5.29, written 3.02 GB of 1.95).
+// frame0: number of the launch's first frame in the stack.
+template <bool E2M1>
+__global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
+    pack_walk_kernel(const uint8_t* __restrict__ frames, int64_t T, int64_t npix, uint32_t frame0,
+                     const int32_t* __restrict__ block_off, const uint4* __restrict__ units,
+                     const uint32_t* __restrict__ spans, int32_t n_chunks, int32_t n_bands,
+                     uint8_t* __restrict__ packed, int64_t pitch, uint32_t row_bytes, Residuals res,
+                     int32_t* __restrict__ err) {
+  using C = Cfg<E2M1>;
+  __shared__ __align__(128) uint8_t s_buf[STAGES][C::F][C::ROW];
+  __shared__ __align__(8) uint64_t full[STAGES];
+  __shared__ __align__(8) uint64_t empty[STAGES];
+  __shared__ int s_abort;
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full[s], 1);        // the copier's arrive.expect_tx, then the bytes
+      mbar_init(&empty[s], MOVERS);  // one arrival per mover warp
+    }
+    s_abort = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  volatile int* abort_flag = &s_abort;
+  const int64_t total_bytes = T * npix;
+  const int64_t n_items = (T + C::F - 1) / C::F * n_bands;
+  uint32_t k = 0;  // staged chunks so far
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ copier
+    if (lane == 0) {
+      bool ok = true;
+      for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        const int64_t g = item / n_bands;
+        const int band = static_cast<int>(item - g * n_bands);
+        const int c0 = static_cast<int>(static_cast<int64_t>(n_chunks) * band / n_bands);
+        const int c1 = static_cast<int>(static_cast<int64_t>(n_chunks) * (band + 1) / n_bands);
+        const int64_t t0 = g * C::F;
+        const int nf = static_cast<int>(T - t0 < C::F ? T - t0 : C::F);
+        for (int c = c0; c < c1; ++c) {
+          if (block_off[c] == block_off[c + 1]) continue;  // no packed byte comes from this chunk
+          const uint32_t span = spans[c];                    // binned pixels [lo, hi) of the chunk
+          const uint32_t s = k % STAGES;
+          if (k >= STAGES && !mbar_wait(&empty[s], ((k / STAGES) & 1u) ^ 1u, abort_flag, err)) {
+            ok = false;
+            break;
+          }
+          const int64_t p0 = static_cast<int64_t>(c) * C::CH;
+          // two passes: the byte count of the stage, then the copies
+          uint32_t bytes = 0;
+#pragma unroll
+          for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+            for (int f = 0; f < C::F; ++f) {
+              if (f >= nf) break;
+              const int64_t start = (t0 + f) * npix + p0;
+              const int64_t a = (start + (span & 0xFFFFu)) & ~int64_t(15);
+              int64_t e = (start + (span >> 16) + 15) & ~int64_t(15);
+              if (e > total_bytes) e = total_bytes;
+              const uint32_t n = static_cast<uint32_t>(e - a), n16 = n & ~15u;
+              uint8_t* dst = &s_buf[s][f][a - (start & ~int64_t(15))];
+              if (pass == 0) {
+                // the stack's last bytes short of a multiple of 16: plain copies,
+                // made visible by the arrive below (only the last frame has them)
+                for (uint32_t i = n16; i < n; ++i) dst[i] = frames[a + i];
+                bytes += n16;
+              } else if (n16) {
+                bulk_load_1d(dst, frames + a, n16, &full[s]);
+              }
+            }
+            if (pass == 0) mbar_arrive_expect_tx(&full[s], bytes);
+          }
+          ++k;
+        }
+      }
+      // after a timed-out wait a copy of this CTA may still be landing
+      if (*abort_flag) {
+        const uint64_t w0 = global_timer_ns();
+        while (global_timer_ns() - w0 < 100000ull) {
+        }
+      }
+    }
+    return;
+  }
+
+  // -------------------------------------------------------------- movers
+  const int mw = warp - 1;
+  bool bad = false, ok = true;
+  for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+    const int64_t g = item / n_bands;
+    const int band = static_cast<int>(item - g * n_bands);
+    const int c0 = static_cast<int>(static_cast<int64_t>(n_chunks) * band / n_bands);
+    const int c1 = static_cast<int>(static_cast<int64_t>(n_chunks) * (band + 1) / n_bands);
+    const int64_t t0 = g * C::F;
+    const int nf = static_cast<int>(T - t0 < C::F ? T - t0 : C::F);
+    const uint32_t t = frame0 + static_cast<uint32_t>(t0);
+    uint8_t* out = packed + static_cast<int64_t>(t) * 128;
+    const uint32_t start = static_cast<uint32_t>(t0 * npix), step = static_cast<uint32_t>(npix);
+    const int band_end = block_off[c1];
+    int b1 = block_off[c0];
+    int j = b1 + (mw + MOVERS - b1 % MOVERS) % MOVERS;  // this warp's next block
+    uint4 u = make_uint4(0, 0, 0, 0);
+    if (j < band_end) u = units[static_cast<int64_t>(j) * 32 + lane];
+    for (int c = c0; c < c1; ++c) {
+      const int b0 = b1;
+      b1 = block_off[c + 1];
+      if (b0 == b1) continue;
+      const uint32_t s = k % STAGES;
+      if (!mbar_wait(&full[s], (k / STAGES) & 1u, abort_flag, err)) {
+        ok = false;
+        break;
+      }
+      ++k;
+      const uint32_t phase = start + static_cast<uint32_t>(c) * C::CH;
+      const uint8_t* base = &s_buf[s][0][0];
+      while (j < b1) {
+        const uint4 w = u;
+        j += MOVERS;
+        if (j < band_end) u = units[static_cast<int64_t>(j) * 32 + lane];
+        if (E2M1) move_e2m1(w, base, phase, step, out, pitch, row_bytes, nf, t, res, err, bad);
+        else move_e4m3(w, base, phase, step, out, pitch, row_bytes, nf, t, res, err, bad);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+    }
+  }
+  if (bad) atomicOr(err, G2_DEVERR_BOUNDS);
+}
+
+// Counts, among the binned pixels of n_sample frames spread over the stack, of
+// the values an e2m1 operand (out[0]) or an e4m3 operand (out[1]) needs a
+// residual for.
+__global__ void __launch_bounds__(256)
+    count_tail_kernel(const uint8_t* __restrict__ frames, int64_t T, int64_t npix, const int32_t* __restrict__ col_src,
+                      int64_t n_cols, int64_t n_sample, uint32_t* __restrict__ out) {
+  uint32_t c4 = 0, c8 = 0;
+  const int64_t total = n_sample * n_cols;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t k = i / n_cols;
+    const int64_t s = col_src[i - k * n_cols];
+    if (s < 0 || s >= npix) continue;
+    const uint32_t v = frames[((2 * k + 1) * T / (2 * n_sample)) * npix + s];
+    c4 += v > 7 ? 1u : 0u;
+    c8 += v > 16 ? 1u : 0u;
+  }
+  c4 = __reduce_add_sync(0xffffffffu, c4);
+  c8 = __reduce_add_sync(0xffffffffu, c8);
+  if ((threadIdx.x & 31) == 0) {
+    if (c4) atomicAdd(&out[0], c4);
+    if (c8) atomicAdd(&out[1], c8);
+  }
+}
+
+// The terms of N and S that the operand's Gram does not hold: r lo(t') for
+// every list entry (its frame t, every frame t'), N(|t - t'|) += r lo(t'),
+// N(0) += 2 r lo(t) + r^2, the products of two residuals of one pixel, and
+// S(t) += r.  A CTA owns one tile of 256 rows and a contiguous share of the
+// operand's 128-byte blocks (entries gather in bright speckles: shares of many
+// blocks even that out, and every tile of a share costs the same).  A block's
+// tile is read as whole lines and staged in shared memory, rows 33 words apart;
+// then each thread takes one row and, for every entry of the block's four e2m1
+// (two e4m3) sectors, adds r lo into one uint32 lag histogram in shared memory
+// (consecutive lanes add to consecutive lags: no bank conflicts), flushed to
+// int64 at each bin change; adds straight to global int64 run at the L2's atomic
+// rate and stay for stacks whose histogram does not fit (HIST false).  Bound by
+// instruction latency (about 8 ps per entry and frame at 8 to 24 warps per SM):
+// 4,500 residuals of 512 x 512 x 3,001 frames (1 photon per pixel, e4m3) 0.15 ms,
+// of which 20 us for the empty lists.  A counter gets at most two adds of at
+// most 248 * 16 per entry, and a CTA flushes before 2^19 entries: no counter
+// wraps.
+constexpr int RES_THREADS = 256;
+constexpr uint32_t RES_MAX_ENTRIES = 1u << 19;
+constexpr int RES_TILE = RES_THREADS;  // rows per tile
+constexpr int RES_ROW = 33;            // words from one staged row to the next
+
+template <bool E2M1, bool HIST>
+__global__ void __launch_bounds__(RES_THREADS)
+    residual_kernel(const uint8_t* __restrict__ packed, int32_t T, int64_t pitch, Residuals res,
+                    const int32_t* __restrict__ sector_bin, int32_t n_bins, unsigned long long* __restrict__ numer,
+                    unsigned long long* __restrict__ sums, uint32_t n_tiles, uint32_t* __restrict__ total,
+                    int32_t* __restrict__ err) {
+  constexpr int W = E2M1 ? 8 : 16;           // words of one row of a sector
+  constexpr int SPB = E2M1 ? 4 : 2;          // sectors per block
+  constexpr int LPS = 32 / SPB;              // lanes per sector for its first entries
+  extern __shared__ uint32_t hist[];
+  __shared__ uint32_t stage[RES_TILE * RES_ROW];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t share = blockIdx.x / n_tiles, n_shares = gridDim.x / n_tiles;
+  const int t0 = static_cast<int>(blockIdx.x % n_tiles) * RES_TILE;
+  const uint32_t n_blocks = res.n_sectors / SPB;
+  const uint32_t sector_end = static_cast<uint32_t>(static_cast<uint64_t>(n_blocks) * (share + 1) / n_shares) * SPB;
+  if (HIST) {
+    for (int i = tid; i < T; i += RES_THREADS) hist[i] = 0;
+  }
+  uint32_t seen = 0, held = 0;  // entries in all, entries in the histogram (block-uniform)
+  int cur = -1;                 // bin of the histogram
+  // Every warp walks the blocks by itself: the counts and bins of 32 sectors
+  // at a time (the next 32 already loaded), the blocks with entries by a mask,
+  // a block's tile and each sector's first entries one block ahead, so that no
+  // load waits for another one.
+  uint32_t group = static_cast<uint32_t>(static_cast<uint64_t>(n_blocks) * share / n_shares) * SPB;
+  uint32_t g_count = 0, g_count_next = 0, mask = 0;
+  int g_bin = -1, g_bin_next = -1;
+  auto load_group = [&](uint32_t base) {
+    const uint32_t k = base + lane;
+    g_count_next = k < sector_end ? min(res.count[k], res.cap) : 0u;
+    g_bin_next = k < sector_end ? sector_bin[k] : -1;
+  };
+  auto take_group = [&]() {
+    g_count = g_count_next;
+    g_bin = g_bin_next;
+    mask = __ballot_sync(0xffffffffu, g_count != 0);
+  };
+  uint32_t first = 0;        // first sector of the block that follows
+  uint32_t n_lane = 0;       // entries of this lane's sector of it
+  int b_next = -1;
+  bool more = true;
+  uint4 v[RES_TILE * 8 / RES_THREADS];  // this thread's part of its tile
+  uint2 e_next = make_uint2(0, 0);
+  auto advance = [&]() {     // to the next block with entries, and start its loads
+    while (mask == 0) {
+      group += 32;
+      if (group >= sector_end) {
+        more = false;
+        return;
+      }
+      take_group();
+      load_group(group + 32);
+    }
+    const int bit = (__ffs(mask) - 1) / SPB * SPB;
+    mask &= ~(((1u << SPB) - 1u) << bit);
+    first = group + bit;
+    const int mine = bit + lane / LPS;
+    n_lane = __shfl_sync(0xffffffffu, g_count, mine);
+    b_next = __shfl_sync(0xffffffffu, g_bin, bit);
+    if (static_cast<uint32_t>(lane % LPS) < n_lane)
+      e_next = res.list[static_cast<size_t>(first + lane / LPS) * res.cap + lane % LPS];
+    const uint8_t* blk = packed + static_cast<int64_t>(first / SPB) * pitch;
+#pragma unroll
+    for (int i = 0; i < RES_TILE * 8 / RES_THREADS; ++i) {
+      const int k = i * RES_THREADS + tid, tp = t0 + k / 8;
+      v[i] = *reinterpret_cast<const uint4*>(blk + static_cast<int64_t>(tp < T ? tp : T - 1) * 128 + (k % 8) * 16);
+    }
+  };
+  load_group(group);
+  take_group();
+  load_group(group + 32);
+  advance();
+  while (more) {
+    const uint32_t s0 = first, ns_lane = n_lane;
+    const int b = b_next;
+    uint2 e = e_next;
+    __syncthreads();  // the tile before has been read (and the histogram zeroed)
+#pragma unroll
+    for (int i = 0; i < RES_TILE * 8 / RES_THREADS; ++i) {
+      const int k = i * RES_THREADS + tid;
+      uint32_t* d = &stage[(k / 8) * RES_ROW + (k % 8) * 4];
+      d[0] = v[i].x;
+      d[1] = v[i].y;
+      d[2] = v[i].z;
+      d[3] = v[i].w;
+    }
+    advance();
+    const bool ok = b >= 0 && b < n_bins;
+    if (!ok && tid == 0) atomicOr(err, G2_DEVERR_BOUNDS);
+    uint32_t all = 0;
+#pragma unroll
+    for (int k = 0; k < SPB; ++k) all += __shfl_sync(0xffffffffu, ns_lane, k * LPS);
+    if (HIST && held && (b != cur || held + all > RES_MAX_ENTRIES)) {
+      __syncthreads();
+      for (int i = tid; i < T; i += RES_THREADS) {
+        const uint32_t h = hist[i];
+        if (h) atomicAdd(&numer[static_cast<int64_t>(cur) * T + i], static_cast<unsigned long long>(h));
+        hist[i] = 0;
+      }
+      held = 0;
+    }
+    __syncthreads();  // the staged tile
+    if (!ok) continue;
+    cur = b;
+    held += all;
+    unsigned long long* nb = numer + static_cast<int64_t>(b) * T;
+    const uint32_t* row = &stage[tid * RES_ROW];
+    const int tp = t0 + tid;
+#pragma unroll 1
+    for (int k = 0; k < SPB; ++k) {
+      const uint32_t n = __shfl_sync(0xffffffffu, ns_lane, k * LPS);
+      const uint2* list = res.list + static_cast<size_t>(s0 + k) * res.cap;
+      if (s0 / SPB % n_tiles == blockIdx.x % n_tiles) {  // a block's own terms: once, spread over the tiles
+        seen += n;
+        for (uint32_t i = tid; i < n; i += RES_THREADS) {
+          const uint2 a = list[i];
+          if (a.x >= static_cast<uint32_t>(T)) continue;
+          atomicAdd(&sums[static_cast<int64_t>(b) * T + a.x], static_cast<unsigned long long>(a.y >> 8));
+          for (uint32_t j = 0; j < i; ++j) {
+            const uint2 d = list[j];
+            if (((a.y ^ d.y) & 255u) || d.x >= static_cast<uint32_t>(T)) continue;
+            const uint32_t lag = a.x > d.x ? a.x - d.x : d.x - a.x;
+            atomicAdd(&nb[lag], static_cast<unsigned long long>(a.y >> 8) * (d.y >> 8));
+          }
+        }
+        __syncwarp();
+      }
+      uint2 f = e;
+      for (uint32_t i0 = 0; i0 < n;) {  // the first LPS entries, then 32 at a time
+        const int from = i0 ? 0 : k * LPS;
+        const uint32_t m = min(n - i0, static_cast<uint32_t>(i0 ? 32 : LPS));
+        if (i0) f = i0 + lane < n ? list[i0 + lane] : make_uint2(0, 0);
+#pragma unroll 2
+        for (uint32_t i = 0; i < m; ++i) {
+          const uint32_t at = __shfl_sync(0xffffffffu, f.x, from + i), ay = __shfl_sync(0xffffffffu, f.y, from + i);
+          const uint32_t col = ay & (SECTOR - 1), rv = ay >> 8;
+          const uint32_t wi = k * W + (E2M1 ? col >> 3 : col >> 2);
+          const uint32_t x = row[wi] >> (E2M1 ? 4 * (col & 7) : 8 * (col & 3));
+          const uint32_t lo = E2M1 ? e2m1_count(x & 15u) : x & 255u;
+          const int lag = abs(tp - static_cast<int>(at));
+          if (lo == 0 && lag != 0) continue;
+          if (tp >= T || at >= static_cast<uint32_t>(T)) continue;
+          if (lag == 0) atomicAdd(&nb[0], static_cast<unsigned long long>(2 * rv * lo + rv * rv));
+          else if (HIST) atomicAdd(&hist[lag], rv * lo);
+          else atomicAdd(&nb[lag], static_cast<unsigned long long>(rv * lo));
+        }
+        i0 += m;
+      }
+    }
+  }
+  if (HIST && held) {
+    __syncthreads();
+    for (int i = tid; i < T; i += RES_THREADS) {
+      const uint32_t h = hist[i];
+      if (h) atomicAdd(&numer[static_cast<int64_t>(cur) * T + i], static_cast<unsigned long long>(h));
+    }
+  }
+  if (tid == 0 && seen) atomicAdd(total, seen);
+}
+
+// The terms of an e2m1 operand's offset, one CTA per bin of P pixels: from
+// the Gram's sums of u u' and of u (int64, two's complement) to those of the
+// low counts lo = u + 3: S(t) += 3 P, and with A the running sums of that S,
+// N(tau) += 3 (A(T - tau) + A(T) - A(tau)) - 9 P (T - tau).
+constexpr int OFF_THREADS = 1024;
+__global__ void __launch_bounds__(OFF_THREADS)
+    offset_kernel(unsigned long long* __restrict__ numer, unsigned long long* __restrict__ sums, int64_t T,
+                  const int64_t* __restrict__ npix, unsigned long long* __restrict__ scratch) {
+  __shared__ unsigned long long part[OFF_THREADS];
+  const int tid = threadIdx.x;
+  const unsigned long long P = static_cast<unsigned long long>(npix[blockIdx.x]);
+  unsigned long long* S = sums + static_cast<int64_t>(blockIdx.x) * T;
+  unsigned long long* N = numer + static_cast<int64_t>(blockIdx.x) * T;
+  unsigned long long* A = scratch + static_cast<int64_t>(blockIdx.x) * (T + 1);  // exclusive running sums
+  const int64_t per = (T + OFF_THREADS - 1) / OFF_THREADS;
+  const int64_t k0 = tid * per < T ? tid * per : T, k1 = k0 + per < T ? k0 + per : T;
+  unsigned long long sum = 0;
+  for (int64_t k = k0; k < k1; ++k) {
+    const unsigned long long v = S[k] + 3 * P;
+    S[k] = v;
+    sum += v;
+  }
+  part[tid] = sum;
+  __syncthreads();
+  for (int d = 1; d < OFF_THREADS; d *= 2) {
+    const unsigned long long x = tid >= d ? part[tid - d] : 0;
+    __syncthreads();
+    part[tid] += x;
+    __syncthreads();
+  }
+  unsigned long long run = part[tid] - sum;
+  for (int64_t k = k0; k < k1; ++k) {
+    A[k] = run;
+    run += S[k];
+  }
+  if (tid == OFF_THREADS - 1) A[T] = part[tid];
+  __syncthreads();
+  const unsigned long long all = part[OFF_THREADS - 1];
+  for (int64_t tau = tid; tau < T; tau += OFF_THREADS)
+    N[tau] += 3 * (A[T - tau] + all - A[tau]) - 9 * P * static_cast<unsigned long long>(T - tau);
+}
+
+// A row-major copy of a packed operand (same column order) in e4m3 bytes or
+// 16-bit counts.  One thread per 8 elements; the row of ones (the last row)
+// tells the columns of padding, which stay 0.
+template <bool E2M1, bool WIDE>
+__global__ void __launch_bounds__(256)
+    expand_kernel(const uint8_t* __restrict__ in, int64_t rows, int64_t cols, uint8_t* __restrict__ out) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= rows * (cols / 8)) return;
+  const int64_t t = i / (cols / 8), c8 = i - t * (cols / 8);
+  uint32_t v[8];
+  if (E2M1) {
+    const uint32_t x = static_cast<uint32_t>(c8 * 4);
+    const uint32_t w = *reinterpret_cast<const uint32_t*>(in + blk_off(x, t, rows * 128));
+    const uint32_t one = *reinterpret_cast<const uint32_t*>(in + blk_off(x, rows - 1, rows * 128));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = t == rows - 1 ? 1u : e2m1_count((w >> (4 * j)) & 15u);
+      if (((one >> (4 * j)) & 15u) == 0) v[j] = 0;
+    }
+  } else {
+    const uint2 w = *reinterpret_cast<const uint2*>(in + blk_off(static_cast<uint32_t>(c8 * 8), t, rows * 128));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = ((j < 4 ? w.x : w.y) >> (8 * (j & 3))) & 255u;
+  }
+  if (WIDE) {
+    reinterpret_cast<uint4*>(out)[i] =
+        make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
+  } else {
+    reinterpret_cast<uint2*>(out)[i] = make_uint2(v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24),
+                                                  v[4] | (v[5] << 8) | (v[6] << 16) | (v[7] << 24));
+  }
+}
+
+// Adds the residuals to the wider copy (each to its own element); an 8-bit
+// element above 16 sets G2_DEVERR_RANGE.
+template <bool WIDE>
+__global__ void __launch_bounds__(64)
+    expand_residual_kernel(Residuals res, int64_t T, int64_t cols, uint8_t* __restrict__ out,
+                           int32_t* __restrict__ err) {
+  const uint32_t s = blockIdx.x;
+  uint32_t n = res.count[s];
+  if (n > res.cap) n = res.cap;
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const uint2 a = res.list[static_cast<size_t>(s) * res.cap + i];
+    const int64_t col = static_cast<int64_t>(s) * SECTOR + (a.y & (SECTOR - 1));
+    if (a.x >= T || col >= cols) continue;
+    const int64_t e = static_cast<int64_t>(a.x) * cols + col;
+    if (WIDE) {
+      reinterpret_cast<uint16_t*>(out)[e] += static_cast<uint16_t>(a.y >> 8);
+    } else {
+      const uint32_t v = out[e] + (a.y >> 8);
+      if (v > 16) atomicOr(err, G2_DEVERR_RANGE);
+      out[e] = static_cast<uint8_t>(v);
+    }
+  }
+}
+
+}  // namespace tail
+}  // namespace g2
+
+namespace {
+using g2::tail::Residuals;
+
+bool residuals_ok(const uint32_t* count, const void* list, int32_t cap, int64_t packed_cols, Residuals* r) {
+  if (!count || !list || cap <= 0 || !g2::aligned(list, 8) || packed_cols <= 0 || packed_cols % G2_PAD != 0 ||
+      packed_cols >= (1ll << 31))
+    return false;
+  r->count = const_cast<uint32_t*>(count);
+  r->list = reinterpret_cast<uint2*>(const_cast<void*>(list));
+  r->cap = static_cast<uint32_t>(cap);
+  r->n_sectors = static_cast<uint32_t>(packed_cols / g2::tail::SECTOR);
+  return true;
+}
+}  // namespace
+
+extern "C" int g2_pack_u8_residual(const void* frames_dev, int64_t nframes, int64_t npix, int64_t frame0,
+                                   int32_t elem_kind, const int32_t* unit_block_off_dev, const uint32_t* units_dev,
+                                   const uint32_t* spans_dev, int64_t n_chunks, void* packed_dev, int64_t packed_rows,
+                                   int64_t packed_cols, uint32_t* res_count_dev, void* res_list_dev, int32_t res_cap,
+                                   int32_t* err_dev, void* stream) {
+  using namespace g2;
+  Residuals res;
+  if (!frames_dev || !unit_block_off_dev || !units_dev || !spans_dev || !packed_dev || !err_dev ||
+      !residuals_ok(res_count_dev, res_list_dev, res_cap, packed_cols, &res) ||
+      (elem_kind != G2_KIND_E2M1 && elem_kind != G2_KIND_E4M3))
+    return G2_ERR_ARG;
+  const bool e2m1 = elem_kind == G2_KIND_E2M1;
+  const int64_t ch = e2m1 ? G2_E2M1_CHUNK : G2_PACK_CHUNK;
+  if (nframes <= 0 || npix <= 0 || frame0 < 0 || packed_rows < frame0 + nframes || packed_rows >= (1ll << 31) ||
+      n_chunks != (npix + ch - 1) / ch || (e2m1 && packed_cols % 256 != 0))
+    return G2_ERR_ARG;
+  if (!aligned(packed_dev, 16) || !aligned(frames_dev, 16) || !aligned(units_dev, 16)) return G2_ERR_ARG;
+  if (n_chunks > 0x7fffffff) return G2_ERR_TOO_LARGE;
+  const int sms = sm_count_current();
+  if (sms <= 0) return G2_ERR_CUDA;
+  // bands: about eight work items per resident CTA, of at least four chunks
+  const int64_t ctas = static_cast<int64_t>(sms) * tail::CTAS_PER_SM;
+  const int F = e2m1 ? tail::Cfg<true>::F : tail::Cfg<false>::F;
+  const int64_t groups = (nframes + F - 1) / F;
+  int64_t bands = (8 * ctas + groups - 1) / groups;
+  if (bands > (n_chunks + 3) / 4) bands = (n_chunks + 3) / 4;
+  if (bands < 1) bands = 1;
+  const unsigned grid = static_cast<unsigned>(groups * bands < ctas ? groups * bands : ctas);
+  auto* fr = reinterpret_cast<const uint8_t*>(frames_dev);
+  auto* un = reinterpret_cast<const uint4*>(units_dev);
+  auto* out = reinterpret_cast<uint8_t*>(packed_dev);
+  const uint32_t f0 = static_cast<uint32_t>(frame0);
+  const int32_t nc = static_cast<int32_t>(n_chunks), nb = static_cast<int32_t>(bands);
+  if (e2m1)
+    tail::pack_walk_kernel<true><<<grid, tail::THREADS, 0, as_stream(stream)>>>(
+        fr, nframes, npix, f0, unit_block_off_dev, un, spans_dev, nc, nb, out, packed_rows * 128,
+        static_cast<uint32_t>(packed_cols / 2), res, err_dev);
+  else
+    tail::pack_walk_kernel<false><<<grid, tail::THREADS, 0, as_stream(stream)>>>(
+        fr, nframes, npix, f0, unit_block_off_dev, un, spans_dev, nc, nb, out, packed_rows * 128,
+        static_cast<uint32_t>(packed_cols), res, err_dev);
+  return launch_status();
+}
+
+extern "C" int g2_count_tail(const void* frames_dev, int64_t nframes, int64_t npix, const int32_t* col_src_dev,
+                             int64_t n_cols, int64_t n_sample, uint32_t* out_dev, void* stream) {
+  using namespace g2;
+  if (!frames_dev || !col_src_dev || !out_dev || nframes <= 0 || npix <= 0 || n_cols <= 0 || n_sample <= 0 ||
+      n_sample > nframes || nframes >= (1ll << 31))
+    return G2_ERR_ARG;
+  const int sms = sm_count_current();
+  if (sms <= 0) return G2_ERR_CUDA;
+  const int64_t want = (n_sample * n_cols + 255) / 256;
+  const unsigned grid = static_cast<unsigned>(want < sms * 8ll ? want : sms * 8ll);
+  tail::count_tail_kernel<<<grid, 256, 0, as_stream(stream)>>>(reinterpret_cast<const uint8_t*>(frames_dev), nframes,
+                                                               npix, col_src_dev, n_cols, n_sample, out_dev);
+  return launch_status();
+}
+
+extern "C" int g2_residual_sums(const void* packed_dev, int64_t packed_rows, int64_t nframes, int64_t packed_cols,
+                                int32_t elem_kind, const uint32_t* res_count_dev, const void* res_list_dev, int32_t res_cap,
+                                const int32_t* sector_bin_dev, int32_t n_bins, uint64_t* numer_dev,
+                                uint64_t* sums_dev, uint32_t* total_dev, int32_t* err_dev, void* stream) {
+  using namespace g2;
+  Residuals res;
+  if (!packed_dev || !sector_bin_dev || !numer_dev || !sums_dev || !total_dev || !err_dev || n_bins <= 0 ||
+      nframes <= 0 || packed_rows < nframes || packed_rows >= (1ll << 31) || !aligned(packed_dev, 16) ||
+      !residuals_ok(res_count_dev, res_list_dev, res_cap, packed_cols, &res) ||
+      (elem_kind != G2_KIND_E2M1 && elem_kind != G2_KIND_E4M3))
+    return G2_ERR_ARG;
+  auto* nm = reinterpret_cast<unsigned long long*>(numer_dev);
+  auto* sm = reinterpret_cast<unsigned long long*>(sums_dev);
+  auto* pk = reinterpret_cast<const uint8_t*>(packed_dev);
+  const int sms = sm_count_current();
+  if (sms <= 0) return G2_ERR_CUDA;
+  const int64_t smem = nframes * 4;
+  const bool hist = smem <= 184 * 1024;
+  // as many CTAs as are resident (228 KB of shared memory, a 33 KB tile each)
+  int64_t per_sm = hist ? 225 * 1024 / (smem + 34 * 1024) : 6;
+  if (per_sm > 6) per_sm = 6;
+  if (per_sm < 1) per_sm = 1;
+  const int64_t tiles = (nframes + tail::RES_TILE - 1) / tail::RES_TILE, blocks = res.n_sectors / (elem_kind == G2_KIND_E2M1 ? 4 : 2);
+  int64_t shares = sms * per_sm / tiles;
+  if (shares > blocks) shares = blocks;
+  if (shares < 1) shares = 1;
+  const unsigned grid = static_cast<unsigned>(tiles * shares);
+  const uint32_t nt = static_cast<uint32_t>(tiles);
+  cudaStream_t st = as_stream(stream);
+  const bool e2m1 = elem_kind == G2_KIND_E2M1;
+#define G2_RESIDUAL_LAUNCH(E, H)                                                                                     \
+  do {                                                                                                               \
+    if (H && cudaFuncSetAttribute(tail::residual_kernel<E, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
+                                  184 * 1024) != cudaSuccess)                                                        \
+      return G2_ERR_CUDA;                                                                                            \
+    tail::residual_kernel<E, H><<<grid, tail::RES_THREADS, H ? smem : 0, st>>>(                                      \
+        pk, static_cast<int32_t>(nframes), packed_rows * 128, res, sector_bin_dev, n_bins, nm, sm, nt, total_dev, err_dev);                \
+  } while (0)
+  if (e2m1 && hist) G2_RESIDUAL_LAUNCH(true, true);
+  else if (e2m1) G2_RESIDUAL_LAUNCH(true, false);
+  else if (hist) G2_RESIDUAL_LAUNCH(false, true);
+  else G2_RESIDUAL_LAUNCH(false, false);
+#undef G2_RESIDUAL_LAUNCH
+  return launch_status();
+}
+
+extern "C" int g2_e2m1_offset(uint64_t* numer_dev, uint64_t* sums_dev, int32_t n_bins, int64_t nframes,
+                              const int64_t* npix_dev, uint64_t* scratch_dev, void* stream) {
+  using namespace g2;
+  if (!numer_dev || !sums_dev || !npix_dev || !scratch_dev || n_bins <= 0 || nframes <= 0 || nframes >= (1ll << 31))
+    return G2_ERR_ARG;
+  tail::offset_kernel<<<static_cast<unsigned>(n_bins), tail::OFF_THREADS, 0, as_stream(stream)>>>(
+      reinterpret_cast<unsigned long long*>(numer_dev), reinterpret_cast<unsigned long long*>(sums_dev), nframes,
+      npix_dev, reinterpret_cast<unsigned long long*>(scratch_dev));
+  return launch_status();
+}
+
+extern "C" int g2_operand_expand(const void* packed_dev, int64_t nrows, int64_t nframes, int64_t packed_cols,
+                                 int32_t elem_kind, int32_t out_kind, const uint32_t* res_count_dev,
+                                 const void* res_list_dev, int32_t res_cap, void* out_dev, int32_t* err_dev,
+                                 void* stream) {
+  using namespace g2;
+  Residuals res;
+  const bool e2m1 = elem_kind == G2_KIND_E2M1, wide = out_kind == G2_KIND_FP16;
+  if (!packed_dev || !out_dev || !err_dev || nframes <= 0 || nrows < nframes || nrows >= (1ll << 31) ||
+      !aligned(packed_dev, 16) || !aligned(out_dev, 16) ||
+      !residuals_ok(res_count_dev, res_list_dev, res_cap, packed_cols, &res) ||
+      (!e2m1 && elem_kind != G2_KIND_E4M3) || (!wide && out_kind != G2_KIND_E4M3))
+    return G2_ERR_ARG;
+  const int64_t n8 = nrows * packed_cols / 8;
+  const int64_t blocks = (n8 + 255) / 256;
+  if (blocks > 0x7fffffff) return G2_ERR_TOO_LARGE;
+  const unsigned g = static_cast<unsigned>(blocks);
+  auto* in = reinterpret_cast<const uint8_t*>(packed_dev);
+  auto* out = reinterpret_cast<uint8_t*>(out_dev);
+  cudaStream_t st = as_stream(stream);
+  if (e2m1 && wide) tail::expand_kernel<true, true><<<g, 256, 0, st>>>(in, nrows, packed_cols, out);
+  else if (e2m1) tail::expand_kernel<true, false><<<g, 256, 0, st>>>(in, nrows, packed_cols, out);
+  else if (wide) tail::expand_kernel<false, true><<<g, 256, 0, st>>>(in, nrows, packed_cols, out);
+  else tail::expand_kernel<false, false><<<g, 256, 0, st>>>(in, nrows, packed_cols, out);
+  if (wide) tail::expand_residual_kernel<true><<<res.n_sectors, 64, 0, st>>>(res, nframes, packed_cols, out, err_dev);
+  else tail::expand_residual_kernel<false><<<res.n_sectors, 64, 0, st>>>(res, nframes, packed_cols, out, err_dev);
+  return launch_status();
+}

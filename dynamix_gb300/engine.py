@@ -23,8 +23,11 @@ import threading
 import numpy as np
 
 from . import _lib
-from .plan import (E4M3_MAX_EXACT, EXACT_LIMIT, FP16_MAX_EXACT, MODE_BYTES, MODE_E4M3, MODE_FP16, TILE_SHAPES,
-                   PackLayout, balance_items, chunk_grams, column_window, e4m3_segment_bound, gram_items)
+from .plan import (E4M3_MAX_EXACT, EXACT_LIMIT, FP16_MAX_EXACT, MODE_BYTES, MODE_E2M1, MODE_E4M3, MODE_FP16,
+                   TILE_SHAPES, NarrowLayout, PackLayout, balance_items, chunk_grams, column_window,
+                   e2m1_segment_bound, e4m3_segment_bound, gram_items, split_items)
+
+MODE_NAMES = {MODE_FP16: "fp16", MODE_BYTES: "bytes", MODE_E4M3: "e4m3", MODE_E2M1: "e2m1"}
 
 
 def _torch():
@@ -113,8 +116,14 @@ def device_layout(qmask, n_bins, mode, dev, digest=None):
         if L is not None:
             _LAYOUTS.move_to_end(key)
             return L
-    L = PackLayout(q, n_bins, mode)
     d = lambda a: torch.as_tensor(a, device=dev)
+    if mode == MODE_E2M1:
+        L = NarrowLayout(q, n_bins)
+        L.d_col_src, L.d_sector_bin = d(L.col_src), d(L.sector_bin)
+        L.d_unit_block_off, L.d_units = d(L.unit_block_off), d(L.units.view(np.int32))
+        L.d_chunk_span = d(L.chunk_span.view(np.int32))
+        return _keep_layout(key, L)
+    L = PackLayout(q, n_bins, mode)
     L.d_col_src = d(L.col_src)
     L.d_chunk_entry_off = d(L.chunk_entry_off)
     L.d_entry_dst = d(L.entry_dst)
@@ -128,6 +137,12 @@ def device_layout(qmask, n_bins, mode, dev, digest=None):
         L.d_word_src = d(L.word_src.view(np.int32))
         L.d_unit_block_off = d(L.unit_block_off)
         L.d_units = d(L.units.view(np.int32))
+        L.d_chunk_span = d(L.chunk_span.view(np.int32))
+        L.d_sector_bin = d(L.seg_bin) if L.n_segs else torch.full((2,), -1, dtype=torch.int32, device=dev)
+    return _keep_layout(key, L)
+
+
+def _keep_layout(key, L):
     with _LAYOUTS_LOCK:
         _LAYOUTS[key] = L
         while len(_LAYOUTS) > _LAYOUTS_MAX:
@@ -188,7 +203,10 @@ class DenseEngine:
         self.denom = z(torch.int64)
         self.g2_f32 = z(torch.float32)
         self.g2_f64 = z(torch.float64)
-        self.err = torch.zeros(1, dtype=torch.int32, device=self.dev)
+        # device words of one call: the error word, the residuals of a narrow
+        # operand, and the sampled counts that e2m1 / e4m3 operands split
+        self.status = torch.zeros(4, dtype=torch.int32, device=self.dev)
+        self.err = self.status[:1]
         self.maxval = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._layouts = {} if layouts is None else layouts   # may be shared by engines of one q-mask
         self._qdigest = qmask_digest
@@ -198,6 +216,10 @@ class DenseEngine:
         self._u8_hint = MODE_E4M3 if method == "tc" else MODE_FP16
         self._u16_hint = MODE_E4M3 if method == "tc" else MODE_FP16
         self.operand_hint = "auto"
+        self._narrow = None       # narrow operand of the next u8 stack (see _narrow_mode): None = look first
+        self._narrow_age = 0
+        self._narrow_over = set()  # narrow operands whose residual lists a stack has overflowed
+        self._residuals = None    # (layout, counts, lists, capacity) of the last narrow run
         self._packed_mode = None
         self.pipeline = True      # chunked copy/pack/Gram overlap where it applies
         self.pipe_chunks = self.PIPE_CHUNKS
@@ -219,6 +241,7 @@ class DenseEngine:
         if operand not in ("auto", "e4m3", "fp16", "bytes"):
             raise ValueError("operand hint must be 'auto', 'e4m3', 'fp16' or 'bytes'")
         self.operand_hint = operand
+        self._narrow = None
         if self.method != "tc" or self.operand != "auto":
             return
         mode = MODE_E4M3 if operand == "auto" else self.MODES[operand]
@@ -318,7 +341,7 @@ class DenseEngine:
         the pack."""
         return bool(L.ones_row or (L.mode == MODE_FP16 and self.method == "tc"))
 
-    def _packed_buffer(self, L):
+    def _packed_buffer(self, L, narrow=False):
         """The packed operand buffer, [T (+1)][packed_cols]; zeroed whenever its
         layout changes, since the pack kernels write only the binned columns
         (padding stays 0).  Layouts with :meth:`ones` get the row of ones after
@@ -328,19 +351,26 @@ class DenseEngine:
         rows = self.T + (1 if ones else 0)
         nbytes = rows * L.packed_bytes_per_frame
         fresh = False
+        # e2m1 layouts of cropped and of whole frames have different column
+        # orders; narrow operands are K-blocked, the others row-major
+        layout = (narrow, L if L.mode == MODE_E2M1 else None)
         if self.packed is None or self.packed.numel() < nbytes:
             self.packed = None
             self.packed = torch.zeros(nbytes, dtype=torch.uint8, device=self.dev)
             fresh = True
-        elif self._packed_mode != L.mode:
+        elif self._packed_mode != L.mode or getattr(self, "_packed_layout", None) != layout:
             self.packed.zero_()
             fresh = True
         if fresh:
             self._packed_mode = L.mode
+            self._packed_layout = layout
             if ones:
                 row = torch.from_numpy(L.ones_row_values().view(np.uint8)).to(self.dev)
-                off = self.T * L.packed_bytes_per_frame
-                self.packed[off:off + row.numel()].copy_(row)
+                if narrow:
+                    self.packed[:nbytes].view(-1, rows, 128)[:, self.T].copy_(row.view(-1, 128))
+                else:
+                    off = self.T * L.packed_bytes_per_frame
+                    self.packed[off:off + row.numel()].copy_(row)
         return self.packed
 
     # -- stages ----------------------------------------------------------
@@ -373,6 +403,7 @@ class DenseEngine:
     def pack(self, frames_dev, mode):
         L = self._layout(mode)
         packed = self._packed_buffer(L)
+        self._residuals = None
         self.sums.zero_()
         emax = self._piece_emax(L)
         emax.zero_()
@@ -395,10 +426,10 @@ class DenseEngine:
             return {"pair": "pair", "wide": "wide"}.get(self.tile, "tc")
         return self.method
 
-    def workers(self):
+    def workers(self, e2m1=False):
         """Persistent workers of a tensor-core Gram launch (CTAs, or CTA pairs
         for the pair tile), as the kernel will use them."""
-        pair = {"pair": 1, "wide": 2}.get(self.tile, 0)
+        pair = 3 if e2m1 else {"pair": 1, "wide": 2}.get(self.tile, 0)
         if self.grid > 0:
             return (self.grid + 1) // 2 if pair else self.grid
         key = (str(self.dev), pair)
@@ -409,12 +440,15 @@ class DenseEngine:
         return _WORKERS[key]
 
     def balanced(self, items, L):
-        """``items`` laid out for the kernel's workers, longest-first balanced
+        """``items`` of one launch, their K cut where they are too few to fill
+        the GPU, laid out for the kernel's workers, longest-first balanced
         (tensor-core launches only)."""
         if self.method != "tc" or items.size == 0:
             return items
-        return balance_items(items, self.workers(), 128 if L.kind == _lib.KIND_E4M3 else 64, self.item_kind,
-                             ones=self.ones(L))
+        e2m1 = L.mode == MODE_E2M1
+        shape = (self.workers(e2m1), 256 if e2m1 else 128 if L.kind == _lib.KIND_E4M3 else 64,
+                 "pair4" if e2m1 else self.item_kind, self.ones(L))
+        return balance_items(split_items(items, *shape), *shape)
 
     pack_units = True         # u8 e4m3 packing by work units (g2_pack_e4m3_units)
 
@@ -476,10 +510,13 @@ class DenseEngine:
                                                 self.numer.numel(), ptr(self.err), st), "g2_plain_direct")
 
     def gram_launch(self, jobs, items_ptr, n_items, stream):
-        """One launch of the tensor-core Gram kernel this engine's tile selects."""
+        """One launch of the tensor-core Gram kernel this engine's tile (or the
+        e2m1 operand) selects."""
         fn, name = {"pair": (self.lib.g2_gram_tc_pair, "g2_gram_tc_pair"),
                     "wide": (self.lib.g2_gram_tc_wide, "g2_gram_tc_wide")}.get(
                         self.tile, (self.lib.g2_gram_tc, "g2_gram_tc"))
+        if jobs[0].elem_kind == _lib.KIND_E2M1:
+            fn, name = self.lib.g2_gram_tc_e2m1, "g2_gram_tc_e2m1"
         _lib.check(fn(jobs, 1, C.c_void_p(items_ptr), n_items, ptr(self.numer), self.numer.numel(), ptr(self.sums),
                       self.sums.numel(), ptr(self.err), self.grid,
                       stream if isinstance(stream, C.c_void_p) else C.c_void_p(stream)), name)
@@ -538,6 +575,7 @@ class DenseEngine:
                 # every count <= 16 (the chunks' largest squares): the next call can use e4m3
                 if frames_dev.element_size() == 1:
                     self._u8_hint = MODE_E4M3
+                    self._narrow = None
                 else:
                     self._u16_hint = MODE_E4M3
             return L, grams
@@ -570,6 +608,19 @@ class DenseEngine:
     # on fp16 operands: 4.04 -> 3.98 ms)
     PIPE_CHUNKS_HOST = 16
 
+    # Stacks on the device: chunks hide the e4m3 pack under a long Gram (514 x
+    # 1030 x 10,000 frames: 11.6 ms against 12.9 in one piece).  A narrow
+    # operand's Gram leaves the pack nothing to hide under (7.82 ms in one
+    # piece, 7.95 in 8 chunks), and a short Gram's launches each cover too few
+    # tiles (256 x 256 x 2,000: 0.31 against 0.40 ms; 128 x 128 x 1,000: 0.16
+    # against 0.20): both run in one piece.
+    PIPE_MIN_MACS = 5.0e11
+
+    def _chunk_count(self, host, narrow):
+        if host:
+            return self.pipe_chunks_host
+        return self.pipe_chunks if not narrow and self._macs() >= self.PIPE_MIN_MACS else 1
+
     @staticmethod
     def pipe_bounds(T, n, growth, taper=0):
         """Frame bounds of ``n`` pipeline chunks (multiples of 128 frames, the
@@ -600,18 +651,21 @@ class DenseEngine:
         e4m3 split, which needs no energies).  ``chunks``: the number of frame
         chunks (default ``pipe_chunks``)."""
         chunks = self.pipe_chunks if chunks is None else int(chunks)
+        kind = "pair4" if L.mode == MODE_E2M1 else self.item_kind
         key = ("pipe", L.mode, self.T, self.exact_limit, self.grid, chunks, self.super_rows, self.kslab,
-               self.item_kind, self.pipe_growth, int(taper), None if grams is None else tuple(grams))
+               kind, self.pipe_growth, int(taper), None if grams is None else tuple(grams),
+               tuple(L.grams()) if L.mode == MODE_E2M1 else None)
         if key not in self._items_cache:
             torch = _torch()
             if grams is None:
-                grams = chunk_grams(L, e4m3_segment_bound(L), self.exact_limit, self.kslab)
-            items = gram_items(self.T, grams, job=0, out_base=0, kind=self.item_kind,
+                bound = e2m1_segment_bound(L) if L.mode == MODE_E2M1 else e4m3_segment_bound(L)
+                grams = chunk_grams(L, bound, self.exact_limit, self.kslab)
+            items = gram_items(self.T, grams, job=0, out_base=0, kind=kind,
                                s_base=0 if self.ones(L) else None, super_rows=self.super_rows)
             T = self.T
             n = max(1, min(chunks, T // 256))
             bounds = self.pipe_bounds(T, n, self.pipe_growth, taper)
-            need = np.minimum(items["j0"].astype(np.int64) + TILE_SHAPES[self.item_kind][1], T)
+            need = np.minimum(items["j0"].astype(np.int64) + TILE_SHAPES[kind][1], T)
             grp = np.searchsorted(bounds[1:], need, side="left")
             # each chunk's launch balanced over the kernel's workers
             parts = [self.balanced(items[grp == g], L) for g in range(bounds.size - 1)]
@@ -640,17 +694,22 @@ class DenseEngine:
 
     def pipelined_ok(self, frames):
         """The chunked pipeline applies on the tensor-core path to u8 stacks
-        while their counts are known (or expected) to be <= 16 (e4m3), and to
-        u8 / u16 stacks in pinned host memory on fp16 operands once a K split
-        can be reused (see :meth:`_speculative_ok`): fp16 packs keep no
-        per-frame state except energy maxima, which chunks combine."""
-        return self._pipeline_mode(frames) is not None
+        on narrow operands (see :meth:`_narrow_ok`), to u8 stacks while their
+        counts are known (or expected) to be <= 16 (e4m3), and to u8 / u16
+        stacks in pinned host memory on fp16 operands once a K split can be
+        reused (see :meth:`_speculative_ok`): fp16 packs keep no per-frame
+        state except energy maxima, which chunks combine."""
+        return (self._narrow_ok(frames) and self._narrow != MODE_FP16) or self._pipeline_mode(frames) is not None
+
+    def _pipeline_input(self, frames):
+        torch = _torch()
+        return (self.method == "tc" and self.pipeline and isinstance(frames, torch.Tensor) and self.n_bins > 0
+                and frames.dtype in (torch.uint8, torch.uint16)
+                and (frames.is_cuda or (frames.is_pinned() and frames.is_contiguous())))
 
     def _pipeline_mode(self, frames):
         torch = _torch()
-        if not (self.method == "tc" and self.pipeline and isinstance(frames, torch.Tensor) and self.n_bins > 0
-                and frames.dtype in (torch.uint8, torch.uint16)
-                and (frames.is_cuda or (frames.is_pinned() and frames.is_contiguous()))):
+        if not self._pipeline_input(frames):
             return None
         if (frames.dtype == torch.uint8 and self.operand in ("auto", "e4m3")
                 and (self.operand == "e4m3" or self._u8_hint == MODE_E4M3)):
@@ -665,27 +724,113 @@ class DenseEngine:
             return MODE_FP16
         return None
 
+    # -- narrow operands (u8 stacks whose large counts are rare) --------------
+    # e2m1 (4 bits: counts 0-7) or e4m3 (0-16) operands with the rest of each
+    # larger count in residual lists (csrc/g2_tail.cu), exact whatever the
+    # counts.  Each residual costs T multiply-adds on the CUDA cores (about
+    # 8 ps each), so a narrow element is taken while its residuals cost less
+    # than the next wider element's Gram: at most NARROW_MAX of the binned
+    # counts (e2m1 against e4m3, e4m3 against fp16; exponential speckle of mean
+    # 0.33 and 1.2 counts).  Which, is sampled on a correlator's first stack
+    # and followed from call to call.  Below NARROW_MIN_MACS the launches cost
+    # more than the Gram whatever the element.
+    NARROW_MIN_MACS = 2.0e10
+    NARROW_MAX = {MODE_E2M1: 1.5e-5, MODE_E4M3: 4.0e-5}
+    TAIL_FRAMES = 32      # frames of a look; from host memory fewer, each is a copy
+    TAIL_FRAMES_HOST = 8
+    NARROW_LOOK = 8       # stacks on fp16 operands between two looks
+
+    def _narrow_ok(self, frames):
+        """Whether a stack may run on a narrow operand (by its type and size)."""
+        torch = _torch()
+        return (self._pipeline_input(frames) and frames.dtype == torch.uint8 and frames.is_contiguous()
+                and self.operand == "auto" and self.operand_hint == "auto" and self.tile == "pair"
+                and self.exact_limit >= EXACT_LIMIT and self.T < 2 ** 31 and self._macs() >= self.NARROW_MIN_MACS)
+
+    def _binned_pixels(self):
+        """Pixels in the bins (an element layout that exists anyway counts them)."""
+        if getattr(self, "_n_binned", None) is None:
+            L = next(iter(self._layouts.values()), None) or self._layout(MODE_E2M1)
+            self._n_binned = int(L.npix.sum())
+        return self._n_binned
+
+    def _macs(self):
+        """Multiply-adds of the Gram's upper triangle (of the whole frame where that is already little)."""
+        tri = float(self.T) * (self.T + 1) / 2
+        return self.npix * tri if self.npix * tri < self.NARROW_MIN_MACS else self._binned_pixels() * tri
+
+    def _pick_narrow(self, sampled, c4, c8):
+        """The element for a stack with ``c4`` / ``c8`` e2m1 / e4m3 residuals
+        among ``sampled`` counts (MODE_FP16: neither)."""
+        for mode, c in ((MODE_E2M1, c4), (MODE_E4M3, c8)):
+            if mode not in self._narrow_over and c <= self.NARROW_MAX[mode] * sampled:
+                return mode
+        return MODE_FP16
+
+    def _narrow_mode(self, frames):
+        """MODE_E2M1 or MODE_E4M3 when the stack runs on that narrow operand,
+        else None.  A correlator's first stack is sampled (one short kernel and
+        a read of two words; frames in host memory are copied in for it)."""
+        if not self._narrow_ok(frames):
+            return None
+        if self._narrow is None:
+            n = min(self.T, self.TAIL_FRAMES if frames.is_cuda else self.TAIL_FRAMES_HOST)
+            src, T = frames, self.T
+            if not frames.is_cuda:
+                pick = [(2 * k + 1) * self.T // (2 * n) for k in range(n)]
+                src, T = _torch().empty((n,) + self.shape, dtype=frames.dtype, device=self.dev), n
+                for k, t in enumerate(pick):
+                    src[k].copy_(frames[t], non_blocking=True)
+            self.status.zero_()
+            self._count_tail(src.data_ptr(), T, self.npix, self._layout(MODE_E2M1), n, stream_handle(self.dev))
+            _, _, c4, c8 = self.status.tolist()
+            self._narrow = self._pick_narrow(n * self._binned_pixels(), c4, c8)
+            if self._narrow == MODE_FP16:
+                self._u8_hint = MODE_FP16             # counts above 16 were seen (or lists overflowed)
+        return None if self._narrow == MODE_FP16 else self._narrow
+
+    def _count_tail(self, frames_ptr, T, npix, L, n, stream):
+        _lib.check(self.lib.g2_count_tail(C.c_void_p(frames_ptr), T, npix, ptr(L.d_col_src), L.col_src.size, n,
+                                          ptr(self.status[2:]), stream if isinstance(stream, C.c_void_p)
+                                          else C.c_void_p(stream)), "g2_count_tail")
+
+    def _residual_buffers(self, L):
+        """(counts, lists, capacity) of the residual lists of layout ``L``: eight
+        times the entries that NARROW_MAX expects per sector, and 64."""
+        torch = _torch()
+        n = L.packed_cols // _lib.RES_SECTOR
+        cap = int(min(8192, 64 + 8 * max(self.NARROW_MAX.values()) * _lib.RES_SECTOR * self.T))
+        have = getattr(self, "_res_bufs", None)
+        if have is None or have[0].numel() < n:
+            self._res_bufs = None
+            have = self._res_bufs = (torch.empty(n, dtype=torch.int32, device=self.dev),
+                                     torch.empty(n * cap * 2, dtype=torch.int32, device=self.dev))
+        return have[0][:n], have[1], cap
+
     def run_pipelined(self, frames):
         """G1 + G2 chunk by chunk of frames: copy (host input) -> pack -> the
         Gram tiles that chunk completes, on three streams, so copies, packing
         and tensor-core work overlap; then G3 + G4.  One synchronisation at the
-        end reads the error word; counts above 16 rerun on fp16 operands."""
+        end reads the error word; counts above 16 rerun on fp16 operands
+        (narrow operands: residual lists that overflow rerun on a wider one)."""
         torch = _torch()
-        mode = self._pipeline_mode(frames)
-        L = self._layout(mode)
-        packed = self._packed_buffer(L)
+        narrow = self._narrow_mode(frames)
+        mode = narrow if narrow is not None else self._pipeline_mode(frames)
+        if mode is None:
+            return self.run(frames, pipelined=False)
         host = not frames.is_cuda
-        if mode == MODE_E4M3:
+        # u8 frames from host memory come in cropped to the q-mask's columns
+        # (the pack then reads the cropped frames with the cropped layout)
+        crop = host and mode in (MODE_E4M3, MODE_E2M1) and frames.element_size() == 1 and self.crop is not None
+        Lp = self._crop_layout(mode) if crop else self._layout(mode)
+        L = Lp if mode == MODE_E2M1 else self._layout(mode)
+        packed = self._packed_buffer(L, narrow is not None)
+        if mode != MODE_FP16:
             grams, bound = None, None
         else:                                 # fp16: the reused K split and the bounds it covers
             _, bound, grams = self._plans[mode]
         items, dev_items, bounds, starts, n_grams = self._pipe_plan(
-            L, self.PIPE_TAPER_HOST if host else 0, grams,
-            self.pipe_chunks_host if host else self.pipe_chunks)
-        # u8 frames from host memory come in cropped to the q-mask's columns
-        # (the pack then reads the cropped frames with the cropped layout)
-        crop = host and mode == MODE_E4M3 and frames.element_size() == 1 and self.crop is not None
-        Lp = self._crop_layout(mode) if crop else L
+            L, self.PIPE_TAPER_HOST if host else 0, grams, self._chunk_count(host, narrow is not None))
         if Lp.packed_cols != L.packed_cols:
             raise RuntimeError("cropped packing layout differs from the frame's")
         npix_in = self.shape[0] * self.crop[1] if crop else self.npix
@@ -706,11 +851,16 @@ class DenseEngine:
         self._mark("pipeline")
         self.numer.zero_()
         self.sums.zero_()
-        self.err.zero_()
+        self.status.zero_()
         emax = None
-        if mode != MODE_E4M3:
+        if mode == MODE_FP16:
             emax = self._piece_emax(L)
             emax.zero_()                      # chunks combine their energy maxima (atomicMax)
+        self._residuals = None
+        res = None
+        if narrow is not None:
+            res = self._residual_buffers(L)
+            res[0].zero_()
         start = torch.cuda.Event()
         start.record(cur)                     # the previous call's work and the zeroing are done first
         copy_s.wait_event(start)
@@ -718,10 +868,11 @@ class DenseEngine:
         gram_s.wait_event(start)
         self._timeline = []
         self._tmark("start", cur)
-        npix, pc = npix_in, L.packed_cols
+        npix = npix_in
         eb = frames_dev.element_size()
         row_bytes = L.packed_bytes_per_frame
-        jobs = _lib.jobs_array([(packed.data_ptr(), self.T, pc, L.kind, self.ones(L))])
+        kind = L.kind + (_lib.KIND_BLOCKED if narrow == MODE_E4M3 else 0)
+        jobs = _lib.jobs_array([(packed.data_ptr(), self.T, L.packed_cols, kind, self.ones(L))])
         item_bytes = _lib.ITEM_DTYPE.itemsize
         for c in range(bounds.size - 1):
             t0, t1 = int(bounds[c]), int(bounds[c + 1])
@@ -738,12 +889,16 @@ class DenseEngine:
                     e.record(copy_s)
                 pack_s.wait_event(e)
             self._tmark("pack%d" % c, pack_s)
-            if mode == MODE_E4M3:
-                self.pack_e4m3(frames_dev.data_ptr() + t0 * npix, 1, t1 - t0, Lp, packed.data_ptr() + t0 * pc,
-                               pack_s.cuda_stream, npix=npix)
+            src, dst = frames_dev.data_ptr() + t0 * npix * eb, packed.data_ptr() + t0 * row_bytes
+            if narrow is not None:
+                _lib.check(self.lib.g2_pack_u8_residual(
+                    C.c_void_p(src), t1 - t0, npix, t0, L.kind, ptr(Lp.d_unit_block_off), ptr(Lp.d_units),
+                    ptr(Lp.d_chunk_span), Lp.n_chunks, ptr(packed), self.T + 1, L.packed_cols, ptr(res[0]), ptr(res[1]), res[2], ptr(self.err),
+                    C.c_void_p(pack_s.cuda_stream)), "g2_pack_u8_residual")
+            elif mode == MODE_E4M3:
+                self.pack_e4m3(src, 1, t1 - t0, Lp, dst, pack_s.cuda_stream, npix=npix)
             else:
-                self.pack_fp16_frames(frames_dev.data_ptr() + t0 * npix * eb, eb, t1 - t0, L,
-                                      packed.data_ptr() + t0 * row_bytes, emax, pack_s.cuda_stream)
+                self.pack_fp16_frames(src, eb, t1 - t0, L, dst, emax, pack_s.cuda_stream)
             self._tmark("pack%d_end" % c, pack_s)
             e = torch.cuda.Event()
             e.record(pack_s)
@@ -759,10 +914,29 @@ class DenseEngine:
                 self._tmark("gram%d" % c, gs)
                 self.gram_launch(jobs, dev_items.data_ptr() + k0 * item_bytes, k1 - k0, gs.cuda_stream)
                 self._tmark("gram%d_end" % c, gs)
+        if narrow == MODE_E4M3:               # whether the next stack could run on e2m1
+            self._count_tail(frames_dev.data_ptr(), self.T, npix, Lp, min(self.T, self.TAIL_FRAMES),
+                             C.c_void_p(pack_s.cuda_stream))
+            done = torch.cuda.Event()
+            done.record(pack_s)
+            cur.wait_event(done)
         if len(gram_streams) > 1:
             done = torch.cuda.Event()
             done.record(gram_s)
             cur.wait_event(done)
+        if narrow is not None:
+            st = stream_handle(self.dev)
+            if mode == MODE_E2M1:
+                if getattr(self, "_offset_scratch", None) is None:
+                    self._offset_scratch = torch.empty(self.n_bins * (self.T + 1), dtype=torch.int64, device=self.dev)
+                    self._npix_dev = torch.as_tensor(L.npix, device=self.dev)
+                _lib.check(self.lib.g2_e2m1_offset(ptr(self.numer), ptr(self.sums), self.n_bins, self.T,
+                                                   ptr(self._npix_dev), ptr(self._offset_scratch), st),
+                           "g2_e2m1_offset")
+            _lib.check(self.lib.g2_residual_sums(
+                ptr(packed), self.T + 1, self.T, L.packed_cols, L.kind, ptr(res[0]), ptr(res[1]), res[2],
+                ptr(L.d_sector_bin), self.n_bins, ptr(self.numer), ptr(self.sums), ptr(self.status[1:]),
+                ptr(self.err), st), "g2_residual_sums")
         self._mark("normalise")
         self._tmark("normalise", cur)
         self.normalise()
@@ -770,7 +944,8 @@ class DenseEngine:
         self._tmark("end", cur)
         if host:
             self._frames_host_ref = frames            # alive until the copies are done
-        if mode != MODE_E4M3:
+        h2d = int(self.T * npix * eb) if host else 0
+        if mode == MODE_FP16:
             # one synchronisation: the error word and whether the stack's
             # energy bounds exceed those the reused split covers
             m = L.n_pieces
@@ -780,15 +955,31 @@ class DenseEngine:
                 return self.run(frames_dev, pipelined=False, reuse_split=False)
             self.last = {"mode": "fp16", "split": int(L.split), "n_items": int(items.size), "n_grams": n_grams,
                          "packed_cols": L.packed_cols, "pipeline_chunks": int(bounds.size - 1), "tile": self.tile,
-                         "plan": "reused", "h2d_bytes": int(self.T * npix * eb) if host else 0, "crop": None}
+                         "plan": "reused", "h2d_bytes": h2d, "crop": None}
+            return self.g2_f32[: self.n_bins]
+        self.last = {"mode": MODE_NAMES[mode], "split": int(L.split), "n_items": int(items.size), "n_grams": n_grams,
+                     "packed_cols": L.packed_cols, "pipeline_chunks": int(bounds.size - 1), "tile": self.tile,
+                     "h2d_bytes": h2d, "crop": list(self.crop) if crop else None}
+        if narrow is not None:
+            code, total, c4, c8 = self.status.tolist()
+            if code & _lib.DEVERR_RESIDUAL:           # more large counts than the lists hold: look again
+                again = frames if crop else frames_dev
+                self._narrow = None
+                if self._narrow_mode(again) == mode:  # a few pixels that are bright in every frame
+                    self._narrow_over.add(mode)
+                    self._narrow = None
+                return self.run(again)
+            self.last["residuals"] = total
+            self._residuals = (L,) + res + (total,)
+            if total > 2 * self.NARROW_MAX[mode] * self._binned_pixels() * self.T:
+                self._narrow = None                   # look at the next stack first
+            elif mode != MODE_E2M1:
+                self._narrow = self._pick_narrow(min(self.T, self.TAIL_FRAMES) * self._binned_pixels(), 2 * c4, c8)
             return self.g2_f32[: self.n_bins]
         code = self.resolve_range_check(int(self.err.item()), frames_dev, cropped=crop)
         if code & _lib.DEVERR_RANGE and self.operand == "auto":
             self._u8_hint = MODE_FP16                 # counts above 16: rerun on fp16 operands
             return self.run(frames if crop else frames_dev, pipelined=False)
-        self.last = {"mode": "e4m3", "split": int(L.split), "n_items": int(items.size), "n_grams": n_grams,
-                     "packed_cols": L.packed_cols, "pipeline_chunks": int(bounds.size - 1), "tile": self.tile,
-                     "h2d_bytes": int(self.T * npix * eb) if host else 0, "crop": list(self.crop) if crop else None}
         return self.g2_f32[: self.n_bins]
 
     # -- whole pipeline ----------------------------------------------------
@@ -804,6 +995,10 @@ class DenseEngine:
                                                                     tuple(frames_dev.shape)))
         if self.n_bins == 0:
             return self.g2_f32[:0]
+        if pipelined and self._narrow == MODE_FP16:
+            self._narrow_age += 1
+            if self._narrow_age % self.NARROW_LOOK == 0:
+                self._narrow = None               # the stacks may have become dim: look again
         if pipelined and self.pipelined_ok(frames_dev):
             return self.run_pipelined(frames_dev)
         if not frames_dev.is_cuda:
@@ -924,6 +1119,33 @@ class DenseEngine:
                      "packed_cols": L.packed_cols}
         return self.g2_f32[: self.n_bins]
 
+    def _last_operand(self, what):
+        """(layout, element kind, buffer) of the last run's packed operand as
+        the single-CTA kernels read it: a narrow operand is expanded to
+        row-major e4m3 bytes, or to fp16 when a count exceeds 16."""
+        torch = _torch()
+        if self.packed is None or self._packed_mode is None:
+            raise RuntimeError("%s needs a preceding run()" % what)
+        if self._residuals is None:
+            L = self._layouts[self._packed_mode]
+            return L, L.kind, self.packed
+        L, counts, lists, cap, total = self._residuals
+        rows = self.T + 1
+        for kind, nb in ((_lib.KIND_E4M3, 1), (_lib.KIND_FP16, 2)):
+            if L.mode == MODE_E4M3 and total and kind == L.kind:
+                continue                              # residuals of e4m3 are counts above 16
+            wide = getattr(self, "_wide", None)
+            if wide is None or wide.numel() < rows * L.packed_cols * nb:
+                self._wide = None
+                wide = self._wide = torch.empty(rows * L.packed_cols * nb, dtype=torch.uint8, device=self.dev)
+            self.err.zero_()
+            _lib.check(self.lib.g2_operand_expand(ptr(self.packed), rows, self.T, L.packed_cols, L.kind, kind,
+                                                  ptr(counts), ptr(lists), cap, ptr(wide), ptr(self.err),
+                                                  stream_handle(self.dev)), "g2_operand_expand")
+            if kind == _lib.KIND_FP16 or not total or not int(self.err.item()) & _lib.DEVERR_RANGE:
+                break
+        return L, kind, wide
+
     def deviation(self):
         """calc_std of the last run (dense.py:58-66): float32 device tensor
         ``(n_bins, T)``; float64 in ``self.dev_f64``.  One more tensor-core pass
@@ -931,12 +1153,10 @@ class DenseEngine:
         torch = _torch()
         if self.method != "tc":
             raise NotImplementedError("calc_std runs on the tensor-core path")
-        L = self._layouts.get(self._packed_mode)
-        if L is None or self.packed is None:
-            raise RuntimeError("deviation() needs a preceding run()")
+        L, kind, packed = self._last_operand("deviation()")
         if L.split:
             return self._deviation_planes(L)
-        key = ("std", L.mode, self.T)
+        key = ("std", L.mode, self.T, tuple(L.grams()))
         if key not in self._items_cache:
             from .plan import std_items
             npix = np.bincount(self.qmask.ravel()[self.qmask.ravel() > 0], minlength=self.n_bins + 1)[1:]
@@ -952,7 +1172,7 @@ class DenseEngine:
         sd2.zero_()
         zeros.zero_()
         st = stream_handle(self.dev)
-        jobs = _lib.jobs_array([(self.packed.data_ptr(), self.T, L.packed_cols, L.kind, self.ones(L))])
+        jobs = _lib.jobs_array([(packed.data_ptr(), self.T, L.packed_cols, kind, self.ones(L))])
         if items.size:
             _lib.check(self.lib.g2_gram_std(jobs, 1, ptr(dev_items), items.size, ptr(self.sums), self.sums.numel(),
                                             ptr(self.g2_f32), ptr(sd), ptr(sd2), ptr(zeros), sd.numel(),
@@ -1016,14 +1236,12 @@ class DenseEngine:
         torch = _torch()
         if self.method != "tc":
             raise NotImplementedError("the two-time correlation runs on the tensor-core path")
-        L = self._layouts.get(self._packed_mode)
-        if L is None or self.packed is None:
-            raise RuntimeError("two_time() needs a preceding run()")
+        L, kind, packed = self._last_operand("two_time()")
         if L.split:
             raise NotImplementedError("the two-time correlation needs counts <= 2048 (no byte planes)")
         if not 0 <= b < self.n_bins:
             raise ValueError("bin %d outside [0, %d)" % (b, self.n_bins))
-        key = ("std", L.mode, self.T)
+        key = ("std", L.mode, self.T, tuple(L.grams()))
         if key not in self._items_cache:
             from .plan import std_items
             npix = np.bincount(self.qmask.ravel()[self.qmask.ravel() > 0], minlength=self.n_bins + 1)[1:]
@@ -1040,7 +1258,7 @@ class DenseEngine:
         mirror = 1 if self.T <= 5 or not np.any(s_h[:-5] * s_h[5:] == 0) else 0
         out = torch.empty((self.T, self.T), dtype=torch.float32, device=self.dev)
         st = stream_handle(self.dev)
-        jobs = _lib.jobs_array([(self.packed.data_ptr(), self.T, L.packed_cols, L.kind, self.ones(L))])
+        jobs = _lib.jobs_array([(packed.data_ptr(), self.T, L.packed_cols, kind, self.ones(L))])
         _lib.check(self.lib.g2_gram_ttcf(jobs, 1, ptr(items_dev), mine.size, ptr(self.sums), self.sums.numel(),
                                          ptr(out), self.T, self.T, mirror, ptr(self.err), self.grid, st),
                    "g2_gram_ttcf")

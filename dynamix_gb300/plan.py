@@ -21,22 +21,27 @@ from __future__ import annotations
 
 import numpy as np
 
-from ._lib import (BK, ITEM_DTYPE, ITEM_EMPTY, KIND_E4M3, KIND_FP16, PACK_CHUNK, PACK_MAX_PIECES, PACK_MAX_SLOTS,
-                   PACK_WORDS_PER_CHUNK, PAD, PLAIN_BM, PLAIN_BN, TC_BM, TC_BN)
+from ._lib import (BK, E2M1_CHUNK, ITEM_DTYPE, ITEM_EMPTY, KIND_E2M1, KIND_E4M3, KIND_FP16, PACK_CHUNK, PACK_MAX_PIECES, PACK_MAX_SLOTS,
+                   PACK_WORDS_PER_CHUNK, PAD, PLAIN_BM, PLAIN_BN, RES_SECTOR, TC_BM, TC_BN)
 
 EXACT_LIMIT = 1 << 24   # fp32 represents every integer up to 2^24 exactly
 FP16_MAX_EXACT = 2048   # fp16 represents every integer up to 2^11 exactly
 E4M3_MAX_EXACT = 16     # e4m3 represents every integer up to 2^4 exactly
 SUPER_ROWS = 2048       # frames per side of a super-tile
 
-MODE_FP16, MODE_BYTES, MODE_E4M3 = 0, 1, 2
+MODE_FP16, MODE_BYTES, MODE_E4M3, MODE_E2M1 = 0, 1, 2, 3
+E2M1_PAD = 256          # e2m1 columns of one 128-byte block
+E2M1_MAX_U = 4          # e2m1 codes hold u = count - 3, counts 0-7
+E2M1_WORD = np.array([0, 4, 1, 5, 2, 6, 3, 7])  # columns of counts a0..a3 b0..b3 in a word of 8
 UNIT_NONE, UNIT_VEC, UNIT_WORD, UNIT_GATHER, UNIT_BYTE = 0, 1, 2, 3, 4   # classes of the e4m3 pack's units
 
 # (rows, columns) of one Gram item per kernel: the single-CTA tensor-core
 # block (g2_gram_tc), the CTA-pair blocks (g2_gram_tc_pair: 256 rows over two
 # SMs; g2_gram_tc_wide: 256 x 512), and the CUDA-core comparators' blocks
 PAIR_BM, PAIR_BN = 256, 256
+F4_BN = 224
 TILE_SHAPES = {"tc": (TC_BM, TC_BN), "pair": (PAIR_BM, PAIR_BN), "wide": (PAIR_BM, 2 * PAIR_BN),
+               "pair4": (PAIR_BM, F4_BN),
                "plain": (PLAIN_BM, PLAIN_BN), "dp4a": (PLAIN_BM, PLAIN_BN)}
 
 
@@ -209,6 +214,7 @@ class PackLayout:
             nxt += nb
         self.unit_block_off = off.astype(np.int32)
         self.units = units.reshape(-1)
+        self.chunk_span = chunk_spans(pix, self.n_chunks, PACK_CHUNK)
 
     def segment_emax(self, piece_emax):
         """Per 64-column output segment, the sum over its pieces of the pieces'
@@ -255,6 +261,168 @@ class PackLayout:
                 out.append((b, lo, h, kp, 8))    # low  x high, weight 2^8
                 out.append((b, lo, lo, kp, 0))   # low  x low
         return out
+
+
+def chunk_spans(pix, n_chunks, size):
+    """lo | hi << 16 of every chunk of ``size`` pixels: its binned pixels
+    (``pix``: all of them) lie in [lo, hi) of the chunk."""
+    ch = pix // size
+    lo = np.full(n_chunks, size, dtype=np.int64)
+    hi = np.zeros(n_chunks, dtype=np.int64)
+    np.minimum.at(lo, ch, pix - ch * size)
+    np.maximum.at(hi, ch, pix - ch * size + 1)
+    return (np.minimum(lo, hi) | (hi << 16)).astype(np.uint32)
+
+
+class NarrowLayout:
+    """Packed-column layout of the bins of one q-mask for e2m1 operands
+    (``g2_pack_u8_residual``, two columns per byte).  The order of a bin's
+    pixels is free (every Gram entry sums over them), so the columns follow
+    the pack's work units: per bin first the 32-column units (16 bytes from two
+    runs of 16 consecutive pixels of one 4080-pixel chunk), then the 8-column
+    units from two runs of 4, then the 8-column units from up to 8 single
+    pixels; bins padded to 256 columns (128 bytes, one block of the K-blocked
+    operand)."""
+
+    mode, kind, split, ones_row, elem_bytes = MODE_E2M1, KIND_E2M1, False, True, 0.5
+    n_pieces = 0
+
+    def __init__(self, qmask, n_bins):
+        q = np.ascontiguousarray(qmask, dtype=np.int32).ravel()
+        self.npix_total, self.n_bins = q.size, int(n_bins)
+        nb = max(self.n_bins, 1)
+        self.n_chunks = -(-q.size // E2M1_CHUNK)
+        pix = np.flatnonzero((q >= 1) & (q <= self.n_bins)).astype(np.int64)
+        b = q[pix].astype(np.int64) - 1
+        self.npix = np.bincount(b, minlength=nb)[: self.n_bins].astype(np.int64)
+        grp = (pix // E2M1_CHUNK) * nb + b                     # (chunk, bin): a unit stays inside one
+        order = np.argsort(grp, kind="stable")
+        pix, grp = pix[order], grp[order]
+        first = np.ones(pix.size, dtype=bool)
+        first[1:] = (np.diff(pix) != 1) | (np.diff(grp) != 0)
+        start = np.flatnonzero(first)
+        n = np.diff(np.append(start, pix.size))
+        rp, rg = pix[start], grp[start]                         # runs: first pixel, group, length
+
+        def pieces(first_pix, group, count, size):
+            """``count`` consecutive pieces of ``size`` pixels from each first pixel."""
+            k = np.arange(count.sum()) - np.repeat(np.cumsum(count) - count, count)
+            return np.repeat(first_pix, count) + size * k, np.repeat(group, count)
+
+        def paired(p, g):
+            """Pieces in pairs of one group, piece j with piece j + m // 2 of its
+            m (the lanes of a warp then read consecutive pieces in both
+            halves), and the pieces left over."""
+            o = np.argsort(g, kind="stable")
+            p, g = p[o], g[o]
+            new = np.ones(g.size, dtype=bool)
+            new[1:] = np.diff(g) != 0
+            s = np.flatnonzero(new)
+            c = np.diff(np.append(s, g.size))
+            rank, half = np.arange(g.size) - np.repeat(s, c), np.repeat(c // 2, c)
+            a = np.flatnonzero(rank < half)
+            odd = rank >= 2 * half
+            return p[a], p[a + half[a]], g[a], p[odd], g[odd]
+
+        p16, g16 = pieces(rp, rg, n // 16, 16)
+        v0, v1, vg, lp, lg = paired(p16, g16)
+        rest = rp + n // 16 * 16
+        p4, g4 = pieces(rest, rg, n % 16 // 4, 4)
+        q4, h4 = pieces(lp, lg, np.full(lp.size, 4), 4)
+        w0, w1, wg, lp, lg = paired(np.concatenate([p4, q4]), np.concatenate([g4, h4]))
+        p1, g1 = pieces(rest + n % 16 // 4 * 4, rg, n % 4, 1)
+        q1, h1 = pieces(lp, lg, np.full(lp.size, 4), 1)
+        p1, g1 = np.concatenate([p1, q1]), np.concatenate([g1, h1])
+        o = np.argsort(g1, kind="stable")
+        p1, g1 = p1[o], g1[o]
+        new = np.ones(g1.size, dtype=bool)
+        new[1:] = np.diff(g1) != 0
+        s = np.flatnonzero(new)
+        c = np.diff(np.append(s, g1.size))
+        rank = np.arange(g1.size) - np.repeat(s, c)
+        unit = np.cumsum(rank % 8 == 0) - 1                      # gather unit of every single pixel
+        gg = g1[rank % 8 == 0]
+        singles = np.full((gg.size, 8), -1, dtype=np.int64)
+        singles[unit, rank % 8] = p1
+
+        def within_bin(g):
+            """Position of every unit among the units of its bin (chunk order)."""
+            bins = g % nb
+            o = np.argsort(bins, kind="stable")
+            c = np.bincount(bins, minlength=nb)
+            pos = np.empty(g.size, dtype=np.int64)
+            pos[o] = np.arange(g.size) - np.repeat(np.cumsum(c) - c, c)
+            return bins, pos, c
+
+        vb, vpos, vc = within_bin(vg)
+        wb, wpos, wc = within_bin(wg)
+        gb, gpos, gc = within_bin(gg)
+        self.kpad = _roundup(32 * vc + 8 * (wc + gc), E2M1_PAD)[: self.n_bins].astype(np.int64)
+        off = np.concatenate([[0], np.cumsum(self.kpad)])
+        self.bin_off = self.plane0 = off[:-1].astype(np.int64)
+        self.plane1 = None
+        self.packed_cols = int(max(E2M1_PAD, off[-1]))
+        if self.packed_cols >= 2 ** 31:
+            raise ValueError("too many binned pixels for one job")
+        vcol = self.bin_off[vb] + 32 * vpos
+        wcol = self.bin_off[wb] + 32 * vc[wb] + 8 * wpos
+        gcol = self.bin_off[gb] + 32 * vc[gb] + 8 * (wc[gb] + gpos)
+        col_src = np.full(self.packed_cols, -1, dtype=np.int32)
+        for col, runs, size in ((vcol, (v0, v1), 16), (wcol, (w0, w1), 4)):
+            j = np.arange(size)
+            for half, p in enumerate(runs):
+                col_src[(col[:, None] + j // 4 * 8 + E2M1_WORD[4 * half + j % 4]).ravel()] = (p[:, None] + j).ravel()
+        col_src[(gcol[:, None] + E2M1_WORD).ravel()] = singles.ravel()
+        self.col_src = col_src                                     # pixel of every packed column, -1: padding
+        self.sector_bin = np.repeat(np.arange(self.n_bins, dtype=np.int32), self.kpad // RES_SECTOR)
+        if self.sector_bin.size < self.packed_cols // RES_SECTOR:
+            self.sector_bin = np.full(self.packed_cols // RES_SECTOR, -1, dtype=np.int32)
+        # blocks of 32 units of one class per chunk
+        local = lambda p, ch: p - ch * E2M1_CHUNK
+        recs = []
+        for cls, g, dst, p in ((UNIT_VEC, vg, vcol // 32, (v0, v1)), (UNIT_WORD, wg, wcol // 8, (w0, w1))):
+            ch = g // nb
+            u = np.zeros((g.size, 4), dtype=np.int64)
+            u[:, 0] = dst | (cls << 30)
+            u[:, 1] = local(p[0], ch) | (local(p[1], ch) << 16)
+            recs.append((ch, u))
+        ch = gg // nb
+        src = np.where(singles >= 0, singles - ch[:, None] * E2M1_CHUNK, 0xFFF)
+        u = np.zeros((gg.size, 4), dtype=np.int64)
+        u[:, 0] = (gcol // 8) | (UNIT_GATHER << 30)
+        for k in range(8):
+            w, sh = divmod(12 * k, 32)
+            u[:, 1 + w] |= (src[:, k] << sh) & 0xFFFFFFFF
+            if sh > 20:
+                u[:, 2 + w] |= src[:, k] >> (32 - sh)
+        recs.append((ch, u))
+        blocks = [-(-np.bincount(ch, minlength=self.n_chunks) // 32) for ch, _ in recs]
+        boff = np.concatenate([[0], np.cumsum(sum(blocks))])
+        units = np.zeros((int(boff[-1]) * 32, 4), dtype=np.uint32)
+        nxt = boff[:-1].copy()
+        for (ch, u), nblk in zip(recs, blocks):
+            o = np.argsort(ch, kind="stable")
+            c = np.bincount(ch, minlength=self.n_chunks)
+            pos = np.arange(ch.size) - np.repeat(np.cumsum(c) - c, c)
+            units[nxt[ch[o]] * 32 + pos] = u[o].astype(np.uint32)
+            nxt += nblk
+        self.unit_block_off = boff.astype(np.int32)
+        self.units = units.reshape(-1)
+        self.chunk_span = chunk_spans(pix, self.n_chunks, E2M1_CHUNK)
+
+    @property
+    def packed_bytes_per_frame(self):
+        return self.packed_cols // 2
+
+    def ones_row_values(self):
+        """Row of ones: code 1 in every binned column, 0 in the padding."""
+        one = (self.col_src >= 0).astype(np.uint8)
+        return one[0::2] | (one[1::2] << 4)
+
+    def grams(self):
+        """The Grams to run per bin: (bin, a_off, b_off, kpad, shift)."""
+        return [(b, int(self.bin_off[b]), int(self.bin_off[b]), int(self.kpad[b]), 0)
+                for b in range(self.n_bins) if self.kpad[b]]
 
 
 def k_chunks(emax_a, emax_b, limit=EXACT_LIMIT):
@@ -359,12 +527,12 @@ def item_costs(items, stage_elems, kind, ones=True):
     (g2_gram_tc_wide); single-CTA items always 256."""
     bn = TILE_SHAPES[kind][1]
     stages = items["k_len"].astype(np.float64) / float(stage_elems)
-    if kind in ("pair", "wide"):
+    if kind in ("pair", "pair4", "wide"):
         live = items["nframes"].astype(np.int64) - items["j0"].astype(np.int64)
         if ones:
             live = live + (items["s_off"] >= 0)
         r = (live + 31) // 32 * 32
-        if kind == "pair":
+        if kind in ("pair", "pair4"):
             n = np.clip(r, 32, bn)
         else:
             n0 = np.where(items["j0"].astype(np.int64) + PAIR_BN <= items["i0"], 0, np.clip(r, 32, PAIR_BN))
@@ -373,6 +541,37 @@ def item_costs(items, stage_elems, kind, ones=True):
             return stages * (n / float(bn)) + ITEM_OVERHEAD_STAGES + n / 64.0
         stages = stages * (n / float(bn))
     return stages + ITEM_OVERHEAD_STAGES
+
+
+# A launch whose items are few next to its workers leaves most of the chip
+# idle: their K is cut so that no item exceeds 1 / SPLIT_SHARE of a worker's
+# even share of the launch, down to SPLIT_MIN_STAGES stages (an item's fixed
+# cost is about ITEM_OVERHEAD_STAGES).
+SPLIT_SHARE = 3
+SPLIT_MIN_STAGES = 16
+
+
+def split_items(items, workers, stage_elems, kind, ones=True):
+    """``items`` of one launch with the K of the long ones cut into equal
+    pieces (multiples of a stage), for launches that would leave workers idle.
+    The sums are added piece by piece, so any cut gives the same results."""
+    if items.size == 0 or workers <= 1:
+        return items
+    share = item_costs(items, stage_elems, kind, ones).sum() / workers
+    most = max(float(SPLIT_MIN_STAGES), share / SPLIT_SHARE)
+    stages = items["k_len"].astype(np.int64) // stage_elems
+    n = np.maximum(1, np.ceil(stages / most).astype(np.int64))
+    n = np.where(stages > 1.25 * most, n, 1)
+    if n.max() == 1:
+        return items
+    out = np.repeat(items, n)
+    k = np.arange(out.size) - np.repeat(np.cumsum(n) - n, n)
+    st, nn = np.repeat(stages, n), np.repeat(n, n)
+    k0, k1 = st * k // nn * stage_elems, st * (k + 1) // nn * stage_elems
+    out["a_k0"] += k0.astype(np.int32)
+    out["b_k0"] += k0.astype(np.int32)
+    out["k_len"] = (k1 - k0).astype(np.int32)
+    return out
 
 
 def balance_items(items, workers, stage_elems, kind, ones=True):
@@ -483,6 +682,12 @@ def e4m3_segment_bound(layout):
     the data: every count is <= 16, so a segment's sum of squares is <= 64 * 256
     (a Gram chunk of up to 65,536 columns stays below 2^24)."""
     return np.full(layout.packed_cols // BK, BK * E4M3_MAX_EXACT ** 2, dtype=np.float64)
+
+
+def e2m1_segment_bound(layout):
+    """The same for e2m1 operands (|u| <= 4), doubled: their lag sums are signed,
+    so a chunk's Gram entries stay below 2^23."""
+    return np.full(layout.packed_cols // BK, 2 * BK * E2M1_MAX_U ** 2, dtype=np.float64)
 
 
 def gram_macs(T, npix):

@@ -39,6 +39,7 @@ extern "C" {
 #define G2_DEVERR_BOUNDS    2  /* an index was out of range and was skipped */
 #define G2_DEVERR_RANGE     4  /* a count does not fit the requested packing */
 #define G2_DEVERR_RANGE_CHECK 8 /* a count may not fit the packing: check the exact maximum */
+#define G2_DEVERR_RESIDUAL 16 /* a residual list overflowed: pack the stack into a wider element */
 
 #define G2_ABI_VERSION      1
 
@@ -52,6 +53,7 @@ extern "C" {
 #define G2_PLAIN_BN   128
 #define G2_PAD        128  /* packed_cols and bin segments are multiples of this */
 #define G2_PACK_CHUNK 2048 /* source pixels per pack chunk */
+#define G2_E2M1_CHUNK 4080 /* source pixels per chunk of the e2m1 pack (12-bit offsets) */
 #define G2_PACK_MAX_SLOTS  128  /* distinct bins per chunk */
 #define G2_PACK_MAX_PIECES 512  /* (64-column segment x chunk) pieces per chunk */
 #define G2_PACK_WORDS_PER_CHUNK 768 /* 4-column words per chunk: 2048/4 + partial words at bin edges */
@@ -60,6 +62,10 @@ extern "C" {
 /* element kinds of a packed operand matrix */
 #define G2_KIND_FP16  0    /* 16-bit raw counts <= 2048, MMA kind::f16 */
 #define G2_KIND_E4M3  1    /* 8-bit raw counts <= 16, MMA kind::f8f6f4 (e4m3) */
+#define G2_KIND_E2M1  2    /* 4-bit codes of u = count - 3, counts 0-7 (e2m1 = u / 2), two per byte
+                              (even column in the low half), padding u = 0, MMA kind::mxf4 */
+#define G2_KIND_BLOCKED 256 /* added to an element kind: the operand is K-blocked */
+#define G2_RES_SECTOR 64   /* packed columns per residual list */
 
 /* One unit of Gram work: rows [i0, i0+BM) of the A operand against rows
  * [j0, j0+BN) of the B operand over packed columns [a_k0, a_k0+k_len) and
@@ -91,12 +97,16 @@ typedef struct g2_gram_item {
 /* A dense job: its packed operand matrix, row-major [nframes][packed_cols]
  * of raw integer counts, 16-bit (G2_KIND_FP16, counts <= 2048, read as fp16 =
  * count * 2^-24) or 8-bit (G2_KIND_E4M3, counts <= 16, read as e4m3 =
- * count * 2^-9); both represent the counts exactly. */
+ * count * 2^-9); both represent the counts exactly.
+ * A K-blocked operand holds its rows in blocks of 128 bytes: byte x of row t
+ * lies at (x / 128) * rows * 128 + t * 128 + x % 128, rows = nframes +
+ * ones_row, so the 128 rows a Gram stage reads are one contiguous span. */
 typedef struct g2_job {
     const void* packed_dev;
     int64_t nframes;
     int64_t packed_cols;   /* multiple of G2_PAD */
-    int32_t elem_kind;     /* G2_KIND_FP16 or G2_KIND_E4M3 */
+    int32_t elem_kind;     /* G2_KIND_FP16 or G2_KIND_E4M3, either + G2_KIND_BLOCKED;
+                              g2_gram_tc_e2m1: G2_KIND_E2M1 (always K-blocked) */
     int32_t ones_row;      /* 1: row nframes of the packed matrix holds 1 in every
                               binned column and 0 in the padding (bin sums) */
 } g2_job;
@@ -194,6 +204,54 @@ int g2_pack_e4m3_units(const void* frames_dev, int64_t nframes, int64_t npix,
                        const int32_t* unit_block_off_dev, const uint32_t* units_dev, int64_t n_chunks,
                        void* packed_dev, int64_t packed_cols, int32_t* err_dev, void* stream);
 
+/* Narrow packing of u8 frames whose large counts are rare: every count v is
+ * split as lo + r, lo = min(v, 7) (elem_kind G2_KIND_E2M1) or min(v, 16)
+ * (G2_KIND_E4M3) going to the operand and r > 0 to the residual list of the count's 64-column sector (column / 64):
+ * res_list_dev[sector * res_cap + k] = {frame0 + frame, column % 64 | r << 8}
+ * (two uint32, 8-byte aligned), res_count_dev[sector] entries (caller zeroes;
+ * above res_cap the entry is dropped and G2_DEVERR_RESIDUAL set).  frame0 is
+ * the number of the first frame in the stack, so a stack may be packed in
+ * pieces.  Units: g2_pack_e4m3_units' for G2_KIND_E4M3; for G2_KIND_E2M1
+ * {class << 30 | destination, ...} with class 1 = 16 bytes from two runs of 16
+ * source bytes (word 1: src0 | src1 << 16), 2 = 4 bytes from two runs of 4, 3 =
+ * 4 bytes from 8 sources of 12 bits in words 1-3 (0xFFF: none), 0 = none; the
+ * 8 columns of a word hold counts 0 2 of the first four (run), 0 2 of the
+ * second, 1 3 of the first, 1 3 of the second.  Every
+ * packed byte belongs to one unit.  Replaces the gather of dense.py:48-50. */
+int g2_pack_u8_residual(const void* frames_dev, int64_t nframes, int64_t npix, int64_t frame0, int32_t elem_kind,
+                        const int32_t* unit_block_off_dev, const uint32_t* units_dev, const uint32_t* spans_dev,
+                        int64_t n_chunks, void* packed_dev, int64_t packed_rows, int64_t packed_cols, uint32_t* res_count_dev,
+                        void* res_list_dev, int32_t res_cap, int32_t* err_dev, void* stream);
+
+/* Adds to out_dev[0] / out_dev[1] the number of binned counts (col_src >= 0)
+ * of n_sample evenly spread frames that an e2m1 / e4m3 operand needs a
+ * residual for.  No reference counterpart. */
+int g2_count_tail(const void* frames_dev, int64_t nframes, int64_t npix, const int32_t* col_src_dev, int64_t n_cols,
+                  int64_t n_sample, uint32_t* out_dev, void* stream);
+
+/* From the sums of u u' and u of an e2m1 Gram to those of its low counts (u + 3
+ * in each of bin b's npix_dev[b] pixels), in place; scratch_dev: n_bins *
+ * (nframes + 1) int64.  Before g2_residual_sums. */
+int g2_e2m1_offset(uint64_t* numer_dev, uint64_t* sums_dev, int32_t n_bins, int64_t nframes,
+                   const int64_t* npix_dev, uint64_t* scratch_dev, void* stream);
+
+/* Adds the terms of a narrow operand's N and S that its Gram does not hold:
+ * r lo', lo r' and r r' of every residual to numer_dev[bin * nframes + lag], r
+ * to sums_dev[bin * nframes + frame] (sector_bin_dev: bin of every sector), and
+ * the number of residuals to total_dev.  Exact in int64. */
+int g2_residual_sums(const void* packed_dev, int64_t packed_rows, int64_t nframes, int64_t packed_cols, int32_t elem_kind,
+                     const uint32_t* res_count_dev, const void* res_list_dev, int32_t res_cap,
+                     const int32_t* sector_bin_dev, int32_t n_bins, uint64_t* numer_dev, uint64_t* sums_dev,
+                     uint32_t* total_dev, int32_t* err_dev, void* stream);
+
+/* A wider, row-major operand with the residuals back in place, same column
+ * order: nrows rows (the frames and the row of ones) of packed_cols elements,
+ * e2m1 to e4m3 or 16-bit, e4m3 to e4m3 or 16-bit counts (a count above 16 in an e4m3 result
+ * sets G2_DEVERR_RANGE). */
+int g2_operand_expand(const void* packed_dev, int64_t nrows, int64_t nframes, int64_t packed_cols, int32_t elem_kind,
+                      int32_t out_kind, const uint32_t* res_count_dev, const void* res_list_dev, int32_t res_cap,
+                      void* out_dev, int32_t* err_dev, void* stream);
+
 /* Largest count over the binned pixels (col_src >= 0): picks split 0/1.
  * No reference counterpart (the reference never checks its dtype range). */
 int g2_binned_max(const void* frames_dev, int32_t elem_bytes, int64_t nframes, int64_t npix,
@@ -238,9 +296,22 @@ int g2_gram_tc_wide(const g2_job* jobs, int32_t n_jobs, const g2_gram_item* item
                     uint64_t* numer_dev, int64_t numer_len, uint64_t* sums_dev, int64_t sums_len,
                     int32_t* err_dev, int32_t grid, void* stream);
 
+/* The same Gram on CTA pairs for e2m1 operands (every job's elem_kind
+ * G2_KIND_E2M1, K-blocked rows of packed_cols / 2 bytes): rows [i0, i0+256)
+ * against rows [j0, j0+224), kind::mxf4 with unit block scales, twice the
+ * e4m3 MMA rate.  k_len, a_k0 and b_k0 are multiples of 256 columns, and a
+ * chunk of at most 524,288 columns keeps every lag sum of a block within int32
+ * (4^2 per column).  numer_dev and sums_dev get the sums of u u' and of u
+ * (int64, two's complement; the row of ones holds u = 1, code 1); g2_e2m1_offset
+ * turns them into those of the counts. */
+int g2_gram_tc_e2m1(const g2_job* jobs, int32_t n_jobs, const g2_gram_item* items_dev, int64_t n_items,
+                    uint64_t* numer_dev, int64_t numer_len, uint64_t* sums_dev, int64_t sums_len,
+                    int32_t* err_dev, int32_t grid, void* stream);
+
 /* Number of persistent workers W a Gram launch with grid <= 0 uses on the
  * current device: CTAs for g2_gram_tc (pair = 0), CTA pairs resident at once
- * for g2_gram_tc_pair (pair = 1) or g2_gram_tc_wide (pair = 2).  No reference counterpart (the reference's
+ * for g2_gram_tc_pair (pair = 1), g2_gram_tc_wide (pair = 2) or
+ * g2_gram_tc_e2m1 (pair = 3).  No reference counterpart (the reference's
  * work-group shapes are fixed, dense.py:184-188). */
 int g2_gram_workers(int32_t pair, int32_t* workers);
 
