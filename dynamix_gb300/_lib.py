@@ -29,7 +29,7 @@ MAX_JOBS = 32
 ITEM_EMPTY = -1
 KIND_FP16, KIND_E4M3, KIND_E2M1 = 0, 1, 2
 KIND_BLOCKED = 256
-E2M1_CHUNK = 4080
+NARROW_CHUNK = 4080
 RES_SECTOR = 64  # packed columns per residual list
 
 # numpy mirror of g2_gram_item (48 bytes, 8-byte aligned)
@@ -102,6 +102,8 @@ SIGNATURES = {
     "g2_stream_compact": (C.c_int, [_p, _p, _p, _i32, _i64, _i32, _p, _i64, _p, _p, _p, _p]),
     "g2_denominator": (C.c_int, [_p, _i32, _i64, _p, _p]),
     "g2_finalize": (C.c_int, [_p, _p, _p, _i32, _i64, _p, _p, _p]),
+    "g2_ntt_scratch": (_i64, [_i32, _i64]),
+    "g2_normalize_ntt": (C.c_int, [_p, _p, _p, _i32, _i64, _p, _p, _i64, _p, _p, _p, _p]),
     "g2_normalize_static": (C.c_int, [_p, _p, _p, _i32, _i64, _p, _p, _p]),
 }
 STATIC_DENOM_MAX = 1 << 19

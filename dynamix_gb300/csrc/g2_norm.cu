@@ -24,6 +24,7 @@ constexpr int THR = 256;
 constexpr int LPT = 4;               // lags per thread, strided by THR
 constexpr int LAGS = THR * LPT;      // lags per block
 constexpr int WIN = 1024;            // frames per shared window
+constexpr int WIN_SHORT = 128;       // the same for launches of few blocks
 
 // S values are split into 32-bit halves in shared memory.  A window whose
 // largest value m is below 2^16 accumulates in 32 bits, added to the 64-bit
@@ -35,10 +36,11 @@ constexpr int WIN = 1024;            // frames per shared window
 // Padded index of the shifted window: one pad word per 32, so lanes 4 words
 // apart (a thread's 4 consecutive lags) fall on distinct banks.
 __device__ __forceinline__ int pad32(int x) { return x + (x >> 5); }
-constexpr int WIN2_PAD = WIN + LAGS + (WIN + LAGS) / 32;
 
+template <int WIN>
 __global__ void __launch_bounds__(THR)
     denom_kernel(const long long* __restrict__ S, int64_t T, long long* __restrict__ D) {
+  constexpr int WIN2_PAD = WIN + LAGS + (WIN + LAGS) / 32;
   __shared__ uint32_t lo1[WIN], hi1[WIN];
   __shared__ uint32_t lo2[WIN2_PAD], hi2[WIN2_PAD];
   __shared__ uint32_t s_wmax[THR / 32];
@@ -142,13 +144,19 @@ inline int launch_denominator(const long long* S, int32_t n_rows, int64_t T, lon
   if (gx > 0x7fffffff) return G2_ERR_TOO_LARGE;
   const int sms = sm_count_current();
   if (sms <= 0) return G2_ERR_CUDA;
-  const int64_t windows = (T + WIN - 1) / WIN;
+  // windows of 128 frames where those of 1024 make fewer than two blocks per
+  // SM: such a launch takes as long as one block, and a block's time is its
+  // window's (1,000 frames x 8 rows: 25 -> 14 us with g2_finalize)
+  const bool small = gx * n_rows * ((T + WIN - 1) / WIN) < 2 * sms;
+  const int64_t win = small ? WIN_SHORT : WIN;
+  const int64_t windows = (T + win - 1) / win;
   int64_t z = (32ll * sms + gx * n_rows - 1) / (gx * n_rows);
-  z = z < 1 ? 1 : (z > windows ? windows : (z > 32 ? 32 : z));
+  z = z < 1 ? 1 : (z > windows ? windows : (z > 32 && !small ? 32 : z));
   if (z > 1 && cudaMemsetAsync(D, 0, static_cast<size_t>(n_rows) * T * sizeof(long long), st) != cudaSuccess)
     return G2_ERR_CUDA;
   dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(n_rows), static_cast<unsigned>(z));
-  denom_kernel<<<grid, THR, 0, st>>>(S, T, D);
+  if (small) denom_kernel<WIN_SHORT><<<grid, THR, 0, st>>>(S, T, D);
+  else denom_kernel<WIN><<<grid, THR, 0, st>>>(S, T, D);
   return launch_status();
 }
 
@@ -322,7 +330,7 @@ extern "C" int g2_normalize_static(const int64_t* numer_dev, const int64_t* sums
   if (sms <= 0) return G2_ERR_CUDA;
   const int64_t gx = (nframes + norm::LAGS - 1) / norm::LAGS;
   dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(n_rows));
-  norm::denom_kernel<<<grid, norm::THR, 0, as_stream(stream)>>>(reinterpret_cast<const long long*>(sums_dev),
+  norm::denom_kernel<norm::WIN><<<grid, norm::THR, 0, as_stream(stream)>>>(reinterpret_cast<const long long*>(sums_dev),
                                                                  nframes, denom);
   const int64_t total = static_cast<int64_t>(n_rows) * nframes;
   int64_t blocks = (total + 255) / 256;

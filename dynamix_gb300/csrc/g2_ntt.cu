@@ -1,0 +1,212 @@
+// G3 and G4 by number-theoretic transforms: the exact denominator
+// D[r][tau] = sum_t S[r][t] S[r][t + tau] of every row (job, bin) and
+// g2 = scale N / D, in O(T log T) instead of the T^2 / 2 multiply-adds of
+// g2_denominator.
+//
+// The autocorrelation is a cyclic convolution modulo the prime
+// p = 2^64 - 2^32 + 1, whose multiplicative group has elements of order 4096
+// (7 generates the group); D < 2^63 < p, so the result modulo p is D itself,
+// whatever the sums.  Transforms have N = 4096 points in shared memory, radix
+// 4, decimation in frequency forward (natural to bit-reversed order) and in
+// time backward, so no reordering pass.  A row is cut into blocks of B = 2048
+// frames, x_I.  transform_kernel writes the spectrum F_I of every block
+// (zero-padded to N = 2 B).  The lags [d B, (d + 1) B) are c_d(tau) +
+// c_{d+1}(tau - B), c_d the correlation of blocks d apart; the shift by B = N / 2
+// is a factor (-1)^k of the spectrum, so lag_kernel needs one backward transform
+// per (row, d) of sum_I F_I(-k) F_{I+d}(k) + (-1)^k sum_I F_I(-k) F_{I+d+1}(k).
+// Bound by the integer instructions of one CTA (about 180 per radix-4 butterfly,
+// 15 us per transform), so it pays for long rows or many: 20,000 frames x 32 rows
+// 719 -> 114 us, 10,000 x 16 116 -> 56 us, 3,000 x 32 39 -> 43 us; the caller's rule
+// is rows * T^2 >= 3e8.
+// Replaces the same reference code as g2_denominator and g2_finalize
+// (densecorrelator.cl:156-176, evtcorrelator.cl:70-75, dense.py:55-64).
+#include "g2_ptx.cuh"
+#include "g2_host.h"
+
+namespace g2 {
+namespace ntt {
+
+using u64 = unsigned long long;
+constexpr u64 PRIME = 0xFFFFFFFF00000001ull;
+constexpr u64 EPS = 0xFFFFFFFFull;  // 2^64 mod p
+constexpr int LOG_MAX = 12;
+constexpr int N_MAX = 1 << LOG_MAX;
+constexpr int BLOCK = N_MAX / 2;    // frames per block of a long row
+constexpr int THREADS = 1024;       // one radix-4 butterfly of a full transform each
+constexpr int SMEM_BYTES = 2 * N_MAX * 8;  // the points and the roots
+
+// Arithmetic modulo p on canonical values (< p).
+__device__ __forceinline__ u64 add(u64 a, u64 b) {
+  u64 s = a + b;
+  if (s < a) s += EPS;
+  return s >= PRIME ? s - PRIME : s;
+}
+__device__ __forceinline__ u64 sub(u64 a, u64 b) {
+  const u64 d = a - b;
+  return a < b ? d + PRIME : d;
+}
+// hi 2^64 + lo with 2^64 = 2^32 - 1 and 2^96 = -1 (mod p)
+__device__ __forceinline__ u64 mul(u64 a, u64 b) {
+  const u64 lo = a * b, hi = __umul64hi(a, b);
+  const u64 hh = hi >> 32, hl = hi & EPS;
+  u64 x = lo - hh;
+  if (lo < hh) x -= EPS;
+  const u64 y = (hl << 32) - hl;
+  u64 r = x + y;
+  if (r < x) r += EPS;
+  return r >= PRIME ? r - PRIME : r;
+}
+// times 2^48, a square root of -1
+__device__ __forceinline__ u64 mul_i(u64 a) { return mul(a, 1ull << 48); }
+
+__device__ __forceinline__ uint32_t brev(uint32_t i) { return __brev(i) >> (32 - LOG_MAX); }
+
+// The points, and the powers of the 4096th root w = 7^((p - 1) / 4096), roots[j] =
+// w^j, copied to shared memory (three reads per butterfly; from global memory a
+// transform of 4096 points took 17 us with 512 threads, from here 15 with 1024).
+__device__ __forceinline__ u64* points(const u64* __restrict__ roots_dev, u64*& roots) {
+  extern __shared__ __align__(16) u64 smem[];
+  roots = smem + N_MAX;
+  for (int i = threadIdx.x; i < N_MAX / 2; i += THREADS)
+    reinterpret_cast<ulonglong2*>(roots)[i] = reinterpret_cast<const ulonglong2*>(roots_dev)[i];
+  return smem;
+}
+
+// Forward: X(k) = sum x(t) w_N^(t k), natural to bit-reversed order.
+__device__ __forceinline__ void forward(u64* s, const u64* roots) {
+  for (int log_len = LOG_MAX; log_len >= 2; log_len -= 2) {  // blocks of len = 4 q
+    const int q = 1 << (log_len - 2), step = N_MAX >> log_len;
+    for (int i = threadIdx.x; i < N_MAX / 4; i += THREADS) {
+      const int j = i & (q - 1);
+      u64* x = s + ((i - j) << 2) + j;
+      const u64 x0 = x[0], x1 = x[q], x2 = x[2 * q], x3 = x[3 * q];
+      const u64 a = add(x0, x2), b = sub(x0, x2), c = add(x1, x3), d = mul_i(sub(x1, x3));
+      x[0] = add(a, c);
+      x[q] = mul(sub(a, c), roots[2 * j * step]);
+      x[2 * q] = mul(add(b, d), roots[j * step]);
+      x[3 * q] = mul(sub(b, d), roots[3 * j * step]);
+    }
+    __syncthreads();
+  }
+}
+
+// Backward, times N: x(t) = sum X(k) w_N^(-t k), bit-reversed to natural order.
+__device__ __forceinline__ void backward(u64* s, const u64* roots) {
+  for (int log_len = 2; log_len <= LOG_MAX; log_len += 2) {
+    const int q = 1 << (log_len - 2), step = N_MAX >> log_len;
+    for (int i = threadIdx.x; i < N_MAX / 4; i += THREADS) {
+      const int j = i & (q - 1);
+      u64* x = s + ((i - j) << 2) + j;
+      // the inverse twiddles w^-m = roots[(4096 - m) mod 4096]
+      const u64 y0 = x[0], y1 = mul(x[q], roots[(N_MAX - 2 * j * step) & (N_MAX - 1)]),
+                y2 = mul(x[2 * q], roots[(N_MAX - j * step) & (N_MAX - 1)]),
+                y3 = mul(x[3 * q], roots[(N_MAX - 3 * j * step) & (N_MAX - 1)]);
+      const u64 a = add(y0, y1), b = sub(y0, y1), c = add(y2, y3), d = mul_i(sub(y3, y2));  // -i (y2 - y3)
+      x[0] = add(a, c);
+      x[q] = add(b, d);
+      x[2 * q] = sub(a, c);
+      x[3 * q] = sub(b, d);
+    }
+    __syncthreads();
+  }
+}
+
+// D of lags lag0 .. lag0 + count - 1 of row r (in s, times N; inv = 1 / N), and g2.
+__device__ __forceinline__ void finish(const u64* s, int64_t r, int64_t T, int64_t lag0, int64_t count,
+                                       u64 inv, const long long* __restrict__ numer,
+                                       const double* __restrict__ scale, long long* __restrict__ denom,
+                                       float* __restrict__ g2f, double* __restrict__ g2d) {
+  const double f = scale[r];
+  for (int64_t k = threadIdx.x; k < count; k += THREADS) {
+    const int64_t at = r * T + lag0 + k;
+    const long long D = static_cast<long long>(mul(s[k], inv));
+    denom[at] = D;
+    const double g = f * static_cast<double>(numer[at]) / static_cast<double>(D);
+    if (g2f) g2f[at] = static_cast<float>(g);
+    if (g2d) g2d[at] = g;
+  }
+}
+
+__global__ void __launch_bounds__(THREADS)
+    transform_kernel(const long long* __restrict__ sums, int64_t T, int n_blocks, const u64* __restrict__ roots_dev,
+                     u64* __restrict__ spectra) {
+  u64* roots;
+  u64* s = points(roots_dev, roots);
+  const int64_t r = blockIdx.x / n_blocks, b = blockIdx.x % n_blocks;
+  for (int i = threadIdx.x; i < N_MAX; i += THREADS) {
+    const int64_t t = b * BLOCK + i;
+    s[i] = i < BLOCK && t < T ? static_cast<u64>(sums[r * T + t]) : 0ull;
+  }
+  __syncthreads();
+  forward(s, roots);
+  u64* out = spectra + static_cast<int64_t>(blockIdx.x) * N_MAX;
+  for (int i = threadIdx.x; i < N_MAX; i += THREADS) out[i] = s[i];
+}
+
+__global__ void __launch_bounds__(THREADS)
+    lag_kernel(const u64* __restrict__ spectra, int64_t T, int n_blocks, const u64* __restrict__ roots_dev,
+               const long long* __restrict__ numer, const double* __restrict__ scale, long long* __restrict__ denom,
+               float* __restrict__ g2f, double* __restrict__ g2d) {
+  u64* roots;
+  u64* s = points(roots_dev, roots);
+  // the first lags sum the most block pairs: d varies slowest
+  const int64_t rows = gridDim.x / n_blocks, r = blockIdx.x % rows;
+  const int d = static_cast<int>(blockIdx.x / rows);
+  const u64* F = spectra + r * n_blocks * N_MAX;
+  for (int i = threadIdx.x; i < N_MAX; i += THREADS) {
+    const int m = static_cast<int>(brev((N_MAX - brev(i)) & (N_MAX - 1)));
+    u64 near = 0, far = 0;
+    u64 ahead = F[static_cast<int64_t>(d) * N_MAX + i];  // F_{I + d}(k)
+    for (int b = 0; b + d < n_blocks; ++b) {
+      const u64 x = F[static_cast<int64_t>(b) * N_MAX + m];
+      near = add(near, mul(x, ahead));
+      if (b + d + 1 < n_blocks) {
+        ahead = F[static_cast<int64_t>(b + d + 1) * N_MAX + i];
+        far = add(far, mul(x, ahead));
+      }
+    }
+    s[i] = i >= N_MAX / 2 ? sub(near, far) : add(near, far);  // position i holds k = brev(i): odd in the upper half
+  }
+  __syncthreads();
+  backward(s, roots);
+  const int64_t lag0 = static_cast<int64_t>(d) * BLOCK;
+  finish(s, r, T, lag0, T - lag0 < BLOCK ? T - lag0 : BLOCK, roots_dev[N_MAX], numer, scale, denom, g2f, g2d);
+}
+
+}  // namespace ntt
+}  // namespace g2
+
+extern "C" int64_t g2_ntt_scratch(int32_t n_rows, int64_t nframes) {
+  using namespace g2::ntt;
+  if (n_rows <= 0 || nframes <= 0) return 0;
+  return n_rows * ((nframes + BLOCK - 1) / BLOCK) * N_MAX;
+}
+
+extern "C" int g2_normalize_ntt(const int64_t* numer_dev, const int64_t* sums_dev, const double* scale_dev,
+                                int32_t n_rows, int64_t nframes, const uint64_t* roots_dev, uint64_t* scratch_dev,
+                                int64_t scratch_len, int64_t* denom_dev, float* g2_f32_dev, double* g2_f64_dev,
+                                void* stream) {
+  using namespace g2;
+  if (!numer_dev || !sums_dev || !scale_dev || !roots_dev || !aligned(roots_dev, 16) || !denom_dev || n_rows <= 0 || nframes <= 0 ||
+      nframes >= (1ll << 31))
+    return G2_ERR_ARG;
+  const int64_t need = g2_ntt_scratch(n_rows, nframes);
+  if (!scratch_dev || scratch_len < need) return G2_ERR_ARG;
+  auto* S = reinterpret_cast<const long long*>(sums_dev);
+  auto* N = reinterpret_cast<const long long*>(numer_dev);
+  auto* D = reinterpret_cast<long long*>(denom_dev);
+  auto* R = reinterpret_cast<const unsigned long long*>(roots_dev);
+  cudaStream_t st = as_stream(stream);
+  for (const void* k : {reinterpret_cast<const void*>(ntt::transform_kernel),
+                        reinterpret_cast<const void*>(ntt::lag_kernel)})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ntt::SMEM_BYTES) != cudaSuccess)
+      return G2_ERR_CUDA;
+  const int64_t nb = (nframes + ntt::BLOCK - 1) / ntt::BLOCK;
+  if (nb * n_rows > 0x7fffffff) return G2_ERR_TOO_LARGE;
+  auto* F = reinterpret_cast<unsigned long long*>(scratch_dev);
+  const unsigned grid = static_cast<unsigned>(nb * n_rows);
+  ntt::transform_kernel<<<grid, ntt::THREADS, ntt::SMEM_BYTES, st>>>(S, nframes, static_cast<int>(nb), R, F);
+  ntt::lag_kernel<<<grid, ntt::THREADS, ntt::SMEM_BYTES, st>>>(F, nframes, static_cast<int>(nb), R, N, scale_dev, D, g2_f32_dev,
+                                                 g2_f64_dev);
+  return launch_status();
+}

@@ -14,13 +14,12 @@
 // caller packs the stack into a wider element.
 //
 // pack_walk_kernel moves the bytes by work units, 32 units of one class per
-// block of a source chunk, a warp per block:
-//  * e2m1: the packed order inside a bin is free (every Gram entry sums over
-//    the bin), so the layout is built from the pack's own units: 16 bytes from
-//    two 16-pixel runs, 4 bytes from two 4-pixel runs, 4 bytes from 8 gathered
-//    pixels.  Eight counts become eight codes in five instructions (code8).
-//    No byte is shared between chunks and no unit is a single byte.
-//  * e4m3: the units of the e4m3 layout (g2_pack_e4m3_units).
+// block of a source chunk, a warp per block.  The packed order inside a bin is
+// free (every Gram entry sums over the bin), so the layout is built from the
+// pack's own units: e2m1 16 bytes from two 16-pixel runs, 4 bytes from two
+// 4-pixel runs, 4 bytes from 8 gathered pixels (e4m3: one run, four pixels).
+// No byte is shared between chunks and no unit is a single byte.  Eight counts
+// become eight e2m1 codes in five instructions (code8).
 // Counts that may need a residual (a byte of 8 or more, or of 16 or
 // more) are found by one OR over the unit's words and take a slow path.
 #include "g2_ptx.cuh"
@@ -29,21 +28,23 @@
 namespace g2 {
 namespace tail {
 
-// Pixels per source chunk, frames per step and bytes of one staged frame row
-// (the chunk from its 16-byte aligned start, and spare words for reads past it).
+constexpr int CH = G2_NARROW_CHUNK;     // source pixels per chunk
+constexpr int F = 4;                    // frames per step
+constexpr int ROW = CH + 48;            // bytes of a staged frame row: the chunk from its 16-byte aligned start, spare words
+static_assert(ROW % 16 == 0 && CH % 16 == 0 && CH <= 0xFFF, "bulk copy rows, 12-bit sources");
+// Warps, ring stages and CTAs per SM: few CTAs, so that a mover's step of F
+// frames stays in registers (80 per thread).  3,000 frames of 514 x 1030, e2m1:
+// 0.54 ms with 5 CTAs of 256 threads and 2 stages (48 registers, spills), 0.43
+// with 3 and 3 stages; 512 x 512 x 3,001, e4m3 (twice the blocks per chunk): 0.37
+// and 0.37, 0.33 with 3 CTAs of 384 threads and 2 stages.
 template <bool E2M1>
 struct Cfg {
-  static constexpr int CH = E2M1 ? G2_E2M1_CHUNK : G2_PACK_CHUNK;
-  static constexpr int F = E2M1 ? 4 : 8;
-  static constexpr int ROW = CH + 48;
-  static_assert(ROW % 16 == 0 && CH % 16 == 0 && CH <= 0xFFF, "bulk copy rows, 12-bit sources");
+  static constexpr int THREADS = E2M1 ? 256 : 384;
+  static constexpr int MOVERS = THREADS / 32 - 1;
+  static constexpr int STAGES = E2M1 ? 3 : 2;
+  static constexpr int CTAS_PER_SM = 3;
 };
-constexpr int THREADS = 256;
-constexpr int MOVERS = THREADS / 32 - 1;
-constexpr int STAGES = 2;
-constexpr int CTAS_PER_SM = 5;
-constexpr uint32_t UNIT_VEC = 1, UNIT_WORD = 2, UNIT_GATHER = 3, UNIT_BYTE = 4;
-constexpr uint32_t NO_SRC = 0xFFF;
+constexpr uint32_t UNIT_VEC = 1, UNIT_WORD = 2, UNIT_GATHER = 3;
 constexpr int SECTOR = 64;                            // packed columns per residual list
 
 struct Residuals {
@@ -143,20 +144,19 @@ __device__ __forceinline__ uint32_t load4(const uint8_t* base, uint32_t o) {
 __device__ __forceinline__ void move_e2m1(const uint4& u, const uint8_t* base, uint32_t phase, uint32_t step,
                                           uint8_t* out, int64_t pitch, uint32_t row_bytes, int nf, uint32_t t,
                                           const Residuals& res, int32_t* err, bool& bad) {
-  using C = Cfg<true>;
   constexpr uint32_t hb = high_bits<true>();
   const uint32_t cls = u.x >> 30, dst = u.x & 0x3FFFFFFFu;
   const uint32_t sa = u.y & 0xFFFFu, sb = u.y >> 16;
   if (cls == UNIT_VEC) {
-    if (dst >= row_bytes / 16 || sa > C::CH - 16 || sb > C::CH - 16) {
+    if (dst >= row_bytes / 16 || sa > CH - 16 || sb > CH - 16) {
       bad = true;
       return;
     }
     uint8_t* o = out + blk_off(16 * dst, 0, pitch);
 #pragma unroll
-    for (int f = 0; f < C::F; ++f) {
+    for (int f = 0; f < F; ++f) {
       if (f >= nf) break;
-      const uint32_t d = ((phase + f * step) & 15u) + f * C::ROW;
+      const uint32_t d = ((phase + f * step) & 15u) + f * ROW;
       uint4 a = load16(base, d + sa);
       uint4 b = load16(base, d + sb);
       if ((a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) & hb) {
@@ -167,15 +167,15 @@ __device__ __forceinline__ void move_e2m1(const uint4& u, const uint8_t* base, u
           make_uint4(code8(a.x, b.x), code8(a.y, b.y), code8(a.z, b.z), code8(a.w, b.w));
     }
   } else if (cls == UNIT_WORD) {
-    if (dst >= row_bytes / 4 || sa > C::CH - 4 || sb > C::CH - 4) {
+    if (dst >= row_bytes / 4 || sa > CH - 4 || sb > CH - 4) {
       bad = true;
       return;
     }
     uint8_t* o = out + blk_off(4 * dst, 0, pitch);
 #pragma unroll
-    for (int f = 0; f < C::F; ++f) {
+    for (int f = 0; f < F; ++f) {
       if (f >= nf) break;
-      const uint32_t d = ((phase + f * step) & 15u) + f * C::ROW;
+      const uint32_t d = ((phase + f * step) & 15u) + f * ROW;
       uint32_t a = load4(base, d + sa), b = load4(base, d + sb);
       if ((a | b) & hb) {
         if (a & hb) a = encode_word<true>(a, 8 * dst, t + f, res, err);
@@ -192,14 +192,14 @@ __device__ __forceinline__ void move_e2m1(const uint4& u, const uint8_t* base, u
                            (u.z >> 16) & 0xFFFu, (u.z >> 28) | ((u.w & 0xFFu) << 4), (u.w >> 8) & 0xFFFu, u.w >> 20};
     uint8_t* o = out + blk_off(4 * dst, 0, pitch);
 #pragma unroll
-    for (int f = 0; f < C::F; ++f) {
+    for (int f = 0; f < F; ++f) {
       if (f >= nf) break;
-      const uint8_t* q = base + ((phase + f * step) & 15u) + f * C::ROW;
+      const uint8_t* q = base + ((phase + f * step) & 15u) + f * ROW;
       uint32_t a = 0, b = 0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {  // 12-bit sources below CH, or NO_SRC: a column of padding (count 3, u = 0)
-        a |= (s[j] < C::CH ? static_cast<uint32_t>(q[s[j]]) : 3u) << (8 * j);
-        b |= (s[4 + j] < C::CH ? static_cast<uint32_t>(q[s[4 + j]]) : 3u) << (8 * j);
+        a |= (s[j] < CH ? static_cast<uint32_t>(q[s[j]]) : 3u) << (8 * j);
+        b |= (s[4 + j] < CH ? static_cast<uint32_t>(q[s[4 + j]]) : 3u) << (8 * j);
       }
       if ((a | b) & hb) {
         if (a & hb) a = encode_word<true>(a, 8 * dst, t + f, res, err);
@@ -210,57 +210,47 @@ __device__ __forceinline__ void move_e2m1(const uint4& u, const uint8_t* base, u
   }
 }
 
-// One e4m3 unit: {destination, sources, sources, class}.
+// One e4m3 unit: one run per destination, four sources of 12 bits.
 __device__ __forceinline__ void move_e4m3(const uint4& u, const uint8_t* base, uint32_t phase, uint32_t step,
                                           uint8_t* out, int64_t pitch, uint32_t row_bytes, int nf, uint32_t t,
                                           const Residuals& res, int32_t* err, bool& bad) {
-  using C = Cfg<false>;
   constexpr uint32_t hb = high_bits<false>();
-  if (u.w == UNIT_VEC) {
-    if (u.x >= row_bytes / 16 || u.y > C::CH - 16) {
+  const uint32_t cls = u.x >> 30, dst = u.x & 0x3FFFFFFFu, sa = u.y & 0xFFFFu;
+  if (cls == UNIT_VEC) {
+    if (dst >= row_bytes / 16 || sa > CH - 16) {
       bad = true;
       return;
     }
-    uint8_t* o = out + blk_off(16 * u.x, 0, pitch);
+    uint8_t* o = out + blk_off(16 * dst, 0, pitch);
 #pragma unroll
-    for (int f = 0; f < C::F; ++f) {
+    for (int f = 0; f < F; ++f) {
       if (f >= nf) break;
-      uint4 v = load16(base, ((phase + f * step) & 15u) + f * C::ROW + u.y);
-      if ((v.x | v.y | v.z | v.w) & hb) encode16<false>(v, 16 * u.x, 4, t + f, res, err);
+      uint4 v = load16(base, ((phase + f * step) & 15u) + f * ROW + sa);
+      if ((v.x | v.y | v.z | v.w) & hb) encode16<false>(v, 16 * dst, 4, t + f, res, err);
       *reinterpret_cast<uint4*>(o + f * 128) = v;
     }
-  } else if (u.w == UNIT_WORD || u.w == UNIT_GATHER) {
-    const uint32_t s0 = u.y & 0xFFFFu, s1 = u.y >> 16, s2 = u.z & 0xFFFFu, s3 = u.z >> 16;
-    const bool word = u.w == UNIT_WORD;
-    if (u.x >= row_bytes / 4 || (word && u.y > C::CH - 4) ||
-        (!word && (s0 >= C::CH || s1 >= C::CH || s2 >= C::CH || s3 >= C::CH))) {
+  } else if (cls == UNIT_WORD || cls == UNIT_GATHER) {
+    const bool word = cls == UNIT_WORD;
+    if (dst >= row_bytes / 4 || (word && sa > CH - 4)) {
       bad = true;
       return;
     }
-    uint8_t* o = out + blk_off(4 * u.x, 0, pitch);
+    const uint32_t s[4] = {u.y & 0xFFFu, (u.y >> 12) & 0xFFFu, (u.y >> 24) | ((u.z & 0xFu) << 8), (u.z >> 4) & 0xFFFu};
+    uint8_t* o = out + blk_off(4 * dst, 0, pitch);
 #pragma unroll
-    for (int f = 0; f < C::F; ++f) {
+    for (int f = 0; f < F; ++f) {
       if (f >= nf) break;
-      const uint32_t d = ((phase + f * step) & 15u) + f * C::ROW;
-      const uint8_t* q = base + d;
-      uint32_t v = word ? load4(base, d + u.y)
-                        : static_cast<uint32_t>(q[s0]) | (static_cast<uint32_t>(q[s1]) << 8) |
-                              (static_cast<uint32_t>(q[s2]) << 16) | (static_cast<uint32_t>(q[s3]) << 24);
-      if (v & hb) v = encode_word<false>(v, 4 * u.x, t + f, res, err);
+      const uint32_t d = ((phase + f * step) & 15u) + f * ROW;
+      uint32_t v = 0;
+      if (word) {
+        v = load4(base, d + sa);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)  // 12-bit sources: NO_SRC or below CH
+          if (s[j] < CH) v |= static_cast<uint32_t>(base[d + s[j]]) << (8 * j);
+      }
+      if (v & hb) v = encode_word<false>(v, 4 * dst, t + f, res, err);
       *reinterpret_cast<uint32_t*>(o + f * 128) = v;
-    }
-  } else if (u.w == UNIT_BYTE) {
-    if (u.x >= row_bytes || u.y >= C::CH) {
-      bad = true;
-      return;
-    }
-    uint8_t* o = out + blk_off(u.x, 0, pitch);
-#pragma unroll
-    for (int f = 0; f < C::F; ++f) {
-      if (f >= nf) break;
-      uint32_t v = base[((phase + f * step) & 15u) + f * C::ROW + u.y];
-      if (v & hb) v = encode_word<false>(v, u.x, t + f, res, err);
-      o[f * 128] = static_cast<uint8_t>(v);
     }
   }
 }
@@ -276,14 +266,15 @@ __device__ __forceinline__ void move_e4m3(const uint4& u, const uint8_t* base, u
 // 514 x 1030, DRAM read 7.05 GB of 5.29, written 3.02 GB of 1.95).
 // frame0: number of the launch's first frame in the stack.
 template <bool E2M1>
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
+__global__ void __launch_bounds__(Cfg<E2M1>::THREADS, Cfg<E2M1>::CTAS_PER_SM)
     pack_walk_kernel(const uint8_t* __restrict__ frames, int64_t T, int64_t npix, uint32_t frame0,
                      const int32_t* __restrict__ block_off, const uint4* __restrict__ units,
                      const uint32_t* __restrict__ spans, int32_t n_chunks, int32_t n_bands,
                      uint8_t* __restrict__ packed, int64_t pitch, uint32_t row_bytes, Residuals res,
                      int32_t* __restrict__ err) {
-  using C = Cfg<E2M1>;
-  __shared__ __align__(128) uint8_t s_buf[STAGES][C::F][C::ROW];
+  constexpr int MOVERS = Cfg<E2M1>::MOVERS, STAGES = Cfg<E2M1>::STAGES;
+  extern __shared__ __align__(128) uint8_t s_dyn[];
+  auto s_buf = reinterpret_cast<uint8_t(*)[F][ROW]>(s_dyn);
   __shared__ __align__(8) uint64_t full[STAGES];
   __shared__ __align__(8) uint64_t empty[STAGES];
   __shared__ int s_abort;
@@ -301,7 +292,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
   __syncthreads();
   volatile int* abort_flag = &s_abort;
   const int64_t total_bytes = T * npix;
-  const int64_t n_items = (T + C::F - 1) / C::F * n_bands;
+  const int64_t n_items = (T + F - 1) / F * n_bands;
   uint32_t k = 0;  // staged chunks so far
 
   if (warp == 0) {
@@ -313,8 +304,8 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
         const int band = static_cast<int>(item - g * n_bands);
         const int c0 = static_cast<int>(static_cast<int64_t>(n_chunks) * band / n_bands);
         const int c1 = static_cast<int>(static_cast<int64_t>(n_chunks) * (band + 1) / n_bands);
-        const int64_t t0 = g * C::F;
-        const int nf = static_cast<int>(T - t0 < C::F ? T - t0 : C::F);
+        const int64_t t0 = g * F;
+        const int nf = static_cast<int>(T - t0 < F ? T - t0 : F);
         for (int c = c0; c < c1; ++c) {
           if (block_off[c] == block_off[c + 1]) continue;  // no packed byte comes from this chunk
           const uint32_t span = spans[c];                    // binned pixels [lo, hi) of the chunk
@@ -323,13 +314,13 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
             ok = false;
             break;
           }
-          const int64_t p0 = static_cast<int64_t>(c) * C::CH;
+          const int64_t p0 = static_cast<int64_t>(c) * CH;
           // two passes: the byte count of the stage, then the copies
           uint32_t bytes = 0;
 #pragma unroll
           for (int pass = 0; pass < 2; ++pass) {
 #pragma unroll
-            for (int f = 0; f < C::F; ++f) {
+            for (int f = 0; f < F; ++f) {
               if (f >= nf) break;
               const int64_t start = (t0 + f) * npix + p0;
               const int64_t a = (start + (span & 0xFFFFu)) & ~int64_t(15);
@@ -369,8 +360,8 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
     const int band = static_cast<int>(item - g * n_bands);
     const int c0 = static_cast<int>(static_cast<int64_t>(n_chunks) * band / n_bands);
     const int c1 = static_cast<int>(static_cast<int64_t>(n_chunks) * (band + 1) / n_bands);
-    const int64_t t0 = g * C::F;
-    const int nf = static_cast<int>(T - t0 < C::F ? T - t0 : C::F);
+    const int64_t t0 = g * F;
+    const int nf = static_cast<int>(T - t0 < F ? T - t0 : F);
     const uint32_t t = frame0 + static_cast<uint32_t>(t0);
     uint8_t* out = packed + static_cast<int64_t>(t) * 128;
     const uint32_t start = static_cast<uint32_t>(t0 * npix), step = static_cast<uint32_t>(npix);
@@ -389,7 +380,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
         break;
       }
       ++k;
-      const uint32_t phase = start + static_cast<uint32_t>(c) * C::CH;
+      const uint32_t phase = start + static_cast<uint32_t>(c) * CH;
       const uint8_t* base = &s_buf[s][0][0];
       while (j < b1) {
         const uint4 w = u;
@@ -742,7 +733,7 @@ extern "C" int g2_pack_u8_residual(const void* frames_dev, int64_t nframes, int6
       (elem_kind != G2_KIND_E2M1 && elem_kind != G2_KIND_E4M3))
     return G2_ERR_ARG;
   const bool e2m1 = elem_kind == G2_KIND_E2M1;
-  const int64_t ch = e2m1 ? G2_E2M1_CHUNK : G2_PACK_CHUNK;
+  constexpr int64_t ch = G2_NARROW_CHUNK;
   if (nframes <= 0 || npix <= 0 || frame0 < 0 || packed_rows < frame0 + nframes || packed_rows >= (1ll << 31) ||
       n_chunks != (npix + ch - 1) / ch || (e2m1 && packed_cols % 256 != 0))
     return G2_ERR_ARG;
@@ -751,26 +742,28 @@ extern "C" int g2_pack_u8_residual(const void* frames_dev, int64_t nframes, int6
   const int sms = sm_count_current();
   if (sms <= 0) return G2_ERR_CUDA;
   // bands: about eight work items per resident CTA, of at least four chunks
-  const int64_t ctas = static_cast<int64_t>(sms) * tail::CTAS_PER_SM;
-  const int F = e2m1 ? tail::Cfg<true>::F : tail::Cfg<false>::F;
-  const int64_t groups = (nframes + F - 1) / F;
+  const int64_t ctas = sms * static_cast<int64_t>(e2m1 ? tail::Cfg<true>::CTAS_PER_SM : tail::Cfg<false>::CTAS_PER_SM);
+  const int64_t groups = (nframes + tail::F - 1) / tail::F;
   int64_t bands = (8 * ctas + groups - 1) / groups;
   if (bands > (n_chunks + 3) / 4) bands = (n_chunks + 3) / 4;
   if (bands < 1) bands = 1;
   const unsigned grid = static_cast<unsigned>(groups * bands < ctas ? groups * bands : ctas);
-  auto* fr = reinterpret_cast<const uint8_t*>(frames_dev);
-  auto* un = reinterpret_cast<const uint4*>(units_dev);
-  auto* out = reinterpret_cast<uint8_t*>(packed_dev);
-  const uint32_t f0 = static_cast<uint32_t>(frame0);
-  const int32_t nc = static_cast<int32_t>(n_chunks), nb = static_cast<int32_t>(bands);
-  if (e2m1)
-    tail::pack_walk_kernel<true><<<grid, tail::THREADS, 0, as_stream(stream)>>>(
-        fr, nframes, npix, f0, unit_block_off_dev, un, spans_dev, nc, nb, out, packed_rows * 128,
-        static_cast<uint32_t>(packed_cols / 2), res, err_dev);
-  else
-    tail::pack_walk_kernel<false><<<grid, tail::THREADS, 0, as_stream(stream)>>>(
-        fr, nframes, npix, f0, unit_block_off_dev, un, spans_dev, nc, nb, out, packed_rows * 128,
-        static_cast<uint32_t>(packed_cols), res, err_dev);
+  const int32_t nb = static_cast<int32_t>(bands);
+#define G2_WALK_LAUNCH(E)                                                                                            \
+  do {                                                                                                               \
+    constexpr int smem = tail::Cfg<E>::STAGES * tail::F * tail::ROW;                                                 \
+    if (cudaFuncSetAttribute(tail::pack_walk_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=        \
+        cudaSuccess)                                                                                                 \
+      return G2_ERR_CUDA;                                                                                            \
+    tail::pack_walk_kernel<E><<<grid, tail::Cfg<E>::THREADS, smem, as_stream(stream)>>>(                             \
+        reinterpret_cast<const uint8_t*>(frames_dev), nframes, npix, static_cast<uint32_t>(frame0),                  \
+        unit_block_off_dev, reinterpret_cast<const uint4*>(units_dev), spans_dev, static_cast<int32_t>(n_chunks),    \
+        nb, reinterpret_cast<uint8_t*>(packed_dev), packed_rows * 128,                                               \
+        static_cast<uint32_t>(E ? packed_cols / 2 : packed_cols), res, err_dev);                                     \
+  } while (0)
+  if (e2m1) G2_WALK_LAUNCH(true);
+  else G2_WALK_LAUNCH(false);
+#undef G2_WALK_LAUNCH
   return launch_status();
 }
 

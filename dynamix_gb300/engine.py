@@ -25,7 +25,7 @@ import numpy as np
 from . import _lib
 from .plan import (E4M3_MAX_EXACT, EXACT_LIMIT, FP16_MAX_EXACT, MODE_BYTES, MODE_E2M1, MODE_E4M3, MODE_FP16,
                    TILE_SHAPES, NarrowLayout, PackLayout, balance_items, chunk_grams, column_window,
-                   e2m1_segment_bound, e4m3_segment_bound, gram_items, split_items)
+                   e2m1_segment_bound, e4m3_segment_bound, gram_items, item_costs, split_items)
 
 MODE_NAMES = {MODE_FP16: "fp16", MODE_BYTES: "bytes", MODE_E4M3: "e4m3", MODE_E2M1: "e2m1"}
 
@@ -103,23 +103,23 @@ def qmask_digest(qmask):
     return "%s:%s" % (q.shape, hashlib.blake2b(q.tobytes(), digest_size=16).hexdigest())
 
 
-def device_layout(qmask, n_bins, mode, dev, digest=None):
-    """The packing layout of a q-mask with its read-only tables on ``dev``,
-    shared process-wide (least recently used of 48 kept): building one costs
+def device_layout(qmask, n_bins, mode, dev, digest=None, narrow=False):
+    """The packing layout of a q-mask (``narrow``: the NarrowLayout of e2m1 or
+    e4m3) with its read-only tables on ``dev``, shared process-wide (least recently used of 48 kept): building one costs
     host time proportional to the frame size.  ``digest``: the q-mask's
     :func:`qmask_digest` when the caller has it."""
     torch = _torch()
     q = np.ascontiguousarray(qmask, dtype=np.int32)
-    key = (str(dev), digest or qmask_digest(q), int(n_bins), int(mode))
+    key = (str(dev), digest or qmask_digest(q), int(n_bins), int(mode), bool(narrow))
     with _LAYOUTS_LOCK:
         L = _LAYOUTS.get(key)
         if L is not None:
             _LAYOUTS.move_to_end(key)
             return L
     d = lambda a: torch.as_tensor(a, device=dev)
-    if mode == MODE_E2M1:
-        L = NarrowLayout(q, n_bins)
-        L.d_col_src, L.d_sector_bin = d(L.col_src), d(L.sector_bin)
+    if narrow:
+        L = NarrowLayout(q, n_bins, mode)
+        L.d_col_src, L.d_sector_bin, L.d_npix = d(L.col_src), d(L.sector_bin), d(L.npix)
         L.d_unit_block_off, L.d_units = d(L.unit_block_off), d(L.units.view(np.int32))
         L.d_chunk_span = d(L.chunk_span.view(np.int32))
         return _keep_layout(key, L)
@@ -137,8 +137,6 @@ def device_layout(qmask, n_bins, mode, dev, digest=None):
         L.d_word_src = d(L.word_src.view(np.int32))
         L.d_unit_block_off = d(L.unit_block_off)
         L.d_units = d(L.units.view(np.int32))
-        L.d_chunk_span = d(L.chunk_span.view(np.int32))
-        L.d_sector_bin = d(L.seg_bin) if L.n_segs else torch.full((2,), -1, dtype=torch.int32, device=dev)
     return _keep_layout(key, L)
 
 
@@ -148,6 +146,49 @@ def _keep_layout(key, L):
         while len(_LAYOUTS) > _LAYOUTS_MAX:
             _LAYOUTS.popitem(last=False)
     return L
+
+
+NTT_PRIME = 2 ** 64 - 2 ** 32 + 1
+_NTT_ROOTS = {}
+
+
+def ntt_roots(dev):
+    """The transform constants of ``g2_normalize_ntt`` on ``dev``."""
+    torch = _torch()
+    key = str(dev)
+    if key not in _NTT_ROOTS:
+        w, x, vals = pow(7, (NTT_PRIME - 1) // 4096, NTT_PRIME), 1, []
+        for _ in range(4096):
+            vals.append(x)
+            x = x * w % NTT_PRIME
+        vals.append(pow(4096, NTT_PRIME - 2, NTT_PRIME))
+        _NTT_ROOTS[key] = torch.from_numpy(np.array(vals, dtype=np.uint64).view(np.int64)).to(dev)
+    return _NTT_ROOTS[key]
+
+
+# rows * T^2 from which G3 runs by transforms: the direct kernel's multiply-adds
+# against about 45 us of transforms (3,000 frames x 32 rows: 39 against 43 us,
+# 5,000 x 32: 89 and 45, 10,000 x 8: 86 and 51, 20,000 x 32: 719 and 114)
+NTT_MIN_WORK = 3.0e8
+
+
+def normalise_rows(eng):
+    """G3 and G4 of an engine's rows (bins): ``eng.denom`` from ``eng.sums``,
+    ``eng.g2_f32`` / ``eng.g2_f64`` from them and ``eng.numer``, on the current
+    stream."""
+    lib, st = eng.lib, stream_handle(eng.dev)
+    if eng.n_bins * float(eng.T) ** 2 < NTT_MIN_WORK:
+        _lib.check(lib.g2_denominator(ptr(eng.sums), eng.n_bins, eng.T, ptr(eng.denom), st), "g2_denominator")
+        _lib.check(lib.g2_finalize(ptr(eng.numer), ptr(eng.denom), ptr(eng.scale), eng.n_bins, eng.T,
+                                   ptr(eng.g2_f32), ptr(eng.g2_f64), st), "g2_finalize")
+        return
+    n = int(lib.g2_ntt_scratch(eng.n_bins, eng.T))
+    buf = getattr(eng, "_ntt_buf", None)
+    if buf is None:
+        buf = eng._ntt_buf = _torch().empty(n, dtype=_torch().int64, device=eng.dev)
+    _lib.check(lib.g2_normalize_ntt(ptr(eng.numer), ptr(eng.sums), ptr(eng.scale), eng.n_bins, eng.T,
+                                    ptr(ntt_roots(eng.dev)), ptr(buf), n, ptr(eng.denom), ptr(eng.g2_f32),
+                                    ptr(eng.g2_f64), st), "g2_normalize_ntt")
 
 
 class DenseEngine:
@@ -306,21 +347,22 @@ class DenseEngine:
         None when the q-mask's binned columns span nearly the whole frame."""
         return column_window(self.qmask.reshape(self.shape), self.n_bins, self.CROP_MIN_SAVING)
 
-    def _crop_layout(self, mode):
+    def _crop_layout(self, mode, narrow=False):
         """The packing layout of the cropped frames (:meth:`_column_window`)."""
-        key = ("crop", mode)
+        key = ("crop", mode, narrow)
         if key not in self._layouts:
             c0, wc = self.crop
             q = np.ascontiguousarray(self.qmask.reshape(self.shape)[:, c0:c0 + wc])
-            self._layouts[key] = device_layout(q, self.n_bins, mode, self.dev)
+            self._layouts[key] = device_layout(q, self.n_bins, mode, self.dev, narrow=narrow)
         return self._layouts[key]
 
-    def _layout(self, mode):
-        if mode not in self._layouts:
+    def _layout(self, mode, narrow=False):
+        key = ("narrow", mode) if narrow else mode
+        if key not in self._layouts:
             if getattr(self, "_qdigest", None) is None:
                 self._qdigest = qmask_digest(self.qmask)
-            self._layouts[mode] = device_layout(self.qmask, self.n_bins, mode, self.dev, self._qdigest)
-        return self._layouts[mode]
+            self._layouts[key] = device_layout(self.qmask, self.n_bins, mode, self.dev, self._qdigest, narrow)
+        return self._layouts[key]
 
     def _piece_emax(self, L):
         """This engine's buffer of per-piece energy maxima for layout L (the
@@ -351,9 +393,9 @@ class DenseEngine:
         rows = self.T + (1 if ones else 0)
         nbytes = rows * L.packed_bytes_per_frame
         fresh = False
-        # e2m1 layouts of cropped and of whole frames have different column
+        # narrow layouts of cropped and of whole frames have different column
         # orders; narrow operands are K-blocked, the others row-major
-        layout = (narrow, L if L.mode == MODE_E2M1 else None)
+        layout = (narrow, L if narrow else None)
         if self.packed is None or self.packed.numel() < nbytes:
             self.packed = None
             self.packed = torch.zeros(nbytes, dtype=torch.uint8, device=self.dev)
@@ -448,7 +490,9 @@ class DenseEngine:
         e2m1 = L.mode == MODE_E2M1
         shape = (self.workers(e2m1), 256 if e2m1 else 128 if L.kind == _lib.KIND_E4M3 else 64,
                  "pair4" if e2m1 else self.item_kind, self.ones(L))
-        return balance_items(split_items(items, *shape), *shape)
+        cost = item_costs(items, *shape[1:])
+        parts = split_items(items, *shape, cost=cost)
+        return balance_items(parts, *shape, cost=cost if parts is items else None)
 
     pack_units = True         # u8 e4m3 packing by work units (g2_pack_e4m3_units)
 
@@ -522,13 +566,8 @@ class DenseEngine:
                       stream if isinstance(stream, C.c_void_p) else C.c_void_p(stream)), name)
 
     def normalise(self):
-        st = stream_handle(self.dev)
-        if self.n_bins == 0:
-            return
-        _lib.check(self.lib.g2_denominator(ptr(self.sums), self.n_bins, self.T, ptr(self.denom), st),
-                   "g2_denominator")
-        _lib.check(self.lib.g2_finalize(ptr(self.numer), ptr(self.denom), ptr(self.scale), self.n_bins, self.T,
-                                        ptr(self.g2_f32), ptr(self.g2_f64), st), "g2_finalize")
+        if self.n_bins:
+            normalise_rows(self)
 
     def check_error(self):
         code = int(self.err.item())
@@ -654,7 +693,7 @@ class DenseEngine:
         kind = "pair4" if L.mode == MODE_E2M1 else self.item_kind
         key = ("pipe", L.mode, self.T, self.exact_limit, self.grid, chunks, self.super_rows, self.kslab,
                kind, self.pipe_growth, int(taper), None if grams is None else tuple(grams),
-               tuple(L.grams()) if L.mode == MODE_E2M1 else None)
+               tuple(L.grams()))
         if key not in self._items_cache:
             torch = _torch()
             if grams is None:
@@ -750,7 +789,7 @@ class DenseEngine:
     def _binned_pixels(self):
         """Pixels in the bins (an element layout that exists anyway counts them)."""
         if getattr(self, "_n_binned", None) is None:
-            L = next(iter(self._layouts.values()), None) or self._layout(MODE_E2M1)
+            L = next(iter(self._layouts.values()), None) or self._layout(MODE_E2M1, True)
             self._n_binned = int(L.npix.sum())
         return self._n_binned
 
@@ -782,7 +821,7 @@ class DenseEngine:
                 for k, t in enumerate(pick):
                     src[k].copy_(frames[t], non_blocking=True)
             self.status.zero_()
-            self._count_tail(src.data_ptr(), T, self.npix, self._layout(MODE_E2M1), n, stream_handle(self.dev))
+            self._count_tail(src.data_ptr(), T, self.npix, self._layout(MODE_E2M1, True), n, stream_handle(self.dev))
             _, _, c4, c8 = self.status.tolist()
             self._narrow = self._pick_narrow(n * self._binned_pixels(), c4, c8)
             if self._narrow == MODE_FP16:
@@ -822,8 +861,8 @@ class DenseEngine:
         # u8 frames from host memory come in cropped to the q-mask's columns
         # (the pack then reads the cropped frames with the cropped layout)
         crop = host and mode in (MODE_E4M3, MODE_E2M1) and frames.element_size() == 1 and self.crop is not None
-        Lp = self._crop_layout(mode) if crop else self._layout(mode)
-        L = Lp if mode == MODE_E2M1 else self._layout(mode)
+        Lp = self._crop_layout(mode, narrow is not None) if crop else self._layout(mode, narrow is not None)
+        L = Lp if narrow is not None else self._layout(mode)
         packed = self._packed_buffer(L, narrow is not None)
         if mode != MODE_FP16:
             grams, bound = None, None
@@ -929,9 +968,8 @@ class DenseEngine:
             if mode == MODE_E2M1:
                 if getattr(self, "_offset_scratch", None) is None:
                     self._offset_scratch = torch.empty(self.n_bins * (self.T + 1), dtype=torch.int64, device=self.dev)
-                    self._npix_dev = torch.as_tensor(L.npix, device=self.dev)
                 _lib.check(self.lib.g2_e2m1_offset(ptr(self.numer), ptr(self.sums), self.n_bins, self.T,
-                                                   ptr(self._npix_dev), ptr(self._offset_scratch), st),
+                                                   ptr(L.d_npix), ptr(self._offset_scratch), st),
                            "g2_e2m1_offset")
             _lib.check(self.lib.g2_residual_sums(
                 ptr(packed), self.T + 1, self.T, L.packed_cols, L.kind, ptr(res[0]), ptr(res[1]), res[2],

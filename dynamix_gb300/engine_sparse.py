@@ -19,7 +19,7 @@ import ctypes as C
 import numpy as np
 
 from . import _lib
-from .engine import DeviceError, _torch, ptr, require_cuda, stream_handle
+from .engine import DeviceError, _torch, normalise_rows, ptr, require_cuda, stream_handle
 
 # shared memory of the shared-counter pair kernel besides its 2 x T counters:
 # 24 warps x 2 half-warp pixels x 2 staging buffers x 128 events x 4 bytes
@@ -382,10 +382,7 @@ class EventEngine:
                     ptr(ro), ptr(rb), n_ranges, ptr(cro), n_ctas, self.T, self.n_bins, mx, ptr(self.numer),
                     ptr(self.sums), ptr(self.err), st), "g2_event_pairsum")
         self._mark("pairsum")
-        _lib.check(self.lib.g2_denominator(ptr(self.sums), self.n_bins, self.T, ptr(self.denom), st),
-                   "g2_denominator")
-        _lib.check(self.lib.g2_finalize(ptr(self.numer), ptr(self.denom), ptr(self.scale), self.n_bins,
-                                        self.T, ptr(self.g2_f32), ptr(self.g2_f64), st), "g2_finalize")
+        normalise_rows(self)
         self._mark("normalize")
         self._host_refs = (vol_times, vol_data, offsets)  # alive until the copies have run
         self._times_checked = True
@@ -421,10 +418,7 @@ class EventEngine:
                 ptr(self.sums), ptr(self.err), st), "g2_event_pairsum")
         self._mark("pairsum")
         if self.n_bins:
-            _lib.check(self.lib.g2_denominator(ptr(self.sums), self.n_bins, self.T, ptr(self.denom), st),
-                       "g2_denominator")
-            _lib.check(self.lib.g2_finalize(ptr(self.numer), ptr(self.denom), ptr(self.scale), self.n_bins,
-                                            self.T, ptr(self.g2_f32), ptr(self.g2_f64), st), "g2_finalize")
+            normalise_rows(self)
         self._mark("normalize")
         self.last = {"n_events": n_ev, "max_count": mx, "kernel": "smem" if use_smem else "global",
                      "n_ranges": n_ranges, "n_ctas": n_ctas}

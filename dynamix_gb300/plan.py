@@ -21,7 +21,7 @@ from __future__ import annotations
 
 import numpy as np
 
-from ._lib import (BK, E2M1_CHUNK, ITEM_DTYPE, ITEM_EMPTY, KIND_E2M1, KIND_E4M3, KIND_FP16, PACK_CHUNK, PACK_MAX_PIECES, PACK_MAX_SLOTS,
+from ._lib import (BK, NARROW_CHUNK, ITEM_DTYPE, ITEM_EMPTY, KIND_E2M1, KIND_E4M3, KIND_FP16, PACK_CHUNK, PACK_MAX_PIECES, PACK_MAX_SLOTS,
                    PACK_WORDS_PER_CHUNK, PAD, PLAIN_BM, PLAIN_BN, RES_SECTOR, TC_BM, TC_BN)
 
 EXACT_LIMIT = 1 << 24   # fp32 represents every integer up to 2^24 exactly
@@ -30,7 +30,6 @@ E4M3_MAX_EXACT = 16     # e4m3 represents every integer up to 2^4 exactly
 SUPER_ROWS = 2048       # frames per side of a super-tile
 
 MODE_FP16, MODE_BYTES, MODE_E4M3, MODE_E2M1 = 0, 1, 2, 3
-E2M1_PAD = 256          # e2m1 columns of one 128-byte block
 E2M1_MAX_U = 4          # e2m1 codes hold u = count - 3, counts 0-7
 E2M1_WORD = np.array([0, 4, 1, 5, 2, 6, 3, 7])  # columns of counts a0..a3 b0..b3 in a word of 8
 UNIT_NONE, UNIT_VEC, UNIT_WORD, UNIT_GATHER, UNIT_BYTE = 0, 1, 2, 3, 4   # classes of the e4m3 pack's units
@@ -214,7 +213,6 @@ class PackLayout:
             nxt += nb
         self.unit_block_off = off.astype(np.int32)
         self.units = units.reshape(-1)
-        self.chunk_span = chunk_spans(pix, self.n_chunks, PACK_CHUNK)
 
     def segment_emax(self, piece_emax):
         """Per 64-column output segment, the sum over its pieces of the pieces'
@@ -275,27 +273,32 @@ def chunk_spans(pix, n_chunks, size):
 
 
 class NarrowLayout:
-    """Packed-column layout of the bins of one q-mask for e2m1 operands
-    (``g2_pack_u8_residual``, two columns per byte).  The order of a bin's
-    pixels is free (every Gram entry sums over them), so the columns follow
-    the pack's work units: per bin first the 32-column units (16 bytes from two
-    runs of 16 consecutive pixels of one 4080-pixel chunk), then the 8-column
-    units from two runs of 4, then the 8-column units from up to 8 single
-    pixels; bins padded to 256 columns (128 bytes, one block of the K-blocked
-    operand)."""
+    """Packed-column layout of the bins of one q-mask for the narrow operands
+    (``g2_pack_u8_residual``): e2m1, two columns per byte, or e4m3.  The order
+    of a bin's pixels is free (every Gram entry sums over them), so the columns
+    follow the pack's work units, each of pixels of one 4080-pixel chunk: per
+    bin first the 16-byte units (e2m1: two runs of 16 consecutive pixels, e4m3:
+    one), then the 4-byte units from runs of 4, then the 4-byte units from
+    single pixels; bins padded to 128 bytes, one block of the K-blocked
+    operand."""
 
-    mode, kind, split, ones_row, elem_bytes = MODE_E2M1, KIND_E2M1, False, True, 0.5
-    n_pieces = 0
+    split, ones_row, n_pieces = False, True, 0
 
-    def __init__(self, qmask, n_bins):
+    def __init__(self, qmask, n_bins, mode=MODE_E2M1):
+        e2m1 = mode == MODE_E2M1
+        self.mode, self.kind = int(mode), KIND_E2M1 if e2m1 else KIND_E4M3
+        self.elem_bytes = 0.5 if e2m1 else 1
+        vec, word = (32, 8) if e2m1 else (16, 4)                # columns per unit
+        pad = 128 * word // 4                                   # columns of 128 bytes
+        order_of = E2M1_WORD if e2m1 else np.arange(4)          # column of every count of a 4-byte word
         q = np.ascontiguousarray(qmask, dtype=np.int32).ravel()
         self.npix_total, self.n_bins = q.size, int(n_bins)
         nb = max(self.n_bins, 1)
-        self.n_chunks = -(-q.size // E2M1_CHUNK)
+        self.n_chunks = -(-q.size // NARROW_CHUNK)
         pix = np.flatnonzero((q >= 1) & (q <= self.n_bins)).astype(np.int64)
         b = q[pix].astype(np.int64) - 1
         self.npix = np.bincount(b, minlength=nb)[: self.n_bins].astype(np.int64)
-        grp = (pix // E2M1_CHUNK) * nb + b                     # (chunk, bin): a unit stays inside one
+        grp = (pix // NARROW_CHUNK) * nb + b                     # (chunk, bin): a unit stays inside one
         order = np.argsort(grp, kind="stable")
         pix, grp = pix[order], grp[order]
         first = np.ones(pix.size, dtype=bool)
@@ -325,14 +328,18 @@ class NarrowLayout:
             return p[a], p[a + half[a]], g[a], p[odd], g[odd]
 
         p16, g16 = pieces(rp, rg, n // 16, 16)
-        v0, v1, vg, lp, lg = paired(p16, g16)
         rest = rp + n // 16 * 16
         p4, g4 = pieces(rest, rg, n % 16 // 4, 4)
-        q4, h4 = pieces(lp, lg, np.full(lp.size, 4), 4)
-        w0, w1, wg, lp, lg = paired(np.concatenate([p4, q4]), np.concatenate([g4, h4]))
         p1, g1 = pieces(rest + n % 16 // 4 * 4, rg, n % 4, 1)
-        q1, h1 = pieces(lp, lg, np.full(lp.size, 4), 1)
-        p1, g1 = np.concatenate([p1, q1]), np.concatenate([g1, h1])
+        if e2m1:                                                # pieces left without a partner: smaller ones
+            v0, v1, vg, lp, lg = paired(p16, g16)
+            q4, h4 = pieces(lp, lg, np.full(lp.size, 4), 4)
+            w0, w1, wg, lp, lg = paired(np.concatenate([p4, q4]), np.concatenate([g4, h4]))
+            q1, h1 = pieces(lp, lg, np.full(lp.size, 4), 1)
+            p1, g1 = np.concatenate([p1, q1]), np.concatenate([g1, h1])
+            vruns, wruns = (v0, v1), (w0, w1)
+        else:
+            vruns, wruns, vg, wg = (p16,), (p4,), g16, g4
         o = np.argsort(g1, kind="stable")
         p1, g1 = p1[o], g1[o]
         new = np.ones(g1.size, dtype=bool)
@@ -340,10 +347,10 @@ class NarrowLayout:
         s = np.flatnonzero(new)
         c = np.diff(np.append(s, g1.size))
         rank = np.arange(g1.size) - np.repeat(s, c)
-        unit = np.cumsum(rank % 8 == 0) - 1                      # gather unit of every single pixel
-        gg = g1[rank % 8 == 0]
-        singles = np.full((gg.size, 8), -1, dtype=np.int64)
-        singles[unit, rank % 8] = p1
+        unit = np.cumsum(rank % word == 0) - 1                   # gather unit of every single pixel
+        gg = g1[rank % word == 0]
+        singles = np.full((gg.size, word), -1, dtype=np.int64)
+        singles[unit, rank % word] = p1
 
         def within_bin(g):
             """Position of every unit among the units of its bin (chunk order)."""
@@ -357,40 +364,40 @@ class NarrowLayout:
         vb, vpos, vc = within_bin(vg)
         wb, wpos, wc = within_bin(wg)
         gb, gpos, gc = within_bin(gg)
-        self.kpad = _roundup(32 * vc + 8 * (wc + gc), E2M1_PAD)[: self.n_bins].astype(np.int64)
+        self.kpad = _roundup(vec * vc + word * (wc + gc), pad)[: self.n_bins].astype(np.int64)
         off = np.concatenate([[0], np.cumsum(self.kpad)])
         self.bin_off = self.plane0 = off[:-1].astype(np.int64)
         self.plane1 = None
-        self.packed_cols = int(max(E2M1_PAD, off[-1]))
+        self.packed_cols = int(max(pad, off[-1]))
         if self.packed_cols >= 2 ** 31:
             raise ValueError("too many binned pixels for one job")
-        vcol = self.bin_off[vb] + 32 * vpos
-        wcol = self.bin_off[wb] + 32 * vc[wb] + 8 * wpos
-        gcol = self.bin_off[gb] + 32 * vc[gb] + 8 * (wc[gb] + gpos)
+        vcol = self.bin_off[vb] + vec * vpos
+        wcol = self.bin_off[wb] + vec * vc[wb] + word * wpos
+        gcol = self.bin_off[gb] + vec * vc[gb] + word * (wc[gb] + gpos)
         col_src = np.full(self.packed_cols, -1, dtype=np.int32)
-        for col, runs, size in ((vcol, (v0, v1), 16), (wcol, (w0, w1), 4)):
+        for col, runs, size in ((vcol, vruns, 16), (wcol, wruns, 4)):
             j = np.arange(size)
             for half, p in enumerate(runs):
-                col_src[(col[:, None] + j // 4 * 8 + E2M1_WORD[4 * half + j % 4]).ravel()] = (p[:, None] + j).ravel()
-        col_src[(gcol[:, None] + E2M1_WORD).ravel()] = singles.ravel()
+                col_src[(col[:, None] + j // 4 * word + order_of[4 * half + j % 4]).ravel()] = (p[:, None] + j).ravel()
+        col_src[(gcol[:, None] + order_of).ravel()] = singles.ravel()
         self.col_src = col_src                                     # pixel of every packed column, -1: padding
         self.sector_bin = np.repeat(np.arange(self.n_bins, dtype=np.int32), self.kpad // RES_SECTOR)
         if self.sector_bin.size < self.packed_cols // RES_SECTOR:
             self.sector_bin = np.full(self.packed_cols // RES_SECTOR, -1, dtype=np.int32)
         # blocks of 32 units of one class per chunk
-        local = lambda p, ch: p - ch * E2M1_CHUNK
+        local = lambda p, ch: p - ch * NARROW_CHUNK
         recs = []
-        for cls, g, dst, p in ((UNIT_VEC, vg, vcol // 32, (v0, v1)), (UNIT_WORD, wg, wcol // 8, (w0, w1))):
+        for cls, g, dst, p in ((UNIT_VEC, vg, vcol // vec, vruns), (UNIT_WORD, wg, wcol // word, wruns)):
             ch = g // nb
             u = np.zeros((g.size, 4), dtype=np.int64)
             u[:, 0] = dst | (cls << 30)
-            u[:, 1] = local(p[0], ch) | (local(p[1], ch) << 16)
+            u[:, 1] = local(p[0], ch) | (local(p[-1], ch) << 16)
             recs.append((ch, u))
         ch = gg // nb
-        src = np.where(singles >= 0, singles - ch[:, None] * E2M1_CHUNK, 0xFFF)
+        src = np.where(singles >= 0, singles - ch[:, None] * NARROW_CHUNK, 0xFFF)
         u = np.zeros((gg.size, 4), dtype=np.int64)
-        u[:, 0] = (gcol // 8) | (UNIT_GATHER << 30)
-        for k in range(8):
+        u[:, 0] = (gcol // word) | (UNIT_GATHER << 30)
+        for k in range(word):
             w, sh = divmod(12 * k, 32)
             u[:, 1 + w] |= (src[:, k] << sh) & 0xFFFFFFFF
             if sh > 20:
@@ -408,16 +415,16 @@ class NarrowLayout:
             nxt += nblk
         self.unit_block_off = boff.astype(np.int32)
         self.units = units.reshape(-1)
-        self.chunk_span = chunk_spans(pix, self.n_chunks, E2M1_CHUNK)
+        self.chunk_span = chunk_spans(pix, self.n_chunks, NARROW_CHUNK)
 
     @property
     def packed_bytes_per_frame(self):
-        return self.packed_cols // 2
+        return self.packed_cols // 2 if self.mode == MODE_E2M1 else self.packed_cols
 
     def ones_row_values(self):
-        """Row of ones: code 1 in every binned column, 0 in the padding."""
+        """Row of ones: 1 (e2m1: code 1) in every binned column, 0 in the padding."""
         one = (self.col_src >= 0).astype(np.uint8)
-        return one[0::2] | (one[1::2] << 4)
+        return one[0::2] | (one[1::2] << 4) if self.mode == MODE_E2M1 else one
 
     def grams(self):
         """The Grams to run per bin: (bin, a_off, b_off, kpad, shift)."""
@@ -551,13 +558,13 @@ SPLIT_SHARE = 3
 SPLIT_MIN_STAGES = 16
 
 
-def split_items(items, workers, stage_elems, kind, ones=True):
+def split_items(items, workers, stage_elems, kind, ones=True, cost=None):
     """``items`` of one launch with the K of the long ones cut into equal
     pieces (multiples of a stage), for launches that would leave workers idle.
     The sums are added piece by piece, so any cut gives the same results."""
     if items.size == 0 or workers <= 1:
         return items
-    share = item_costs(items, stage_elems, kind, ones).sum() / workers
+    share = (item_costs(items, stage_elems, kind, ones) if cost is None else cost).sum() / workers
     most = max(float(SPLIT_MIN_STAGES), share / SPLIT_SHARE)
     stages = items["k_len"].astype(np.int64) // stage_elems
     n = np.maximum(1, np.ceil(stages / most).astype(np.int64))
@@ -574,7 +581,7 @@ def split_items(items, workers, stage_elems, kind, ones=True):
     return out
 
 
-def balance_items(items, workers, stage_elems, kind, ones=True):
+def balance_items(items, workers, stage_elems, kind, ones=True, cost=None):
     """Static longest-first list schedule of one launch's items over
     ``workers`` persistent workers (CTAs, or CTA pairs for "pair" items):
     each item, largest cost first, goes to the least-loaded worker, and the
@@ -585,7 +592,9 @@ def balance_items(items, workers, stage_elems, kind, ones=True):
     n = items.size
     if workers <= 1 or n <= workers:
         return items
-    cost = np.ascontiguousarray(item_costs(items, stage_elems, kind, ones), dtype=np.float64)
+    if cost is None:
+        cost = item_costs(items, stage_elems, kind, ones)
+    cost = np.ascontiguousarray(cost, dtype=np.float64)
     slots, n_slots = lpt_slots(cost, workers)
     out = np.zeros(n_slots, dtype=ITEM_DTYPE)
     out["job"] = ITEM_EMPTY

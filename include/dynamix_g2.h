@@ -53,7 +53,7 @@ extern "C" {
 #define G2_PLAIN_BN   128
 #define G2_PAD        128  /* packed_cols and bin segments are multiples of this */
 #define G2_PACK_CHUNK 2048 /* source pixels per pack chunk */
-#define G2_E2M1_CHUNK 4080 /* source pixels per chunk of the e2m1 pack (12-bit offsets) */
+#define G2_NARROW_CHUNK 4080 /* source pixels per chunk of the narrow pack (12-bit offsets) */
 #define G2_PACK_MAX_SLOTS  128  /* distinct bins per chunk */
 #define G2_PACK_MAX_PIECES 512  /* (64-column segment x chunk) pieces per chunk */
 #define G2_PACK_WORDS_PER_CHUNK 768 /* 4-column words per chunk: 2048/4 + partial words at bin edges */
@@ -211,12 +211,12 @@ int g2_pack_e4m3_units(const void* frames_dev, int64_t nframes, int64_t npix,
  * (two uint32, 8-byte aligned), res_count_dev[sector] entries (caller zeroes;
  * above res_cap the entry is dropped and G2_DEVERR_RESIDUAL set).  frame0 is
  * the number of the first frame in the stack, so a stack may be packed in
- * pieces.  Units: g2_pack_e4m3_units' for G2_KIND_E4M3; for G2_KIND_E2M1
- * {class << 30 | destination, ...} with class 1 = 16 bytes from two runs of 16
- * source bytes (word 1: src0 | src1 << 16), 2 = 4 bytes from two runs of 4, 3 =
- * 4 bytes from 8 sources of 12 bits in words 1-3 (0xFFF: none), 0 = none; the
- * 8 columns of a word hold counts 0 2 of the first four (run), 0 2 of the
- * second, 1 3 of the first, 1 3 of the second.  Every
+ * pieces.  Units, in blocks of 32 of one class as for g2_pack_e4m3_units:
+ * {class << 30 | destination, sources ...} with class 1 = 16 bytes from runs of
+ * 16 source bytes (word 1: e4m3 src, e2m1 src0 | src1 << 16), 2 = 4 bytes from
+ * runs of 4, 3 = 4 bytes from 4 (e2m1: 8) sources of 12 bits in words 1-3
+ * (0xFFF: none), 0 = none; the 8 columns of an e2m1 word hold counts 0 2 of the
+ * first four (run), 0 2 of the second, 1 3 of the first, 1 3 of the second.  Every
  * packed byte belongs to one unit.  Replaces the gather of dense.py:48-50. */
 int g2_pack_u8_residual(const void* frames_dev, int64_t nframes, int64_t npix, int64_t frame0, int32_t elem_kind,
                         const int32_t* unit_block_off_dev, const uint32_t* units_dev, const uint32_t* spans_dev,
@@ -575,6 +575,17 @@ int g2_denominator(const int64_t* sums_dev, int32_t n_rows, int64_t nframes,
 int g2_finalize(const int64_t* numer_dev, const int64_t* denom_dev, const double* scale_dev,
                 int32_t n_rows, int64_t nframes, float* g2_f32_dev, double* g2_f64_dev,
                 void* stream);
+
+/* ---- G3 and G4 by number-theoretic transforms -----------------------------
+ * The same D (denom_dev) and g2 as g2_denominator + g2_finalize, in O(T log T)
+ * (arithmetic modulo 2^64 - 2^32 + 1: exact for D < 2^63).  roots_dev: the 4096
+ * powers of the 4096th root of unity 7^((p - 1) / 4096), then the inverse of
+ * 4096, uint64, 16-byte aligned.  scratch_dev: g2_ntt_scratch(n_rows, nframes)
+ * uint64.  Either g2 array may be NULL. */
+int64_t g2_ntt_scratch(int32_t n_rows, int64_t nframes);
+int g2_normalize_ntt(const int64_t* numer_dev, const int64_t* sums_dev, const double* scale_dev, int32_t n_rows,
+                     int64_t nframes, const uint64_t* roots_dev, uint64_t* scratch_dev, int64_t scratch_len,
+                     int64_t* denom_dev, float* g2_f32_dev, double* g2_f64_dev, void* stream);
 
 /* ---- G3+G4 without allocation -------------------------------------------
  * No counterpart in the reference.  Same result as g2_denominator followed by
