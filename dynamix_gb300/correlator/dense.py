@@ -58,10 +58,7 @@ class _DenseBase(BaseCorrelator):
         ``CorrelationResult(res, dev)`` whose ``dev`` is the deviation of
         dense.py:58-66 (float32, computed in float on the tensor cores and
         reduced in float64; NaN where the reference divides by zero)."""
-        out = self.correlate_device(frames)
-        res = out.cpu().numpy()
-        self.engine.check_error()
-        self.engine.check_denominator_range()
+        res = self.engine.correlate(lambda: self.correlate_device(frames))
         if calc_std:
             dev = self.engine.deviation().cpu().numpy()
             self.engine.check_error()

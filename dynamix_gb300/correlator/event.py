@@ -59,10 +59,7 @@ class EventCorrelator(BaseCorrelator):
 
     def correlate(self, vol_times, vol_data, offsets):
         self._check_event_arrays(vol_times, vol_data, offsets)
-        out = self.engine.run(vol_times, vol_data, offsets)
-        res = out.cpu().numpy()
-        self.engine.check_error()
-        return res
+        return self.engine.correlate(lambda: self.engine.run(vol_times, vol_data, offsets))
 
     @property
     def numerator(self):

@@ -42,9 +42,7 @@ class SparseCorrelator(BaseCorrelator):
         return self.engine.run(data, indices, indptr, offsets)
 
     def correlate(self, data, indices, indptr, offsets, output=None):
-        out = self.engine.run(data, indices, indptr, offsets)
-        res = out.cpu().numpy()
-        self.engine.check_error()
+        res = self.engine.events.correlate(lambda: self.engine.run(data, indices, indptr, offsets))
         if self._single_q:
             res = res.ravel()
         if output is not None:

@@ -173,6 +173,18 @@ __global__ void finalize_kernel(const long long* __restrict__ N, const long long
   }
 }
 
+// The largest of n non-negative values, into *out (zeroed by the caller).
+__global__ void __launch_bounds__(256)
+    max_kernel(const long long* __restrict__ x, int64_t n, unsigned long long* __restrict__ out) {
+  long long m = 0;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    m = max(m, x[i]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(out, static_cast<unsigned long long>(m));
+}
+
 // calc_std deviation (dense.py:58-66): dev(tau) = std_t(r) / sqrt(T - tau),
 // from the sums of d = r - centre and d^2 over the T - tau pairs of the lag
 // (population variance, as numpy's std); NaN when a pair had S(t) S(t') = 0
@@ -272,6 +284,18 @@ extern "C" int g2_denominator(const int64_t* sums_dev, int32_t n_rows, int64_t n
   if (n_rows > 65535) return G2_ERR_TOO_LARGE;
   return norm::launch_denominator(reinterpret_cast<const long long*>(sums_dev), n_rows, nframes,
                                   reinterpret_cast<long long*>(denom_dev), as_stream(stream));
+}
+
+extern "C" int g2_max_i64(const int64_t* x_dev, int64_t n, uint64_t* max_dev, void* stream) {
+  using namespace g2;
+  if (!x_dev || !max_dev || n <= 0 || !aligned(max_dev, 8)) return G2_ERR_ARG;
+  const int sms = sm_count_current();
+  if (sms <= 0) return G2_ERR_CUDA;
+  int64_t blocks = (n + 1023) / 1024;
+  if (blocks > sms * 2) blocks = sms * 2;
+  norm::max_kernel<<<static_cast<unsigned>(blocks), 256, 0, as_stream(stream)>>>(
+      reinterpret_cast<const long long*>(x_dev), n, reinterpret_cast<unsigned long long*>(max_dev));
+  return launch_status();
 }
 
 extern "C" int g2_finalize(const int64_t* numer_dev, const int64_t* denom_dev, const double* scale_dev,

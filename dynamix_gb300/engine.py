@@ -148,6 +148,65 @@ def _keep_layout(key, L):
     return L
 
 
+class ResultBuffers:
+    """Device memory of one engine's sums and results, laid out so that a call
+    zeroes them with one fill and reads its result with one copy:
+
+        numer | sums (int64 rows x T each) | status (8 int32) | g2 (float32 rows x T)
+
+    ``status`` holds the error word, two counters of the narrow operands (see
+    DenseEngine) or a flag, and, written by :meth:`read_result`, the largest
+    bin sum (int64 at word 4).  ``numer`` and ``sums`` may be the caller's
+    (views into an arena)."""
+
+    def _init_results(self, rows, numer=None, sums=None):
+        torch = _torch()
+        n = rows * self.T
+        own = numer is None and sums is None
+        buf = torch.zeros((2 * n if own else 0) + 4 + (n + 1) // 2, dtype=torch.int64, device=self.dev)
+        tail = buf[2 * n:] if own else buf
+        self.numer = buf[:n].view(rows, self.T) if own else numer
+        self.sums = buf[n:2 * n].view(rows, self.T) if own else sums
+        if not own:
+            z = lambda x: torch.zeros((rows, self.T), dtype=torch.int64, device=self.dev) if x is None else x
+            self.numer, self.sums = z(self.numer), z(self.sums)
+        self._zeroed = buf[:2 * n + 4] if own else None
+        words = tail.view(torch.int32)
+        self._ret = words[:8 + n]
+        self.status = words[:8]
+        self.err = words[:1]
+        self._sum_max = words[4:6]
+        self.g2_f32 = words[8:8 + n].view(torch.float32).view(rows, self.T)
+        self._result = None       # (status words, g2) of the run that correlate() reads
+
+    def zero_results(self):
+        """Zero N, S and the status words (one fill when they are the engine's own)."""
+        if self._zeroed is not None:
+            self._zeroed.zero_()
+        else:
+            self.numer.zero_()
+            self.sums.zero_()
+            self.status.zero_()
+
+    def read_result(self, largest=True):
+        """The status words and g2 as numpy (one synchronising copy), with the
+        ``largest`` bin sum in words 4-5."""
+        n = 8 + self.n_bins * self.T
+        if largest and self.n_bins:
+            _lib.check(self.lib.g2_max_i64(ptr(self.sums), self.n_bins * self.T, ptr(self._sum_max),
+                                           stream_handle(self.dev)), "g2_max_i64")
+        # into fresh pageable memory: on this host's coherent link as fast as
+        # into pinned memory, and no second copy (2.56 MB: 32 us, pinned and
+        # copied out 178 us)
+        a = self._ret[:n].cpu().numpy()
+        return a[:8], a[8:].view(np.float32).reshape(self.n_bins, self.T)
+
+    def take_result(self):
+        """The result of the last run, read now unless the run has done so."""
+        res, self._result = self._result, None
+        return self.read_result() if res is None else res
+
+
 NTT_PRIME = 2 ** 64 - 2 ** 32 + 1
 _NTT_ROOTS = {}
 
@@ -191,7 +250,7 @@ def normalise_rows(eng):
                                     ptr(eng.g2_f64), st), "g2_normalize_ntt")
 
 
-class DenseEngine:
+class DenseEngine(ResultBuffers):
     """Exact g2 of a dense (T, H, W) stack for the bins of one q-mask.
 
     ``operand`` selects the packed element type of the tensor-core Gram:
@@ -238,16 +297,14 @@ class DenseEngine:
         rows = max(self.n_bins, 1)
         z = lambda dt: torch.zeros((rows, self.T), dtype=dt, device=self.dev)
         # N and S may be views into a caller's arena (grouped launches address
-        # several jobs' sums through one base pointer)
-        self.sums = z(torch.int64) if sums is None else sums
-        self.numer = z(torch.int64) if numer is None else numer
+        # several jobs' sums through one base pointer).  Status words of one
+        # call: the error word, the residuals of a narrow operand (or whether a
+        # stack exceeds the reused K split), and the sampled counts that e2m1 /
+        # e4m3 operands split
+        self._init_results(rows, numer, sums)
+        self.want_result = False  # read g2 with the run's last synchronisation (correlate)
         self.denom = z(torch.int64)
-        self.g2_f32 = z(torch.float32)
         self.g2_f64 = z(torch.float64)
-        # device words of one call: the error word, the residuals of a narrow
-        # operand, and the sampled counts that e2m1 / e4m3 operands split
-        self.status = torch.zeros(4, dtype=torch.int32, device=self.dev)
-        self.err = self.status[:1]
         self.maxval = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._layouts = {} if layouts is None else layouts   # may be shared by engines of one q-mask
         self._qdigest = qmask_digest
@@ -449,7 +506,7 @@ class DenseEngine:
         self.sums.zero_()
         emax = self._piece_emax(L)
         emax.zero_()
-        self.err.zero_()
+        self.status.zero_()
         st = stream_handle(self.dev)
         if mode == MODE_E4M3:
             self.pack_e4m3(frames_dev.data_ptr(), frames_dev.element_size(), self.T, L, packed.data_ptr(), st)
@@ -822,7 +879,7 @@ class DenseEngine:
                     src[k].copy_(frames[t], non_blocking=True)
             self.status.zero_()
             self._count_tail(src.data_ptr(), T, self.npix, self._layout(MODE_E2M1, True), n, stream_handle(self.dev))
-            _, _, c4, c8 = self.status.tolist()
+            c4, c8 = self.status.tolist()[2:4]
             self._narrow = self._pick_narrow(n * self._binned_pixels(), c4, c8)
             if self._narrow == MODE_FP16:
                 self._u8_hint = MODE_FP16             # counts above 16 were seen (or lists overflowed)
@@ -888,9 +945,7 @@ class DenseEngine:
         gram_streams = (cur, gram_s) if self.pipe_gram_streams > 1 else (cur,)
         self._events = []
         self._mark("pipeline")
-        self.numer.zero_()
-        self.sums.zero_()
-        self.status.zero_()
+        self.zero_results()
         emax = None
         if mode == MODE_FP16:
             emax = self._piece_emax(L)
@@ -987,8 +1042,8 @@ class DenseEngine:
             # one synchronisation: the error word and whether the stack's
             # energy bounds exceed those the reused split covers
             m = L.n_pieces
-            above = ((emax[:m].to(torch.int64) & 0xFFFFFFFF) > bound).any().to(torch.int32)
-            code, over = (int(x) for x in torch.stack([self.err[0], above]).cpu())
+            self.status[1:2].copy_(((emax[:m].to(torch.int64) & 0xFFFFFFFF) > bound).any().view(1))
+            code, over = self._end_words()[:2]
             if code or over:                          # out of range, or a brighter stack: planned path
                 return self.run(frames_dev, pipelined=False, reuse_split=False)
             self.last = {"mode": "fp16", "split": int(L.split), "n_items": int(items.size), "n_grams": n_grams,
@@ -999,7 +1054,7 @@ class DenseEngine:
                      "packed_cols": L.packed_cols, "pipeline_chunks": int(bounds.size - 1), "tile": self.tile,
                      "h2d_bytes": h2d, "crop": list(self.crop) if crop else None}
         if narrow is not None:
-            code, total, c4, c8 = self.status.tolist()
+            code, total, c4, c8 = self._end_words()[:4]
             if code & _lib.DEVERR_RESIDUAL:           # more large counts than the lists hold: look again
                 again = frames if crop else frames_dev
                 self._narrow = None
@@ -1014,11 +1069,21 @@ class DenseEngine:
             elif mode != MODE_E2M1:
                 self._narrow = self._pick_narrow(min(self.T, self.TAIL_FRAMES) * self._binned_pixels(), 2 * c4, c8)
             return self.g2_f32[: self.n_bins]
-        code = self.resolve_range_check(int(self.err.item()), frames_dev, cropped=crop)
+        code = self.resolve_range_check(self._end_words()[0], frames_dev, cropped=crop)
         if code & _lib.DEVERR_RANGE and self.operand == "auto":
             self._u8_hint = MODE_FP16                 # counts above 16: rerun on fp16 operands
             return self.run(frames if crop else frames_dev, pipelined=False)
+        if self._result is not None:
+            self._result[0][0] = code                 # as resolved
         return self.g2_f32[: self.n_bins]
+
+    def _end_words(self):
+        """The status words at the end of a run (its synchronisation), with
+        :attr:`want_result` in one copy with g2."""
+        if self.want_result:
+            self._result = self.read_result()
+            return [int(x) for x in self._result[0]]
+        return self.status.tolist()
 
     # -- whole pipeline ----------------------------------------------------
     def run(self, frames_dev, pipelined=True, reuse_split=True):
@@ -1031,6 +1096,7 @@ class DenseEngine:
         if tuple(frames_dev.shape) != (self.T,) + self.shape:
             raise ValueError("frames should have shape %s, got %s" % ((self.T,) + self.shape,
                                                                     tuple(frames_dev.shape)))
+        self._result = None
         if self.n_bins == 0:
             return self.g2_f32[:0]
         if pipelined and self._narrow == MODE_FP16:
@@ -1118,14 +1184,14 @@ class DenseEngine:
         if L is not L0:
             return None
         m = L.n_pieces * (2 if L.split else 1)
-        above = ((self._piece_emax(L)[:m].to(torch.int64) & 0xFFFFFFFF) > bound).any().to(torch.int32)
+        self.status[1:2].copy_(((self._piece_emax(L)[:m].to(torch.int64) & 0xFFFFFFFF) > bound).any().view(1))
         items, items_dev, n_chunks = self.items_for(L, grams)
         self._mark("gram_" + self.method)
         self.numerator(L, items_dev, items.size)
         self._mark("normalise")
         self.normalise()
         self._mark("end")
-        code, over = (int(x) for x in torch.stack([self.err[0], above]).cpu())
+        code, over = self._end_words()[:2]
         if code or over:
             return None
         self.last = {"mode": ["fp16", "bytes", "e4m3"][L.mode], "split": int(L.split), "n_items": int(items.size),
@@ -1304,8 +1370,23 @@ class DenseEngine:
         self.check_error()
         return out
 
-    def check_denominator_range(self):
-        """Raise if int64 D could have overflowed (checked from S on the host)."""
-        S = self.sums[: self.n_bins].cpu().numpy()
-        if S.size and float(S.max()) ** 2 * self.T >= 2.0 ** 63:
+    def check_denominator_range(self, largest=None):
+        """Raise if int64 D could have overflowed (checked from the largest S)."""
+        if largest is None:
+            S = self.sums[: self.n_bins].cpu().numpy()
+            largest = S.max() if S.size else 0
+        if float(largest) ** 2 * self.T >= 2.0 ** 63:
             raise OverflowError("denominator exceeds int64 for these counts")
+
+    def correlate(self, run):
+        """g2 as numpy of the run that ``run()`` makes: one copy back, errors raised."""
+        self.want_result = True
+        try:
+            run()
+            words, g2 = self.take_result()
+        finally:
+            self.want_result, self._result = False, None
+        if words[0]:
+            raise DeviceError(_lib.device_error_message(int(words[0])))
+        self.check_denominator_range(int(words[4:6].view(np.int64)[0]))
+        return g2

@@ -19,7 +19,7 @@ import ctypes as C
 import numpy as np
 
 from . import _lib
-from .engine import DeviceError, _torch, normalise_rows, ptr, require_cuda, stream_handle
+from .engine import DeviceError, ResultBuffers, _torch, normalise_rows, ptr, require_cuda, stream_handle
 
 # shared memory of the shared-counter pair kernel besides its 2 x T counters:
 # 24 warps x 2 half-warp pixels x 2 staging buffers x 128 events x 4 bytes
@@ -170,7 +170,7 @@ def cta_ranges(binned_bin, n_ctas):
     return range_off, range_bin, cta_range_off
 
 
-class EventEngine:
+class EventEngine(ResultBuffers):
     """Exact g2 from per-pixel event lists (G6 pair sums, then G3, G4)."""
 
     SMEM_CTAS_PER_SM = 1   # the shared-memory kernel holds 2 x T counters per CTA
@@ -199,9 +199,8 @@ class EventEngine:
         self.scale = torch.as_tensor(np.asarray(scale, dtype=np.float64), device=self.dev)
         rows = max(self.n_bins, 1)
         z = lambda dt: torch.zeros((rows, self.T), dtype=dt, device=self.dev)
-        self.sums, self.numer, self.denom = z(torch.int64), z(torch.int64), z(torch.int64)
-        self.g2_f32, self.g2_f64 = z(torch.float32), z(torch.float64)
-        self.err = torch.zeros(1, dtype=torch.int32, device=self.dev)
+        self._init_results(rows)
+        self.denom, self.g2_f64 = z(torch.int64), z(torch.float64)
         self.last = {}
         self.profile = False
         self._events = []
@@ -329,9 +328,7 @@ class EventEngine:
         if counts is None or counts.numel() < max(n_ev, 1) or counts.dtype != vol_data.dtype:
             self._counts_buf = None
             counts = self._counts_buf = torch.empty(max(n_ev, 1), dtype=vol_data.dtype, device=self.dev)
-        self.numer.zero_()
-        self.sums.zero_()
-        self.err.zero_()
+        self.zero_results()
         st = stream_handle(self.dev)
         start = torch.cuda.Event()
         start.record(cur)
@@ -396,10 +393,11 @@ class EventEngine:
         ``counts``, or packed words ``(t << 16) | v`` with ``counts=None``
         (``reset_error=False`` keeps the flags an earlier stage of the same
         call has set)."""
-        self.numer.zero_()
-        self.sums.zero_()
         if reset_error:
-            self.err.zero_()
+            self.zero_results()
+        else:
+            self.numer.zero_()
+            self.sums.zero_()
         st = stream_handle(self.dev)
         # the C side makes the same choice (shared counters for 2 x T frames,
         # times below 2^16, products below 2^31)
@@ -424,8 +422,15 @@ class EventEngine:
                      "n_ranges": n_ranges, "n_ctas": n_ctas}
         return self.g2_f32[: self.n_bins]
 
-    def check_error(self):
-        code = int(self.err.item())
+    def correlate(self, run):
+        """g2 as numpy of the run that ``run()`` makes: one copy back, errors raised."""
+        run()
+        words, g2 = self.read_result(largest=False)
+        self.check_error(int(words[0]))
+        return g2
+
+    def check_error(self, code=None):
+        code = int(self.err.item()) if code is None else code
         times_checked, csr_checked = getattr(self, "_times_checked", False), getattr(self, "_csr_checked", False)
         self._times_checked = self._csr_checked = False
         offsets_bad, self._offsets_bad = getattr(self, "_offsets_bad", None), None
