@@ -1297,11 +1297,11 @@ def run_compress(args):
     stack_bytes = T * npix
     out_bytes = n_ev * 5 + (npix + 1) * 8
     peaks, peak_kind = measured_peaks()
-    # dominant kernel: the stage pass (reads the stack, writes a 4-byte word per event);
-    # the count pass reads the stack once more, the gather moves the words to the lists
+    # dominant kernel: the emit pass (reads the stack, writes the lists); the count
+    # pass reads the stack once more
     count_gbs = stack_bytes / (st["count"] / 1e3) / 1e9
-    stage_bytes = stack_bytes + n_ev * 4
-    stage_gbs = stage_bytes / (st["stage"] / 1e3) / 1e9
+    emit_bytes = stack_bytes + n_ev * 5
+    emit_gbs = emit_bytes / (st["emit"] / 1e3) / 1e9
     traffic = profile_traffic("launches_compress_514x1030_T10000.md")
     if traffic is not None:
         traffic *= T / COMPRESS_WORKLOAD["nframes"]
@@ -1312,13 +1312,13 @@ def run_compress(args):
         "config": compress_config(T, n_events=n_ev, parallelism="replicas" if world > 1 else "single"),
         "hbm_GB_per_s_step": (stack_bytes + out_bytes) / (ms / 1e3) / 1e9,
         "stages_ms": st,
-        "roofline": {"bound": "hbm", "achieved": stage_gbs, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
-                     "frac": stage_gbs / peaks.get("hbm_gbs"), "traffic": traffic, "kernel": "g2_compress_stage",
+        "roofline": {"bound": "hbm", "achieved": emit_gbs, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
+                     "frac": emit_gbs / peaks.get("hbm_gbs"), "traffic": traffic, "kernel": "g2_compress_emit",
                      "peak_source": "%s hbm_gbs" % peak_kind,
-                     "algorithmic_bytes_per_launch": stage_bytes, "launch_ms": st["stage"],
+                     "algorithmic_bytes_per_launch": emit_bytes, "launch_ms": st["emit"],
                      "count_pass_GB_per_s": count_gbs,
-                     "note": "two passes read the stack (count, stage); the algorithmic minimum reads it once"},
-        "clocks": clocks, "gpu_launches": 8 * args.steps,
+                     "note": "two passes read the stack (count, emit); the algorithmic minimum reads it once"},
+        "clocks": clocks, "gpu_launches": 6 * args.steps,
     }
     if rank == 0 and not args.no_e2e:
         host = torch.empty((T, npix), dtype=torch.uint8, pin_memory=True)

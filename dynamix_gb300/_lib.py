@@ -96,6 +96,7 @@ SIGNATURES = {
     "g2_events_unpack": (C.c_int, [_p, _i64, _i32, _p, _p, _p]),
     "g2_compress_count": (C.c_int, [_p, _i32, _i32, _i64, _i32, _p, _p, _p, _p, _p, _p]),
     "g2_compress_finish": (C.c_int, [_p, _p, _p, _i32, _i64, _p, _p, _p, _p, _p]),
+    "g2_compress_emit": (C.c_int, [_p, _i32, _i32, _i64, _p, _p, _i64, _p, _p, _p, _p]),
     "g2_compress_stage": (C.c_int, [_p, _i32, _i32, _i64, _p, _p, _p, _p, _p, _i64, _p, _p]),
     "g2_events_gather_rel": (C.c_int, [_p, _p, _p, _i32, _i64, _i64, _p, _i32, _p, _p, _p, _p, _p]),
     "g2_stream_compress": (C.c_int, [_p, _i32, _i32, _i64, _i64, _i32, _i32, _p, _p, _p, _p, _p, _p, _p]),

@@ -9,10 +9,11 @@ above the threshold masks its pixel from that frame on, a masked pixel gives
 no events, and the sum frame adds every raw value.
 
 Kernels (``csrc/g2_compress.cu``, gather in ``csrc/g2_csr.cu``): count per
-(1024-frame sub-block, pixel), the sticky-mask pass, two scans, a stage pass
-that writes each kept value as ``((t - sub-block start) << 16) | v`` in
-(sub-block, pixel, frame) order, and the tiled gather into the per-pixel lists
-(frame order within a pixel, the reference's layout).  Frames are uint8,
+(1024-frame sub-block, pixel), the sticky-mask pass and a scan; then the lists
+straight from the frames (frame order within a pixel, the reference's layout),
+or, with a cut (threshold or mask) or for packed words, a stage pass that writes
+each kept value as ``((t - sub-block start) << 16) | v`` in (sub-block, pixel,
+frame) order and the tiled gather into the per-pixel lists.  Frames are uint8,
 uint16, int8 or int16; only values > 0 are events.
 """
 from __future__ import annotations
@@ -161,21 +162,31 @@ class StackCompressor:
         _lib.check(self.lib.g2_exclusive_scan_u32(ptr(self.counts), self.npix, ptr(self.ev_off),
                                                   ptr(self.scan_scratch), self.scan_scratch.numel(), st),
                    "g2_exclusive_scan_u32")
-        nb = self.n_sb * self.n_blk
-        _lib.check(self.lib.g2_exclusive_scan_u32(ptr(self.blk_totals), nb, ptr(self.blk_base),
-                                                  ptr(self.blk_scratch), self.blk_scratch.numel(), st),
-                   "g2_exclusive_scan_u32")
         self._mark("scans")
         self.n_events = int(self.ev_off[-1].to(torch.int64).item()) & 0xFFFFFFFF
         return self.n_events
 
     def emit(self, frames, packed=False):
-        """Passes 4-5 after :meth:`count`: ``(data, times int32, offsets int64)``
+        """The lists after :meth:`count`: ``(data, times int32, offsets int64)``
         device tensors (data in the frames' dtype), or ``(words, offsets)``
         with ``packed`` (``(t << 16) | v`` as int32; at most 65,536 frames)."""
         torch = _torch()
         n = self.n_events
         st = stream_handle(self.dev)
+        if not packed and not self._cut:
+            times = torch.empty(max(n, 1), dtype=torch.int32, device=self.dev)
+            data = torch.empty(max(n, 1), dtype=frames.dtype, device=self.dev)
+            self._mark("host_read")
+            _lib.check(self.lib.g2_compress_emit(ptr(frames), elem_kind(frames.dtype), self.T, self.npix,
+                                                 ptr(self.sb_counts), ptr(self.ev_off), n, ptr(times), ptr(data),
+                                                 ptr(self.err), st), "g2_compress_emit")
+            self._mark("emit")
+            self.check_error()
+            return data[:n], times[:n], self.offsets()
+        nb = self.n_sb * self.n_blk
+        _lib.check(self.lib.g2_exclusive_scan_u32(ptr(self.blk_totals), nb, ptr(self.blk_base),
+                                                  ptr(self.blk_scratch), self.blk_scratch.numel(), st),
+                   "g2_exclusive_scan_u32")
         stage = self._stage_buffer(n)
         self._mark("host_read")  # from the scans to here: the event count read and the output allocation
         _lib.check(self.lib.g2_compress_stage(ptr(frames), elem_kind(frames.dtype), self.T, self.npix,

@@ -12,6 +12,8 @@
 //               above the threshold: that frame and every later one drop out),
 //               corrected sub-block counts, the pixel's total, the cut frame;
 //   3. scans  : pixel totals -> event offsets; block totals -> block bases;
+//   4. emit   : without a cut, the lists straight from the frames;
+//   or, with a cut or for packed words,
 //   4. stage  : the same CTAs read their frames again and write every kept
 //               value as one word ((t - sub-block start) << 16) | v into the
 //               staging area, ordered by sub-block, then pixel, then frame;
@@ -24,6 +26,7 @@
 // batch of frames' positive values to the (pixels x max_nnz) event and time
 // arrays; compaction (get_compacted_events, event.py:298-321) copies each
 // pixel's row to its offset.
+#include <type_traits>
 #include "g2_ptx.cuh"
 #include "g2_host.h"
 
@@ -96,6 +99,29 @@ template <typename Tv>
 __device__ __forceinline__ int32_t lane_value(uint2 w, int j) {
   const uint32_t h = ((j < 2 ? w.x : w.y) >> (16 * (j & 1))) & 0xFFFFu;
   return static_cast<Tv>(-1) < 0 ? static_cast<int32_t>(static_cast<int16_t>(h)) : static_cast<int32_t>(h);
+}
+
+// The raw word of 4 consecutive values at any alignment of the type (frames
+// whose pixel count is not a multiple of 4): the aligned 32-bit words around
+// them, shifted together.  Values beyond n_valid are 0, and no word without a
+// valid value is read.
+__device__ __forceinline__ uint32_t raw4(const uint8_t* src, int64_t n_valid, uint32_t) {
+  const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(src) & 3u);
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(src - off);
+  const uint32_t n = static_cast<uint32_t>(n_valid);
+  const uint32_t hi = off + n > 4 ? q[1] : 0u;
+  const uint32_t w = n ? __funnelshift_r(q[0], hi, 8 * off) : 0u;
+  return n >= 4 ? w : w & ((1u << (8 * n)) - 1u);
+}
+__device__ __forceinline__ uint2 raw4(const uint8_t* src, int64_t n_valid, uint2) {
+  const uint32_t n = static_cast<uint32_t>(n_valid);
+  return make_uint2(raw4(src, n < 2 ? 2 * n : 4, 0u), raw4(src + 4, n < 2 ? 0 : 2 * n - 4, 0u));
+}
+template <typename Tv, bool VEC>
+__device__ __forceinline__ typename Word4<Tv>::type load_raw(const Tv* src, int64_t n_valid) {
+  using W = typename Word4<Tv>::type;
+  if (VEC) return *reinterpret_cast<const W*>(src);
+  return raw4(reinterpret_cast<const uint8_t*>(src), n_valid, W{});
 }
 
 // Positive-value flags of a 32-bit word of packed values, all lanes at once:
@@ -179,10 +205,10 @@ __device__ __forceinline__ void walk_frames(const Tv* __restrict__ src, int64_t 
   }
 }
 
-// Positive values of frames [0, n) of 4 pixels at src (VEC loads), added to
-// cnt: lane counters flushed every 128 frames.
-template <typename Tv>
-__device__ __forceinline__ void count_positive(const Tv* __restrict__ src, int64_t npix, int64_t n,
+// Positive values of frames [0, n) of 4 pixels at src, added to cnt: lane
+// counters flushed every 128 frames.
+template <typename Tv, bool VEC>
+__device__ __forceinline__ void count_positive(const Tv* __restrict__ src, int64_t npix, int64_t n, int64_t n_valid,
                                                uint32_t cnt[PX]) {
   using W = typename Word4<Tv>::type;
   constexpr int TU = InFlight<Tv>::frames;
@@ -191,12 +217,12 @@ __device__ __forceinline__ void count_positive(const Tv* __restrict__ src, int64
   for (int g = 1; t + TU <= n; t += TU, ++g) {
     W raw[TU];
 #pragma unroll
-    for (int u = 0; u < TU; ++u) raw[u] = *reinterpret_cast<const W*>(src + (t + u) * npix);
+    for (int u = 0; u < TU; ++u) raw[u] = load_raw<Tv, VEC>(src + (t + u) * npix, n_valid);
 #pragma unroll
     for (int u = 0; u < TU; ++u) add_positive<Tv>(raw[u], a0, a1);
     if (g % (128 / TU) == 0) flush_positive<Tv>(a0, a1, cnt);
   }
-  for (; t < n; ++t) add_positive<Tv>(*reinterpret_cast<const W*>(src + t * npix), a0, a1);
+  for (; t < n; ++t) add_positive<Tv>(load_raw<Tv, VEC>(src + t * npix, n_valid), a0, a1);
   flush_positive<Tv>(a0, a1, cnt);
 }
 
@@ -243,8 +269,8 @@ __global__ void __launch_bounds__(THREADS)
   uint32_t first[PX] = {NONE, NONE, NONE, NONE};
   long long sum[PX] = {0, 0, 0, 0};
   if (n_valid > 0) {
-    if (VEC && !THR && !SUM) {
-      count_positive<Tv>(frames + t0 * npix + p0, npix, t1 - t0, cnt);
+    if (!THR && !SUM) {
+      count_positive<Tv, VEC>(frames + t0 * npix + p0, npix, t1 - t0, n_valid, cnt);
     } else {
       walk_frames<Tv, VEC>(
           frames + t0 * npix + p0, npix, t0, t1, n_valid,
@@ -477,6 +503,182 @@ __global__ void __launch_bounds__(THREADS)
   if (bad) atomicOr(err, G2_DEVERR_BOUNDS);
 }
 
+// Passes 4 and 5 in one for stacks without a cut: the event lists straight
+// from the frames.  A CTA owns 128 pixels of one sub-block and walks its frames
+// in steps of 8 warps x CHUNK frames.  A warp reads its CHUNK frames of the 128
+// pixels (4 pixels per lane, all loads in flight together), keeps the words in
+// shared memory and, per pixel, a mask of the frames with an event; the masks'
+// counts tell where each warp's events of each pixel begin.  Then every lane
+// goes through its masks bit by bit and places the events pixel-major in shared
+// memory, and each warp writes 8 pixels' pieces of the lists, one after the other
+// (about 46 events of 8-bit frames at 9 % filled: 184 and 46 contiguous bytes).  A
+// step with more events than the buffer goes in 2, 4 or 8 rounds of warps.  The
+// stack is read once and nothing is staged in global memory: 514 x 1030 x 4,000
+// u8 at 0.1 per pixel 1.37 ms against 1.43 (stage) + 0.48 (gather).  Bound by
+// instructions and their latency (50 % of the issue slots); testing every value and
+// placing it under a predicate took 1.60 ms, CTAs of 16 warps 1.49
+// (21 instructions per value).
+constexpr int EMIT_PX = 128;
+constexpr int EMIT_WARPS = 8;
+constexpr int EMIT_BUF = 4864;  // words of events placed before they are written
+template <typename Tv> struct Emit { static constexpr int CHUNK = sizeof(Tv) == 1 ? 32 : 16; };
+constexpr int EMIT_SMEM = EMIT_BUF * 4 + EMIT_WARPS * 32 * 128;
+static_assert(EMIT_BUF >= 32 * EMIT_PX, "a round of one warp always fits");
+
+// Masks of the frames whose value is positive, per pixel, from the flags of
+// 8 (16-bit: 16) frames at a time: shifting a word of flags right once per frame
+// leaves frame k's flag in bit k of the pixel's byte (half word).
+template <typename Tv>
+__device__ __forceinline__ void frame_masks(const uint32_t (&raw)[32], uint32_t m[PX]) {
+  uint32_t a[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    a[g] = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a[g] = (a[g] >> 1) | positive_flags<Tv>(raw[8 * g + k]);
+  }
+#pragma unroll
+  for (int j = 0; j < PX; ++j) {
+    const uint32_t lo = __byte_perm(a[0], a[1], j | ((4 + j) << 4)), hi = __byte_perm(a[2], a[3], j | ((4 + j) << 4));
+    m[j] = __byte_perm(lo, hi, 0x5410);
+  }
+}
+template <typename Tv>
+__device__ __forceinline__ void frame_masks(const uint2 (&raw)[16], uint32_t m[PX]) {
+  uint32_t x = 0, y = 0;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    x = (x >> 1) | positive_flags<Tv>(raw[k].x);
+    y = (y >> 1) | positive_flags<Tv>(raw[k].y);
+  }
+  m[0] = x & 0xFFFFu;
+  m[1] = x >> 16;
+  m[2] = y & 0xFFFFu;
+  m[3] = y >> 16;
+}
+
+template <typename Tv, bool VEC>
+__global__ void __launch_bounds__(EMIT_WARPS * 32, 4)
+    emit_kernel(const Tv* __restrict__ frames, int32_t T, int64_t npix, const uint16_t* __restrict__ sb_counts,
+                const uint32_t* __restrict__ ev_off, int64_t n_events, int32_t* __restrict__ times,
+                Tv* __restrict__ data, int32_t* __restrict__ err) {
+  using W = typename Word4<Tv>::type;
+  using U = typename std::conditional<sizeof(Tv) == 1, uint8_t, uint16_t>::type;
+  constexpr int CHUNK = Emit<Tv>::CHUNK;
+  constexpr int STEP = EMIT_WARPS * CHUNK;
+  extern __shared__ __align__(16) uint32_t buf[];                 // EMIT_BUF words, then the warps' frames
+  __shared__ __align__(8) uint16_t s_cnt[EMIT_WARPS + 1][EMIT_PX];  // events of the pixel before warp w
+  __shared__ uint32_t s_start[EMIT_PX + 1];                       // first word of every pixel in the buffer
+  __shared__ uint32_t s_delta[EMIT_PX];
+  __shared__ uint32_t s_scan[EMIT_PX / 32];
+  __shared__ uint32_t s_total[EMIT_WARPS];                        // events of every warp
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t px0 = static_cast<int64_t>(blockIdx.x) * EMIT_PX;
+  const int64_t sb = blockIdx.y, t0 = sb * SUBBLOCK;
+  const int64_t t1 = t0 + SUBBLOCK < T ? t0 + SUBBLOCK : T;
+  const int64_t p0 = px0 + lane * PX;                             // this lane's pixels
+  const int64_t n_valid = p0 < npix ? (npix - p0 < PX ? npix - p0 : PX) : 0;
+  W* mine = reinterpret_cast<W*>(buf + EMIT_BUF) + warp * CHUNK * 32;
+  const U* values = reinterpret_cast<const U*>(mine + lane);      // value j of frame u: values[u * 128 + j]
+  // thread i < 128: where pixel i's next events go in its list, and its end
+  uint32_t out = 0, end = 0;
+  if (tid < EMIT_PX && px0 + tid < npix) {
+    const int64_t p = px0 + tid;
+    out = ev_off[p];
+    end = ev_off[p + 1] < n_events ? ev_off[p + 1] : static_cast<uint32_t>(n_events);
+    for (int64_t b = 0; b < sb; ++b) out += sb_counts[b * npix + p];
+  }
+  bool bad = false;
+  for (int64_t ts = t0; ts < t1; ts += STEP) {
+    const int64_t tw = ts + warp * CHUNK;                         // this warp's frames [tw, tw + nf)
+    const int nf = static_cast<int>(t1 - tw < CHUNK ? t1 - tw : CHUNK);
+    uint32_t m[PX];
+    {
+      W raw[CHUNK];
+      const Tv* src = frames + tw * npix + p0;
+#pragma unroll
+      for (int u = 0; u < CHUNK; ++u)
+        raw[u] = n_valid > 0 && u < nf ? load_raw<Tv, VEC>(src + u * npix, n_valid) : W{};
+#pragma unroll
+      for (int u = 0; u < CHUNK; ++u) mine[u * 32 + lane] = raw[u];
+      frame_masks<Tv>(raw, m);
+    }
+    const uint32_t n0 = __popc(m[0]), n1 = __popc(m[1]), n2 = __popc(m[2]), n3 = __popc(m[3]);
+    *reinterpret_cast<uint2*>(&s_cnt[warp][lane * PX]) = make_uint2(n0 | (n1 << 16), n2 | (n3 << 16));
+    const uint32_t all = __reduce_add_sync(0xffffffffu, n0 + n1 + n2 + n3);
+    if (lane == 0) s_total[warp] = all;
+    __syncthreads();
+    if (tid < EMIT_PX) {  // the pixel's events before every warp
+      uint32_t sum = 0;
+#pragma unroll
+      for (int w = 0; w < EMIT_WARPS; ++w) {
+        const uint32_t x = s_cnt[w][tid];
+        s_cnt[w][tid] = static_cast<uint16_t>(sum);
+        sum += x;
+      }
+      s_cnt[EMIT_WARPS][tid] = static_cast<uint16_t>(sum);
+    }
+    // warps per round: the most whose events fit the buffer in every round
+    int per = EMIT_WARPS;
+    for (; per > 1; per /= 2) {
+      bool fits = true;
+      for (int w = 0; w < EMIT_WARPS; w += per) {
+        uint32_t x = 0;
+        for (int k = 0; k < per; ++k) x += s_total[w + k];
+        fits &= x <= static_cast<uint32_t>(EMIT_BUF);
+      }
+      if (fits) break;
+    }
+    __syncthreads();
+    for (int w0 = 0; w0 < EMIT_WARPS; w0 += per) {
+      uint32_t n = 0, inc = 0;
+      if (tid < EMIT_PX) {  // where the round's events of every pixel begin
+        n = s_cnt[w0 + per][tid] - s_cnt[w0][tid];
+        inc = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += y;
+        }
+        if (lane == 31) s_scan[warp] = inc;
+      }
+      __syncthreads();
+      bool over = false;
+      if (tid < EMIT_PX) {
+        for (int w = 0; w < warp; ++w) inc += s_scan[w];
+        s_start[tid] = inc - n;
+        if (tid == EMIT_PX - 1) s_start[EMIT_PX] = inc;
+        s_delta[tid] = out - (inc - n);  // list position of an event less its place in the buffer
+        over = out + n > end;            // the stack changed between the passes
+        out += n;
+      }
+      bad |= over;
+      const bool skip = __syncthreads_or(over);
+      if (warp >= w0 && warp < w0 + per) {
+        const uint32_t rel = static_cast<uint32_t>(warp * CHUNK) << 16;
+#pragma unroll
+        for (int j = 0; j < PX; ++j) {
+          uint32_t* at = buf + s_start[lane * PX + j] + (s_cnt[warp][lane * PX + j] - s_cnt[w0][lane * PX + j]);
+          const uint32_t tag = rel + (static_cast<uint32_t>(lane * PX + j) << 25);
+          for (uint32_t k = m[j]; k; k &= k - 1) {
+            const int u = __ffs(k) - 1;
+            *at++ = tag + (u << 16) + values[u * 128 + j];
+          }
+        }
+      }
+      __syncthreads();
+      const uint32_t total = skip ? 0 : s_start[EMIT_PX];
+      for (uint32_t i = tid; i < total; i += EMIT_WARPS * 32) {
+        const uint32_t w = buf[i], g = s_delta[w >> 25] + i;
+        times[g] = static_cast<int32_t>(ts) + static_cast<int32_t>((w >> 16) & 511u);
+        data[g] = static_cast<Tv>(w & 0xFFFFu);
+      }
+      __syncthreads();
+    }
+  }
+  if (bad) atomicOr(err, G2_DEVERR_BOUNDS);
+}
+
 // Streaming: a thread per pixel appends the positive values of nb frames
 // (frame numbers frame0, frame0 + 1, ...) to its row of the (npix x max_nnz)
 // event and time arrays.  With a threshold, a value above it masks the pixel
@@ -676,6 +878,48 @@ extern "C" int g2_compress_finish(uint16_t* sb_counts_dev, const uint16_t* sb_fi
                                                                static_cast<int>(n_sb), nframes, npix, mask_dev,
                                                                blk_totals_dev, n_blk, counts_dev, t_cut_dev);
   return launch_status();
+}
+
+namespace {
+template <typename Tv>
+int launch_emit(const void* frames, bool vec, int32_t T, int64_t npix, const uint16_t* sbc, const uint32_t* off,
+                int64_t n_events, int32_t* times, void* data, int32_t* err, cudaStream_t st) {
+  constexpr int smem = cmp::EMIT_SMEM;
+  auto* kernel = vec ? cmp::emit_kernel<Tv, true> : cmp::emit_kernel<Tv, false>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return G2_ERR_CUDA;
+  const int64_t gx = (npix + cmp::EMIT_PX - 1) / cmp::EMIT_PX;
+  const int64_t gy = (static_cast<int64_t>(T) + cmp::SUBBLOCK - 1) / cmp::SUBBLOCK;
+  if (gx > 0x7fffffff || gy > 65535) return G2_ERR_TOO_LARGE;
+  kernel<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), cmp::EMIT_WARPS * 32, smem, st>>>(
+      reinterpret_cast<const Tv*>(frames), T, npix, sbc, off, n_events, times, reinterpret_cast<Tv*>(data), err);
+  return launch_status();
+}
+}  // namespace
+
+extern "C" int g2_compress_emit(const void* frames_dev, int32_t elem_kind, int32_t nframes, int64_t npix,
+                                const uint16_t* sb_counts_dev, const uint32_t* ev_offsets_dev, int64_t n_events,
+                                int32_t* ev_times_dev, void* ev_data_dev, int32_t* err_dev, void* stream) {
+  if (!frames_dev || !sb_counts_dev || !ev_offsets_dev || !ev_times_dev || !ev_data_dev || !err_dev ||
+      !kind_ok(elem_kind) || nframes <= 0 || npix <= 0 || n_events < 0)
+    return G2_ERR_ARG;
+  if (n_events >= (1ll << 32)) return G2_ERR_UNSUPPORTED;
+  const bool vec = npix % cmp::PX == 0 && aligned(frames_dev, static_cast<uintptr_t>(kind_bytes(elem_kind) * cmp::PX));
+  cudaStream_t st = as_stream(stream);
+  switch (elem_kind) {
+    case 1:
+      return launch_emit<uint8_t>(frames_dev, vec, nframes, npix, sb_counts_dev, ev_offsets_dev, n_events,
+                                  ev_times_dev, ev_data_dev, err_dev, st);
+    case -1:
+      return launch_emit<int8_t>(frames_dev, vec, nframes, npix, sb_counts_dev, ev_offsets_dev, n_events,
+                                 ev_times_dev, ev_data_dev, err_dev, st);
+    case 2:
+      return launch_emit<uint16_t>(frames_dev, vec, nframes, npix, sb_counts_dev, ev_offsets_dev, n_events,
+                                   ev_times_dev, ev_data_dev, err_dev, st);
+    default:
+      return launch_emit<int16_t>(frames_dev, vec, nframes, npix, sb_counts_dev, ev_offsets_dev, n_events,
+                                  ev_times_dev, ev_data_dev, err_dev, st);
+  }
 }
 
 extern "C" int g2_compress_stage(const void* frames_dev, int32_t elem_kind, int32_t nframes, int64_t npix,

@@ -492,6 +492,15 @@ int g2_events_gather_rel(const uint32_t* stage_dev, const uint32_t* tile_pos_dev
                          int32_t elem_bytes, uint32_t* ev_words_dev, int32_t* ev_times_dev, void* ev_data_dev,
                          int32_t* err_dev, void* stream);
 
+/* The event lists of a stack without threshold and mask straight from the
+ * frames, after g2_compress_count and the scan of the counts (sb_counts as
+ * g2_compress_count wrote them): the same ev_times_dev and ev_data_dev (the
+ * frames' type, n_events entries each) as g2_compress_stage and
+ * g2_events_gather_rel give. */
+int g2_compress_emit(const void* frames_dev, int32_t elem_kind, int32_t nframes, int64_t npix,
+                     const uint16_t* sb_counts_dev, const uint32_t* ev_offsets_dev, int64_t n_events,
+                     int32_t* ev_times_dev, void* ev_data_dev, int32_t* err_dev, void* stream);
+
 /* Streaming (process_frame and get_compacted_events, event.py:286-321): one
  * call appends n_batch frames (frame numbers frame0, frame0 + 1, ...) to the
  * per-pixel rows of events_dev (npix x max_nnz, the frames' type) and
