@@ -19,6 +19,7 @@ G2_OK = 0
 STATUS = {0: "ok", 1: "invalid argument", 2: "CUDA runtime error", 3: "unsupported device or feature",
           4: "size exceeds a kernel limit"}
 DEVERR_TIMEOUT, DEVERR_BOUNDS, DEVERR_RANGE, DEVERR_RANGE_CHECK, DEVERR_RESIDUAL = 1, 2, 4, 8, 16
+DEVERR_ENERGY = 32
 
 BK = 64          # source segment width (pixels)
 PAD = 128        # packed bins and packed_cols are multiples of this
@@ -28,7 +29,7 @@ PLAIN_BM, PLAIN_BN = 128, 128
 MAX_JOBS = 32
 ITEM_EMPTY = -1
 KIND_FP16, KIND_E4M3, KIND_E2M1 = 0, 1, 2
-KIND_BLOCKED = 256
+KIND_BLOCKED, KIND_SIGNED, KIND_CHECK = 256, 512, 1024
 NARROW_CHUNK = 4080
 RES_SECTOR = 64  # packed columns per residual list
 
@@ -66,6 +67,9 @@ SIGNATURES = {
     "g2_gram_tc_e2m1": (C.c_int, [_p, _i32, _p, _i64, _p, _i64, _p, _i64, _p, _i32, _p]),
     "g2_pack_u8_residual": (C.c_int, [_p, _i64, _i64, _i64, _i32, _p, _p, _p, _i64, _p, _i64, _i64, _p, _p, _i32, _p,
                                       _p]),
+    "g2_pack_blocked": (C.c_int, [_p, _i32, _i64, _i64, _i64, _i32, _p, _p, _p, _i64, _p, _i64, _i64, _p, _p]),
+    "g2_sample_energy": (C.c_int, [_p, _i32, _i64, _i64, _p, _i64, _p, _i64, _i64, _i32, _p, _p, _p]),
+    "g2_operand_rows": (C.c_int, [_p, _i64, _i64, _p, _p]),
     "g2_count_tail": (C.c_int, [_p, _i64, _i64, _p, _i64, _i64, _p, _p]),
     "g2_residual_sums": (C.c_int, [_p, _i64, _i64, _i64, _i32, _p, _p, _i32, _p, _i32, _p, _p, _p, _p, _p]),
     "g2_e2m1_offset": (C.c_int, [_p, _p, _i32, _i64, _p, _p, _p]),
@@ -169,4 +173,6 @@ def device_error_message(code):
         msgs.append("a count may not fit the packing (unchecked)")
     if code & DEVERR_RESIDUAL:
         msgs.append("more large counts than the narrow operand's residual lists hold")
+    if code & DEVERR_ENERGY:
+        msgs.append("a Gram's energy exceeds what its K split was planned for")
     return "; ".join(msgs) or "device error %d" % code

@@ -60,6 +60,8 @@ struct MapsParam {
   int32_t kind[G2_MAX_JOBS];
   int32_t ones[G2_MAX_JOBS];
   uint32_t blocked;              // bit per job: K-blocked operand, 3-D map (128 B, rows, blocks)
+  uint32_t is_signed;            // bit per job: signed elements
+  uint32_t check;                // bit per job: the items' diagonals are checked (G2_DEVERR_ENERGY)
 };
 
 __device__ __forceinline__ int stage_elems(int kind) { return kind == G2_KIND_E4M3 ? 128 : 64; }
@@ -95,7 +97,8 @@ __device__ __forceinline__ bool item_ok(const g2_gram_item& w, const MapsParam& 
   return w.k_len > 0 && (w.k_len % bk) == 0 && (w.a_k0 % bk) == 0 && (w.b_k0 % bk) == 0 && w.nframes > 0 &&
          w.i0 >= 0 && w.j0 >= 0 && w.j0 < w.nframes + 1 && w.out_off >= 0 && w.out_off + w.nframes <= numer_len &&
          w.shift >= 0 && w.shift <= 32 &&
-         (w.s_off < 0 || (maps.ones[w.job] && w.shift == 0 && w.s_off + w.nframes <= sums_len));
+         (w.s_off < 0 || (maps.ones[w.job] && (w.shift == 0 || ((maps.blocked >> w.job) & 1u)) &&
+                          w.s_off + w.nframes <= sums_len));
 }
 
 __device__ __forceinline__ bool named_bar_any(uint32_t id, uint32_t n, bool v) {
@@ -120,11 +123,10 @@ struct PairMaps<true> {
   using type = MapsParamF4;
 };
 
-// An epilogue sum as int64: e2m1 sums are signed (two's complement throughout).
-template <bool F4>
-__device__ __forceinline__ unsigned long long widen(uint32_t v) {
-  return F4 ? static_cast<unsigned long long>(static_cast<long long>(static_cast<int32_t>(v)))
-            : static_cast<unsigned long long>(v);
+// An epilogue sum as int64: signed sums are two's complement throughout.
+__device__ __forceinline__ unsigned long long widen(uint32_t v, bool is_signed) {
+  return is_signed ? static_cast<unsigned long long>(static_cast<long long>(static_cast<int32_t>(v)))
+                   : static_cast<unsigned long long>(v);
 }
 
 // F4: e2m1 operands on kind::mxf4 (every job); else e4m3 / fp16 operands.
@@ -339,12 +341,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       const bool row_live = i0 + row < w.nframes;
       const int n = item_n<F4>(w, maps);
       const int lag0 = w.j0 - i0 - (HALF - 1);
-      const int ones_col = w.s_off >= 0 ? w.nframes - w.j0 : -1;  // -1 or >= n: not in this block
+      const int ones_col = maps.ones[w.job] ? w.nframes - w.j0 : -1;  // -1 or >= n: not in this block
       // rows past the frames (the row of ones among them) contribute nothing;
       // columns past the frames are TMA zero fill, except the row of ones,
       // whose column goes to the bin sums
       const float us = row_live ? unscale : 0.0f;
       const int dwarp = (HALF - 1) - q * 32 + lane;  // lag index of offset `lane` in chunk 0
+      const bool sgn = F4 || ((maps.is_signed >> w.job) & 1u);
+      // the column of this row's own product, in an item of a plane with itself
+      const int own = !F4 && ((maps.check >> w.job) & 1u) && w.a_k0 == w.b_k0 ? i0 + row - w.j0 : -1;
+      const uint32_t most = sgn ? 1u << 23 : 1u << 24;
       uint32_t carry = 0;
 #pragma unroll 1
       for (int cc = 0; cc < n / 32; ++cc) {
@@ -355,14 +361,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           const float x = __uint_as_float(v[j]) * us;
-          v[j] = F4 ? static_cast<uint32_t>(__float2int_rn(x)) : __float2uint_rn(x);
+          v[j] = static_cast<uint32_t>(__float2int_rn(x));  // |x| < 2^31: a checked diagonal may be above 2^24
+        }
+        if (!F4 && __any_sync(0xffffffffu, (own >> 5) == cc)) {  // the rows' energies are in this chunk (own < 0: -1)
+          uint32_t e = 0;
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (own == cc * 32 + j) e = v[j];
+          if (row_live && e >= most) atomicOr(err, G2_DEVERR_ENERGY);
         }
         const int jx = ones_col - cc * 32;
         if (jx >= 0 && jx < 32) {  // warp-uniform
 #pragma unroll
           for (int j = 0; j < 32; ++j)
             if (j == jx) {
-              if (v[j]) atomicAdd(&sums[w.s_off + i0 + row], widen<F4>(v[j]));
+              // (byte planes: the high plane's Gram has shift 16, its bin sums 8)
+              if (v[j] && w.s_off >= 0)
+                atomicAdd(&sums[w.s_off + i0 + row], widen(v[j], sgn) << (w.shift >> 1));
               v[j] = 0;
             }
         }
@@ -385,7 +400,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         if (s) {
           const int tau = lag0 + d;
           if (tau >= 0 && tau < w.nframes)
-            atomicAdd(&numer[w.out_off + tau], widen<F4>(s) << w.shift);
+            atomicAdd(&numer[w.out_off + tau], widen(s, sgn) << w.shift);
           dacc[d] = 0;
         }
       }
@@ -715,20 +730,21 @@ int wide_max_clusters(int* out) {
   return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_wide_kernel), g2::pair::W_SMEM_BYTES, out);
 }
 
-// Checks the jobs and fills the tensor maps (box: 128 rows of one stage row).
-int pair_maps(const g2_job* jobs, int32_t n_jobs, g2::pair::MapsParam* maps) {
+// Checks the jobs (element kinds with the given flags) and fills the tensor
+// maps (box: 128 rows of one stage row).
+int pair_maps(const g2_job* jobs, int32_t n_jobs, int32_t flags, g2::pair::MapsParam* maps) {
   using namespace g2;
   for (int j = 0; j < n_jobs; ++j) {
     const g2_job& jb = jobs[j];
     if (!jb.packed_dev || !aligned(jb.packed_dev, 16) || jb.nframes <= 0 || jb.nframes >= (1ll << 31) ||
         jb.packed_cols <= 0 || jb.packed_cols % G2_PAD != 0 || jb.packed_cols >= (1ll << 31) ||
-        ((jb.elem_kind & ~G2_KIND_BLOCKED) != G2_KIND_FP16 && (jb.elem_kind & ~G2_KIND_BLOCKED) != G2_KIND_E4M3) ||
-        (jb.ones_row != 0 && jb.ones_row != 1))
+        ((jb.elem_kind & 255) != G2_KIND_FP16 && (jb.elem_kind & 255) != G2_KIND_E4M3) ||
+        (jb.elem_kind & ~(255 | flags)) != 0 || (jb.ones_row != 0 && jb.ones_row != 1))
       return G2_ERR_ARG;
   }
   std::memset(maps, 0, sizeof(*maps));
   for (int j = 0; j < n_jobs; ++j) {
-    const int32_t kind = jobs[j].elem_kind & ~G2_KIND_BLOCKED;
+    const int32_t kind = jobs[j].elem_kind & 255;
     const bool blocked = (jobs[j].elem_kind & G2_KIND_BLOCKED) != 0;
     const int eb = kind == G2_KIND_E4M3 ? 1 : 2;
     const uint64_t rows = static_cast<uint64_t>(jobs[j].nframes) + (jobs[j].ones_row ? 1 : 0);
@@ -738,6 +754,8 @@ int pair_maps(const g2_job* jobs, int32_t n_jobs, g2::pair::MapsParam* maps) {
                                             pair::ROW_BYTES / eb, pair::HALF);
     if (st != G2_OK) return st;
     if (blocked) maps->blocked |= 1u << j;
+    if (jobs[j].elem_kind & G2_KIND_SIGNED) maps->is_signed |= 1u << j;
+    if (jobs[j].elem_kind & G2_KIND_CHECK) maps->check |= 1u << j;
     maps->kind[j] = kind;
     maps->ones[j] = jobs[j].ones_row;
   }
@@ -773,7 +791,7 @@ int launch_pair(bool wide, const g2_job* jobs, int32_t n_jobs, const g2_gram_ite
   static pair::MapsParam maps;  // large; filled under the lock below
   static std::mutex* mu = new std::mutex;
   std::lock_guard<std::mutex> lk(*mu);
-  int st = pair_maps(jobs, n_jobs, &maps);
+  int st = pair_maps(jobs, n_jobs, wide ? G2_KIND_BLOCKED : G2_KIND_BLOCKED | G2_KIND_SIGNED | G2_KIND_CHECK, &maps);
   if (st != G2_OK) return st;
   if (n_items == 0) return G2_OK;
   int max_cl = 0;

@@ -22,6 +22,14 @@
 // become eight e2m1 codes in five instructions (code8).
 // Counts that may need a residual (a byte of 8 or more, or of 16 or
 // more) are found by one OR over the unit's words and take a slow path.
+//
+// The same walk packs 16-bit operands (g2_pack_blocked): counts up to 2048 as
+// fp16 patterns, or two planes of signed digits for larger ones.  It computes
+// no energy bounds (sample_energy_kernel and the Gram's own diagonal take their
+// place) and no bin sums (row of ones), so that only the bytes bound it: 5,000
+// u16 frames of 256 x 256 0.46 -> 0.22 ms (1.14 GB of DRAM traffic, 5.1 TB/s),
+// 1,500 of 195 x 487 in digits 0.51 -> 0.14 ms.  Signed digits halve a byte's
+// square: fewer K chunks, and no unsigned plane of energy 255^2 per pixel.
 #include "g2_ptx.cuh"
 #include "g2_host.h"
 
@@ -30,19 +38,24 @@ namespace tail {
 
 constexpr int CH = G2_NARROW_CHUNK;     // source pixels per chunk
 constexpr int F = 4;                    // frames per step
-constexpr int ROW = CH + 48;            // bytes of a staged frame row: the chunk from its 16-byte aligned start, spare words
+constexpr int ROW = CH + 48;            // bytes of a staged u8 frame row: the chunk from its 16-byte aligned start, spare words
 static_assert(ROW % 16 == 0 && CH % 16 == 0 && CH <= 0xFFF, "bulk copy rows, 12-bit sources");
 // Warps, ring stages and CTAs per SM: few CTAs, so that a mover's step of F
 // frames stays in registers (80 per thread).  3,000 frames of 514 x 1030, e2m1:
 // 0.54 ms with 5 CTAs of 256 threads and 2 stages (48 registers, spills), 0.43
 // with 3 and 3 stages; 512 x 512 x 3,001, e4m3 (twice the blocks per chunk): 0.37
 // and 0.37, 0.33 with 3 CTAs of 384 threads and 2 stages.
-template <bool E2M1>
+// What a walk packs: e2m1 or e4m3 with residuals, fp16 from u8 or u16 counts,
+// two planes of signed digits from u16 counts.
+enum Element { EL_E2M1, EL_E4M3, EL_FP16_U8, EL_FP16_U16, EL_DIGITS };
+template <Element EL>
 struct Cfg {
-  static constexpr int THREADS = E2M1 ? 256 : 384;
+  static constexpr int THREADS = EL == EL_E2M1 ? 256 : 384;
   static constexpr int MOVERS = THREADS / 32 - 1;
-  static constexpr int STAGES = E2M1 ? 3 : 2;
+  static constexpr int STAGES = EL == EL_E2M1 ? 3 : 2;
   static constexpr int CTAS_PER_SM = 3;
+  static constexpr int ES = EL == EL_FP16_U16 || EL == EL_DIGITS ? 2 : 1;  // bytes of a source count
+  static constexpr int ROW = CH * ES + 48;
 };
 constexpr uint32_t UNIT_VEC = 1, UNIT_WORD = 2, UNIT_GATHER = 3;
 constexpr int SECTOR = 64;                            // packed columns per residual list
@@ -255,6 +268,94 @@ __device__ __forceinline__ void move_e4m3(const uint4& u, const uint8_t* base, u
   }
 }
 
+// A word of two u16 counts as two signed digits each, count = 256 high + low,
+// low in [-128, 127] as an fp16 pattern (sign and magnitude).
+__device__ __forceinline__ void digits2(uint32_t w, uint32_t& high, uint32_t& low) {
+  const uint32_t lo = w & 0x00FF00FFu, neg = (lo >> 7) & 0x00010001u;
+  high = ((w >> 8) & 0x00FF00FFu) + neg;
+  low = ((lo ^ (neg * 0xFFu)) + neg) | (neg << 15);  // 256 - lo where negative
+}
+__device__ __forceinline__ bool above2048(uint32_t w) { return (w & 0xFFFFu) > 2048u || (w >> 16) > 2048u; }
+
+// One unit of a 16-bit operand: 8 or 2 consecutive counts or two gathered ones
+// to 16 or 4 bytes, with EL_DIGITS in two planes, the low one u.w bytes on.
+template <Element EL>
+__device__ __forceinline__ void move_wide(const uint4& u, const uint8_t* base, uint32_t phase, uint32_t step,
+                                          uint8_t* out, int64_t pitch, uint32_t row_bytes, int nf, bool& big,
+                                          bool& bad) {
+  constexpr int ES = Cfg<EL>::ES, ROW_B = Cfg<EL>::ROW;
+  const uint32_t cls = u.x >> 30, dst = u.x & 0x3FFFFFFFu, sa = u.y & 0xFFFFu;
+  const uint32_t plane = EL == EL_DIGITS ? u.w : 0u;
+  if (cls == UNIT_VEC) {
+    if (dst >= row_bytes / 16 || plane % 128 != 0 || plane >= row_bytes || 16 * dst >= row_bytes - plane ||
+        sa > CH - 8) {
+      bad = true;
+      return;
+    }
+    uint8_t* o = out + blk_off(16 * dst, 0, pitch);
+    uint8_t* o_low = o + static_cast<int64_t>(plane >> 7) * pitch;
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      if (f >= nf) break;
+      const uint32_t d = ((phase + f * step) & 15u) + f * ROW_B + ES * sa;
+      uint4 v;
+      if (ES == 2) {
+        v = load16(base, d);
+      } else {
+        const uint32_t a = load4(base, d), b = load4(base, d + 4);
+        v = make_uint4(__byte_perm(a, 0, 0x4140), __byte_perm(a, 0, 0x4342), __byte_perm(b, 0, 0x4140),
+                       __byte_perm(b, 0, 0x4342));
+      }
+      if (EL == EL_DIGITS) {
+        uint4 h, l;
+        digits2(v.x, h.x, l.x);
+        digits2(v.y, h.y, l.y);
+        digits2(v.z, h.z, l.z);
+        digits2(v.w, h.w, l.w);
+        *reinterpret_cast<uint4*>(o + f * 128) = h;
+        *reinterpret_cast<uint4*>(o_low + f * 128) = l;
+      } else {
+        if (EL == EL_FP16_U16 && ((v.x | v.y | v.z | v.w) & 0xF800F800u))
+          big |= above2048(v.x) || above2048(v.y) || above2048(v.z) || above2048(v.w);
+        *reinterpret_cast<uint4*>(o + f * 128) = v;
+      }
+    }
+  } else if (cls == UNIT_WORD || cls == UNIT_GATHER) {
+    const bool word = cls == UNIT_WORD;
+    if (dst >= row_bytes / 4 || plane % 128 != 0 || plane >= row_bytes || 4 * dst >= row_bytes - plane ||
+        (word && sa > CH - 2)) {
+      bad = true;
+      return;
+    }
+    // 12-bit sources; a gathered word's second one is NO_SRC (at least CH) in a column of padding
+    const uint32_t s0 = word ? sa : u.y & 0xFFFu, s1 = word ? sa + 1 : (u.y >> 12) & 0xFFFu;
+    uint8_t* o = out + blk_off(4 * dst, 0, pitch);
+    uint8_t* o_low = o + static_cast<int64_t>(plane >> 7) * pitch;
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      if (f >= nf) break;
+      const uint8_t* q = base + ((phase + f * step) & 15u) + f * ROW_B;
+      uint32_t v = 0;
+      if (ES == 2) {
+        if (s0 < CH) v = *reinterpret_cast<const uint16_t*>(q + 2 * s0);
+        if (s1 < CH) v |= static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(q + 2 * s1)) << 16;
+      } else {
+        if (s0 < CH) v = q[s0];
+        if (s1 < CH) v |= static_cast<uint32_t>(q[s1]) << 16;
+      }
+      if (EL == EL_DIGITS) {
+        uint32_t h, l;
+        digits2(v, h, l);
+        *reinterpret_cast<uint32_t*>(o + f * 128) = h;
+        *reinterpret_cast<uint32_t*>(o_low + f * 128) = l;
+      } else {
+        if (EL == EL_FP16_U16) big |= above2048(v);
+        *reinterpret_cast<uint32_t*>(o + f * 128) = v;
+      }
+    }
+  }
+}
+
 // Persistent CTAs; a work item is a step of F frames over one band of chunks.
 // The CTA walks the band chunk by chunk through a ring of STAGES staged chunks:
 // warp 0 lane 0 bulk-copies the F frames' binned span of the chunk, the mover
@@ -265,16 +366,16 @@ __device__ __forceinline__ void move_e4m3(const uint4& u, const uint8_t* base, u
 // of the written bytes left L2 as partly filled lines (T = 10,000 frames of
 // 514 x 1030, DRAM read 7.05 GB of 5.29, written 3.02 GB of 1.95).
 // frame0: number of the launch's first frame in the stack.
-template <bool E2M1>
-__global__ void __launch_bounds__(Cfg<E2M1>::THREADS, Cfg<E2M1>::CTAS_PER_SM)
+template <Element EL>
+__global__ void __launch_bounds__(Cfg<EL>::THREADS, Cfg<EL>::CTAS_PER_SM)
     pack_walk_kernel(const uint8_t* __restrict__ frames, int64_t T, int64_t npix, uint32_t frame0,
                      const int32_t* __restrict__ block_off, const uint4* __restrict__ units,
                      const uint32_t* __restrict__ spans, int32_t n_chunks, int32_t n_bands,
                      uint8_t* __restrict__ packed, int64_t pitch, uint32_t row_bytes, Residuals res,
                      int32_t* __restrict__ err) {
-  constexpr int MOVERS = Cfg<E2M1>::MOVERS, STAGES = Cfg<E2M1>::STAGES;
+  constexpr int MOVERS = Cfg<EL>::MOVERS, STAGES = Cfg<EL>::STAGES, ES = Cfg<EL>::ES;
   extern __shared__ __align__(128) uint8_t s_dyn[];
-  auto s_buf = reinterpret_cast<uint8_t(*)[F][ROW]>(s_dyn);
+  auto s_buf = reinterpret_cast<uint8_t(*)[F][Cfg<EL>::ROW]>(s_dyn);
   __shared__ __align__(8) uint64_t full[STAGES];
   __shared__ __align__(8) uint64_t empty[STAGES];
   __shared__ int s_abort;
@@ -291,7 +392,7 @@ __global__ void __launch_bounds__(Cfg<E2M1>::THREADS, Cfg<E2M1>::CTAS_PER_SM)
   }
   __syncthreads();
   volatile int* abort_flag = &s_abort;
-  const int64_t total_bytes = T * npix;
+  const int64_t total_bytes = T * npix * ES;
   const int64_t n_items = (T + F - 1) / F * n_bands;
   uint32_t k = 0;  // staged chunks so far
 
@@ -322,9 +423,9 @@ __global__ void __launch_bounds__(Cfg<E2M1>::THREADS, Cfg<E2M1>::CTAS_PER_SM)
 #pragma unroll
             for (int f = 0; f < F; ++f) {
               if (f >= nf) break;
-              const int64_t start = (t0 + f) * npix + p0;
-              const int64_t a = (start + (span & 0xFFFFu)) & ~int64_t(15);
-              int64_t e = (start + (span >> 16) + 15) & ~int64_t(15);
+              const int64_t start = ((t0 + f) * npix + p0) * ES;
+              const int64_t a = (start + ES * (span & 0xFFFFu)) & ~int64_t(15);
+              int64_t e = (start + ES * (span >> 16) + 15) & ~int64_t(15);
               if (e > total_bytes) e = total_bytes;
               const uint32_t n = static_cast<uint32_t>(e - a), n16 = n & ~15u;
               uint8_t* dst = &s_buf[s][f][a - (start & ~int64_t(15))];
@@ -354,7 +455,7 @@ __global__ void __launch_bounds__(Cfg<E2M1>::THREADS, Cfg<E2M1>::CTAS_PER_SM)
 
   // -------------------------------------------------------------- movers
   const int mw = warp - 1;
-  bool bad = false, ok = true;
+  bool bad = false, ok = true, big = false;
   for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
     const int64_t g = item / n_bands;
     const int band = static_cast<int>(item - g * n_bands);
@@ -364,7 +465,7 @@ __global__ void __launch_bounds__(Cfg<E2M1>::THREADS, Cfg<E2M1>::CTAS_PER_SM)
     const int nf = static_cast<int>(T - t0 < F ? T - t0 : F);
     const uint32_t t = frame0 + static_cast<uint32_t>(t0);
     uint8_t* out = packed + static_cast<int64_t>(t) * 128;
-    const uint32_t start = static_cast<uint32_t>(t0 * npix), step = static_cast<uint32_t>(npix);
+    const uint32_t start = static_cast<uint32_t>(t0 * npix * ES), step = static_cast<uint32_t>(npix * ES);
     const int band_end = block_off[c1];
     int b1 = block_off[c0];
     int j = b1 + (mw + MOVERS - b1 % MOVERS) % MOVERS;  // this warp's next block
@@ -380,20 +481,79 @@ __global__ void __launch_bounds__(Cfg<E2M1>::THREADS, Cfg<E2M1>::CTAS_PER_SM)
         break;
       }
       ++k;
-      const uint32_t phase = start + static_cast<uint32_t>(c) * CH;
+      const uint32_t phase = start + static_cast<uint32_t>(c) * (CH * ES);
       const uint8_t* base = &s_buf[s][0][0];
       while (j < b1) {
         const uint4 w = u;
         j += MOVERS;
         if (j < band_end) u = units[static_cast<int64_t>(j) * 32 + lane];
-        if (E2M1) move_e2m1(w, base, phase, step, out, pitch, row_bytes, nf, t, res, err, bad);
-        else move_e4m3(w, base, phase, step, out, pitch, row_bytes, nf, t, res, err, bad);
+        if constexpr (EL == EL_E2M1) move_e2m1(w, base, phase, step, out, pitch, row_bytes, nf, t, res, err, bad);
+        else if constexpr (EL == EL_E4M3) move_e4m3(w, base, phase, step, out, pitch, row_bytes, nf, t, res, err, bad);
+        else move_wide<EL>(w, base, phase, step, out, pitch, row_bytes, nf, big, bad);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
     }
   }
   if (bad) atomicOr(err, G2_DEVERR_BOUNDS);
+  if (big) atomicOr(err, G2_DEVERR_RANGE);
+}
+
+// Energies of 128-column units (sums of squares, digits: of each plane) in
+// n_sample frames spread over the stack, a warp per frame and unit, and the
+// largest count.  A unit's sum of squares is below 128 * 65535^2 < 2^40.
+template <typename E, bool DIGITS>
+__global__ void __launch_bounds__(256)
+    sample_energy_kernel(const E* __restrict__ frames, int64_t T, int64_t npix, const int32_t* __restrict__ col_src,
+                         int64_t n_cols, const int32_t* __restrict__ unit_col, int64_t n_units, int64_t n_sample,
+                         unsigned long long* __restrict__ energy, uint32_t* __restrict__ most) {
+  const int lane = threadIdx.x & 31;
+  const int64_t total = n_sample * n_units, n_warps = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
+  uint32_t top = 0;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32; i < total; i += n_warps) {
+    const int64_t k = i / n_units, u = i - k * n_units;
+    const E* f = frames + ((2 * k + 1) * T / (2 * n_sample)) * npix;
+    unsigned long long e0 = 0, e1 = 0;
+    for (int j = lane; j < G2_PAD; j += 32) {
+      const int64_t c = unit_col[u] + j;
+      const int64_t s = c >= 0 && c < n_cols ? col_src[c] : -1;
+      const uint32_t v = s >= 0 && s < npix ? f[s] : 0u;
+      top = max(top, v);
+      if (DIGITS) {
+        const int l = static_cast<int>((v & 255u) ^ 128u) - 128;
+        const uint32_t h = (v >> 8) + ((v >> 7) & 1u);
+        e0 += h * h;
+        e1 += static_cast<uint32_t>(l * l);
+      } else {
+        e0 += static_cast<unsigned long long>(v) * v;
+      }
+    }
+#pragma unroll
+    for (int d = 16; d; d /= 2) {
+      e0 += __shfl_xor_sync(0xffffffffu, e0, d);
+      if (DIGITS) e1 += __shfl_xor_sync(0xffffffffu, e1, d);
+    }
+    if (lane == 0) {
+      if (DIGITS) {
+        energy[2 * k * n_units + u] = e0;
+        energy[(2 * k + 1) * n_units + u] = e1;
+      } else {
+        energy[k * n_units + u] = e0;
+      }
+    }
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0 && top) atomicMax(most, top);
+}
+
+// A row-major copy of a K-blocked operand, 16 bytes per thread.
+__global__ void __launch_bounds__(256)
+    rows_kernel(const uint8_t* __restrict__ in, int64_t rows, int64_t row_bytes, uint8_t* __restrict__ out) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x, per = row_bytes / 16;
+  if (i >= rows * per) return;
+  const int64_t t = i / per;
+  reinterpret_cast<uint4*>(out)[i] =
+      *reinterpret_cast<const uint4*>(in + blk_off(static_cast<uint32_t>((i - t * per) * 16), t, rows * 128));
 }
 
 // Counts, among the binned pixels of n_sample frames spread over the stack, of
@@ -703,6 +863,42 @@ __global__ void __launch_bounds__(64)
   }
 }
 
+// Arguments of one walk.
+struct Walk {
+  const uint8_t* frames;
+  int64_t nframes, npix, frame0;
+  const int32_t* block_off;
+  const uint4* units;
+  const uint32_t* spans;
+  int64_t n_chunks;
+  uint8_t* packed;
+  int64_t packed_rows, row_bytes;
+  Residuals res;
+  int32_t* err;
+  cudaStream_t stream;
+};
+
+template <Element EL>
+int launch_walk(const Walk& w) {
+  const int sms = sm_count_current();
+  if (sms <= 0) return G2_ERR_CUDA;
+  // bands: about eight work items per resident CTA, of at least four chunks
+  const int64_t ctas = sms * static_cast<int64_t>(Cfg<EL>::CTAS_PER_SM);
+  const int64_t groups = (w.nframes + F - 1) / F;
+  int64_t bands = (8 * ctas + groups - 1) / groups;
+  if (bands > (w.n_chunks + 3) / 4) bands = (w.n_chunks + 3) / 4;
+  if (bands < 1) bands = 1;
+  const unsigned grid = static_cast<unsigned>(groups * bands < ctas ? groups * bands : ctas);
+  constexpr int smem = Cfg<EL>::STAGES * F * Cfg<EL>::ROW;
+  if (cudaFuncSetAttribute(pack_walk_kernel<EL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return G2_ERR_CUDA;
+  pack_walk_kernel<EL><<<grid, Cfg<EL>::THREADS, smem, w.stream>>>(
+      w.frames, w.nframes, w.npix, static_cast<uint32_t>(w.frame0), w.block_off, w.units, w.spans,
+      static_cast<int32_t>(w.n_chunks), static_cast<int32_t>(bands), w.packed, w.packed_rows * 128,
+      static_cast<uint32_t>(w.row_bytes), w.res, w.err);
+  return launch_status();
+}
+
 }  // namespace tail
 }  // namespace g2
 
@@ -739,31 +935,69 @@ extern "C" int g2_pack_u8_residual(const void* frames_dev, int64_t nframes, int6
     return G2_ERR_ARG;
   if (!aligned(packed_dev, 16) || !aligned(frames_dev, 16) || !aligned(units_dev, 16)) return G2_ERR_ARG;
   if (n_chunks > 0x7fffffff) return G2_ERR_TOO_LARGE;
+  tail::Walk w{reinterpret_cast<const uint8_t*>(frames_dev), nframes, npix, frame0, unit_block_off_dev,
+               reinterpret_cast<const uint4*>(units_dev), spans_dev, n_chunks, reinterpret_cast<uint8_t*>(packed_dev),
+               packed_rows, e2m1 ? packed_cols / 2 : packed_cols, res, err_dev, as_stream(stream)};
+  return e2m1 ? tail::launch_walk<tail::EL_E2M1>(w) : tail::launch_walk<tail::EL_E4M3>(w);
+}
+
+extern "C" int g2_pack_blocked(const void* frames_dev, int32_t elem_bytes, int64_t nframes, int64_t npix,
+                               int64_t frame0, int32_t mode, const int32_t* unit_block_off_dev,
+                               const uint32_t* units_dev, const uint32_t* spans_dev, int64_t n_chunks,
+                               void* packed_dev, int64_t packed_rows, int64_t packed_cols, int32_t* err_dev,
+                               void* stream) {
+  using namespace g2;
+  constexpr int64_t ch = G2_NARROW_CHUNK;
+  if (!frames_dev || !unit_block_off_dev || !units_dev || !spans_dev || !packed_dev || !err_dev ||
+      (elem_bytes != 1 && elem_bytes != 2) || (mode != 0 && mode != 1) || (mode == 1 && elem_bytes != 2) ||
+      nframes <= 0 || npix <= 0 || frame0 < 0 || packed_rows < frame0 + nframes || packed_rows >= (1ll << 31) ||
+      n_chunks != (npix + ch - 1) / ch || packed_cols <= 0 || packed_cols % G2_PAD != 0 || packed_cols >= (1ll << 30))
+    return G2_ERR_ARG;
+  if (!aligned(packed_dev, 16) || !aligned(frames_dev, 16) || !aligned(units_dev, 16)) return G2_ERR_ARG;
+  if (n_chunks > 0x7fffffff) return G2_ERR_TOO_LARGE;
+  tail::Walk w{reinterpret_cast<const uint8_t*>(frames_dev), nframes, npix, frame0, unit_block_off_dev,
+               reinterpret_cast<const uint4*>(units_dev), spans_dev, n_chunks, reinterpret_cast<uint8_t*>(packed_dev),
+               packed_rows, 2 * packed_cols, Residuals{}, err_dev, as_stream(stream)};
+  if (mode == 1) return tail::launch_walk<tail::EL_DIGITS>(w);
+  return elem_bytes == 2 ? tail::launch_walk<tail::EL_FP16_U16>(w) : tail::launch_walk<tail::EL_FP16_U8>(w);
+}
+
+extern "C" int g2_sample_energy(const void* frames_dev, int32_t elem_bytes, int64_t nframes, int64_t npix,
+                                const int32_t* col_src_dev, int64_t n_cols, const int32_t* unit_col_dev,
+                                int64_t n_units, int64_t n_sample, int32_t mode, uint64_t* energy_dev,
+                                uint32_t* max_dev, void* stream) {
+  using namespace g2;
+  if (!frames_dev || !col_src_dev || !unit_col_dev || !energy_dev || !max_dev || (elem_bytes != 1 && elem_bytes != 2) ||
+      (mode != 0 && mode != 1) || nframes <= 0 || nframes >= (1ll << 31) || npix <= 0 || n_cols <= 0 || n_units <= 0 ||
+      n_sample <= 0 || n_sample > nframes || (elem_bytes == 2 && !aligned(frames_dev, 2)))
+    return G2_ERR_ARG;
   const int sms = sm_count_current();
   if (sms <= 0) return G2_ERR_CUDA;
-  // bands: about eight work items per resident CTA, of at least four chunks
-  const int64_t ctas = sms * static_cast<int64_t>(e2m1 ? tail::Cfg<true>::CTAS_PER_SM : tail::Cfg<false>::CTAS_PER_SM);
-  const int64_t groups = (nframes + tail::F - 1) / tail::F;
-  int64_t bands = (8 * ctas + groups - 1) / groups;
-  if (bands > (n_chunks + 3) / 4) bands = (n_chunks + 3) / 4;
-  if (bands < 1) bands = 1;
-  const unsigned grid = static_cast<unsigned>(groups * bands < ctas ? groups * bands : ctas);
-  const int32_t nb = static_cast<int32_t>(bands);
-#define G2_WALK_LAUNCH(E)                                                                                            \
-  do {                                                                                                               \
-    constexpr int smem = tail::Cfg<E>::STAGES * tail::F * tail::ROW;                                                 \
-    if (cudaFuncSetAttribute(tail::pack_walk_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=        \
-        cudaSuccess)                                                                                                 \
-      return G2_ERR_CUDA;                                                                                            \
-    tail::pack_walk_kernel<E><<<grid, tail::Cfg<E>::THREADS, smem, as_stream(stream)>>>(                             \
-        reinterpret_cast<const uint8_t*>(frames_dev), nframes, npix, static_cast<uint32_t>(frame0),                  \
-        unit_block_off_dev, reinterpret_cast<const uint4*>(units_dev), spans_dev, static_cast<int32_t>(n_chunks),    \
-        nb, reinterpret_cast<uint8_t*>(packed_dev), packed_rows * 128,                                               \
-        static_cast<uint32_t>(E ? packed_cols / 2 : packed_cols), res, err_dev);                                     \
-  } while (0)
-  if (e2m1) G2_WALK_LAUNCH(true);
-  else G2_WALK_LAUNCH(false);
-#undef G2_WALK_LAUNCH
+  const int64_t want = (n_sample * n_units + 7) / 8;
+  const unsigned grid = static_cast<unsigned>(want < sms * 8ll ? want : sms * 8ll);
+  auto* e = reinterpret_cast<unsigned long long*>(energy_dev);
+  cudaStream_t st = as_stream(stream);
+#define G2_SAMPLE_LAUNCH(E, D)                                                                                       \
+  tail::sample_energy_kernel<E, D><<<grid, 256, 0, st>>>(reinterpret_cast<const E*>(frames_dev), nframes, npix,      \
+                                                         col_src_dev, n_cols, unit_col_dev, n_units, n_sample, e,   \
+                                                         max_dev)
+  if (elem_bytes == 2 && mode == 1) G2_SAMPLE_LAUNCH(uint16_t, true);
+  else if (elem_bytes == 2) G2_SAMPLE_LAUNCH(uint16_t, false);
+  else if (mode == 1) G2_SAMPLE_LAUNCH(uint8_t, true);
+  else G2_SAMPLE_LAUNCH(uint8_t, false);
+#undef G2_SAMPLE_LAUNCH
+  return launch_status();
+}
+
+extern "C" int g2_operand_rows(const void* packed_dev, int64_t rows, int64_t row_bytes, void* out_dev, void* stream) {
+  using namespace g2;
+  if (!packed_dev || !out_dev || rows <= 0 || rows >= (1ll << 31) || row_bytes <= 0 || row_bytes % 128 != 0 ||
+      row_bytes >= (1ll << 31) || !aligned(packed_dev, 16) || !aligned(out_dev, 16))
+    return G2_ERR_ARG;
+  const int64_t blocks = (rows * (row_bytes / 16) + 255) / 256;
+  if (blocks > 0x7fffffff) return G2_ERR_TOO_LARGE;
+  tail::rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, as_stream(stream)>>>(
+      reinterpret_cast<const uint8_t*>(packed_dev), rows, row_bytes, reinterpret_cast<uint8_t*>(out_dev));
   return launch_status();
 }
 

@@ -104,8 +104,8 @@ def qmask_digest(qmask):
 
 
 def device_layout(qmask, n_bins, mode, dev, digest=None, narrow=False):
-    """The packing layout of a q-mask (``narrow``: the NarrowLayout of e2m1 or
-    e4m3) with its read-only tables on ``dev``, shared process-wide (least recently used of 48 kept): building one costs
+    """The packing layout of a q-mask (``narrow``: the K-blocked NarrowLayout)
+    with its read-only tables on ``dev``, shared process-wide (least recently used of 48 kept): building one costs
     host time proportional to the frame size.  ``digest``: the q-mask's
     :func:`qmask_digest` when the caller has it."""
     torch = _torch()
@@ -121,7 +121,7 @@ def device_layout(qmask, n_bins, mode, dev, digest=None, narrow=False):
         L = NarrowLayout(q, n_bins, mode)
         L.d_col_src, L.d_sector_bin, L.d_npix = d(L.col_src), d(L.sector_bin), d(L.npix)
         L.d_unit_block_off, L.d_units = d(L.unit_block_off), d(L.units.view(np.int32))
-        L.d_chunk_span = d(L.chunk_span.view(np.int32))
+        L.d_chunk_span, L.d_unit_col = d(L.chunk_span.view(np.int32)), d(L.unit_col)
         return _keep_layout(key, L)
     L = PackLayout(q, n_bins, mode)
     L.d_col_src = d(L.col_src)
@@ -317,6 +317,10 @@ class DenseEngine(ResultBuffers):
         self._narrow = None       # narrow operand of the next u8 stack (see _narrow_mode): None = look first
         self._narrow_age = 0
         self._narrow_over = set()  # narrow operands whose residual lists a stack has overflowed
+        self._wide_plan = None    # 16-bit operand and K split of the next stack (see _wide_mode): None = look first
+        self._wide_age = 0
+        self._wide_from = MODE_FP16   # MODE_BYTES after a stack's counts above 2048
+        self._wide_margin = 0     # index into WIDE_MARGIN, raised when a stack exceeded its K split's energies
         self._residuals = None    # (layout, counts, lists, capacity) of the last narrow run
         self._packed_mode = None
         self.pipeline = True      # chunked copy/pack/Gram overlap where it applies
@@ -339,7 +343,8 @@ class DenseEngine(ResultBuffers):
         if operand not in ("auto", "e4m3", "fp16", "bytes"):
             raise ValueError("operand hint must be 'auto', 'e4m3', 'fp16' or 'bytes'")
         self.operand_hint = operand
-        self._narrow = None
+        self._narrow = self._wide_plan = None
+        self._wide_from, self._wide_margin = MODE_FP16, 0
         if self.method != "tc" or self.operand != "auto":
             return
         mode = MODE_E4M3 if operand == "auto" else self.MODES[operand]
@@ -749,7 +754,7 @@ class DenseEngine(ResultBuffers):
         chunks = self.pipe_chunks if chunks is None else int(chunks)
         kind = "pair4" if L.mode == MODE_E2M1 else self.item_kind
         key = ("pipe", L.mode, self.T, self.exact_limit, self.grid, chunks, self.super_rows, self.kslab,
-               kind, self.pipe_growth, int(taper), None if grams is None else tuple(grams),
+               kind, self.ones(L), self.pipe_growth, int(taper), None if grams is None else tuple(grams),
                tuple(L.grams()))
         if key not in self._items_cache:
             torch = _torch()
@@ -790,12 +795,14 @@ class DenseEngine(ResultBuffers):
 
     def pipelined_ok(self, frames):
         """The chunked pipeline applies on the tensor-core path to u8 stacks
-        on narrow operands (see :meth:`_narrow_ok`), to u8 stacks while their
+        on narrow operands (see :meth:`_narrow_ok`), to larger stacks on K-blocked
+        16-bit ones (:meth:`_wide_ok`), to u8 stacks while their
         counts are known (or expected) to be <= 16 (e4m3), and to u8 / u16
         stacks in pinned host memory on fp16 operands once a K split can be
         reused (see :meth:`_speculative_ok`): fp16 packs keep no per-frame
         state except energy maxima, which chunks combine."""
-        return (self._narrow_ok(frames) and self._narrow != MODE_FP16) or self._pipeline_mode(frames) is not None
+        return ((self._narrow_ok(frames) and self._narrow != MODE_FP16) or self._wide_ok(frames)
+                or self._pipeline_mode(frames) is not None)
 
     def _pipeline_input(self, frames):
         torch = _torch()
@@ -836,12 +843,15 @@ class DenseEngine(ResultBuffers):
     TAIL_FRAMES_HOST = 8
     NARROW_LOOK = 8       # stacks on fp16 operands between two looks
 
-    def _narrow_ok(self, frames):
-        """Whether a stack may run on a narrow operand (by its type and size)."""
-        torch = _torch()
-        return (self._pipeline_input(frames) and frames.dtype == torch.uint8 and frames.is_contiguous()
+    def _blocked_ok(self, frames):
+        """Whether a stack may run on a K-blocked operand (by its type and size)."""
+        return (self._pipeline_input(frames) and frames.is_contiguous()
                 and self.operand == "auto" and self.operand_hint == "auto" and self.tile == "pair"
                 and self.exact_limit >= EXACT_LIMIT and self.T < 2 ** 31 and self._macs() >= self.NARROW_MIN_MACS)
+
+    def _narrow_ok(self, frames):
+        """Whether a stack may run on a narrow operand."""
+        return self._blocked_ok(frames) and frames.element_size() == 1
 
     def _binned_pixels(self):
         """Pixels in the bins (an element layout that exists anyway counts them)."""
@@ -870,13 +880,7 @@ class DenseEngine(ResultBuffers):
         if not self._narrow_ok(frames):
             return None
         if self._narrow is None:
-            n = min(self.T, self.TAIL_FRAMES if frames.is_cuda else self.TAIL_FRAMES_HOST)
-            src, T = frames, self.T
-            if not frames.is_cuda:
-                pick = [(2 * k + 1) * self.T // (2 * n) for k in range(n)]
-                src, T = _torch().empty((n,) + self.shape, dtype=frames.dtype, device=self.dev), n
-                for k, t in enumerate(pick):
-                    src[k].copy_(frames[t], non_blocking=True)
+            src, T, n = self._sampled(frames)
             self.status.zero_()
             self._count_tail(src.data_ptr(), T, self.npix, self._layout(MODE_E2M1, True), n, stream_handle(self.dev))
             c4, c8 = self.status.tolist()[2:4]
@@ -884,6 +888,82 @@ class DenseEngine(ResultBuffers):
             if self._narrow == MODE_FP16:
                 self._u8_hint = MODE_FP16             # counts above 16 were seen (or lists overflowed)
         return None if self._narrow == MODE_FP16 else self._narrow
+
+    def _sampled(self, frames):
+        """(device frames, their number, frames to look at) for a look at a
+        stack: frames in host memory are copied in."""
+        n = min(self.T, self.TAIL_FRAMES if frames.is_cuda else self.TAIL_FRAMES_HOST)
+        if frames.is_cuda:
+            return frames, self.T, n
+        src = _torch().empty((n,) + self.shape, dtype=frames.dtype, device=self.dev)
+        for k in range(n):
+            src[k].copy_(frames[(2 * k + 1) * self.T // (2 * n)], non_blocking=True)
+        return src, n, n
+
+    # -- K-blocked 16-bit operands ---------------------------------------------
+    # u16 stacks, and u8 stacks too bright for a narrow operand: counts up to
+    # 2048 as fp16 patterns, larger ones as two planes of signed digits
+    # (g2_pack_blocked).  A K chunk is exact while every frame's energy (sum of
+    # squares) in it is below 2^24 (2^23 for signed digits, so that a lag's sum
+    # over a tile fits 32 bits).  The chunks are cut from the energies of a few
+    # sampled frames with a margin, and the Gram checks its own diagonal, which
+    # is every frame's energy: a stack above the limit is run again, cut finer,
+    # and after that on the row-major operands, whose pack computes bounds for
+    # every stack.  256 x 256 x 5,000 u16 (mean 50): 1.71 ms on row-major operands,
+    # 1.35 on these; 195 x 487 x 1,500 with counts above 2048: 1.45 and 1.01.
+    # Stacks of few counts (e4m3) and small ones (NARROW_MIN_MACS: 275 x 263 x
+    # 300, 0.40 ms either way) keep the row-major operands.
+    WIDE_MARGIN = (1.25, 4.0)
+
+    def _wide_ok(self, frames):
+        """Whether a stack may run on a K-blocked 16-bit operand."""
+        if not self._blocked_ok(frames) or self._wide_margin >= len(self.WIDE_MARGIN):
+            return False
+        if frames.element_size() == 1:
+            return self._narrow == MODE_FP16
+        return self._wide_plan is not False or self._u16_hint != MODE_E4M3
+
+    def _wide_mode(self, frames):
+        """(mode, layout, K split) when the stack runs on a K-blocked 16-bit
+        operand, else None.  The first stack and every NARROW_LOOK-th are
+        looked at (one kernel and a read of its energies); a split is kept while
+        the energies stay between a quarter of what it allows and that."""
+        if not self._wide_ok(frames):
+            return None
+        self._wide_age += 1
+        if not self._wide_plan or self._wide_age % self.NARROW_LOOK == 0:
+            self._wide_plan = self._look_wide(frames)
+        return self._wide_plan or None
+
+    def _look_wide(self, frames):
+        torch = _torch()
+        src, T, n = self._sampled(frames)
+        for mode in (MODE_FP16, MODE_BYTES)[int(self._wide_from == MODE_BYTES):]:
+            if mode == MODE_BYTES and frames.element_size() == 1:
+                break                                    # u8 counts are never above 2048
+            L = self._layout(mode, True)
+            planes = 2 if L.split else 1
+            energy = torch.empty(n * planes * max(L.unit_col.size, 1) + 1, dtype=torch.int64, device=self.dev)
+            energy[-1:].zero_()
+            _lib.check(self.lib.g2_sample_energy(
+                ptr(src), src.element_size(), T, self.npix, ptr(L.d_col_src), L.col_src.size, ptr(L.d_unit_col),
+                L.unit_col.size, n, int(L.split), ptr(energy), ptr(energy[-1:]), stream_handle(self.dev)),
+                "g2_sample_energy")
+            e = energy.cpu().numpy()
+            most, e = int(e[-1]), e[:-1].reshape(n, planes, -1).astype(np.float64)
+            if frames.element_size() == 2 and most <= E4M3_MAX_EXACT and self._wide_from == MODE_FP16:
+                self._u16_hint = MODE_E4M3
+                return False
+            if mode == MODE_FP16 and most > FP16_MAX_EXACT:
+                continue
+            limit = EXACT_LIMIT / planes
+            have = self._wide_plan
+            if have and have[0] == mode and limit / 4 <= L.split_peak(e, have[2]) < limit:
+                return have
+            cut = L.sampled_grams(e, limit / self.WIDE_MARGIN[self._wide_margin])
+            if cut is not None:
+                return mode, L, cut
+        return False
 
     def _count_tail(self, frames_ptr, T, npix, L, n, stream):
         _lib.check(self.lib.g2_count_tail(C.c_void_p(frames_ptr), T, npix, ptr(L.d_col_src), L.col_src.size, n,
@@ -911,22 +991,27 @@ class DenseEngine(ResultBuffers):
         (narrow operands: residual lists that overflow rerun on a wider one)."""
         torch = _torch()
         narrow = self._narrow_mode(frames)
-        mode = narrow if narrow is not None else self._pipeline_mode(frames)
+        wide = self._wide_mode(frames) if narrow is None else None
+        blocked = narrow is not None or wide is not None
+        mode = narrow if narrow is not None else wide[0] if wide is not None else self._pipeline_mode(frames)
         if mode is None:
             return self.run(frames, pipelined=False)
         host = not frames.is_cuda
         # u8 frames from host memory come in cropped to the q-mask's columns
         # (the pack then reads the cropped frames with the cropped layout)
         crop = host and mode in (MODE_E4M3, MODE_E2M1) and frames.element_size() == 1 and self.crop is not None
-        Lp = self._crop_layout(mode, narrow is not None) if crop else self._layout(mode, narrow is not None)
-        L = Lp if narrow is not None else self._layout(mode)
-        packed = self._packed_buffer(L, narrow is not None)
-        if mode != MODE_FP16:
+        Lp = self._crop_layout(mode, blocked) if crop else self._layout(mode, blocked)
+        L = Lp if blocked else self._layout(mode)
+        packed = self._packed_buffer(L, blocked)
+        if wide is not None:
+            _, L, grams = wide
+            Lp = L
+        elif mode != MODE_FP16:
             grams, bound = None, None
         else:                                 # fp16: the reused K split and the bounds it covers
             _, bound, grams = self._plans[mode]
         items, dev_items, bounds, starts, n_grams = self._pipe_plan(
-            L, self.PIPE_TAPER_HOST if host else 0, grams, self._chunk_count(host, narrow is not None))
+            L, self.PIPE_TAPER_HOST if host else 0, grams, self._chunk_count(host, blocked))
         if Lp.packed_cols != L.packed_cols:
             raise RuntimeError("cropped packing layout differs from the frame's")
         npix_in = self.shape[0] * self.crop[1] if crop else self.npix
@@ -947,7 +1032,7 @@ class DenseEngine(ResultBuffers):
         self._mark("pipeline")
         self.zero_results()
         emax = None
-        if mode == MODE_FP16:
+        if mode == MODE_FP16 and wide is None:
             emax = self._piece_emax(L)
             emax.zero_()                      # chunks combine their energy maxima (atomicMax)
         self._residuals = None
@@ -965,7 +1050,9 @@ class DenseEngine(ResultBuffers):
         npix = npix_in
         eb = frames_dev.element_size()
         row_bytes = L.packed_bytes_per_frame
-        kind = L.kind + (_lib.KIND_BLOCKED if narrow == MODE_E4M3 else 0)
+        kind = L.kind + (_lib.KIND_BLOCKED if blocked and narrow != MODE_E2M1 else 0)
+        if wide is not None:
+            kind += _lib.KIND_CHECK + (_lib.KIND_SIGNED if L.split else 0)
         jobs = _lib.jobs_array([(packed.data_ptr(), self.T, L.packed_cols, kind, self.ones(L))])
         item_bytes = _lib.ITEM_DTYPE.itemsize
         for c in range(bounds.size - 1):
@@ -989,6 +1076,11 @@ class DenseEngine(ResultBuffers):
                     C.c_void_p(src), t1 - t0, npix, t0, L.kind, ptr(Lp.d_unit_block_off), ptr(Lp.d_units),
                     ptr(Lp.d_chunk_span), Lp.n_chunks, ptr(packed), self.T + 1, L.packed_cols, ptr(res[0]), ptr(res[1]), res[2], ptr(self.err),
                     C.c_void_p(pack_s.cuda_stream)), "g2_pack_u8_residual")
+            elif wide is not None:
+                _lib.check(self.lib.g2_pack_blocked(
+                    C.c_void_p(src), eb, t1 - t0, npix, t0, int(L.split), ptr(L.d_unit_block_off), ptr(L.d_units),
+                    ptr(L.d_chunk_span), L.n_chunks, ptr(packed), self.T + 1, L.packed_cols, ptr(self.err),
+                    C.c_void_p(pack_s.cuda_stream)), "g2_pack_blocked")
             elif mode == MODE_E4M3:
                 self.pack_e4m3(src, 1, t1 - t0, Lp, dst, pack_s.cuda_stream, npix=npix)
             else:
@@ -1038,6 +1130,20 @@ class DenseEngine(ResultBuffers):
         if host:
             self._frames_host_ref = frames            # alive until the copies are done
         h2d = int(self.T * npix * eb) if host else 0
+        if wide is not None:
+            code = self._end_words()[0]
+            if code & (_lib.DEVERR_RANGE | _lib.DEVERR_ENERGY):   # counts above 2048, or a brighter stack: look again
+                if code & _lib.DEVERR_RANGE:
+                    self._wide_from = MODE_BYTES
+                else:
+                    self._wide_margin += 1
+                self._wide_plan = None
+                return self.run(frames_dev)
+            self.last = {"mode": MODE_NAMES[mode], "split": int(L.split), "n_items": int(items.size),
+                         "n_grams": n_grams, "packed_cols": L.packed_cols,
+                         "pipeline_chunks": int(bounds.size - 1), "tile": self.tile, "plan": "sampled",
+                         "h2d_bytes": h2d, "crop": None}
+            return self.g2_f32[: self.n_bins]
         if mode == MODE_FP16:
             # one synchronisation: the error word and whether the stack's
             # energy bounds exceed those the reused split covers
@@ -1231,17 +1337,21 @@ class DenseEngine(ResultBuffers):
         if self.packed is None or self._packed_mode is None:
             raise RuntimeError("%s needs a preceding run()" % what)
         if self._residuals is None:
-            L = self._layouts[self._packed_mode]
-            return L, L.kind, self.packed
+            blocked, L = self._packed_layout
+            if not blocked:
+                L = self._layouts[self._packed_mode]
+                return L, L.kind, self.packed
+            rows, row_bytes = self.T + 1, L.packed_bytes_per_frame
+            wide = self._expand_buffer(rows * row_bytes)
+            _lib.check(self.lib.g2_operand_rows(ptr(self.packed), rows, row_bytes, ptr(wide),
+                                                stream_handle(self.dev)), "g2_operand_rows")
+            return L, L.kind, wide
         L, counts, lists, cap, total = self._residuals
         rows = self.T + 1
         for kind, nb in ((_lib.KIND_E4M3, 1), (_lib.KIND_FP16, 2)):
             if L.mode == MODE_E4M3 and total and kind == L.kind:
                 continue                              # residuals of e4m3 are counts above 16
-            wide = getattr(self, "_wide", None)
-            if wide is None or wide.numel() < rows * L.packed_cols * nb:
-                self._wide = None
-                wide = self._wide = torch.empty(rows * L.packed_cols * nb, dtype=torch.uint8, device=self.dev)
+            wide = self._expand_buffer(rows * L.packed_cols * nb)
             self.err.zero_()
             _lib.check(self.lib.g2_operand_expand(ptr(self.packed), rows, self.T, L.packed_cols, L.kind, kind,
                                                   ptr(counts), ptr(lists), cap, ptr(wide), ptr(self.err),
@@ -1249,6 +1359,13 @@ class DenseEngine(ResultBuffers):
             if kind == _lib.KIND_FP16 or not total or not int(self.err.item()) & _lib.DEVERR_RANGE:
                 break
         return L, kind, wide
+
+    def _expand_buffer(self, nbytes):
+        buf = getattr(self, "_expanded", None)
+        if buf is None or buf.numel() < nbytes:
+            self._expanded = None
+            buf = self._expanded = _torch().empty(nbytes, dtype=_torch().uint8, device=self.dev)
+        return buf
 
     def deviation(self):
         """calc_std of the last run (dense.py:58-66): float32 device tensor
@@ -1259,7 +1376,7 @@ class DenseEngine(ResultBuffers):
             raise NotImplementedError("calc_std runs on the tensor-core path")
         L, kind, packed = self._last_operand("deviation()")
         if L.split:
-            return self._deviation_planes(L)
+            return self._deviation_planes(L, packed)
         key = ("std", L.mode, self.T, tuple(L.grams()))
         if key not in self._items_cache:
             from .plan import std_items
@@ -1286,7 +1403,7 @@ class DenseEngine(ResultBuffers):
         self.dev_f64 = d64
         return d32[: self.n_bins]
 
-    def _deviation_planes(self, L):
+    def _deviation_planes(self, L, packed):
         """calc_std of a byte-plane stack (counts above 2048): the per-pair
         ratio needs the four plane Grams of a pair together, so each bin's
         Gram G = 2^16 G_hh + 2^8 (G_hl + G_lh) + G_ll is assembled in a T x T
@@ -1306,7 +1423,7 @@ class DenseEngine(ResultBuffers):
         npix = np.bincount(self.qmask.ravel()[self.qmask.ravel() > 0], minlength=self.n_bins + 1)[1:]
         i0, j0 = _tiles(T, TILE_SHAPES["tc"][0], TILE_SHAPES["tc"][1])
         st = stream_handle(self.dev)
-        jobs = _lib.jobs_array([(self.packed.data_ptr(), T, L.packed_cols, L.kind, 0)])
+        jobs = _lib.jobs_array([(packed.data_ptr(), T, L.packed_cols, L.kind, 0)])
         by_bin = {}
         for (b, a_off, b_off, kp, shift) in L.grams():
             by_bin.setdefault(b, []).append((a_off, b_off, kp, shift))

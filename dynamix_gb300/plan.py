@@ -273,24 +273,27 @@ def chunk_spans(pix, n_chunks, size):
 
 
 class NarrowLayout:
-    """Packed-column layout of the bins of one q-mask for the narrow operands
-    (``g2_pack_u8_residual``): e2m1, two columns per byte, or e4m3.  The order
-    of a bin's pixels is free (every Gram entry sums over them), so the columns
+    """Packed-column layout of the bins of one q-mask for the K-blocked
+    operands: e2m1 (two columns per byte) and e4m3 of ``g2_pack_u8_residual``,
+    16-bit counts and 16-bit byte planes of ``g2_pack_blocked``.  The order of a
+    bin's pixels is free (every Gram entry sums over them), so the columns
     follow the pack's work units, each of pixels of one 4080-pixel chunk: per
-    bin first the 16-byte units (e2m1: two runs of 16 consecutive pixels, e4m3:
-    one), then the 4-byte units from runs of 4, then the 4-byte units from
-    single pixels; bins padded to 128 bytes, one block of the K-blocked
-    operand."""
+    bin first the 16-byte units (from runs of 16 consecutive pixels, e2m1 two,
+    16-bit 8 pixels), then the 4-byte units from runs of 4 (16-bit: 2), then the
+    4-byte units from single pixels; bins padded to whole 128-byte blocks of the
+    operand.  Byte planes follow each other bin by bin, high then low."""
 
-    split, ones_row, n_pieces = False, True, 0
+    ones_row, n_pieces = True, 0
 
     def __init__(self, qmask, n_bins, mode=MODE_E2M1):
-        e2m1 = mode == MODE_E2M1
-        self.mode, self.kind = int(mode), KIND_E2M1 if e2m1 else KIND_E4M3
-        self.elem_bytes = 0.5 if e2m1 else 1
-        vec, word = (32, 8) if e2m1 else (16, 4)                # columns per unit
-        pad = 128 * word // 4                                   # columns of 128 bytes
-        order_of = E2M1_WORD if e2m1 else np.arange(4)          # column of every count of a 4-byte word
+        e2m1, wide = mode == MODE_E2M1, mode in (MODE_FP16, MODE_BYTES)
+        self.mode, self.split = int(mode), mode == MODE_BYTES
+        self.kind = KIND_E2M1 if e2m1 else KIND_FP16 if wide else KIND_E4M3
+        self.elem_bytes = 0.5 if e2m1 else 2 if wide else 1
+        vrun, wrun = (8, 2) if wide else (16, 4)                # pixels of a run
+        vec, word = (32, 8) if e2m1 else (vrun, wrun)           # columns per unit
+        pad = max(PAD, 128 * word // 4)                         # columns of whole blocks
+        order_of = E2M1_WORD if e2m1 else np.arange(wrun)       # column of every count of a 4-byte word
         q = np.ascontiguousarray(qmask, dtype=np.int32).ravel()
         self.npix_total, self.n_bins = q.size, int(n_bins)
         nb = max(self.n_bins, 1)
@@ -327,10 +330,10 @@ class NarrowLayout:
             odd = rank >= 2 * half
             return p[a], p[a + half[a]], g[a], p[odd], g[odd]
 
-        p16, g16 = pieces(rp, rg, n // 16, 16)
-        rest = rp + n // 16 * 16
-        p4, g4 = pieces(rest, rg, n % 16 // 4, 4)
-        p1, g1 = pieces(rest + n % 16 // 4 * 4, rg, n % 4, 1)
+        p16, g16 = pieces(rp, rg, n // vrun, vrun)
+        rest = rp + n // vrun * vrun
+        p4, g4 = pieces(rest, rg, n % vrun // wrun, wrun)
+        p1, g1 = pieces(rest + n % vrun // wrun * wrun, rg, n % wrun, 1)
         if e2m1:                                                # pieces left without a partner: smaller ones
             v0, v1, vg, lp, lg = paired(p16, g16)
             q4, h4 = pieces(lp, lg, np.full(lp.size, 4), 4)
@@ -365,9 +368,9 @@ class NarrowLayout:
         wb, wpos, wc = within_bin(wg)
         gb, gpos, gc = within_bin(gg)
         self.kpad = _roundup(vec * vc + word * (wc + gc), pad)[: self.n_bins].astype(np.int64)
-        off = np.concatenate([[0], np.cumsum(self.kpad)])
+        off = np.concatenate([[0], np.cumsum(self.kpad * (2 if self.split else 1))])
         self.bin_off = self.plane0 = off[:-1].astype(np.int64)
-        self.plane1 = None
+        self.plane1 = self.plane0 + self.kpad if self.split else None
         self.packed_cols = int(max(pad, off[-1]))
         if self.packed_cols >= 2 ** 31:
             raise ValueError("too many binned pixels for one job")
@@ -375,13 +378,24 @@ class NarrowLayout:
         wcol = self.bin_off[wb] + vec * vc[wb] + word * wpos
         gcol = self.bin_off[gb] + vec * vc[gb] + word * (wc[gb] + gpos)
         col_src = np.full(self.packed_cols, -1, dtype=np.int32)
-        for col, runs, size in ((vcol, vruns, 16), (wcol, wruns, 4)):
+        for col, runs, size in ((vcol, vruns, vrun), (wcol, wruns, wrun)):
             j = np.arange(size)
             for half, p in enumerate(runs):
-                col_src[(col[:, None] + j // 4 * word + order_of[4 * half + j % 4]).ravel()] = (p[:, None] + j).ravel()
+                at = col[:, None] + j // wrun * word + order_of[wrun * half + j % wrun]
+                col_src[at.ravel()] = (p[:, None] + j).ravel()
         col_src[(gcol[:, None] + order_of).ravel()] = singles.ravel()
+        # 128-column units (of the first plane), for energies
+        self.unit_bin = np.repeat(np.arange(self.n_bins), self.kpad // PAD)
+        first = np.concatenate([[0], np.cumsum(self.kpad // PAD)])[:-1]
+        self.unit_col = (self.plane0[self.unit_bin]
+                         + PAD * (np.arange(self.unit_bin.size) - first[self.unit_bin])).astype(np.int32)
+        if self.split:                                          # the low planes hold the same pixels
+            for b in range(self.n_bins):
+                o, k = int(self.plane0[b]), int(self.kpad[b])
+                col_src[o + k:o + 2 * k] = col_src[o:o + k]
         self.col_src = col_src                                     # pixel of every packed column, -1: padding
-        self.sector_bin = np.repeat(np.arange(self.n_bins, dtype=np.int32), self.kpad // RES_SECTOR)
+        self.sector_bin = np.repeat(np.arange(self.n_bins, dtype=np.int32),
+                                    self.kpad * (2 if self.split else 1) // RES_SECTOR)
         if self.sector_bin.size < self.packed_cols // RES_SECTOR:
             self.sector_bin = np.full(self.packed_cols // RES_SECTOR, -1, dtype=np.int32)
         # blocks of 32 units of one class per chunk
@@ -392,6 +406,8 @@ class NarrowLayout:
             u = np.zeros((g.size, 4), dtype=np.int64)
             u[:, 0] = dst | (cls << 30)
             u[:, 1] = local(p[0], ch) | (local(p[-1], ch) << 16)
+            if self.split:
+                u[:, 3] = 2 * self.kpad[g % nb]                  # bytes from the high to the low plane
             recs.append((ch, u))
         ch = gg // nb
         src = np.where(singles >= 0, singles - ch[:, None] * NARROW_CHUNK, 0xFFF)
@@ -402,6 +418,8 @@ class NarrowLayout:
             u[:, 1 + w] |= (src[:, k] << sh) & 0xFFFFFFFF
             if sh > 20:
                 u[:, 2 + w] |= src[:, k] >> (32 - sh)
+        if self.split:
+            u[:, 3] = 2 * self.kpad[gg % nb]
         recs.append((ch, u))
         blocks = [-(-np.bincount(ch, minlength=self.n_chunks) // 32) for ch, _ in recs]
         boff = np.concatenate([[0], np.cumsum(sum(blocks))])
@@ -419,17 +437,53 @@ class NarrowLayout:
 
     @property
     def packed_bytes_per_frame(self):
-        return self.packed_cols // 2 if self.mode == MODE_E2M1 else self.packed_cols
+        return int(self.packed_cols * self.elem_bytes)
 
     def ones_row_values(self):
         """Row of ones: 1 (e2m1: code 1) in every binned column, 0 in the padding."""
-        one = (self.col_src >= 0).astype(np.uint8)
+        one = (self.col_src >= 0).astype(np.uint16 if self.elem_bytes == 2 else np.uint8)
         return one[0::2] | (one[1::2] << 4) if self.mode == MODE_E2M1 else one
 
     def grams(self):
         """The Grams to run per bin: (bin, a_off, b_off, kpad, shift)."""
-        return [(b, int(self.bin_off[b]), int(self.bin_off[b]), int(self.kpad[b]), 0)
-                for b in range(self.n_bins) if self.kpad[b]]
+        out = []
+        for b in range(self.n_bins):
+            h, k = int(self.plane0[b]), int(self.kpad[b])
+            lo = h + k
+            if k and self.split:
+                out += [(b, h, h, k, 16), (b, h, lo, k, 8), (b, lo, h, k, 8), (b, lo, lo, k, 0)]
+            elif k:
+                out.append((b, h, h, k, 0))
+        return out
+
+    def split_peak(self, energy, grams):
+        """The largest energy of a frame and plane in a K chunk of ``grams``."""
+        rel = self.unit_col - self.plane0[self.unit_bin]
+        peak = 0.0
+        for b, k0, kl in {(b, k0, kl) for (b, _, _, k0, kl, _) in grams}:
+            mine = (self.unit_bin == b) & (rel >= k0) & (rel < k0 + kl)
+            peak = max(peak, float(energy[:, :, mine].sum(axis=2).max()))
+        return peak
+
+    def sampled_grams(self, energy, limit):
+        """The Grams cut along K so that a chunk's energy (sum of squares) stays
+        below ``limit`` in every sampled frame and plane: ``energy`` is (frames,
+        planes, 128-column units).  Returns ``(bin, a_off, b_off, k0, k_len,
+        shift)`` tuples, or None when a single unit is above the limit."""
+        e = np.asarray(energy, dtype=np.float64)
+        if e.shape[2] and e.max() > limit:
+            return None
+        cuts = {}
+        for b in range(self.n_bins):
+            mine = e[:, :, self.unit_bin == b]
+            cum = np.concatenate([np.zeros(mine.shape[:2] + (1,)), np.cumsum(mine, axis=2)], axis=2)
+            u0, n, cuts[b] = 0, mine.shape[2], []
+            while u0 < n:
+                over = np.flatnonzero((cum[:, :, u0 + 1:] - cum[:, :, u0:u0 + 1]).max(axis=(0, 1)) > limit)
+                u1 = n if over.size == 0 else u0 + int(over[0])
+                cuts[b].append((u0 * PAD, (u1 - u0) * PAD))
+                u0 = u1
+        return [(b, a, c, k0, kl, shift) for (b, a, c, _, shift) in self.grams() for (k0, kl) in cuts[b]]
 
 
 def k_chunks(emax_a, emax_b, limit=EXACT_LIMIT):
@@ -513,7 +567,8 @@ def gram_items(T, chunked_grams, job=0, out_base=0, kind="tc", s_base=None, supe
         it["shift"] = shift
         it["nframes"] = T
         it["out_off"] = out_base + b * T
-        it["s_off"] = -1 if s_base is None else s_base + b * T
+        # byte planes: S = 256 S_high + S_low from the Grams of a plane with itself
+        it["s_off"] = -1 if s_base is None or a_off != b_off else s_base + b * T
         parts.append(it)
     if not parts:
         return np.empty(0, dtype=ITEM_DTYPE)

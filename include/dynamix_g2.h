@@ -41,6 +41,8 @@ extern "C" {
 #define G2_DEVERR_RANGE_CHECK 8 /* a count may not fit the packing: check the exact maximum */
 #define G2_DEVERR_RESIDUAL 16 /* a residual list overflowed: pack the stack into a wider element */
 
+#define G2_DEVERR_ENERGY 32 /* a checked Gram's own diagonal exceeds the exact range: cut its K finer */
+
 #define G2_ABI_VERSION      1
 
 /* Tile sizes of the tensor-core Gram: an item covers a 128 x 256 block of
@@ -65,6 +67,10 @@ extern "C" {
 #define G2_KIND_E2M1  2    /* 4-bit codes of u = count - 3, counts 0-7 (e2m1 = u / 2), two per byte
                               (even column in the low half), padding u = 0, MMA kind::mxf4 */
 #define G2_KIND_BLOCKED 256 /* added to an element kind: the operand is K-blocked */
+/* more flags of an element kind, g2_gram_tc_pair only: */
+#define G2_KIND_SIGNED 512  /* signed elements (16-bit: sign and magnitude): signed lag sums */
+#define G2_KIND_CHECK 1024  /* set G2_DEVERR_ENERGY when an item's G(t, t) reaches 2^24 (signed: 2^23):
+                               below it every entry of the item is exact (Cauchy-Schwarz) */
 #define G2_RES_SECTOR 64   /* packed columns per residual list */
 
 /* One unit of Gram work: rows [i0, i0+BM) of the A operand against rows
@@ -105,7 +111,7 @@ typedef struct g2_job {
     const void* packed_dev;
     int64_t nframes;
     int64_t packed_cols;   /* multiple of G2_PAD */
-    int32_t elem_kind;     /* G2_KIND_FP16 or G2_KIND_E4M3, either + G2_KIND_BLOCKED;
+    int32_t elem_kind;     /* G2_KIND_FP16 or G2_KIND_E4M3, either + flags (G2_KIND_BLOCKED ...);
                               g2_gram_tc_e2m1: G2_KIND_E2M1 (always K-blocked) */
     int32_t ones_row;      /* 1: row nframes of the packed matrix holds 1 in every
                               binned column and 0 in the padding (bin sums) */
@@ -222,6 +228,30 @@ int g2_pack_u8_residual(const void* frames_dev, int64_t nframes, int64_t npix, i
                         const int32_t* unit_block_off_dev, const uint32_t* units_dev, const uint32_t* spans_dev,
                         int64_t n_chunks, void* packed_dev, int64_t packed_rows, int64_t packed_cols, uint32_t* res_count_dev,
                         void* res_list_dev, int32_t res_cap, int32_t* err_dev, void* stream);
+
+/* Pack of u8 (mode 0) or u16 frames into a K-blocked 16-bit operand: mode 0
+ * the counts (<= 2048, else G2_DEVERR_RANGE), mode 1 two planes of signed
+ * digits, count = 256 high + low, low in [-128, 127] as sign and magnitude, the
+ * low plane word 3 of the unit bytes after the high one.  Units as for
+ * g2_pack_u8_residual's e4m3 with runs of 8 and 2 pixels and two sources per
+ * gathered word.  Energies are not computed: K is cut from sampled ones
+ * (g2_sample_energy) and checked by the Gram (G2_KIND_CHECK).  Replaces the
+ * gather of dense.py:48-50. */
+int g2_pack_blocked(const void* frames_dev, int32_t elem_bytes, int64_t nframes, int64_t npix, int64_t frame0,
+                    int32_t mode, const int32_t* unit_block_off_dev, const uint32_t* units_dev,
+                    const uint32_t* spans_dev, int64_t n_chunks, void* packed_dev, int64_t packed_rows,
+                    int64_t packed_cols, int32_t* err_dev, void* stream);
+
+/* Sums of squares of the 128-column units (first column unit_col_dev[u], pixels
+ * col_src_dev) of n_sample evenly spread frames: energy_dev[(f * planes + p) *
+ * n_units + u], planes = 1 (mode 0) or the signed digits' 2 (mode 1); raises
+ * max_dev (caller zeroes it) to the largest count seen. */
+int g2_sample_energy(const void* frames_dev, int32_t elem_bytes, int64_t nframes, int64_t npix,
+                     const int32_t* col_src_dev, int64_t n_cols, const int32_t* unit_col_dev, int64_t n_units,
+                     int64_t n_sample, int32_t mode, uint64_t* energy_dev, uint32_t* max_dev, void* stream);
+
+/* A row-major copy of a K-blocked operand (row_bytes a multiple of 128). */
+int g2_operand_rows(const void* packed_dev, int64_t rows, int64_t row_bytes, void* out_dev, void* stream);
 
 /* Adds to out_dev[0] / out_dev[1] the number of binned counts (col_src >= 0)
  * of n_sample evenly spread frames that an e2m1 / e4m3 operand needs a
