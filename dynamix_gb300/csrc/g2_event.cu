@@ -12,10 +12,11 @@
 // keeps the current bin's lag histogram and frame-sum histogram as uint32
 // counters in shared memory (2 x T words) and flushes them at each range end.  A warp takes one pixel at a time, stages up to EV of its
 // events in shared memory as (t << 16 | v) and walks the pairs: for each i (warp
-// uniform) the lanes take j = i + lane, i + lane + 32, ...  A counter whose
-// value reaches 2^31 is drained with an atomic exchange into the int64 global
-// sums by the thread that saw it cross, so no uint32 counter can wrap (each
-// increment is < 2^31 and at most a few thousand threads add concurrently).
+// uniform) the lanes take j = i + lane, i + lane + 32, ...  A counter
+// that wraps carries 2^32 into the int64 global sums.  The adds set the pace: 32
+// lags in random banks take 3.5 turns on average, and 6 useful pairs per clock
+// and SM are done (0.75 ms for 2^18 pixels of 100 events); a warp per pixel in
+// tiles of 8 x 8 events is 5 % slower there and 12 % faster at 300 events.
 // At the end the CTA adds its counters to the global N and S.
 // When 2 T words do not fit in shared memory, or counts are large, a second
 // kernel adds every pair directly to the global int64 sums.
@@ -32,16 +33,14 @@ constexpr int LANES = 16;                  // lanes per pixel: a warp walks two 
 constexpr int HALVES = 32 / LANES;
 constexpr int EV = 128;                    // events of one pixel staged per block of pairs
 constexpr int ROWS = 8;                    // rows of the pair block walked together
-constexpr uint32_t DRAIN = 1u << 31;
 constexpr int SMEM_FIXED = WARPS * HALVES * 2 * EV * 4;
 constexpr int SMEM_STATIC = WARPS * 8;    // block-reduction slots
 
+// A uint32 counter's add; the one add that wraps it carries 2^32 into the int64
+// sum, so counter + sum is exact whatever adds run at the same time.
 __device__ __forceinline__ void add_counter(uint32_t* c, unsigned long long* g, uint32_t x) {
   const uint32_t old = atomicAdd(c, x);
-  if (old + x >= DRAIN || old + x < old) {
-    const uint32_t val = atomicExch(c, 0u);
-    if (val) atomicAdd(g, static_cast<unsigned long long>(val));
-  }
+  if (old + x < old) atomicAdd(g, 1ull << 32);
 }
 
 // One event as (t << 16) | v with its validity: from the caller's split
@@ -63,7 +62,7 @@ __device__ __forceinline__ uint32_t load_event(const int32_t* __restrict__ times
 // Pair sums of one pixel's events by one warp.  FAST: every counter of the
 // range is known to stay below 2^32 (checked per range from its event count),
 // so the shared adds need no returned value (the warp does not wait on them)
-// and no drain check.
+// and no carry.
 template <bool FAST, bool PACKED, typename Tv>
 __device__ __forceinline__ void pixel_pairs(const int32_t* __restrict__ times, const Tv* __restrict__ data,
                                             int64_t base, int n, int T, uint32_t maxc, uint32_t* hist,
@@ -167,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     // events of the range: a lag counter gains at most max^2 per event and a
     // frame counter at most max per pixel, so max^2 * events < 2^32 keeps
-    // every counter of the range in uint32 without draining
+    // every counter of the range in uint32 without a carry
     unsigned long long ev = 0;
     for (int li = range_off[r] + threadIdx.x; li < range_off[r + 1]; li += THREADS) {
       const int32_t p = pix_list[li];
