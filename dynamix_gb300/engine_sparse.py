@@ -79,6 +79,10 @@ def events_to_device(vol_times, vol_data, offsets, npix, nframes, dev):
         raise ValueError("vol_times and vol_data must have the same size")
     if len(offsets) != npix + 1:
         raise ValueError("offsets should have size %d, got %d" % (npix + 1, len(offsets)))
+    if (all(_is_cuda(x) and x.device == dev and x.is_contiguous() for x in (vol_times, vol_data, offsets))
+            and vol_times.dtype == torch.int32 and vol_data.dtype in (torch.uint8, torch.uint16)
+            and offsets.dtype in (torch.int32, torch.int64) and 0 < len(vol_times) and nframes < 2 ** 31):
+        return _checked_events(vol_times, vol_data, offsets, npix, nframes, dev)
     if _is_cuda(offsets):
         o = offsets.to(dev).to(torch.int64)
         if int(o[0].item()) != 0 or not bool(torch.all(o[1:] >= o[:-1])):
@@ -110,6 +114,31 @@ def events_to_device(vol_times, vol_data, offsets, npix, nframes, dev):
             raise ValueError("event times must lie in [0, nframes)")
     counts, mx = _int_counts_to_device(vol_data, n_ev, dev)
     return times, counts, offs_d, n_ev, mx
+
+
+def _checked_events(times, counts, offsets, npix, nframes, dev):
+    """:func:`events_to_device` for tensors that are used where they are: the
+    checks run in two kernels and come back in one read."""
+    torch = _torch()
+    lib, st = _lib.load(), stream_handle(dev)
+    offs = torch.empty(npix + 1, dtype=torch.int32, device=dev)
+    stats = torch.zeros(5, dtype=torch.int64, device=dev)
+    _lib.check(lib.g2_check_offsets(ptr(offsets), offsets.element_size(), npix + 1, ptr(offs), ptr(stats), st),
+               "g2_check_offsets")
+    _lib.check(lib.g2_check_events(ptr(times), ptr(counts), counts.element_size(), len(times), ptr(stats[1:]),
+                                   nframes, ptr(stats), st), "g2_check_events")
+    first, n_ev, falls, bad_times, mx = stats.tolist()
+    if first != 0 or falls:
+        raise ValueError("offsets must start at 0 and be non-decreasing")
+    if n_ev >= 2 ** 32:
+        raise ValueError("too many events for uint32 offsets")
+    if len(times) < n_ev:
+        raise ValueError("offsets reference %d events but only %d are given" % (n_ev, len(times)))
+    if bad_times:
+        raise ValueError("event times must lie in [0, nframes)")
+    if n_ev == 0:
+        return times, torch.zeros(1, dtype=torch.uint8, device=dev), offs, 0, 0
+    return times[:n_ev], counts[:n_ev], offs, n_ev, mx
 
 
 def csr_to_device(data, indices, indptr, offsets, shape, nframes, dev):
@@ -490,14 +519,15 @@ class SparseEngine:
     SUBBLOCK = 1024
     TILE_P = 64
 
-    def to_words(self, data, indices, indptr, offsets, ib, n, sort=False):
+    def to_words(self, data, indices, indptr, offsets, ib, n, sort=False, after_count=None):
         """CSR on the device -> packed event words and event offsets (uint32
         as int32) on the device; requires :meth:`packed_for`.  Counts per
         (1024-frame sub-block, pixel) and per (sub-block, row), their scans,
         the stage pass (runs grouped by sub-block, row and pixel) and the
         gather pass (64-pixel tiles; each pixel's runs in sub-block order, in
         frame order inside each run with ``sort``, so the whole list is in
-        frame order)."""
+        frame order).  ``after_count`` is called when the count pass and the
+        scans are launched."""
         torch = _torch()
         H, W = self.shape
         st = stream_handle(self.dev)
@@ -518,6 +548,8 @@ class SparseEngine:
                    "g2_exclusive_scan_u32")
         _lib.check(self.lib.g2_exclusive_scan_u32(ptr(rt), n_rows, ptr(base), ptr(rscr), rscr.numel(), st),
                    "g2_exclusive_scan_u32")
+        if after_count is not None:
+            after_count()
         stage = self._buffer("stage_words", n, torch.int32)
         tpos = self._buffer("tile_pos", n_sb * -(-self.npix // self.TILE_P), torch.int32)
         _lib.check(self.lib.g2_csr_stage_blocked(ptr(data), data.element_size(), ptr(indices), ptr(rb), ib, n,
@@ -663,9 +695,52 @@ class SparseEngine:
         self.last = dict(self.events.last, n_elements=n, packed=True, host_sb_per_chunk=G)
         return out
 
+    def _in_place_ok(self, data, indices, indptr, offsets):
+        """Device tensors that the packed transposition reads where they are."""
+        torch = _torch()
+        H = self.shape[0]
+        return (all(_is_cuda(x) and x.device == self.dev and x.is_contiguous() and x.dim() == 1
+                    for x in (data, indices, indptr, offsets))
+                and data.dtype in (torch.uint8, torch.uint16) and indices.dtype == indptr.dtype == torch.int32
+                and offsets.dtype in (torch.int32, torch.int64) and 0 < len(data) == len(indices) < 2 ** 31
+                and len(indptr) == (H + 1) * self.T and len(offsets) == self.T + 1 and self.packed_for(len(data)))
+
+    def _run_in_place(self, data, indices, indptr, offsets):
+        """:meth:`run` without a reading of the columns before the count pass,
+        which checks those it walks: when it flags one, or has not walked every
+        element, the columns are looked at before anything else is launched."""
+        torch = _torch()
+        ev, n = self.events, len(data)
+        if offsets.dtype == torch.int64:
+            if int(offsets[-1].item()) >= 2 ** 31:        # not the int32 it is read as
+                offsets = torch.full_like(offsets, -1)    # reported by the count pass
+            offsets = offsets.to(torch.int32)
+        stats = torch.zeros(5, dtype=torch.int64, device=self.dev)
+        largest = []
+
+        def look():
+            _lib.check(self.lib.g2_check_events(None, ptr(data), data.element_size(), n, None, self.T, ptr(stats),
+                                                stream_handle(self.dev)), "g2_check_events")
+            stats[0:1].copy_(ev.err)
+            stats[1:2].copy_(self.ev_off[self.npix:])
+            code, walked, _, _, mx = stats.tolist()
+            if code or walked != n:
+                lo, hi = torch.aminmax(indices)
+                if int(lo.item()) < 0 or int(hi.item()) >= self.shape[1]:
+                    raise ValueError("column indices must lie in [0, width)")
+            largest.append(mx)
+
+        ev.err.zero_()
+        words, evoff = self.to_words(data, indices, indptr, offsets, 4, n, after_count=look)
+        out = ev.run_device(words, None, evoff, n, largest[0], reset_error=False)
+        self.last = dict(ev.last, n_elements=n, packed=True)
+        return out
+
     def run(self, data, indices, indptr, offsets):
         if self.host_pipeline_ok(data, indices, indptr, offsets):
             return self.run_host_pipelined(data, indices, indptr, offsets)
+        if self._in_place_ok(data, indices, indptr, offsets):
+            return self._run_in_place(data, indices, indptr, offsets)
         counts, ind, ip, off, ib, n, mx = csr_to_device(data, indices, indptr, offsets, self.shape, self.T,
                                                         self.dev)
         packed = self.packed_for(n)

@@ -374,6 +374,18 @@ int g2_plain_dp4a(const g2_job* jobs, int32_t n_jobs, const g2_gram_item* items_
  * grid * iters * 4 * 128 * 256 * K. */
 int g2_tc_rate_probe(int32_t kind, int64_t iters, int32_t grid, int32_t* err_dev, void* stream);
 
+/* Checks of event offsets (int32 or int64, n of them) in one read, with their
+ * uint32 copy: stats_dev[0], [1] = first and last offset, [2] = 1 if one is
+ * smaller than the one before.  Caller zeroes stats_dev (5 words). */
+int g2_check_offsets(const void* offsets_dev, int32_t offset_bytes, int64_t n, uint32_t* out_dev,
+                     int64_t* stats_dev, void* stream);
+
+/* Checks of the first min(n, *limit_dev) (limit_dev may be NULL) events:
+ * stats_dev[3] = 1 if a time lies outside [0, nframes) (times_dev may be NULL),
+ * stats_dev[4] raised to the largest count (u8 or u16). */
+int g2_check_events(const int32_t* times_dev, const void* data_dev, int32_t elem_bytes, int64_t n,
+                    const int64_t* limit_dev, int32_t nframes, int64_t* stats_dev, void* stream);
+
 /* ---- G6: event-list pair sums -------------------------------------------
  * Replaces event_correlator (dynamix/resources/opencl/evtcorrelator.cl:3-47)
  * behind EventCorrelator.correlate (dynamix/correlator/event.py:162-204).
