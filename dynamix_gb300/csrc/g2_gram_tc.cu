@@ -16,14 +16,14 @@
 // diagonals of each 32 x 32 block in registers and then in uint32 shared
 // counters (<= 128 * 2^24 < 2^32), which are added to the int64 numerator.
 //
-// Roles (192 threads, one CTA per SM, persistent over a static item schedule):
+// Roles (192 or 320 threads, one CTA per SM, persistent over a static item schedule):
 //   warp 0 lane 0  TMA producer: A (128 x 64) and B (256 x 64) fp16 tiles per
 //                  stage, 4-stage ring, 128-byte swizzle
 //   warp 1 lane 0  MMA issuer: 4 x (M128 N256 K16) per stage into one of two
 //                  TMEM accumulators (2 x 256 columns)
 //   warps 2..5     epilogue: tcgen05.ld 32 columns at a time, lag sums by
 //                  lane rotation and warp reductions, int64 atomics to the
-//                  numerator
+//                  numerator (deviation and two-time modes: warps 2..9)
 // Replaces dense.py:54,61-64 (numpy sgemm + diagonal loop), cuda.py:67-116
 // (cuBLAS sgemm + extract_upper_diags) and densecorrelator.cl:6-56.
 #include <cstring>
@@ -45,15 +45,18 @@ constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int NDIAG = BM + BN - 1;  // lags covered by one item
 constexpr int NDIAG_PAD = 384;
 constexpr int TMEM_COLS = 2 * BN;
-constexpr int NUM_THREADS = 192;
-constexpr int EPI_THREADS = 128;
+// Epilogue threads: four warps, one per TMEM sub-partition; the modes that work
+// on every element (a division, or stores) take eight, two per sub-partition
+// with half of the columns each (two-time matrix of 2,000 frames: 47 us with four
+// warps, 39 with eight; 75 with four-byte stores and sums read per element).
+constexpr int epi_threads(bool numer) { return numer ? 128 : 256; }
 constexpr uint32_t IDESC = idesc_f32acc(BM, BN);  // same bits for fp16 and e4m3 operands
 
 constexpr int SMEM_BAR_OFF = STAGES * STAGE_BYTES;
 constexpr int SMEM_BYTES = 1024 /*alignment slack*/ + SMEM_BAR_OFF + 256 + 2 * NDIAG_PAD * 4;
-// deviation mode: per TMEM buffer the lag centres, sums of d, sums of d^2 and
-// zero-denominator counts (4 x NDIAG_PAD words)
-constexpr int STD_WORDS = 4 * NDIAG_PAD;
+// deviation mode: per TMEM buffer the lag centres, sums of d, sums of d^2,
+// zero-denominator counts (4 x NDIAG_PAD words) and the columns' bin sums (BN)
+constexpr int STD_WORDS = 4 * NDIAG_PAD + BN;
 constexpr int SMEM_BYTES_STD = 1024 + SMEM_BAR_OFF + 256 + 2 * STD_WORDS * 4;
 
 // Outputs of the deviation mode (calc_std of dense.py:58-66): for every pair
@@ -124,11 +127,12 @@ __device__ __forceinline__ bool item_ok(const g2_gram_item& w, const MapsParam& 
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(64 + epi_threads(MODE == MODE_NUMER), 1)
     gram_tc_kernel(const __grid_constant__ MapsParam maps, int n_jobs, const g2_gram_item* __restrict__ items,
                    int64_t n_items, unsigned long long* __restrict__ numer, int64_t numer_len,
                    unsigned long long* __restrict__ sums, int64_t sums_len, int32_t* __restrict__ err,
                    const StdOut so) {
+  constexpr int EPI_THREADS = epi_threads(MODE == MODE_NUMER);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -159,7 +163,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     fence_mbar_init();
   }
   constexpr bool STD = MODE != MODE_NUMER;
-  for (int i = threadIdx.x; i < (STD ? 2 * STD_WORDS : 2 * NDIAG_PAD); i += NUM_THREADS) diag[i] = 0;
+  for (int i = threadIdx.x; i < (STD ? 2 * STD_WORDS : 2 * NDIAG_PAD); i += 64 + EPI_THREADS) diag[i] = 0;
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
@@ -262,6 +266,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     const int q = warp & 3;  // TMEM sub-partition this warp may access
     const int row = q * 32 + lane;
     const int etid = threadIdx.x - 64;
+    constexpr int CHUNKS = BN / 32 / (EPI_THREADS / 128);  // 32-column chunks per warp
+    const int cc0 = etid / 128 * CHUNKS;
     int64_t local = 0;
     for (int64_t it = blockIdx.x; it < n_items; it += gridDim.x, ++local) {
       const g2_gram_item w = items[it];
@@ -297,7 +303,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         const float wgt = unscale * static_cast<float>(1u << w.shift);
         const int64_t t = static_cast<int64_t>(w.i0) + row;
 #pragma unroll 1
-        for (int cc = 0; cc < BN / 32; ++cc) {
+        for (int cc = cc0; cc < cc0 + CHUNKS; ++cc) {
           uint32_t v[32];
           __syncwarp();
           tmem_ld_32x32b_x32(tbase + static_cast<uint32_t>(cc * 32), v);
@@ -322,22 +328,37 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         const float P = static_cast<float>(w.shift);
         const int64_t t = static_cast<int64_t>(w.i0) + row;
         const float St = row_live ? static_cast<float>(so.S[w.s_off + t]) : 0.0f;
+        float* col_sum = reinterpret_cast<float*>(diag) + (local & 1) * STD_WORDS;
+        for (int c = etid; c < BN; c += EPI_THREADS)
+          col_sum[c] = c < col_end ? static_cast<float>(so.S[w.s_off + w.j0 + c]) : 0.0f;
+        named_bar_sync(1, EPI_THREADS);
 #pragma unroll 1
-        for (int cc = 0; cc < BN / 32; ++cc) {
+        for (int cc = cc0; cc < cc0 + CHUNKS; ++cc) {
           uint32_t v[32];
           __syncwarp();
           tmem_ld_32x32b_x32(tbase + static_cast<uint32_t>(cc * 32), v);
           tmem_wait_ld();
           if (!row_live) continue;
+          const int64_t t2 = static_cast<int64_t>(w.j0) + cc * 32;
+          float* o = so.ttcf + t * so.ld + t2;
+          float r[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int c = cc * 32 + j;
-            const int64_t t2 = static_cast<int64_t>(w.j0) + c;
-            if (c >= col_end || t2 <= t) continue;  // t' >= T, or not above the diagonal
-            const float den = St * static_cast<float>(so.S[w.s_off + t2]);
-            const float r = P * (__uint_as_float(v[j]) * unscale) / den;  // 0/0 -> NaN as in the reference
-            so.ttcf[t * so.ld + t2] = r;
-            if (so.mirror) so.ttcf[t2 * so.ld + t] = r;
+          for (int j = 0; j < 32; ++j)  // 0/0 -> NaN as in the reference
+            r[j] = P * (__uint_as_float(v[j]) * unscale) / (St * col_sum[cc * 32 + j]);
+          // pairs t' > t, t' < T; a whole run of a row in 16-byte stores
+          if (cc * 32 + 32 <= col_end && t2 > t && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+              *reinterpret_cast<float4*>(o + j) = make_float4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (cc * 32 + j < col_end && t2 + j > t) o[j] = r[j];
+          }
+          if (so.mirror) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (cc * 32 + j < col_end && t2 + j > t) so.ttcf[(t2 + j) * so.ld + t] = r[j];
           }
         }
         tc_fence_before();
@@ -350,35 +371,69 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         float* sd = cen + NDIAG_PAD;
         float* sd2 = sd + NDIAG_PAD;
         unsigned int* zc = reinterpret_cast<unsigned int*>(sd2 + NDIAG_PAD);
+        float* col_sum = reinterpret_cast<float*>(zc + NDIAG_PAD);
         for (int d = etid; d < NDIAG; d += EPI_THREADS) {
           const int tau = lag0 + d;
           const float c = (tau >= 0 && tau < w.nframes) ? so.centre[w.out_off + tau] : 0.0f;
           cen[d] = isfinite(c) ? c : 0.0f;
         }
+        for (int c = etid; c < BN; c += EPI_THREADS)
+          col_sum[c] = c < col_end ? static_cast<float>(so.S[w.s_off + w.j0 + c]) : 0.0f;
         named_bar_sync(1, EPI_THREADS);
         const float P = static_cast<float>(w.shift);
         const float St = row_live ? static_cast<float>(so.S[w.s_off + w.i0 + row]) : 0.0f;
+        // Lag sums without an add per element in shared memory: lane L, row L of
+        // the warp's 32, carries the partial sums of the lag that it adds to at
+        // this column; from one column to the next they move up a lane (a lag's
+        // next element is one row down), lane 0 starts a new lag and lane 31's is
+        // complete, which lane j of the chunk keeps.  Float adds in shared memory
+        // are compare-and-swap loops: two per element made this epilogue 90 us a
+        // tile (8 bins of 2,000 frames of 256 x 256, e4m3: 378 us; without them 160,
+        // with eight warps 110; the numerator's Gram on CTA pairs 86).
+        const int top = row_live ? (w.j0 - w.i0) - row : -(1 << 30);  // columns c >= -top have t' >= t
+        float a = 0.0f, a2 = 0.0f;
 #pragma unroll 1
-        for (int cc = 0; cc < BN / 32; ++cc) {
+        for (int cc = cc0; cc < cc0 + CHUNKS; ++cc) {
           uint32_t v[32];
           __syncwarp();
           tmem_ld_32x32b_x32(tbase + static_cast<uint32_t>(cc * 32), v);
           tmem_wait_ld();
-          if (!row_live) continue;
           const int dbase = cc * 32 - row + (BM - 1);
+          float dv[32];
+          uint32_t none = 0;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if (cc * 32 + j >= col_end || dbase + j < (BM - 1) - (w.j0 - w.i0)) continue;  // t' >= T or t' < t
-            const float den = St * static_cast<float>(so.S[w.s_off + w.j0 + cc * 32 + j]);
-            if (den == 0.0f) {
-              atomicAdd(&zc[dbase + j], 1u);
-            } else {
-              const float r = P * (__uint_as_float(v[j]) * unscale) / den;
-              const float dv = r - cen[dbase + j];
-              atomicAdd(&sd[dbase + j], dv);
-              atomicAdd(&sd2[dbase + j], dv * dv);
+            const int c = cc * 32 + j;
+            const bool pair = c < col_end && c + top >= 0;  // t <= t' < T
+            const float den = St * col_sum[c];
+            const float r = P * (__uint_as_float(v[j]) * unscale) / (den == 0.0f ? 1.0f : den);
+            dv[j] = pair && den != 0.0f ? r - cen[dbase + j] : 0.0f;
+            none |= pair && den == 0.0f ? 1u << j : 0u;
+          }
+          for (; none; none &= none - 1) atomicAdd(&zc[dbase + __ffs(none) - 1], 1u);
+          __syncwarp();
+          float keep = 0.0f, keep2 = 0.0f;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            a = __shfl_up_sync(0xffffffffu, a, 1);
+            a2 = __shfl_up_sync(0xffffffffu, a2, 1);
+            if (lane == 0) a = a2 = 0.0f;
+            a += dv[j];
+            a2 += dv[j] * dv[j];
+            const float e = __shfl_sync(0xffffffffu, a, 31), e2 = __shfl_sync(0xffffffffu, a2, 31);
+            if (lane == j) {
+              keep = e;
+              keep2 = e2;
             }
           }
+          const int d = cc * 32 + lane - (q * 32 + 31) + (BM - 1);  // the lag of row 31 at column cc * 32 + lane
+          atomicAdd(&sd[d], keep);
+          atomicAdd(&sd2[d], keep2);
+        }
+        if (lane < 31) {  // the lags that no later column of this warp completes
+          const int d = (cc0 + CHUNKS) * 32 - 1 - row + (BM - 1);
+          atomicAdd(&sd[d], a);
+          atomicAdd(&sd2[d], a2);
         }
         tc_fence_before();
         mbar_arrive(&acce[buf]);
@@ -492,7 +547,7 @@ int launch_gram(const g2_job* jobs, int32_t n_jobs, const g2_gram_item* items_de
   if (sms <= 0) return G2_ERR_CUDA;
   int64_t g = grid > 0 ? grid : sms;
   if (g > n_items) g = n_items;
-  tc::gram_tc_kernel<MODE><<<static_cast<unsigned>(g), tc::NUM_THREADS, smem, as_stream(stream)>>>(
+  tc::gram_tc_kernel<MODE><<<static_cast<unsigned>(g), 64 + tc::epi_threads(MODE == tc::MODE_NUMER), smem, as_stream(stream)>>>(
       maps, n_jobs, items_dev, n_items, reinterpret_cast<unsigned long long*>(numer_dev), numer_len,
       reinterpret_cast<unsigned long long*>(sums_dev), sums_len, err_dev, so);
   return launch_status();
