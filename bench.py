@@ -201,6 +201,21 @@ def tc_rate(dev, kind, iters=40000, reps=5):
                                               "mma": "tcgen05 M128 N256 K%d x4 per iteration" % k}
 
 
+def piece_stage_ms(corr, frames, n):
+    """Mean milliseconds of the pack and of the Gram over ``n`` steps that run in
+    one piece on their production path (events round the two launches)."""
+    eng = corr.engine
+    eng.profile = True
+    rows = []
+    for _ in range(n):
+        corr.correlate_device(frames)
+        eng.take_events()
+        rows.append(eng.take_timeline())
+    eng.profile = False
+    eng.check_error()
+    return {k: sum(r[k + "0_end"] - r[k + "0"] for r in rows) / n for k in ("pack", "gram")}
+
+
 def make_workload(dev, T):
     from dynamix_gb300.speckle import annular_qmask, speckle_torch
     H, W = WORKLOAD["frame_shape"]
@@ -361,6 +376,12 @@ def run_ours(args):
     # launch), denominator, finalize
     merged = max(1, min(int(eng.PIPE_MERGE_FIRST), chunks)) - 1
     launches_per_step = 2 * chunks - merged + 2 if "pipeline_chunks" in info else 4
+    narrow = "residuals" in info
+    if narrow:                  # residual sums, and the e2m1 offset or the look at the counts
+        launches_per_step += 2
+    # a narrow step runs in one piece: its pack and Gram are timed as they run
+    whole = piece_stage_ms(corr, frames, max(3, min(args.steps, 10))) if chunks == 1 and "pipeline_chunks" in info \
+        else None
 
     # stage attribution: the same step run as one pack and one Gram launch,
     # with CUDA events on the launching stream around each stage
@@ -383,6 +404,8 @@ def run_ours(args):
         by_tile[tile] = (g_ms, p_ms)
     eng.tile = tile0
     gram_ms, pack_ms = by_tile[tile0]
+    if whole:
+        gram_ms, pack_ms = [whole["gram"]], [whole["pack"]]
     # one pipelined step with events at every pack and Gram launch of it
     eng.pipeline = True
     corr.correlate_device(frames)
@@ -397,14 +420,19 @@ def run_ours(args):
     # ran on, measured in this run by the library's own tcgen05 probe (the
     # kernel runs at full clock, below the power cap, like the probe).
     from dynamix_gb300 import _lib as L
-    kind = L.KIND_E4M3 if info.get("mode") == "e4m3" else L.KIND_FP16
+    kind = L.KIND_E4M3 if info.get("mode") in ("e4m3", "e2m1") else L.KIND_FP16
     peak, probe = tc_rate(dev, kind)
+    e2m1 = info.get("mode") == "e2m1"
+    elem_bytes = {"e2m1": 0.5, "e4m3": 1}.get(info.get("mode"), 2)
     peak_f16, _ = tc_rate(dev, L.KIND_FP16) if kind == L.KIND_E4M3 else (peak, None)
     peak_src = ("tcgen05 kind::%s rate measured in this run (g2_tc_rate_probe: %d CTAs x %d iterations of "
                 "4 x M128 N256 MMAs on shared-memory operands, best of 5, %.3f ms)"
                 % ("f8f6f4 e4m3" if kind == L.KIND_E4M3 else "f16", probe["ctas"], probe["iters"],
                    probe["launch_ms"]))
-    pack_bytes = T * H * W + T * info["packed_cols"] * (1 if info.get("mode") == "e4m3" else 2)
+    if e2m1:                    # K = 64 per instruction in the time of e4m3's K = 32
+        peak *= 2
+        peak_src = "kind::mxf4 as twice the " + peak_src
+    pack_bytes = T * H * W + T * info["packed_cols"] * elem_bytes
     pack_avg = sum(pack_ms) / len(pack_ms)
     # DRAM bytes of one Gram launch from the committed ncu summary of the tile measured there
     traffic = profile_traffic("gram_pair_dense_514x1030_%s.md" % info.get("mode")) if tile0 == "pair" else None
@@ -414,20 +442,25 @@ def run_ours(args):
         "warmup": max(args.warmup, 3), "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "u8", "data": "synthetic",
         "config": dict(WORKLOAD, nframes=T, parallelism="replicas" if world > 1 else "single"),
-        "mma_kind": {"e4m3": "tcgen05 kind::f8f6f4 (e4m3 counts <= 16, fp32 accumulate, exact below 2^24)",
+        "mma_kind": {"e2m1": "tcgen05 kind::mxf4 (e2m1 codes of count - 3, unit block scales, fp32 accumulate, exact "
+                             "below 2^24; counts above 7 as residuals, int64)",
+                     "e4m3": "tcgen05 kind::f8f6f4 (e4m3 counts <= 16, fp32 accumulate, exact below 2^24)",
                      "fp16": "tcgen05 kind::f16 (fp16 counts <= 2048, fp32 accumulate, exact below 2^24)",
                      "bytes": "tcgen05 kind::f16 on hi/lo byte planes (4 Grams)"}[info["mode"]],
         "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak, "traffic": traffic,
-                     "kernel": {"pair": "g2_gram_tc_pair", "wide": "g2_gram_tc_wide"}.get(tile0, "g2_gram_tc"),
+                     "kernel": "g2_gram_tc_e2m1" if e2m1 else
+                     {"pair": "g2_gram_tc_pair", "wide": "g2_gram_tc_wide"}.get(tile0, "g2_gram_tc"),
                      "peak_source": peak_src,
                      "algorithmic_ops_per_launch": 2 * macs, "launch_ms": gram_avg,
                      "other_peaks": {"tcgen05_f16_probe": peak_f16, "bf16_cublas_" + peak_kind: peaks.get(
                          "bf16_tflops")}},
+        # whole e4m3 (or fp16) operands, one launch, by tile
         "gram_ms_by_tile": {t: sum(v[0]) / len(v[0]) for t, v in by_tile.items()},
         "pipeline_timeline_ms": {k: round(v, 4) for k, v in timeline.items()},
         "stages_ms": {"pack": pack_avg, "gram_tc": gram_avg, "tile": tile0,
-                      "note": "stage times from %d steps run unpipelined (one pack, one Gram launch); the timed "
+                      "note": "stage times of the timed path (one pack, one Gram launch)" if whole else
+                              "stage times from %d steps run unpipelined (one pack, one Gram launch); the timed "
                               "steps overlap the pack of frame chunk c+1 with the Gram tiles chunk c completes "
                               "(%d chunks)" % (n_attr, chunks)},
         "dtype_detail": "integer counts (u8) packed as %s, N/S/D int64, g2 float64 -> float32" % info.get("mode"),
@@ -712,14 +745,16 @@ def measure_sparse(args, dev, T, steps, warmup, which=("sparse", "event"), shape
         stage_report = {"pairsum": {"ms": pair_ms, "GB_per_s": achieved, "bytes": pair_bytes,
                                     "pair_ops_per_s": pairs / (pair_ms / 1e3)},
                         "normalize": {"ms": stages.get("normalize", float("nan")), "bytes": norm_bytes}}
-        launches = 3   # pair sums, denominator, finalize
+        launches = 3   # pair sums, two of the normalisation
         if kind == "sparse":
             tms = stages.get("transpose", float("nan"))
             stage_report["transpose"] = {"ms": tms, "GB_per_s": transpose_bytes / (tms / 1e3) / 1e9,
                                          "bytes": transpose_bytes,
                                          "kernels": "row bounds, row counts, sub-block sums, two scans (3 each), "
                                                     "stage, gather"}
-            launches += 11
+            launches += 12     # with the largest count
+        else:
+            launches += 2      # checks of the offsets and of the events
         cfg = dict(SPARSE_WORKLOAD, nframes=T, frame_shape=[H, W], workload=SPARSE_WORKLOAD["workload"].replace(
             "sparse", "sparse_csr" if kind == "sparse" else "event_lists"),
             parallelism="replicas" if world > 1 else "single", n_elements=n_elem,
@@ -1137,7 +1172,11 @@ def measure_u16(args, dev, T, steps, warmup, cpu=True, e2e=True):
         eng.profile = True
         corr.correlate_device(frames)
         st = eng.stage_times(eng.take_events())
+        eng.take_timeline()
         eng.profile = False
+        if info.get("pipeline_chunks") == 1:
+            t = piece_stage_ms(corr, frames, max(3, min(steps, 10)))
+            st = {"pack": t["pack"], "gram_tc": t["gram"], "normalise": st.get("normalise", float("nan"))}
         planes = 4 if info["mode"] == "bytes" else 1
         gram = st.get("gram_tc", float("nan"))
         executed = 2.0 * macs * planes / (gram / 1e3) / 1e12
