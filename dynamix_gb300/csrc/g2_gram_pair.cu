@@ -18,9 +18,9 @@
 // registers (g2_epilogue.cuh), then adds one value per lane and lag group to
 // uint32 shared counters.
 //
-// Roles per CTA (192 threads): warp 0 lane 0 TMA producer (both CTAs), warp 1
+// Roles per CTA (192 or 320 threads): warp 0 lane 0 TMA producer (both CTAs), warp 1
 // lane 0 MMA issuer (leader only; warp 1 of both CTAs allocates TMEM), warps
-// 2..5 epilogue (both CTAs, each on its own TMEM rows).
+// 2..5 (or 2..9) epilogue (both CTAs, each on its own TMEM rows).
 // Barriers: full[s] of the leader collects both CTAs' TMA bytes of stage s;
 // empty[s] of each CTA and accf[b] of each CTA are signalled by the leader's
 // commits (multicast); acce[b] of the leader collects one arrival per
@@ -50,6 +50,13 @@ constexpr int TMEM_COLS = 2 * BN;
 constexpr int NUM_THREADS = 192;
 constexpr int EPI_THREADS = 128;
 constexpr int EPI_WARPS = EPI_THREADS / 32;
+// Epilogue threads of gram_pair_kernel: with eight warps, two per sub-partition
+// with half of an item's columns each, an item's epilogue is down from 7.6 us, so
+// that items of few stages (small bins, byte planes, K cut for exactness) wait
+// less for their accumulators: 195 x 487 x 1,500 u16 in digits 0.609 -> 0.546 ms,
+// 128 x 128 x 1,000 u8 30 -> 27 us.  e2m1 items, whose columns hold twice the
+// counts per stage, keep four: 514 x 1030 x 10,000 5.79 ms, 5.85 with eight.
+constexpr int pair_epi(bool f4) { return f4 ? 128 : 256; }
 constexpr int SMEM_BAR_OFF = STAGES * STAGE_BYTES;
 constexpr int SMEM_BYTES = 1024 /*alignment slack*/ + SMEM_BAR_OFF + 256 + 2 * NDIAG_PAD * 4;
 constexpr int F4_SMEM_BYTES = SMEM_BYTES - STAGES * (B_BYTES - 112 * ROW_BYTES);  // e2m1 items: 112 B rows per CTA
@@ -131,11 +138,12 @@ __device__ __forceinline__ unsigned long long widen(uint32_t v, bool is_signed) 
 
 // F4: e2m1 operands on kind::mxf4 (every job); else e4m3 / fp16 operands.
 template <bool F4>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + pair_epi(F4), 1)
     gram_pair_kernel(const __grid_constant__ typename PairMaps<F4>::type maps, int n_jobs, const g2_gram_item* __restrict__ items,
                      int64_t n_items, unsigned long long* __restrict__ numer, int64_t numer_len,
                      unsigned long long* __restrict__ sums, int64_t sums_len, int32_t* __restrict__ err) {
   constexpr int SB = F4 ? F4_B_BYTES : B_BYTES;  // B bytes per stage and CTA
+  constexpr int PAIR_EPI = pair_epi(F4);         // epilogue threads
   constexpr int ACC_STEP = F4 ? F4_BN : BN;      // TMEM columns from one accumulator to the next
   constexpr int BAR_OFF = STAGES * (A_BYTES + SB);
   extern __shared__ uint8_t smem_raw[];
@@ -164,13 +172,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&accf[b], 1);
-      mbar_init(&acce[b], 2 * EPI_WARPS);  // one per epilogue warp of both CTAs (leader's copy)
+      mbar_init(&acce[b], 2 * PAIR_EPI / 32);  // one per epilogue warp of both CTAs (leader's copy)
     }
     mbar_init(drain, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
-  for (int i = threadIdx.x; i < 2 * NDIAG_PAD; i += NUM_THREADS) diag[i] = 0;
+  for (int i = threadIdx.x; i < 2 * NDIAG_PAD; i += 64 + PAIR_EPI) diag[i] = 0;
   // both CTAs have initialised their barriers (and are running) before any
   // signal crosses between them
   cluster_sync_all();
@@ -181,7 +189,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   const uint32_t tmem_base = *tmem_slot;
   if (F4) {
     // the scale columns of both CTAs hold ones before the leader's first MMA
-    if (warp >= 2)
+    if (warp >= 2 && warp < 6)
       tmem_fill_x32(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + F4_SCALE_COL, F4_SCALE_ONES);
     tc_fence_before();
     cluster_sync_all();
@@ -332,7 +340,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       const uint32_t ap = static_cast<uint32_t>((local >> 1) & 1);
       uint32_t* dacc = diag + (local & 1) * NDIAG_PAD;
       const bool ok = mbar_wait_cluster(&accf[buf], ap, abort_flag, err);
-      if (named_bar_any(1, EPI_THREADS, !ok)) break;
+      if (named_bar_any(1, PAIR_EPI, !ok)) break;
       tc_fence_after();
       // e2m1 codes hold u / 2
       const float unscale = F4 ? 4.0f : (maps.kind[w.job] == G2_KIND_E4M3 ? 262144.0f : 281474976710656.0f);
@@ -351,9 +359,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       // the column of this row's own product, in an item of a plane with itself
       const int own = !F4 && ((maps.check >> w.job) & 1u) && w.a_k0 == w.b_k0 ? i0 + row - w.j0 : -1;
       const uint32_t most = sgn ? 1u << 23 : 1u << 24;
+      // this warp's chunks of 32 columns: with eight warps the first or the second half
+      const int c0 = etid < 128 ? 0 : n / 64, c1 = PAIR_EPI > 128 && etid < 128 ? n / 64 : n / 32;
       uint32_t carry = 0;
 #pragma unroll 1
-      for (int cc = 0; cc < n / 32; ++cc) {
+      for (int cc = c0; cc < c1; ++cc) {
         uint32_t v[32];
         __syncwarp();  // tcgen05.ld is warp-collective
         tmem_ld_32x32b_x32(tbase + static_cast<uint32_t>(cc * 32), v);
@@ -389,13 +399,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         if (val && d >= 0) atomicAdd(&dacc[d], val);
         carry = hi;
       }
-      if (carry) atomicAdd(&dacc[(n / 32 - 1) * 32 + dwarp], carry);
+      if (carry) atomicAdd(&dacc[(c1 - 1) * 32 + dwarp], carry);
       // this warp's TMEM reads are done: release the buffer to the leader's MMA
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_addr(&acce[buf]), 0));
-      named_bar_sync(1, EPI_THREADS);
-      for (int d = etid; d < NDIAG; d += EPI_THREADS) {
+      named_bar_sync(1, PAIR_EPI);
+      for (int d = etid; d < NDIAG; d += PAIR_EPI) {
         const uint32_t s = dacc[d];
         if (s) {
           const int tau = lag0 + d;
@@ -702,7 +712,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 
 namespace {
 // CTA pairs of `kernel` (one CTA per SM, `smem` bytes) that can be resident at once.
-int max_clusters(const void* kernel, int smem, int* out) {
+int max_clusters(const void* kernel, int threads, int smem, int* out) {
   using namespace g2;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return G2_ERR_CUDA;
@@ -710,7 +720,7 @@ int max_clusters(const void* kernel, int smem, int* out) {
   if (sms <= 0) return G2_ERR_CUDA;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1), 1, 1);
-  cfg.blockDim = dim3(pair::NUM_THREADS, 1, 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
   cfg.dynamicSmemBytes = smem;
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) return G2_ERR_CUDA;
@@ -719,15 +729,18 @@ int max_clusters(const void* kernel, int smem, int* out) {
 }
 
 int pair_max_clusters(int* out) {
-  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<false>), g2::pair::SMEM_BYTES, out);
+  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<false>), 64 + g2::pair::pair_epi(false),
+                      g2::pair::SMEM_BYTES, out);
 }
 
 int f4_max_clusters(int* out) {
-  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<true>), g2::pair::F4_SMEM_BYTES, out);
+  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<true>), 64 + g2::pair::pair_epi(true),
+                      g2::pair::F4_SMEM_BYTES, out);
 }
 
 int wide_max_clusters(int* out) {
-  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_wide_kernel), g2::pair::W_SMEM_BYTES, out);
+  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_wide_kernel), g2::pair::NUM_THREADS,
+                      g2::pair::W_SMEM_BYTES, out);
 }
 
 // Checks the jobs (element kinds with the given flags) and fills the tensor
@@ -807,7 +820,7 @@ int launch_pair(bool wide, const g2_job* jobs, int32_t n_jobs, const g2_gram_ite
     pair::gram_wide_kernel<<<g, pair::NUM_THREADS, pair::W_SMEM_BYTES, as_stream(stream)>>>(
         maps, n_jobs, items_dev, n_items, nm, numer_len, sm, sums_len, err_dev);
   else
-    pair::gram_pair_kernel<false><<<g, pair::NUM_THREADS, pair::SMEM_BYTES, as_stream(stream)>>>(
+    pair::gram_pair_kernel<false><<<g, 64 + pair::pair_epi(false), pair::SMEM_BYTES, as_stream(stream)>>>(
         maps, n_jobs, items_dev, n_items, nm, numer_len, sm, sums_len, err_dev);
   return launch_status();
 }
@@ -859,7 +872,7 @@ extern "C" int g2_gram_tc_e2m1(const g2_job* jobs, int32_t n_jobs, const g2_gram
   int64_t clusters = grid > 0 ? (grid + 1) / 2 : max_cl;
   if (clusters > max_cl) clusters = max_cl;
   if (clusters > n_items) clusters = n_items;
-  pair::gram_pair_kernel<true><<<static_cast<unsigned>(2 * clusters), pair::NUM_THREADS, pair::F4_SMEM_BYTES,
+  pair::gram_pair_kernel<true><<<static_cast<unsigned>(2 * clusters), 64 + pair::pair_epi(true), pair::F4_SMEM_BYTES,
                                  as_stream(stream)>>>(
       maps, n_jobs, items_dev, n_items, reinterpret_cast<unsigned long long*>(numer_dev), numer_len,
       reinterpret_cast<unsigned long long*>(sums_dev), sums_len, err_dev);
