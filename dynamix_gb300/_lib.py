@@ -29,7 +29,7 @@ PLAIN_BM, PLAIN_BN = 128, 128
 MAX_JOBS = 32
 ITEM_EMPTY = -1
 KIND_FP16, KIND_E4M3, KIND_E2M1 = 0, 1, 2
-KIND_BLOCKED, KIND_SIGNED, KIND_CHECK = 256, 512, 1024
+KIND_BLOCKED, KIND_SIGNED, KIND_CHECK, KIND_ALONE = 256, 512, 1024, 2048
 NARROW_CHUNK = 4080
 RES_SECTOR = 64  # packed columns per residual list
 

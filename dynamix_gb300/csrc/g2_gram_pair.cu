@@ -50,13 +50,16 @@ constexpr int TMEM_COLS = 2 * BN;
 constexpr int NUM_THREADS = 192;
 constexpr int EPI_THREADS = 128;
 constexpr int EPI_WARPS = EPI_THREADS / 32;
-// Epilogue threads of gram_pair_kernel: with eight warps, two per sub-partition
-// with half of an item's columns each, an item's epilogue is down from 7.6 us, so
-// that items of few stages (small bins, byte planes, K cut for exactness) wait
-// less for their accumulators: 195 x 487 x 1,500 u16 in digits 0.609 -> 0.546 ms,
-// 128 x 128 x 1,000 u8 30 -> 27 us.  e2m1 items, whose columns hold twice the
-// counts per stage, keep four: 514 x 1030 x 10,000 5.79 ms, 5.85 with eight.
-constexpr int pair_epi(bool f4) { return f4 ? 128 : 256; }
+// Epilogue threads of gram_pair_kernel: four warps, or eight (G2_KIND_ALONE), two
+// per TMEM sub-partition with half of an item's columns each.  With eight an
+// item's epilogue is down from 7.6 us, so that items of few stages (small bins,
+// byte planes, K cut for exactness) wait less for their accumulators: 195 x 487 x
+// 1,500 u16 in digits 0.609 -> 0.546 ms, 128 x 128 x 1,000 u8 30 -> 27 us.  But
+// its 320 threads leave a pack beside it no registers (e4m3 of 514 x 1030 x
+// 10,000 in 8 chunks, each packed under the Gram of the one before: 11.6 -> 12.6
+// ms), so that callers that overlap the two keep four, as do e2m1 items, whose
+// columns hold twice the counts per stage (5.79 ms there, 5.85 with eight).
+constexpr int EPI_ALONE = 256;
 constexpr int SMEM_BAR_OFF = STAGES * STAGE_BYTES;
 constexpr int SMEM_BYTES = 1024 /*alignment slack*/ + SMEM_BAR_OFF + 256 + 2 * NDIAG_PAD * 4;
 constexpr int F4_SMEM_BYTES = SMEM_BYTES - STAGES * (B_BYTES - 112 * ROW_BYTES);  // e2m1 items: 112 B rows per CTA
@@ -137,13 +140,13 @@ __device__ __forceinline__ unsigned long long widen(uint32_t v, bool is_signed) 
 }
 
 // F4: e2m1 operands on kind::mxf4 (every job); else e4m3 / fp16 operands.
-template <bool F4>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + pair_epi(F4), 1)
+// PAIR_EPI: epilogue threads.
+template <bool F4, int PAIR_EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + PAIR_EPI, 1)
     gram_pair_kernel(const __grid_constant__ typename PairMaps<F4>::type maps, int n_jobs, const g2_gram_item* __restrict__ items,
                      int64_t n_items, unsigned long long* __restrict__ numer, int64_t numer_len,
                      unsigned long long* __restrict__ sums, int64_t sums_len, int32_t* __restrict__ err) {
   constexpr int SB = F4 ? F4_B_BYTES : B_BYTES;  // B bytes per stage and CTA
-  constexpr int PAIR_EPI = pair_epi(F4);         // epilogue threads
   constexpr int ACC_STEP = F4 ? F4_BN : BN;      // TMEM columns from one accumulator to the next
   constexpr int BAR_OFF = STAGES * (A_BYTES + SB);
   extern __shared__ uint8_t smem_raw[];
@@ -729,13 +732,18 @@ int max_clusters(const void* kernel, int threads, int smem, int* out) {
 }
 
 int pair_max_clusters(int* out) {
-  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<false>), 64 + g2::pair::pair_epi(false),
-                      g2::pair::SMEM_BYTES, out);
+  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<false, g2::pair::EPI_THREADS>),
+                      g2::pair::NUM_THREADS, g2::pair::SMEM_BYTES, out);
+}
+
+int alone_max_clusters(int* out) {
+  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<false, g2::pair::EPI_ALONE>),
+                      64 + g2::pair::EPI_ALONE, g2::pair::SMEM_BYTES, out);
 }
 
 int f4_max_clusters(int* out) {
-  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<true>), 64 + g2::pair::pair_epi(true),
-                      g2::pair::F4_SMEM_BYTES, out);
+  return max_clusters(reinterpret_cast<const void*>(g2::pair::gram_pair_kernel<true, g2::pair::EPI_THREADS>),
+                      g2::pair::NUM_THREADS, g2::pair::F4_SMEM_BYTES, out);
 }
 
 int wide_max_clusters(int* out) {
@@ -804,11 +812,13 @@ int launch_pair(bool wide, const g2_job* jobs, int32_t n_jobs, const g2_gram_ite
   static pair::MapsParam maps;  // large; filled under the lock below
   static std::mutex* mu = new std::mutex;
   std::lock_guard<std::mutex> lk(*mu);
-  int st = pair_maps(jobs, n_jobs, wide ? G2_KIND_BLOCKED : G2_KIND_BLOCKED | G2_KIND_SIGNED | G2_KIND_CHECK, &maps);
+  int st = pair_maps(jobs, n_jobs, wide ? G2_KIND_BLOCKED
+                                        : G2_KIND_BLOCKED | G2_KIND_SIGNED | G2_KIND_CHECK | G2_KIND_ALONE, &maps);
   if (st != G2_OK) return st;
   if (n_items == 0) return G2_OK;
   int max_cl = 0;
-  st = wide ? wide_max_clusters(&max_cl) : pair_max_clusters(&max_cl);
+  const bool alone = (jobs[0].elem_kind & G2_KIND_ALONE) != 0;
+  st = wide ? wide_max_clusters(&max_cl) : alone ? alone_max_clusters(&max_cl) : pair_max_clusters(&max_cl);
   if (st != G2_OK) return st;
   int64_t clusters = grid > 0 ? (grid + 1) / 2 : max_cl;
   if (clusters > max_cl) clusters = max_cl;
@@ -819,8 +829,11 @@ int launch_pair(bool wide, const g2_job* jobs, int32_t n_jobs, const g2_gram_ite
   if (wide)
     pair::gram_wide_kernel<<<g, pair::NUM_THREADS, pair::W_SMEM_BYTES, as_stream(stream)>>>(
         maps, n_jobs, items_dev, n_items, nm, numer_len, sm, sums_len, err_dev);
+  else if (alone)
+    pair::gram_pair_kernel<false, pair::EPI_ALONE><<<g, 64 + pair::EPI_ALONE, pair::SMEM_BYTES, as_stream(stream)>>>(
+        maps, n_jobs, items_dev, n_items, nm, numer_len, sm, sums_len, err_dev);
   else
-    pair::gram_pair_kernel<false><<<g, 64 + pair::pair_epi(false), pair::SMEM_BYTES, as_stream(stream)>>>(
+    pair::gram_pair_kernel<false, pair::EPI_THREADS><<<g, pair::NUM_THREADS, pair::SMEM_BYTES, as_stream(stream)>>>(
         maps, n_jobs, items_dev, n_items, nm, numer_len, sm, sums_len, err_dev);
   return launch_status();
 }
@@ -872,7 +885,7 @@ extern "C" int g2_gram_tc_e2m1(const g2_job* jobs, int32_t n_jobs, const g2_gram
   int64_t clusters = grid > 0 ? (grid + 1) / 2 : max_cl;
   if (clusters > max_cl) clusters = max_cl;
   if (clusters > n_items) clusters = n_items;
-  pair::gram_pair_kernel<true><<<static_cast<unsigned>(2 * clusters), 64 + pair::pair_epi(true), pair::F4_SMEM_BYTES,
+  pair::gram_pair_kernel<true, pair::EPI_THREADS><<<static_cast<unsigned>(2 * clusters), pair::NUM_THREADS, pair::F4_SMEM_BYTES,
                                  as_stream(stream)>>>(
       maps, n_jobs, items_dev, n_items, reinterpret_cast<unsigned long long*>(numer_dev), numer_len,
       reinterpret_cast<unsigned long long*>(sums_dev), sums_len, err_dev);

@@ -603,7 +603,8 @@ class DenseEngine(ResultBuffers):
 
     def numerator(self, L, items_dev, n_items):
         self.numer.zero_()
-        jobs = _lib.jobs_array([(self.packed.data_ptr(), self.T, L.packed_cols, L.kind, self.ones(L))])
+        alone = _lib.KIND_ALONE if self.method == "tc" and self.tile == "pair" else 0
+        jobs = _lib.jobs_array([(self.packed.data_ptr(), self.T, L.packed_cols, L.kind + alone, self.ones(L))])
         st = stream_handle(self.dev)
         if self.method == "tc":
             self.gram_launch(jobs, items_dev.data_ptr(), n_items, st)
@@ -1053,6 +1054,8 @@ class DenseEngine(ResultBuffers):
         kind = L.kind + (_lib.KIND_BLOCKED if blocked and narrow != MODE_E2M1 else 0)
         if wide is not None:
             kind += _lib.KIND_CHECK + (_lib.KIND_SIGNED if L.split else 0)
+        if bounds.size == 2 and self.tile == "pair" and mode != MODE_E2M1:
+            kind += _lib.KIND_ALONE               # one piece: no pack runs beside the Gram
         jobs = _lib.jobs_array([(packed.data_ptr(), self.T, L.packed_cols, kind, self.ones(L))])
         item_bytes = _lib.ITEM_DTYPE.itemsize
         for c in range(bounds.size - 1):

@@ -71,6 +71,8 @@ extern "C" {
 #define G2_KIND_SIGNED 512  /* signed elements (16-bit: sign and magnitude): signed lag sums */
 #define G2_KIND_CHECK 1024  /* set G2_DEVERR_ENERGY when an item's G(t, t) reaches 2^24 (signed: 2^23):
                                below it every entry of the item is exact (Cauchy-Schwarz) */
+#define G2_KIND_ALONE 2048  /* (the first job's) no other kernel is to run beside the launch: it may take
+                               all of an SM's registers */
 #define G2_RES_SECTOR 64   /* packed columns per residual list */
 
 /* One unit of Gram work: rows [i0, i0+BM) of the A operand against rows
