@@ -1332,36 +1332,45 @@ class DenseEngine(ResultBuffers):
                      "packed_cols": L.packed_cols}
         return self.g2_f32[: self.n_bins]
 
-    def _last_operand(self, what):
-        """(layout, element kind, buffer) of the last run's packed operand as
-        the single-CTA kernels read it: a narrow operand is expanded to
-        row-major e4m3 bytes, or to fp16 when a count exceeds 16."""
-        torch = _torch()
+    def _last_layout(self, what):
+        """(layout, K-blocked) of the last run's packed operand."""
         if self.packed is None or self._packed_mode is None:
             raise RuntimeError("%s needs a preceding run()" % what)
-        if self._residuals is None:
-            blocked, L = self._packed_layout
-            if not blocked:
-                L = self._layouts[self._packed_mode]
-                return L, L.kind, self.packed
-            rows, row_bytes = self.T + 1, L.packed_bytes_per_frame
-            wide = self._expand_buffer(rows * row_bytes)
-            _lib.check(self.lib.g2_operand_rows(ptr(self.packed), rows, row_bytes, ptr(wide),
-                                                stream_handle(self.dev)), "g2_operand_rows")
-            return L, L.kind, wide
-        L, counts, lists, cap, total = self._residuals
+        blocked, L = self._packed_layout
+        return (L if blocked else self._layouts[self._packed_mode]), blocked
+
+    def _last_operand(self, what, b=None):
+        """(layout, element kind, buffer, first column, columns) of the last
+        run's packed operand as the single-CTA kernels read it.  A K-blocked
+        operand is copied to rows, with ``b`` only that bin's columns, a narrow
+        one in e4m3 bytes, or in fp16 when a count exceeds 16."""
+        L, blocked = self._last_layout(what)
+        if not blocked:
+            return L, L.kind, self.packed, 0, L.packed_cols
         rows = self.T + 1
+        col0, cols = (0, L.packed_cols) if b is None else (int(L.plane0[b]), int(L.kpad[b]))
+        src = C.c_void_p(self.packed.data_ptr() + int(col0 * L.elem_bytes) * rows)   # whole 128-byte blocks
+        st = stream_handle(self.dev)
+        if cols == 0:
+            return L, L.kind, self.packed, col0, cols
+        if self._residuals is None:
+            row_bytes = int(cols * L.elem_bytes)
+            wide = self._expand_buffer(rows * row_bytes)
+            _lib.check(self.lib.g2_operand_rows(src, rows, row_bytes, ptr(wide), st), "g2_operand_rows")
+            return L, L.kind, wide, col0, cols
+        L, counts, lists, cap, total = self._residuals
+        s0 = col0 // _lib.RES_SECTOR
         for kind, nb in ((_lib.KIND_E4M3, 1), (_lib.KIND_FP16, 2)):
             if L.mode == MODE_E4M3 and total and kind == L.kind:
                 continue                              # residuals of e4m3 are counts above 16
-            wide = self._expand_buffer(rows * L.packed_cols * nb)
+            wide = self._expand_buffer(rows * cols * nb)
             self.err.zero_()
-            _lib.check(self.lib.g2_operand_expand(ptr(self.packed), rows, self.T, L.packed_cols, L.kind, kind,
-                                                  ptr(counts), ptr(lists), cap, ptr(wide), ptr(self.err),
-                                                  stream_handle(self.dev)), "g2_operand_expand")
+            _lib.check(self.lib.g2_operand_expand(src, rows, self.T, cols, L.kind, kind, ptr(counts[s0:]),
+                                                  ptr(lists[2 * s0 * cap:]), cap, ptr(wide), ptr(self.err), st),
+                       "g2_operand_expand")
             if kind == _lib.KIND_FP16 or not total or not int(self.err.item()) & _lib.DEVERR_RANGE:
                 break
-        return L, kind, wide
+        return L, kind, wide, col0, cols
 
     def _expand_buffer(self, nbytes):
         buf = getattr(self, "_expanded", None)
@@ -1377,7 +1386,7 @@ class DenseEngine(ResultBuffers):
         torch = _torch()
         if self.method != "tc":
             raise NotImplementedError("calc_std runs on the tensor-core path")
-        L, kind, packed = self._last_operand("deviation()")
+        L, kind, packed, _, _ = self._last_operand("deviation()")
         if L.split:
             return self._deviation_planes(L, packed)
         key = ("std", L.mode, self.T, tuple(L.grams()))
@@ -1460,11 +1469,11 @@ class DenseEngine(ResultBuffers):
         torch = _torch()
         if self.method != "tc":
             raise NotImplementedError("the two-time correlation runs on the tensor-core path")
-        L, kind, packed = self._last_operand("two_time()")
-        if L.split:
+        if self._last_layout("two_time()")[0].split:
             raise NotImplementedError("the two-time correlation needs counts <= 2048 (no byte planes)")
         if not 0 <= b < self.n_bins:
             raise ValueError("bin %d outside [0, %d)" % (b, self.n_bins))
+        L, kind, packed, col0, cols = self._last_operand("two_time()", b)
         key = ("std", L.mode, self.T, tuple(L.grams()))
         if key not in self._items_cache:
             from .plan import std_items
@@ -1475,6 +1484,8 @@ class DenseEngine(ResultBuffers):
         mine = items[items["out_off"] == b * self.T]
         if mine.size == 0:
             raise ValueError("bin %d has no pixels" % (b + 1))
+        mine["a_k0"] -= col0
+        mine["b_k0"] -= col0
         items_dev = torch.from_numpy(mine.view(np.uint8).copy()).to(self.dev)
         S = self.sums[b * self.T:(b + 1) * self.T] if self.sums.dim() == 1 else self.sums[b]
         s_h = S.cpu().numpy().astype(np.float64)
@@ -1482,7 +1493,7 @@ class DenseEngine(ResultBuffers):
         mirror = 1 if self.T <= 5 or not np.any(s_h[:-5] * s_h[5:] == 0) else 0
         out = torch.empty((self.T, self.T), dtype=torch.float32, device=self.dev)
         st = stream_handle(self.dev)
-        jobs = _lib.jobs_array([(packed.data_ptr(), self.T, L.packed_cols, kind, self.ones(L))])
+        jobs = _lib.jobs_array([(packed.data_ptr(), self.T, cols, kind, self.ones(L))])
         _lib.check(self.lib.g2_gram_ttcf(jobs, 1, ptr(items_dev), mine.size, ptr(self.sums), self.sums.numel(),
                                          ptr(out), self.T, self.T, mirror, ptr(self.err), self.grid, st),
                    "g2_gram_ttcf")

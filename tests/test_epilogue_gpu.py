@@ -45,3 +45,28 @@ def test_two_time_tile_edges(built_lib, cuda_device, T, empty):
         assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
         ok = np.isfinite(want)
         assert np.all(np.abs(got[ok] - want[ok]) <= 5e-6 * np.abs(want[ok]) + 1e-30)
+
+
+@pytest.mark.parametrize("dtype,top", [(np.uint8, 6), (np.uint8, 40), (np.uint16, 300)])
+def test_two_time_of_a_bin_of_a_blocked_operand(built_lib, cuda_device, dtype, top):
+    """Only the bin's columns of a K-blocked operand are copied to rows: bins at
+    the start, in the middle and at the end, an empty one, residuals in others."""
+    import torch
+    from dynamix_gb300.correlator import MatMulCorrelator
+    rng = np.random.default_rng(top)
+    T, shape = 270, (30, 40)
+    fr = rng.poisson(top / 3.0 * rng.random((1,) + shape), (T,) + shape).clip(0, top).astype(dtype)
+    fr[5, 3, 7], fr[9, 20, 30] = top, min(3 * top, 255)
+    qm = np.repeat([1, 2, 0, 4], 300).reshape(shape).astype(np.int32)
+    c = MatMulCorrelator(shape, T, qmask=qm)
+    c.engine.NARROW_MIN_MACS = 0.0
+    c.engine.NARROW_MAX = {3: 1e-2, 2: 1e-2}
+    c.correlate(torch.from_numpy(fr).to(cuda_device))
+    assert c.engine._packed_layout[0]
+    for q in (1, 2, c.n_bins):
+        if not np.any(qm == q):
+            continue
+        got, want = c.two_time(q), o.ttcf_exact(fr, qm, q)
+        ok = np.isfinite(want)
+        assert np.array_equal(np.isfinite(got), ok)
+        assert np.all(np.abs(got[ok] - want[ok]) <= 5e-6 * np.abs(want[ok]) + 1e-30)
