@@ -1023,12 +1023,15 @@ class DenseEngine(ResultBuffers):
         if not host and frames_dev.data_ptr() % 16:
             frames_dev = frames_dev.clone()
         cur = torch.cuda.current_stream(self.dev)
-        copy_s, pack_s, gram_s = self._streams()
+        # one piece has nothing to overlap: its launches follow each other on the
+        # caller's stream, without events between streams
+        one = not host and bounds.size == 2
+        copy_s, pack_s, gram_s = (cur, cur, cur) if one else self._streams()
         # consecutive chunks' Gram launches alternate between the caller's
         # stream and a second one, so a launch's CTAs take the SMs that the
         # previous launch's last items leave (sums are atomic adds: exact in
         # any order)
-        gram_streams = (cur, gram_s) if self.pipe_gram_streams > 1 else (cur,)
+        gram_streams = (cur, gram_s) if self.pipe_gram_streams > 1 and not one else (cur,)
         self._events = []
         self._mark("pipeline")
         self.zero_results()
@@ -1041,11 +1044,12 @@ class DenseEngine(ResultBuffers):
         if narrow is not None:
             res = self._residual_buffers(L)
             res[0].zero_()
-        start = torch.cuda.Event()
-        start.record(cur)                     # the previous call's work and the zeroing are done first
-        copy_s.wait_event(start)
-        pack_s.wait_event(start)
-        gram_s.wait_event(start)
+        if not one:
+            start = torch.cuda.Event()
+            start.record(cur)                 # the previous call's work and the zeroing are done first
+            copy_s.wait_event(start)
+            pack_s.wait_event(start)
+            gram_s.wait_event(start)
         self._timeline = []
         self._tmark("start", cur)
         npix = npix_in
@@ -1089,8 +1093,9 @@ class DenseEngine(ResultBuffers):
             else:
                 self.pack_fp16_frames(src, eb, t1 - t0, L, dst, emax, pack_s.cuda_stream)
             self._tmark("pack%d_end" % c, pack_s)
-            e = torch.cuda.Event()
-            e.record(pack_s)
+            if not one:
+                e = torch.cuda.Event()
+                e.record(pack_s)
             # the first PIPE_MERGE_FIRST chunks' tiles go in one launch (the
             # first chunk alone completes too few tiles to fill the GPU)
             merge = max(1, min(int(self.PIPE_MERGE_FIRST), bounds.size - 1))
@@ -1099,16 +1104,18 @@ class DenseEngine(ResultBuffers):
             k0, k1 = int(starts[0 if c == merge - 1 else c]), int(starts[c + 1])
             if k1 > k0:
                 gs = gram_streams[c % len(gram_streams)]
-                gs.wait_event(e)
+                if not one:
+                    gs.wait_event(e)
                 self._tmark("gram%d" % c, gs)
                 self.gram_launch(jobs, dev_items.data_ptr() + k0 * item_bytes, k1 - k0, gs.cuda_stream)
                 self._tmark("gram%d_end" % c, gs)
         if narrow == MODE_E4M3:               # whether the next stack could run on e2m1
             self._count_tail(frames_dev.data_ptr(), self.T, npix, Lp, min(self.T, self.TAIL_FRAMES),
                              C.c_void_p(pack_s.cuda_stream))
-            done = torch.cuda.Event()
-            done.record(pack_s)
-            cur.wait_event(done)
+            if not one:
+                done = torch.cuda.Event()
+                done.record(pack_s)
+                cur.wait_event(done)
         if len(gram_streams) > 1:
             done = torch.cuda.Event()
             done.record(gram_s)
