@@ -1095,7 +1095,9 @@ extern "C" int g2_operand_expand(const void* packed_dev, int64_t nrows, int64_t 
   if (e2m1 && wide) tail::expand_kernel<true, true><<<g, 256, 0, st>>>(in, nrows, packed_cols, out);
   else if (e2m1) tail::expand_kernel<true, false><<<g, 256, 0, st>>>(in, nrows, packed_cols, out);
   else if (wide) tail::expand_kernel<false, true><<<g, 256, 0, st>>>(in, nrows, packed_cols, out);
-  else tail::expand_kernel<false, false><<<g, 256, 0, st>>>(in, nrows, packed_cols, out);
+  else  // the same bytes in rows
+    tail::rows_kernel<<<static_cast<unsigned>((nrows * (packed_cols / 16) + 255) / 256), 256, 0, st>>>(
+        in, nrows, packed_cols, out);
   if (wide) tail::expand_residual_kernel<true><<<res.n_sectors, 64, 0, st>>>(res, nframes, packed_cols, out, err_dev);
   else tail::expand_residual_kernel<false><<<res.n_sectors, 64, 0, st>>>(res, nframes, packed_cols, out, err_dev);
   return launch_status();
