@@ -108,6 +108,7 @@ SIGNATURES = {
     "g2_stream_compress": (C.c_int, [_p, _i32, _i32, _i64, _i64, _i32, _i32, _p, _p, _p, _p, _p, _p, _p]),
     "g2_stream_compact": (C.c_int, [_p, _p, _p, _i32, _i64, _i32, _p, _i64, _p, _p, _p, _p]),
     "g2_denominator": (C.c_int, [_p, _i32, _i64, _p, _p]),
+    "g2_normalize": (C.c_int, [_p, _p, _p, _i32, _i64, _p, _i64, _p, _p, _p, _p]),
     "g2_finalize": (C.c_int, [_p, _p, _p, _i32, _i64, _p, _p, _p]),
     "g2_max_i64": (C.c_int, [_p, _i64, _p, _p]),
     "g2_ntt_scratch": (_i64, [_i32, _i64]),

@@ -37,9 +37,22 @@ constexpr int WIN_SHORT = 128;       // the same for launches of few blocks
 // apart (a thread's 4 consecutive lags) fall on distinct banks.
 __device__ __forceinline__ int pad32(int x) { return x + (x >> 5); }
 
-template <int WIN>
+// What g2_normalize does beyond G3, in the block that is the last to add to its
+// lags: G4 for them (and the largest S, found by the first lag block of a row).
+// Short stacks are bound by launches: denominator, finalize and maximum in one
+// (a call on 128 x 128 x 1,000 u8 168 -> 160 us).
+struct Finish {
+  const long long* N;
+  const double* scale;
+  float* g32;
+  double* g64;
+  uint32_t* arrived;          // per row and lag block, zeroed by the caller
+  unsigned long long* most;   // raised to the largest S; may be null
+};
+
+template <int WIN, bool FINISH>
 __global__ void __launch_bounds__(THR)
-    denom_kernel(const long long* __restrict__ S, int64_t T, long long* __restrict__ D) {
+    denom_kernel(const long long* __restrict__ S, int64_t T, long long* D, const Finish fin) {
   constexpr int WIN2_PAD = WIN + LAGS + (WIN + LAGS) / 32;
   __shared__ uint32_t lo1[WIN], hi1[WIN];
   __shared__ uint32_t lo2[WIN2_PAD], hi2[WIN2_PAD];
@@ -48,7 +61,7 @@ __global__ void __launch_bounds__(THR)
   const int64_t tau0 = static_cast<int64_t>(blockIdx.x) * LAGS;
   const long long* row = S + r * T;
   const int l0 = LPT * threadIdx.x;  // this thread's lags: tau0 + l0 + k
-  unsigned long long acc[LPT] = {0, 0, 0, 0};
+  unsigned long long acc[LPT] = {0, 0, 0, 0}, most = 0;
   // split z of gridDim.z takes every gridDim.z-th window of frames
   for (int64_t t0 = static_cast<int64_t>(blockIdx.z) * WIN; t0 < T - tau0;
        t0 += static_cast<int64_t>(gridDim.z) * WIN) {
@@ -57,6 +70,7 @@ __global__ void __launch_bounds__(THR)
     for (int i = threadIdx.x; i < WIN; i += THR) {
       const int64_t t = t0 + i;
       const unsigned long long v = t < T ? static_cast<unsigned long long>(row[t]) : 0ull;
+      if (FINISH) most = max(most, v);
       lo1[i] = static_cast<uint32_t>(v);
       hi1[i] = static_cast<uint32_t>(v >> 32);
       wide |= (v >> 32) != 0;
@@ -132,6 +146,28 @@ __global__ void __launch_bounds__(THR)
         atomicAdd(reinterpret_cast<unsigned long long*>(&D[r * T + tau]), acc[k]);  // D zeroed by the host
     }
   }
+  if (FINISH) {
+    if (fin.most && blockIdx.x == 0) {  // the windows of a row's first lag block cover the row
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+      if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(fin.most, most);
+    }
+    __shared__ bool s_last;
+    __threadfence();  // this thread's part of D before the block's arrival
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&fin.arrived[r * gridDim.x + blockIdx.x], 1u) == gridDim.z - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const double scale = fin.scale[r];
+    for (int i = threadIdx.x; i < LAGS; i += THR) {
+      const int64_t tau = tau0 + i;
+      if (tau >= T) break;
+      const double g = scale * static_cast<double>(fin.N[r * T + tau]) / static_cast<double>(__ldcg(&D[r * T + tau]));
+      if (fin.g32) fin.g32[r * T + tau] = static_cast<float>(g);
+      if (fin.g64) fin.g64[r * T + tau] = g;
+    }
+  }
 }
 
 // Launch G3 with enough blocks to fill the GPU: the frame windows are split
@@ -139,7 +175,9 @@ __global__ void __launch_bounds__(THR)
 // The work of a lag block falls with its lags (fewer frames pair up), so the
 // first blocks set the time: z aims at 32 blocks per SM, not just enough to
 // occupy every SM (2162x2068x20k events, 32 bins: 1.01 -> 0.71 ms).
-inline int launch_denominator(const long long* S, int32_t n_rows, int64_t T, long long* D, cudaStream_t st) {
+// With `fin` (its counters behind D): g2 too, in the same launch.
+inline int launch_denominator(const long long* S, int32_t n_rows, int64_t T, long long* D, const Finish* fin,
+                              cudaStream_t st) {
   const int64_t gx = (T + LAGS - 1) / LAGS;
   if (gx > 0x7fffffff) return G2_ERR_TOO_LARGE;
   const int sms = sm_count_current();
@@ -152,11 +190,13 @@ inline int launch_denominator(const long long* S, int32_t n_rows, int64_t T, lon
   const int64_t windows = (T + win - 1) / win;
   int64_t z = (32ll * sms + gx * n_rows - 1) / (gx * n_rows);
   z = z < 1 ? 1 : (z > windows ? windows : (z > 32 && !small ? 32 : z));
-  if (z > 1 && cudaMemsetAsync(D, 0, static_cast<size_t>(n_rows) * T * sizeof(long long), st) != cudaSuccess)
-    return G2_ERR_CUDA;
+  const size_t clear = static_cast<size_t>(n_rows) * T * sizeof(long long) + (fin ? n_rows * gx * sizeof(uint32_t) : 0);
+  if ((fin || z > 1) && cudaMemsetAsync(D, 0, clear, st) != cudaSuccess) return G2_ERR_CUDA;
   dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(n_rows), static_cast<unsigned>(z));
-  if (small) denom_kernel<WIN_SHORT><<<grid, THR, 0, st>>>(S, T, D);
-  else denom_kernel<WIN><<<grid, THR, 0, st>>>(S, T, D);
+  if (fin && small) denom_kernel<WIN_SHORT, true><<<grid, THR, 0, st>>>(S, T, D, *fin);
+  else if (fin) denom_kernel<WIN, true><<<grid, THR, 0, st>>>(S, T, D, *fin);
+  else if (small) denom_kernel<WIN_SHORT, false><<<grid, THR, 0, st>>>(S, T, D, Finish{});
+  else denom_kernel<WIN, false><<<grid, THR, 0, st>>>(S, T, D, Finish{});
   return launch_status();
 }
 
@@ -283,7 +323,25 @@ extern "C" int g2_denominator(const int64_t* sums_dev, int32_t n_rows, int64_t n
   if (n_rows == 0) return G2_OK;
   if (n_rows > 65535) return G2_ERR_TOO_LARGE;
   return norm::launch_denominator(reinterpret_cast<const long long*>(sums_dev), n_rows, nframes,
-                                  reinterpret_cast<long long*>(denom_dev), as_stream(stream));
+                                  reinterpret_cast<long long*>(denom_dev), nullptr, as_stream(stream));
+}
+
+extern "C" int g2_normalize(const int64_t* numer_dev, const int64_t* sums_dev, const double* scale_dev, int32_t n_rows,
+                            int64_t nframes, int64_t* denom_dev, int64_t denom_len, float* g2_f32_dev,
+                            double* g2_f64_dev, uint64_t* max_dev, void* stream) {
+  using namespace g2;
+  if (!numer_dev || !sums_dev || !scale_dev || !denom_dev || n_rows < 0 || nframes <= 0 ||
+      (!g2_f32_dev && !g2_f64_dev) || (max_dev && !aligned(max_dev, 8)))
+    return G2_ERR_ARG;
+  if (n_rows == 0) return G2_OK;
+  if (n_rows > 65535) return G2_ERR_TOO_LARGE;
+  const int64_t blocks = (nframes + norm::LAGS - 1) / norm::LAGS;
+  if (denom_len < n_rows * nframes + (n_rows * blocks + 1) / 2) return G2_ERR_ARG;
+  const norm::Finish fin{reinterpret_cast<const long long*>(numer_dev), scale_dev, g2_f32_dev, g2_f64_dev,
+                         reinterpret_cast<uint32_t*>(denom_dev + n_rows * nframes),
+                         reinterpret_cast<unsigned long long*>(max_dev)};
+  return norm::launch_denominator(reinterpret_cast<const long long*>(sums_dev), n_rows, nframes,
+                                  reinterpret_cast<long long*>(denom_dev), &fin, as_stream(stream));
 }
 
 extern "C" int g2_max_i64(const int64_t* x_dev, int64_t n, uint64_t* max_dev, void* stream) {
@@ -354,8 +412,8 @@ extern "C" int g2_normalize_static(const int64_t* numer_dev, const int64_t* sums
   if (sms <= 0) return G2_ERR_CUDA;
   const int64_t gx = (nframes + norm::LAGS - 1) / norm::LAGS;
   dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(n_rows));
-  norm::denom_kernel<norm::WIN><<<grid, norm::THR, 0, as_stream(stream)>>>(reinterpret_cast<const long long*>(sums_dev),
-                                                                 nframes, denom);
+  norm::denom_kernel<norm::WIN, false><<<grid, norm::THR, 0, as_stream(stream)>>>(
+      reinterpret_cast<const long long*>(sums_dev), nframes, denom, norm::Finish{});
   const int64_t total = static_cast<int64_t>(n_rows) * nframes;
   int64_t blocks = (total + 255) / 256;
   if (blocks > sms * 8) blocks = sms * 8;

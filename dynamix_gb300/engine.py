@@ -178,6 +178,10 @@ class ResultBuffers:
         self._sum_max = words[4:6]
         self.g2_f32 = words[8:8 + n].view(torch.float32).view(rows, self.T)
         self._result = None       # (status words, g2) of the run that correlate() reads
+        # D, and behind it the counters of g2_normalize
+        self._denom = torch.zeros(n + (rows * -(-self.T // 1024) + 1) // 2, dtype=torch.int64, device=self.dev)
+        self.denom = self._denom[:n].view(rows, self.T)
+        self._largest_known = False   # whether the last normalisation wrote the largest bin sum
 
     def zero_results(self):
         """Zero N, S and the status words (one fill when they are the engine's own)."""
@@ -192,7 +196,7 @@ class ResultBuffers:
         """The status words and g2 as numpy (one synchronising copy), with the
         ``largest`` bin sum in words 4-5."""
         n = 8 + self.n_bins * self.T
-        if largest and self.n_bins:
+        if largest and self.n_bins and not self._largest_known:
             _lib.check(self.lib.g2_max_i64(ptr(self.sums), self.n_bins * self.T, ptr(self._sum_max),
                                            stream_handle(self.dev)), "g2_max_i64")
         # into fresh pageable memory: on this host's coherent link as fast as
@@ -236,10 +240,11 @@ def normalise_rows(eng):
     ``eng.g2_f32`` / ``eng.g2_f64`` from them and ``eng.numer``, on the current
     stream."""
     lib, st = eng.lib, stream_handle(eng.dev)
-    if eng.n_bins * float(eng.T) ** 2 < NTT_MIN_WORK:
-        _lib.check(lib.g2_denominator(ptr(eng.sums), eng.n_bins, eng.T, ptr(eng.denom), st), "g2_denominator")
-        _lib.check(lib.g2_finalize(ptr(eng.numer), ptr(eng.denom), ptr(eng.scale), eng.n_bins, eng.T,
-                                   ptr(eng.g2_f32), ptr(eng.g2_f64), st), "g2_finalize")
+    eng._largest_known = eng.n_bins * float(eng.T) ** 2 < NTT_MIN_WORK
+    if eng._largest_known:
+        _lib.check(lib.g2_normalize(ptr(eng.numer), ptr(eng.sums), ptr(eng.scale), eng.n_bins, eng.T,
+                                    ptr(eng._denom), eng._denom.numel(), ptr(eng.g2_f32), ptr(eng.g2_f64),
+                                    ptr(eng._sum_max), st), "g2_normalize")
         return
     n = int(lib.g2_ntt_scratch(eng.n_bins, eng.T))
     buf = getattr(eng, "_ntt_buf", None)
@@ -303,7 +308,6 @@ class DenseEngine(ResultBuffers):
         # e4m3 operands split
         self._init_results(rows, numer, sums)
         self.want_result = False  # read g2 with the run's last synchronisation (correlate)
-        self.denom = z(torch.int64)
         self.g2_f64 = z(torch.float64)
         self.maxval = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._layouts = {} if layouts is None else layouts   # may be shared by engines of one q-mask

@@ -229,7 +229,7 @@ class EventEngine(ResultBuffers):
         rows = max(self.n_bins, 1)
         z = lambda dt: torch.zeros((rows, self.T), dtype=dt, device=self.dev)
         self._init_results(rows)
-        self.denom, self.g2_f64 = z(torch.int64), z(torch.float64)
+        self.g2_f64 = z(torch.float64)
         self.last = {}
         self.profile = False
         self._events = []

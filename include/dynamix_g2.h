@@ -632,6 +632,13 @@ int g2_finalize(const int64_t* numer_dev, const int64_t* denom_dev, const double
 /* Raises max_dev (caller zeroes it) to the largest of n non-negative int64. */
 int g2_max_i64(const int64_t* x_dev, int64_t n, uint64_t* max_dev, void* stream);
 
+/* g2_denominator, g2_finalize and the largest bin sum (raised into max_dev,
+ * uint64, may be NULL; the caller zeroes it) in one launch.  denom_dev holds
+ * denom_len int64: D, and behind it n_rows * ceil(nframes / 1024) uint32 counters. */
+int g2_normalize(const int64_t* numer_dev, const int64_t* sums_dev, const double* scale_dev, int32_t n_rows,
+                 int64_t nframes, int64_t* denom_dev, int64_t denom_len, float* g2_f32_dev, double* g2_f64_dev,
+                 uint64_t* max_dev, void* stream);
+
 /* ---- G3 and G4 by number-theoretic transforms -----------------------------
  * The same D (denom_dev) and g2 as g2_denominator + g2_finalize, in O(T log T)
  * (arithmetic modulo 2^64 - 2^32 + 1: exact for D < 2^63).  roots_dev: the 4096
