@@ -105,9 +105,9 @@ def qmask_digest(qmask):
 
 def device_layout(qmask, n_bins, mode, dev, digest=None, narrow=False):
     """The packing layout of a q-mask (``narrow``: the K-blocked NarrowLayout)
-    with its read-only tables on ``dev``, shared process-wide (least recently used of 48 kept): building one costs
-    host time proportional to the frame size.  ``digest``: the q-mask's
-    :func:`qmask_digest` when the caller has it."""
+    with its read-only tables on ``dev``, shared process-wide (least recently
+    used of 48 kept): building one costs host time proportional to the frame size.  ``digest``: the q-mask's
+    :func:`qmask_digest`, or another name for it, when the caller has one."""
     torch = _torch()
     q = np.ascontiguousarray(qmask, dtype=np.int32)
     key = (str(dev), digest or qmask_digest(q), int(n_bins), int(mode), bool(narrow))
@@ -419,16 +419,21 @@ class DenseEngine(ResultBuffers):
         if key not in self._layouts:
             c0, wc = self.crop
             q = np.ascontiguousarray(self.qmask.reshape(self.shape)[:, c0:c0 + wc])
-            self._layouts[key] = device_layout(q, self.n_bins, mode, self.dev, narrow=narrow)
+            # the whole mask's digest, known anyway, and the window name the cropped mask
+            name = (self._mask_digest(), self.shape, c0, wc)
+            self._layouts[key] = device_layout(q, self.n_bins, mode, self.dev, name, narrow)
         return self._layouts[key]
 
     def _layout(self, mode, narrow=False):
         key = ("narrow", mode) if narrow else mode
         if key not in self._layouts:
-            if getattr(self, "_qdigest", None) is None:
-                self._qdigest = qmask_digest(self.qmask)
-            self._layouts[key] = device_layout(self.qmask, self.n_bins, mode, self.dev, self._qdigest, narrow)
+            self._layouts[key] = device_layout(self.qmask, self.n_bins, mode, self.dev, self._mask_digest(), narrow)
         return self._layouts[key]
+
+    def _mask_digest(self):
+        if getattr(self, "_qdigest", None) is None:
+            self._qdigest = qmask_digest(self.qmask)
+        return self._qdigest
 
     def _piece_emax(self, L):
         """This engine's buffer of per-piece energy maxima for layout L (the
