@@ -143,9 +143,10 @@ __device__ __forceinline__ unsigned long long widen(uint32_t v, bool is_signed) 
 // PAIR_EPI: epilogue threads.
 template <bool F4, int PAIR_EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + PAIR_EPI, 1)
-    gram_pair_kernel(const __grid_constant__ typename PairMaps<F4>::type maps, int n_jobs, const g2_gram_item* __restrict__ items,
-                     int64_t n_items, unsigned long long* __restrict__ numer, int64_t numer_len,
-                     unsigned long long* __restrict__ sums, int64_t sums_len, int32_t* __restrict__ err) {
+    gram_pair_kernel(const __grid_constant__ typename PairMaps<F4>::type maps, int n_jobs,
+                     const g2_gram_item* __restrict__ items, int64_t n_items, unsigned long long* __restrict__ numer,
+                     int64_t numer_len, unsigned long long* __restrict__ sums, int64_t sums_len,
+                     int32_t* __restrict__ err) {
   constexpr int SB = F4 ? F4_B_BYTES : B_BYTES;  // B bytes per stage and CTA
   constexpr int ACC_STEP = F4 ? F4_BN : BN;      // TMEM columns from one accumulator to the next
   constexpr int BAR_OFF = STAGES * (A_BYTES + SB);
@@ -885,8 +886,8 @@ extern "C" int g2_gram_tc_e2m1(const g2_job* jobs, int32_t n_jobs, const g2_gram
   int64_t clusters = grid > 0 ? (grid + 1) / 2 : max_cl;
   if (clusters > max_cl) clusters = max_cl;
   if (clusters > n_items) clusters = n_items;
-  pair::gram_pair_kernel<true, pair::EPI_THREADS><<<static_cast<unsigned>(2 * clusters), pair::NUM_THREADS, pair::F4_SMEM_BYTES,
-                                 as_stream(stream)>>>(
+  pair::gram_pair_kernel<true, pair::EPI_THREADS><<<static_cast<unsigned>(2 * clusters), pair::NUM_THREADS,
+                                                    pair::F4_SMEM_BYTES, as_stream(stream)>>>(
       maps, n_jobs, items_dev, n_items, reinterpret_cast<unsigned long long*>(numer_dev), numer_len,
       reinterpret_cast<unsigned long long*>(sums_dev), sums_len, err_dev);
   return launch_status();

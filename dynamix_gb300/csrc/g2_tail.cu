@@ -38,7 +38,8 @@ namespace tail {
 
 constexpr int CH = G2_NARROW_CHUNK;     // source pixels per chunk
 constexpr int F = 4;                    // frames per step
-constexpr int ROW = CH + 48;            // bytes of a staged u8 frame row: the chunk from its 16-byte aligned start, spare words
+// bytes of a staged u8 frame row: the chunk from its 16-byte aligned start, spare words
+constexpr int ROW = CH + 48;
 static_assert(ROW % 16 == 0 && CH % 16 == 0 && CH <= 0xFFF, "bulk copy rows, 12-bit sources");
 // Warps, ring stages and CTAs per SM: few CTAs, so that a mover's step of F
 // frames stays in registers (80 per thread).  3,000 frames of 514 x 1030, e2m1:
@@ -1038,7 +1039,8 @@ extern "C" int g2_residual_sums(const void* packed_dev, int64_t packed_rows, int
   int64_t per_sm = hist ? 225 * 1024 / (smem + 34 * 1024) : 6;
   if (per_sm > 6) per_sm = 6;
   if (per_sm < 1) per_sm = 1;
-  const int64_t tiles = (nframes + tail::RES_TILE - 1) / tail::RES_TILE, blocks = res.n_sectors / (elem_kind == G2_KIND_E2M1 ? 4 : 2);
+  const int64_t tiles = (nframes + tail::RES_TILE - 1) / tail::RES_TILE;
+  const int64_t blocks = res.n_sectors / (elem_kind == G2_KIND_E2M1 ? 4 : 2);
   int64_t shares = sms * per_sm / tiles;
   if (shares > blocks) shares = blocks;
   if (shares < 1) shares = 1;
@@ -1052,7 +1054,8 @@ extern "C" int g2_residual_sums(const void* packed_dev, int64_t packed_rows, int
                                   184 * 1024) != cudaSuccess)                                                        \
       return G2_ERR_CUDA;                                                                                            \
     tail::residual_kernel<E, H><<<grid, tail::RES_THREADS, H ? smem : 0, st>>>(                                      \
-        pk, static_cast<int32_t>(nframes), packed_rows * 128, res, sector_bin_dev, n_bins, nm, sm, nt, total_dev, err_dev);                \
+        pk, static_cast<int32_t>(nframes), packed_rows * 128, res, sector_bin_dev, n_bins, nm, sm, nt, total_dev,    \
+        err_dev);                                                                                                    \
   } while (0)
   if (e2m1 && hist) G2_RESIDUAL_LAUNCH(true, true);
   else if (e2m1) G2_RESIDUAL_LAUNCH(true, false);

@@ -1090,8 +1090,8 @@ class DenseEngine(ResultBuffers):
             if narrow is not None:
                 _lib.check(self.lib.g2_pack_u8_residual(
                     C.c_void_p(src), t1 - t0, npix, t0, L.kind, ptr(Lp.d_unit_block_off), ptr(Lp.d_units),
-                    ptr(Lp.d_chunk_span), Lp.n_chunks, ptr(packed), self.T + 1, L.packed_cols, ptr(res[0]), ptr(res[1]), res[2], ptr(self.err),
-                    C.c_void_p(pack_s.cuda_stream)), "g2_pack_u8_residual")
+                    ptr(Lp.d_chunk_span), Lp.n_chunks, ptr(packed), self.T + 1, L.packed_cols, ptr(res[0]),
+                    ptr(res[1]), res[2], ptr(self.err), C.c_void_p(pack_s.cuda_stream)), "g2_pack_u8_residual")
             elif wide is not None:
                 _lib.check(self.lib.g2_pack_blocked(
                     C.c_void_p(src), eb, t1 - t0, npix, t0, int(L.split), ptr(L.d_unit_block_off), ptr(L.d_units),

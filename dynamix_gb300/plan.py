@@ -21,8 +21,9 @@ from __future__ import annotations
 
 import numpy as np
 
-from ._lib import (BK, NARROW_CHUNK, ITEM_DTYPE, ITEM_EMPTY, KIND_E2M1, KIND_E4M3, KIND_FP16, PACK_CHUNK, PACK_MAX_PIECES, PACK_MAX_SLOTS,
-                   PACK_WORDS_PER_CHUNK, PAD, PLAIN_BM, PLAIN_BN, RES_SECTOR, TC_BM, TC_BN)
+from ._lib import (BK, NARROW_CHUNK, ITEM_DTYPE, ITEM_EMPTY, KIND_E2M1, KIND_E4M3, KIND_FP16, PACK_CHUNK,
+                   PACK_MAX_PIECES, PACK_MAX_SLOTS, PACK_WORDS_PER_CHUNK, PAD, PLAIN_BM, PLAIN_BN, RES_SECTOR,
+                   TC_BM, TC_BN)
 
 EXACT_LIMIT = 1 << 24   # fp32 represents every integer up to 2^24 exactly
 FP16_MAX_EXACT = 2048   # fp16 represents every integer up to 2^11 exactly
